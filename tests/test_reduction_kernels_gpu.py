@@ -1,0 +1,69 @@
+"""The kernels that merge partial results: attention partials of a split context, expert outputs of a row."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def C():
+    from b200serve.ops import cuda_ops
+
+    cuda_ops.lib()
+    return cuda_ops
+
+
+def _combine(C, acc, ml, gate):
+    rows, n_q, Z, D = acc.shape
+    out = torch.empty(rows, n_q * D, dtype=torch.bfloat16, device="cuda")
+    C._check(C.lib().b200_attn_combine(acc.data_ptr(), ml.data_ptr(), gate.data_ptr(), out.data_ptr(), rows, n_q, D, Z,
+                                       C._stream()), "attn_combine")
+    return out
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("valid,Z", [(1, 1), (1, 8), (15, 15), (13, 16), (16, 17), (33, 63), (7, 64), (64, 64), (177, 512), (512, 512)])
+def test_attention_partials_against_64_bits(C, D, valid, Z):
+    g = torch.Generator(device="cuda").manual_seed(valid * 1000 + Z)
+    rows, n_q = 3, 2
+    acc = torch.randn(rows, n_q, Z, D, device="cuda", generator=g)
+    ml = torch.stack([torch.randn(rows, n_q, Z, device="cuda", generator=g) * 4,
+                      torch.rand(rows, n_q, Z, device="cuda", generator=g) * 30 + 1], -1).contiguous()
+    acc[:, :, valid:] = float("nan")  # a split without keys writes only its (-inf, 0) pair
+    ml[:, :, valid:, 0], ml[:, :, valid:, 1] = float("-inf"), 0.0
+    gate = torch.randn(rows, n_q * D, device="cuda", generator=g).bfloat16()
+    got = _combine(C, acc, ml, gate)
+    w = torch.exp(ml[..., 0].double() - ml[..., 0].double().amax(-1, keepdim=True))
+    o = (w[..., :valid, None] * acc[:, :, :valid].double()).sum(2) / (w * ml[..., 1].double()).sum(-1)[..., None]
+    ref = o.reshape(rows, -1) * torch.sigmoid(gate.double())
+    # two roundings to bf16 (8 significant bits: at most 2^-8 each) and fp32 sums of at most 512 terms
+    assert ((got.double() - ref).abs() <= 2.0 ** -7 * 1.01 * ref.abs() + 1e-5).all()
+    # the order of the sums follows the partials that hold keys, not the width of the table behind them
+    wide = torch.full((rows, n_q, 520, D), float("nan"), device="cuda")
+    wide_ml = torch.zeros(rows, n_q, 520, 2, device="cuda")
+    wide_ml[..., 0] = float("-inf")
+    wide[:, :, :valid], wide_ml[:, :, :valid] = acc[:, :, :valid], ml[:, :, :valid]
+    assert torch.equal(_combine(C, wide, wide_ml, gate), got)
+
+
+@pytest.mark.parametrize("T,P,H", [(1, 1, 8), (3, 9, 2048), (5, 10, 2056), (130, 8, 128), (2, 33, 4096)])
+def test_expert_outputs_of_a_row(C, T, P, H):
+    g = torch.Generator(device="cuda").manual_seed(T + P)
+    pairs = torch.randn(T * P, H, device="cuda", generator=g).bfloat16()
+    wts = torch.rand(T, P, device="cuda", generator=g).bfloat16().float()
+    inv = torch.randperm(T * P, device="cuda", generator=g).int().view(T, P)
+    inv[torch.rand(T, P, device="cuda", generator=g) < 0.2] = -1  # pairs that another rank serves
+    src = pairs.double()[inv.clamp(min=0).long()] * (wts * (inv >= 0)).double()[..., None]
+    ref = src.sum(1)
+    out = torch.empty(T, H, device="cuda", dtype=torch.float32)
+    C._check(C.lib().b200_moe_combine(pairs.data_ptr(), wts.data_ptr(), inv.data_ptr(), T, P, H, None, out.data_ptr(),
+                                      C._stream()), "moe_combine")
+    assert ((out.double() - ref).abs() <= 1e-6 * P * src.abs().sum(1) + 1e-12).all()
+    res = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    norm_w = torch.randn(H, device="cuda", generator=g).bfloat16() * 0.1
+    new, y = torch.empty_like(res), torch.empty_like(res)
+    C._check(C.lib().b200_moe_combine_norm(pairs.data_ptr(), wts.data_ptr(), inv.data_ptr(), T, P, H, res.data_ptr(),
+                                           norm_w.data_ptr(), new.data_ptr(), y.data_ptr(), 1e-6, C._stream()), "combine_norm")
+    ref_new, ref_y = C.add_rmsnorm(out.bfloat16(), res, norm_w, 1e-6)
+    assert torch.equal(new, ref_new) and torch.equal(y, ref_y)
