@@ -67,3 +67,17 @@ def test_expert_outputs_of_a_row(C, T, P, H):
                                            norm_w.data_ptr(), new.data_ptr(), y.data_ptr(), 1e-6, C._stream()), "combine_norm")
     ref_new, ref_y = C.add_rmsnorm(out.bfloat16(), res, norm_w, 1e-6)
     assert torch.equal(new, ref_new) and torch.equal(y, ref_y)
+
+
+@pytest.mark.parametrize("T,V", [(1, 128), (2, 1000), (17, 129), (64, 4096), (200, 777), (256, 1280), (300, 2500)])
+def test_greedy_head_takes_the_lowest_id_among_equal_logits(C, T, V):
+    """Small whole numbers: every logit is exact, and a row has many columns with the same largest one."""
+    g = torch.Generator(device="cuda").manual_seed(T * 7 + V)
+    x = torch.randint(-2, 3, (T, 64), device="cuda", generator=g).bfloat16()
+    w = torch.randint(-1, 2, (V, 64), device="cuda", generator=g).bfloat16()
+    w[V // 2:] = w[: V - V // 2].clone()  # every logit appears twice
+    logits = x.double() @ w.double().t()
+    top = logits.amax(1, keepdim=True)
+    first = torch.where(logits == top, torch.arange(V, device="cuda"), V).amin(1)
+    idx, val = C.lm_head_argmax(x, w, return_value=True)
+    assert torch.equal(idx, first) and torch.equal(val.double(), top[:, 0])
