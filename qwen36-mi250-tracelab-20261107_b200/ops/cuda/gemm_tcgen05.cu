@@ -64,19 +64,30 @@ struct GemmParams {
   int w_tiles;       // packed: weight tiles per expert
 };
 
-template <int BT, int EPI>
+// RT: weight rows per tile. 128 fills the MMA's M; the thin forms (64, 32) load that many rows into the first rows of the
+// operand tile and let the MMA read whatever shared memory holds behind them: an accumulator row depends on its own operand
+// row only, the surplus rows are never read back, and the instruction shape, and with it every bit of the result, stay
+// those of RT = 128. They exist for launches whose 128-row tiles would leave most SMs without work.
+// KPS: k-blocks per pipeline stage. One trip through the pipeline (wait, expect, TMA, wait, MMAs, commit) costs a CTA about
+// 0.2 us however little it moves, and at decode sizes a CTA's time is the sum of its trips; a stage of KPS k-blocks comes
+// with one TMA instruction per operand. Tile-packed weights only.
+template <int BT, int EPI, int RT = BM, int KPS = 1>
 struct Cfg {
   static constexpr int A_TILES = (EPI == EPI_SILU_MUL) ? 2 : 1;
-  static constexpr int A_BYTES = BM * BK * 2;
+  static constexpr int A_BYTES = RT * BK * 2;
   static constexpr int B_BYTES = BT * BK * 2;
-  static constexpr int STAGE_BYTES = A_TILES * A_BYTES + B_BYTES;
+  static constexpr int STAGE_BYTES = KPS * (A_TILES * A_BYTES + B_BYTES);
+  static constexpr int A_STEP = (RT == BM ? A_TILES : 1) * A_BYTES;  // bytes between the k-blocks of a stage
+  static constexpr int UP_OFF = RT == BM ? A_BYTES : KPS * A_BYTES;  // from a gate tile to its up tile
+  static constexpr int B_OFF = KPS * A_TILES * A_BYTES;
+  static constexpr bool THIN = RT < BM || KPS > 1;
   // small token tiles (decode) leave room for two CTAs per SM: one CTA's pipeline fill and epilogue
   // overlap the other's main loop, which matters when K is short (the MoE down projection has 8 k-blocks)
   // The fused gate/up GEMM at 16-row token tiles runs three CTAs per SM with two deep stages each: the same bytes in
   // flight per SM, but a decode step's ~1300 tiles then fill 2.9 waves of 444 CTAs instead of 4.4 waves of 296, and
   // the partial last wave is what the weight-streaming time loses.
-  static constexpr int CTAS_PER_SM = (BT <= 16 && EPI == EPI_SILU_MUL) ? 3 : BT <= 64 ? 2 : 1;
-  static constexpr int BUDGET = CTAS_PER_SM == 3 ? 72 * 1024 : BT <= 64 ? 108 * 1024 : 200 * 1024;
+  static constexpr int CTAS_PER_SM = THIN ? 2 : (BT <= 16 && EPI == EPI_SILU_MUL) ? 3 : BT <= 64 ? 2 : 1;
+  static constexpr int BUDGET = THIN ? (RT < BM ? 96 * 1024 : 108 * 1024) : CTAS_PER_SM == 3 ? 72 * 1024 : BT <= 64 ? 108 * 1024 : 200 * 1024;
   static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int ACC_COLS = A_TILES * BT;  // one accumulator stage
@@ -85,13 +96,14 @@ struct Cfg {
   static constexpr int ACC_STAGES = (2 * ACC_COLS * CTAS_PER_SM <= 512) ? 2 : 1;
   static constexpr int TMEM_COLS_RAW = ACC_COLS * ACC_STAGES;
   static constexpr int TMEM_COLS = TMEM_COLS_RAW <= 32 ? 32 : TMEM_COLS_RAW <= 64 ? 64 : TMEM_COLS_RAW <= 128 ? 128 : TMEM_COLS_RAW <= 256 ? 256 : 512;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int OVERREAD = (BM - RT) * BK * 2;  // bytes behind the last stage that a thin tile's MMA may read
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + (OVERREAD > 256 ? OVERREAD : 256) /*barriers first*/;
 };
 
-template <int BT, int EPI, bool GROUPED, bool SPLIT = false>
-__global__ void __launch_bounds__(192, Cfg<BT, EPI>::CTAS_PER_SM)
+template <int BT, int EPI, bool GROUPED, bool SPLIT = false, int RT = BM, int KPS = 1>
+__global__ void __launch_bounds__(192, Cfg<BT, EPI, RT, KPS>::CTAS_PER_SM)
 gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, GemmParams p) {
-  using C = Cfg<BT, EPI>;
+  using C = Cfg<BT, EPI, RT, KPS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -110,14 +122,14 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (GROUPED) pdl_wait();
   // Persistent tile loop: CTA b takes output tiles b, b + gridDim.x, ... (weight tile fastest, so CTAs that run
   // together share the activation tile). A split-K cluster takes the single tile its grid position names.
-  const int tiles_n = (p.N + BM - 1) / BM;
+  const int tiles_n = (p.N + RT - 1) / RT;
   const int tiles_y = GROUPED ? *p.n_tiles : p.grid_y;
   const int total = tiles_n * tiles_y;
   const int tile0 = SPLIT ? static_cast<int>(blockIdx.y) * tiles_n + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
   const int tstep = SPLIT ? (1 << 30) : static_cast<int>(gridDim.x);
   constexpr int ACC = SPLIT ? 1 : C::ACC_STAGES;
   if (SPLIT && tile0 >= total) return;  // the whole cluster leaves together, before any barrier or TMEM use
-  const int num_k_all = (p.K + BK - 1) / BK;
+  const int num_k_all = (p.K + BK * KPS - 1) / (BK * KPS);  // in stages
   // split-K: the cluster's CTAs (blockIdx.z = rank in the cluster) take consecutive runs of k-blocks; their fp32
   // partial tiles meet in the leader through distributed shared memory, added in rank order
   const int k_per = SPLIT ? (num_k_all + p.splits - 1) / p.splits : num_k_all;
@@ -144,7 +156,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   // geometry of output tile `tile`
   auto tile_geom = [&](int tile, int& n0, int& by, int& expert, int& row0, int& nrows) {
     const int nx = tile % tiles_n, byr = tile / tiles_n;
-    n0 = nx * BM;
+    n0 = nx * RT;
     by = (!GROUPED && p.y_rot) ? (byr + p.y_rot) % tiles_y : byr;
     expert = 0;
     if (GROUPED) {
@@ -153,6 +165,23 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     } else {
       row0 = by * BT;
       nrows = min(BT, p.T - row0);
+    }
+  };
+
+  // weight rows [n0, n0 + RT) of pipeline step `kb` (and the matching up rows) into stage `st`
+  auto load_weights = [&](uint8_t* st, uint64_t* bar, int n0, int expert, int kb) {
+    if constexpr (C::THIN) {  // packed only: [expert, tile, k-block][rows of the tile][64], KPS k-blocks per box
+      const int z = ((expert * p.w_tiles + n0 / BM) * num_k_all + kb) * KPS;
+      tma_load_3d(st, &tmW, bar, 0, n0 % BM, z);  // RT = 128: gate and up rows are one box
+      if (RT < BM && EPI == EPI_SILU_MUL) tma_load_3d(st + C::UP_OFF, &tmW, bar, 0, BM + n0 % BM, z);
+    } else if (p.packed) {
+      tma_load_2d(st, &tmW, bar, 0, ((expert * p.w_tiles + n0 / BM) * num_k_all + kb) * (BM * C::A_TILES));
+    } else if (GROUPED) {
+      tma_load_3d(st, &tmW, bar, kb * BK, n0, expert);
+      if (EPI == EPI_SILU_MUL) tma_load_3d(st + C::A_BYTES, &tmW, bar, kb * BK, p.up_offset + n0, expert);
+    } else {
+      tma_load_2d(st, &tmW, bar, kb * BK, n0);
+      if (EPI == EPI_SILU_MUL) tma_load_2d(st + C::A_BYTES, &tmW, bar, kb * BK, p.up_offset + n0);
     }
   };
 
@@ -182,22 +211,19 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
         uint8_t* st = smem + s * C::STAGE_BYTES;
         if (lane == 0) {
-          mbar_expect_tx(&full[s], C::A_TILES * C::A_BYTES);
-          if (p.packed) {
-            tma_load_2d(st, &tmW, &full[s], 0,
-                        ((expert * p.w_tiles + n0 / BM) * num_k_all + kb0 + kb) * (BM * C::A_TILES));
-          } else {
-            tma_load_3d(st, &tmW, &full[s], (kb0 + kb) * BK, n0, expert);
-            if (EPI == EPI_SILU_MUL) tma_load_3d(st + C::A_BYTES, &tmW, &full[s], (kb0 + kb) * BK, p.up_offset + n0, expert);
-          }
+          mbar_expect_tx(&full[s], C::B_OFF);
+          load_weights(st, &full[s], n0, expert, kb0 + kb);
         }
-        const uint32_t xb = smem_u32(st + C::A_TILES * C::A_BYTES);
+        const uint32_t xb = smem_u32(st + C::B_OFF);
 #pragma unroll
         for (int i = 0; i < PER_LANE; ++i) {
           const int r = (lane >> 3) + 4 * i;
           if (src[i] != nullptr) {
             const uint32_t dst = xb + (r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src[i] + (kb0 + kb) * BK) : "memory");
+#pragma unroll
+            for (int ks = 0; ks < KPS; ++ks)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + ks * C::B_BYTES),
+                           "l"(src[i] + ((kb0 + kb) * KPS + ks) * BK) : "memory");
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
@@ -218,12 +244,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         for (int kb = 0; kb < pre; ++kb) {
           uint8_t* st = smem + kb * C::STAGE_BYTES;
           mbar_expect_tx(&full[kb], C::STAGE_BYTES);
-          if (p.packed) {
-            tma_load_2d(st, &tmW, &full[kb], 0, ((n0 / BM) * num_k_all + kb) * (BM * C::A_TILES));
-          } else {
-            tma_load_2d(st, &tmW, &full[kb], kb * BK, n0);
-            if (EPI == EPI_SILU_MUL) tma_load_2d(st + C::A_BYTES, &tmW, &full[kb], kb * BK, p.up_offset + n0);
-          }
+          load_weights(st, &full[kb], n0, 0, kb);
         }
       }
       pdl_wait();
@@ -241,18 +262,10 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (it >= pre) {
         if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
         mbar_expect_tx(&full[s], C::STAGE_BYTES);
-        if (p.packed) {
-          tma_load_2d(st, &tmW, &full[s], 0,
-                      ((expert * p.w_tiles + n0 / BM) * num_k_all + kb0 + kb) * (BM * C::A_TILES));
-        } else if (GROUPED) {
-          tma_load_3d(st, &tmW, &full[s], (kb0 + kb) * BK, n0, expert);
-          if (EPI == EPI_SILU_MUL) tma_load_3d(st + C::A_BYTES, &tmW, &full[s], (kb0 + kb) * BK, p.up_offset + n0, expert);
-        } else {
-          tma_load_2d(st, &tmW, &full[s], (kb0 + kb) * BK, n0);
-          if (EPI == EPI_SILU_MUL) tma_load_2d(st + C::A_BYTES, &tmW, &full[s], (kb0 + kb) * BK, p.up_offset + n0);
+        load_weights(st, &full[s], n0, expert, kb0 + kb);
         }
-        }
-        tma_load_2d(st + C::A_TILES * C::A_BYTES, &tmX, &full[s], (kb0 + kb) * BK, row0);
+        if constexpr (C::THIN) tma_load_3d(st + C::B_OFF, &tmX, &full[s], 0, row0, (kb0 + kb) * KPS);
+        else tma_load_2d(st + C::B_OFF, &tmX, &full[s], (kb0 + kb) * BK, row0);
       }
       }
     }
@@ -277,14 +290,15 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-        const uint32_t b_addr = a_addr + C::A_TILES * C::A_BYTES;
+        const uint32_t b_addr = a_addr + C::B_OFF;
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          const uint32_t koff = k * UMMA_K * 2;  // bytes inside the 128-byte swizzled row
-          const uint64_t db = umma_smem_desc(b_addr + koff);
-          umma_bf16(tmem, umma_smem_desc(a_addr + koff), db, idesc, (kb | k) != 0);
+        for (int k = 0; k < KPS * BK / UMMA_K; ++k) {
+          const uint32_t koff = (k % (BK / UMMA_K)) * UMMA_K * 2;  // bytes inside the 128-byte swizzled row
+          const uint32_t aoff = k / (BK / UMMA_K) * C::A_STEP + koff;
+          const uint64_t db = umma_smem_desc(b_addr + k / (BK / UMMA_K) * C::B_BYTES + koff);
+          umma_bf16(tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
           if (EPI == EPI_SILU_MUL)
-            umma_bf16(tmem + BT, umma_smem_desc(a_addr + C::A_BYTES + koff), db, idesc, (kb | k) != 0);
+            umma_bf16(tmem + BT, umma_smem_desc(a_addr + C::UP_OFF + aoff), db, idesc, (kb | k) != 0);
         }
         umma_commit(&empty[s]);  // stage reusable once these MMAs have read it
       }
@@ -301,13 +315,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     int n0, by, expert, row0, nrows;
     tile_geom(tile, n0, by, expert, row0, nrows);
     (void)expert;
-    const int nx = n0 / BM;
+    const int nx = n0 / RT;
     const int acc = lt % ACC;
     const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
     const bool ok = mbar_wait(&acc_full[acc], (lt / ACC) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
     tc_fence_after();
     const int n = n0 + q * 32 + lane;
-    const bool n_ok = n < p.N;
+    const bool n_ok = n < p.N && (RT == BM || q * 32 + lane < RT);
     if (EPI == EPI_ALLREDUCE) {
       // Fused GEMM -> one-shot all-reduce: this tile's fp32 partial goes straight from TMEM into every
       // rank's receive slot over NVLink; when all R partials of the tile have arrived they are added in
@@ -404,7 +418,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       cluster_sync();  // first cluster barrier (every thread of the cluster takes part exactly once)
     } else {
     if (SPLIT) cluster_sync();  // first cluster barrier: the followers' partial tiles are in place
-    if (ok) {
+    if (ok && q * 32 < RT) {
       const uint32_t red_local = smem_u32(smem);
 #pragma unroll 1
       for (int c = 0; c < BT; c += 16) {
@@ -595,6 +609,22 @@ static int make_map_packed(CUtensorMap* m, const void* base, uint64_t total_rows
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// Maps of the thin forms: `kps` k-blocks of `rows` rows per box. Packed weights: [tile, k-block][tile rows][64]; activations:
+// the k-blocks of a row are 128 bytes apart.
+static int make_map_kblocks(CUtensorMap* m, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t blocks,
+                            uint64_t block_bytes, uint32_t box_rows, uint32_t kps) {
+  EncodeFn fn = encode_fn();
+  if (!fn) return -1;
+  cuuint64_t dims[3] = {BK, rows, blocks};
+  cuuint64_t strides[2] = {row_bytes, block_bytes};
+  cuuint32_t box[3] = {BK, box_rows, kps};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -2;
+}
+
 // Weight map of a launch: `packed` selects the tile-packed layout (N padded to a multiple of 128 per expert, K a
 // multiple of 64; with the SiLU-mul epilogue the gate and up tiles of a k-block are stored back to back).
 static int weight_map(CUtensorMap* m, const void* W, int E, int N, int w_rows, int K, int ldw, bool silu, int packed,
@@ -636,13 +666,13 @@ static int launch_split(const CUtensorMap& tw, const CUtensorMap& tx, const Gemm
   return cudaLaunchKernelEx(&cfg, kern, tw, tx, q) == cudaSuccess ? 0 : -4;
 }
 
-template <int BT, int EPI, bool GROUPED>
+template <int BT, int EPI, bool GROUPED, int RT = BM, int KPS = 1>
 static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, int grid_y, cudaStream_t st) {
-  using C = Cfg<BT, EPI>;
-  if constexpr (EPI == EPI_BF16 || EPI == EPI_F32 || EPI == EPI_SILU_MUL) {
+  using C = Cfg<BT, EPI, RT, KPS>;
+  if constexpr (!C::THIN && (EPI == EPI_BF16 || EPI == EPI_F32 || EPI == EPI_SILU_MUL)) {
     if (p.splits > 1) return launch_split<BT, EPI, GROUPED>(tw, tx, p, grid_y, st);
   }
-  auto kern = gemm_swapab_kernel<BT, EPI, GROUPED, false>;
+  auto kern = gemm_swapab_kernel<BT, EPI, GROUPED, false, RT, KPS>;
   // per device: the shared-memory attribute is set on the device that is current, and the persistent grid is sized
   // from that device's SM count (a process may drive several GPUs)
   static bool configured[MAX_DEVICES] = {};
@@ -659,7 +689,7 @@ static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams
   const int resident = resident_of[dev];
   GemmParams q = p;
   q.grid_y = grid_y;
-  const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * grid_y;
+  const long long tiles = static_cast<long long>((p.N + RT - 1) / RT) * grid_y;
   return launch_pdl(kern, dim3(static_cast<unsigned>(tiles < resident ? tiles : resident)), dim3(192), C::SMEM, st, tw,
                     tx, q) == cudaSuccess ? 0 : -4;
 }
@@ -678,6 +708,96 @@ static int dispatch_bt(int bt, const CUtensorMap& tw, const CUtensorMap& tx, con
   }
 }
 
+static int sm_count() {  // of the current device; 148 on a B200
+  static int of[MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 148;
+  if (of[dev] == 0 && cudaDeviceGetAttribute(&of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  return of[dev];
+}
+
+struct DenseForm {
+  int bt, rt, kps;  // token rows per tile, weight rows per tile, k-blocks per stage
+};
+
+// The form of a dense bf16 / fp32 GEMM. It never changes a row's bits (every element sees the same k order in the same
+// instruction shape), so it may follow the number of rows. Measured in chains of launches on weights that are not in L2, us,
+// plain form -> chosen form; 12352 x 2048 is a GDN layer's input projection, 9216 x 2048 an attention layer's, 2048 x 4096
+// the output projection, 257 x 2048 the router:
+//   up to 16 rows     12352: 13.0 -> 12.0   9216: 11.6 -> 10.4   2048: 15.4 -> 10.9   257: 8.5 -> 6.3
+//   32 rows           12352: 14.5 -> 13.0   9216: 13.3 -> 12.1   2048: 15.2 -> 11.1   257: 8.5 -> 6.3
+//   61 rows           12352: 16.6 -> 15.4   9216: 15.5 -> 14.2   2048: 14.7 -> 12.5   257: 8.4 -> 6.5
+//   128 rows          12352: 16.9           9216: 16.2 -> 14.5   2048: 15.0 -> 13.8   257: 8.4 -> 6.5
+//   256 rows          12352: 25.1           9216: 24.2 -> 17.6   2048: 16.1           257: 8.4 -> 7.0
+static DenseForm dense_form(int T, int N, int K, bool packed) {
+  const int sms = sm_count();
+  const auto tiles = [&](int rt, int bt) { return static_cast<long long>((N + rt - 1) / rt) * ((T + bt - 1) / bt); };
+  const bool by2 = packed && K % (2 * BK) == 0, by4 = packed && K % (4 * BK) == 0;
+  if (T <= 16) {
+    // one token tile: the weights are streamed once whatever the tile, so the thinnest tile whose CTAs (two per SM) are
+    // all resident wins; beyond that the second wave costs more (386 CTAs of 32 rows: 14.2 us for the 12352 rows)
+    if (by4 && tiles(32, 16) <= 2 * sms) return {16, 32, 4};
+    if (by2 && tiles(64, 16) <= 2 * sms) return {16, 64, 2};
+    return {16, BM, 1};
+  }
+  if (T <= 256 && N <= 32 * BM) {
+    // few weight tiles: 16-row token tiles put 8x more CTAs on the K loop. Several token tiles re-read the weights, so
+    // thin tiles pay only while the CTAs have an SM each, with a little room (144 CTAs already share some)
+    const int lim = sms * 7 / 8;
+    if (by4 && tiles(32, 16) <= lim) return {16, 32, 4};
+    if (by2 && tiles(64, 16) <= lim) return {16, 64, 2};
+    if (by2 && tiles(64, 32) <= lim) return {32, 64, 2};
+    return {16, BM, 1};
+  }
+  if (by2 && T <= 64 && tiles(64, 64) <= 2 * sms) return {T <= 32 ? 32 : 64, 64, 2};
+  if (by2 && T <= 128 && tiles(64, 64) <= 2 * sms) return {64, 64, 2};
+  if (by2 && T > 128 && T <= 256 && tiles(BM, 64) <= 2 * sms) return {64, BM, 2};
+  return {T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256, BM, 1};
+}
+
+// Thin dense launch; 1 when the form is the plain one.
+template <int EPI>
+static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, GemmParams p, int ldx, cudaStream_t st) {
+  CUtensorMap tw, tx;
+  const uint64_t nk = p.K / BK;
+  p.packed = 1;
+  p.w_tiles = (p.N + BM - 1) / BM;
+  if (make_map_kblocks(&tw, W, BM, BK * 2, p.w_tiles * nk, BM * BK * 2, f.rt, f.kps)) return -1;
+  if (make_map_kblocks(&tx, X, p.T, static_cast<uint64_t>(ldx) * 2, nk, BK * 2, f.bt, f.kps)) return -1;
+  const int gy = (p.T + f.bt - 1) / f.bt;
+  if (f.bt == 16 && f.rt == 32 && f.kps == 4) return launch<16, EPI, false, 32, 4>(tw, tx, p, gy, st);
+  if (f.bt == 16 && f.rt == 64 && f.kps == 2) return launch<16, EPI, false, 64, 2>(tw, tx, p, gy, st);
+  if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
+  if (f.bt == 64 && f.rt == 64 && f.kps == 2) return launch<64, EPI, false, 64, 2>(tw, tx, p, gy, st);
+  if (f.bt == 64 && f.rt == BM && f.kps == 2) return launch<64, EPI, false, BM, 2>(tw, tx, p, gy, st);
+  return -5;
+}
+
+// Gate/up GEMM of the experts of a few rows (16-row token tiles, at most one per pair, tile-packed weights): each 128-row
+// tile becomes four when that still leaves at most one CTA per SM, two when at most two. Whole block, us: 1 row 41.5 ->
+// 30.7, 2 rows 46.1 -> 39.4, 4 rows 54.8 -> 52.7; at 8 rows the plain tiles are as good (77.3, thin 78.9). The down
+// projection (16 weight tiles per expert) has CTAs enough at one row. Returns 1 when the plain form is to run.
+static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
+                               int max_tiles, cudaStream_t st) {
+  const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
+  const int sms = sm_count(), rt = 4 * tiles <= sms ? 32 : 2 * tiles <= 2 * sms ? 64 : BM;
+  if (rt == BM || p.K % (2 * BK) || p.N % BM) return 1;
+  CUtensorMap tw, tx;
+  const uint64_t nk = p.K / BK;
+  p.packed = 1;
+  p.w_tiles = p.N / BM;
+  if (make_map_kblocks(&tw, W, 2 * BM, BK * 2, static_cast<uint64_t>(E) * p.w_tiles * nk, 2 * BM * BK * 2, rt, 2)) return -1;
+  if (gather_rows != nullptr) {
+    p.gather_rows = gather_rows;
+    p.gx = static_cast<const bf16*>(X);
+    p.ldgx = ldx;
+  }
+  // with row indices the producer never reads through this map, but it has to be a valid one
+  if (make_map_kblocks(&tx, X, gather_rows ? 16 : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, 16, 2)) return -1;
+  if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 2>(tw, tx, p, max_tiles, st);
+  return launch<16, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -692,18 +812,24 @@ extern "C" int b200_pick_bt(int T) {
   return 256;
 }
 
-// Dense: out[T, N] = X[T, K] W[N, K]^T.   epi: 0 bf16, 1 fp32, 2 silu(gate)*up (N = rows of each half, W has 2N rows
+// Dense: out[T, N] = X[T, K] W[N, K]^T. bt <= 0: the launcher picks the form, otherwise the token tile is `bt` rows.   epi: 0 bf16, 1 fp32, 2 silu(gate)*up (N = rows of each half, W has 2N rows
 // with the up half at row `up_offset`), 3 argmax partials (part_max/part_idx sized [ceil(N/128), T]).
 extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, int N, int K, int ldx, int ldw, int ldo,
                                int epi, int up_offset, int bt, float* part_max, int* part_idx, int* err,
                                int splits, int packed, cudaStream_t st) {
   if (T <= 0) return 0;
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
+  const int w_rows = (epi == EPI_SILU_MUL) ? up_offset + N : N;
+  GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
+  if (bt <= 0 && (epi == EPI_BF16 || epi == EPI_F32)) {
+    const DenseForm f = dense_form(T, N, K, packed && splits == 1);
+    if (f.rt < BM || f.kps > 1)
+      return epi == EPI_F32 ? launch_thin_dense<EPI_F32>(f, X, W, p, ldx, st) : launch_thin_dense<EPI_BF16>(f, X, W, p, ldx, st);
+    bt = f.bt;
+  }
   if (bt <= 0) bt = b200_pick_bt(T);
   if (epi == EPI_SILU_MUL && bt > 128) bt = 128;
   CUtensorMap tw, tx;
-  const int w_rows = (epi == EPI_SILU_MUL) ? up_offset + N : N;
-  GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
   if (weight_map(&tw, W, 0, N, w_rows, K, ldw, epi == EPI_SILU_MUL, packed, &p)) return -1;
   if (make_map(&tx, X, K, T, 0, ldx, 0, bt)) return -1;
   const int gy = (T + bt - 1) / bt;
@@ -729,6 +855,10 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   CUtensorMap tw, tx;
   GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
+  if (packed && splits == 1 && bt == 16 && epi == EPI_SILU_MUL) {
+    const int rc = launch_thin_grouped(X, W, p, E, gather_rows, ldx, max_tiles, st);
+    if (rc <= 0) return rc;
+  }
   if (weight_map(&tw, W, E, N, w_rows, K, K, epi == EPI_SILU_MUL, packed, &p)) return -1;
   if (gather_rows != nullptr) {
     p.gather_rows = gather_rows;
