@@ -25,8 +25,9 @@ namespace b200 {
 
 constexpr int BM = 128;  // weight rows per tile (TMEM lanes)
 constexpr int BK = 64;   // bf16 per operand row per stage (128 bytes)
-constexpr int GATHER_BT_MAX = 64;  // widest token tile whose rows the grouped GEMM's producer warp can fetch by index
+constexpr int GATHER_BT_MAX = 128;  // widest token tile whose rows the grouped GEMM's producer warps can fetch by index
 constexpr int UMMA_K = 16;
+constexpr int VAR_BOX = 32;  // rows per activation load of a wide expert tile: a tile with 40 rows loads 64
 constexpr int MAX_DEVICES = 64;  // per-device launch state (function attributes, SM counts)
 
 enum Epilogue : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_SILU_MUL = 2, EPI_ARGMAX = 3, EPI_ALLREDUCE = 4, EPI_SCATTER = 5, EPI_REDUCE_SCATTER = 6 };
@@ -81,6 +82,20 @@ struct Cfg {
   static constexpr int UP_OFF = RT == BM ? A_BYTES : KPS * A_BYTES;  // from a gate tile to its up tile
   static constexpr int B_OFF = KPS * A_TILES * A_BYTES;
   static constexpr bool THIN = RT < BM || KPS > 1;
+  // Wide expert tiles (prefill): the MMA's N follows the tile's row count (a 128-row tile with 40 rows costs 48 columns and
+  // loads 64 rows), and two producer warps fetch the rows by index. Grouped launches only. What bounds the expert GEMMs is
+  // shared memory: each k-block is written once and its weight half is read again for every MMA, so a wider tile moves
+  // fewer bytes per product. Gate/up at 8192 rows of 9 pairs: 496 us with 64-row tiles, 365 with these (L2 prefetches of
+  // the weights 4 to 16 k-blocks ahead made it 388 to 419).
+  static constexpr bool VAR_N = BT == 128 && (EPI == EPI_SILU_MUL || EPI == EPI_BF16);
+  static constexpr int GATHER_WARPS = (BT == 128 && EPI == EPI_SILU_MUL) ? 2 : 1;
+  // Staged stores: 16 token rows at a time go through shared memory and leave as 16-byte pieces of 256-byte rows, instead of
+  // 16 two-byte-per-lane stores per warp. Input projection and output projection of a pass, mean: 195 -> 186 us at 8192
+  // rows, 57 -> 52 at 2048, 47 -> 42 at 1531 (one 256-byte bulk copy per row instead: no better, and 20 us slower in the
+  // down projection).
+  static constexpr bool STAGED = !THIN && BT >= 64 && (EPI == EPI_SILU_MUL || EPI == EPI_BF16);
+  static constexpr int OUT_BUFS = STAGED ? 2 : 0;
+  static constexpr int OUT_BYTES = OUT_BUFS * 16 * BM * 2;
   // small token tiles (decode) leave room for two CTAs per SM: one CTA's pipeline fill and epilogue
   // overlap the other's main loop, which matters when K is short (the MoE down projection has 8 k-blocks)
   // The fused gate/up GEMM at 16-row token tiles runs three CTAs per SM with two deep stages each: the same bytes in
@@ -97,11 +112,23 @@ struct Cfg {
   static constexpr int TMEM_COLS_RAW = ACC_COLS * ACC_STAGES;
   static constexpr int TMEM_COLS = TMEM_COLS_RAW <= 32 ? 32 : TMEM_COLS_RAW <= 64 ? 64 : TMEM_COLS_RAW <= 128 ? 128 : TMEM_COLS_RAW <= 256 ? 256 : 512;
   static constexpr int OVERREAD = (BM - RT) * BK * 2;  // bytes behind the last stage that a thin tile's MMA may read
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + (OVERREAD > 256 ? OVERREAD : 256) /*barriers first*/;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + (OVERREAD > 256 ? OVERREAD : 256) /*barriers first*/ + OUT_BYTES;
 };
 
+// Whether `ok` holds in all 128 epilogue threads.
+__device__ __forceinline__ bool epilogue_all(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.aligned.pred q, 2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r) : "r"(static_cast<uint32_t>(ok)) : "memory");
+  return r != 0;
+}
+
 template <int BT, int EPI, bool GROUPED, bool SPLIT = false, int RT = BM, int KPS = 1>
-__global__ void __launch_bounds__(192, Cfg<BT, EPI, RT, KPS>::CTAS_PER_SM)
+__global__ void __launch_bounds__(GROUPED ? 160 + 32 * Cfg<BT, EPI, RT, KPS>::GATHER_WARPS : 192, Cfg<BT, EPI, RT, KPS>::CTAS_PER_SM)
 gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, GemmParams p) {
   using C = Cfg<BT, EPI, RT, KPS>;
   extern __shared__ uint8_t smem_raw[];
@@ -113,8 +140,10 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   uint64_t* acc_empty = bars + 2 * C::STAGES + 2;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  __shared__ float red_max[4][BT > 0 ? BT : 1];
-  __shared__ int red_idx[4][BT > 0 ? BT : 1];
+  uint8_t* out_stage = smem + C::STAGES * C::STAGE_BYTES + 256;  // behind the barriers
+  constexpr int RED = EPI == EPI_ARGMAX ? BT : 1;
+  __shared__ float red_max[4][RED];
+  __shared__ int red_idx[4][RED];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // The grouped tile table is written by the kernel just before this one: wait for it before the first read.
@@ -138,8 +167,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (threadIdx.x == 0) {
     // a gathering producer: lane 0's expect_tx arrival for the weight tile plus one arrival per lane when that
-    // lane's row copies have landed
-    const uint32_t full_count = (GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) ? 33 : 1;
+    // lane's row copies have landed (all lanes of all gathering warps)
+    const uint32_t full_count = (GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) ? 1 + 32 * C::GATHER_WARPS : 1;
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], full_count); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
     *abort_flag = 0;
@@ -154,13 +183,17 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
 
   // geometry of output tile `tile`
+  // (the table entry of the role's next tile is requested one tile ahead: its latency would otherwise open every tile)
+  int4 t_next = make_int4(0, 0, 0, 0);
+  if (GROUPED && tile0 < total) t_next = p.tiles[tile0 / tiles_n];
   auto tile_geom = [&](int tile, int& n0, int& by, int& expert, int& row0, int& nrows) {
     const int nx = tile % tiles_n, byr = tile / tiles_n;
     n0 = nx * RT;
     by = (!GROUPED && p.y_rot) ? (byr + p.y_rot) % tiles_y : byr;
     expert = 0;
     if (GROUPED) {
-      const int4 t = p.tiles[by];
+      const int4 t = t_next;
+      if (!SPLIT && total - tile > tstep) t_next = p.tiles[(tile + tstep) / tiles_n];
       expert = t.x; row0 = t.y; nrows = t.z;
     } else {
       row0 = by * BT;
@@ -185,13 +218,16 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   };
 
-  if (warp == 0 && GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) {
-    // ---------------- gathering producer (all 32 lanes): weights by TMA from lane 0, activation rows by index.
+  constexpr int GW = GROUPED ? C::GATHER_WARPS : 1;
+  if ((warp == 0 || warp >= 6) && GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) {
+    // ---------------- gathering producer (all 32 lanes): weights by TMA from lane 0 of warp 0, activation rows by index
+    // (with two gathering warps, each takes half of the tile's rows).
     // Chunk q = lane + 32 i of a k-block is bytes [16 (q & 7), +16) of tile row q >> 3; it lands where the 128-byte
     // swizzle of the K-major operand layout puts it: row r at (r >> 3) * 1024 + (r & 7) * 128, chunk j at
     // ((j ^ (r & 7)) * 16). Rows beyond the tile's row count are left as they are: an MMA column depends on its own
     // row only, and the epilogue never stores those columns.
-    constexpr int PER_LANE = BT / 4 > 0 ? BT / 4 : 1;
+    constexpr int PER_LANE = BT / 4 / GW > 0 ? BT / 4 / GW : 1;
+    const int rbase = GW == 2 && warp >= 6 ? BT / 2 : 0;
     int it = 0;
     bool live = true;
     const int j = lane & 7;
@@ -201,7 +237,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const bf16* src[PER_LANE];
 #pragma unroll
       for (int i = 0; i < PER_LANE; ++i) {
-        const int r = (lane >> 3) + 4 * i;
+        const int r = rbase + (lane >> 3) + 4 * i;
         const int g = r < nrows ? p.gather_rows[row0 + r] : -1;
         src[i] = g >= 0 ? p.gx + static_cast<size_t>(g) * p.ldgx + j * 8 : nullptr;
       }
@@ -210,14 +246,14 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const uint32_t ph = (it / C::STAGES) & 1;
         if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
         uint8_t* st = smem + s * C::STAGE_BYTES;
-        if (lane == 0) {
+        if (lane == 0 && (GW == 1 || warp == 0)) {
           mbar_expect_tx(&full[s], C::B_OFF);
           load_weights(st, &full[s], n0, expert, kb0 + kb);
         }
         const uint32_t xb = smem_u32(st + C::B_OFF);
 #pragma unroll
         for (int i = 0; i < PER_LANE; ++i) {
-          const int r = (lane >> 3) + 4 * i;
+          const int r = rbase + (lane >> 3) + 4 * i;
           if (src[i] != nullptr) {
             const uint32_t dst = xb + (r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4);
 #pragma unroll
@@ -230,6 +266,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");  // no copy of this lane may outlive the CTA's shared memory
+  } else if (warp >= 6) {
+    // the second gathering warp has nothing to do when the rows come through the tensor map
   } else if (warp == 0) {
     if (elect_one()) {
       int it = 0;  // k-blocks issued so far, over all tiles of this CTA
@@ -261,10 +299,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         uint8_t* st = smem + s * C::STAGE_BYTES;
         if (it >= pre) {
         if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
-        mbar_expect_tx(&full[s], C::STAGE_BYTES);
+        mbar_expect_tx(&full[s], GROUPED && C::VAR_N ? C::B_OFF + (nrows + VAR_BOX - 1) / VAR_BOX * (VAR_BOX * BK * 2) : C::STAGE_BYTES);
         load_weights(st, &full[s], n0, expert, kb0 + kb);
         }
-        if constexpr (C::THIN) tma_load_3d(st + C::B_OFF, &tmX, &full[s], 0, row0, (kb0 + kb) * KPS);
+        if constexpr (GROUPED && C::VAR_N) {
+          for (int r = 0; r < nrows; r += VAR_BOX)
+            tma_load_2d(st + C::B_OFF + r * (BK * 2), &tmX, &full[s], (kb0 + kb) * BK, row0 + r);
+        } else if constexpr (C::THIN) tma_load_3d(st + C::B_OFF, &tmX, &full[s], 0, row0, (kb0 + kb) * KPS);
         else tma_load_2d(st + C::B_OFF, &tmX, &full[s], (kb0 + kb) * BK, row0);
       }
       }
@@ -272,10 +313,15 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (SPLIT) { __syncwarp(); cluster_sync(); }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BT);
+      uint32_t idesc = umma_idesc_bf16(BM, BT);
       bool ok = true;
       int it = 0, lt = 0;  // k-blocks and tiles consumed so far
       for (int tile = tile0; tile < total && ok; tile += tstep, ++lt) {
+      if (GROUPED && C::VAR_N) {
+        int n0, by, expert, row0, nrows;
+        tile_geom(tile, n0, by, expert, row0, nrows);
+        idesc = umma_idesc_bf16(BM, (nrows + 15) / 16 * 16);
+      }
       const int acc = lt % ACC;
       const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
       // the epilogue must have drained this accumulator stage (two tiles ago) before it is overwritten
@@ -311,6 +357,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     pdl_wait();  // first global write of the CTA comes from here
     const int q = warp & 3;
     int lt = 0;
+    int out_buf = 0;  // staging buffer of the next 16 rows
+    const bool staged = C::STAGED && p.ldo % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
     for (int tile = tile0; tile < total; tile += tstep, ++lt) {
     int n0, by, expert, row0, nrows;
     tile_geom(tile, n0, by, expert, row0, nrows);
@@ -318,7 +366,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const int nx = n0 / RT;
     const int acc = lt % ACC;
     const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
-    const bool ok = mbar_wait(&acc_full[acc], (lt / ACC) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
+    bool ok = mbar_wait(&acc_full[acc], (lt / ACC) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
+    if (C::STAGED && staged) ok = epilogue_all(ok);  // the batches below hold barriers: all four warps take them, or none
     tc_fence_after();
     const int n = n0 + q * 32 + lane;
     const bool n_ok = n < p.N && (RT == BM || q * 32 + lane < RT);
@@ -493,6 +542,22 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 p.pair_out[m.x][static_cast<size_t>(m.y) * p.ldo + n] = __float2bfloat16(v[j]);
               }
             }
+          }
+        } else if (C::STAGED && staged) {
+          // [16 rows][128 weight rows] bf16, two buffers: a lane writes its column, and behind the barrier the 128 threads
+          // send the rows. A thread's reads of a buffer precede its next barrier, behind which the buffer is written again.
+          bf16* ob = reinterpret_cast<bf16*>(out_stage) + out_buf * (16 * BM);
+          out_buf ^= 1;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) ob[j * BM + q * 32 + lane] = __float2bfloat16(v[j]);
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          const int col = (lane & 15) * 8;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int r = i * 8 + q * 2 + (lane >> 4);
+            const uint4 o = *reinterpret_cast<const uint4*>(ob + r * BM + col);
+            if (c + r < nrows && n0 + col < p.N)
+              *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + static_cast<size_t>(row0 + c + r) * p.ldo + n0 + col) = o;
           }
         } else if (n_ok) {
 #pragma unroll
@@ -690,7 +755,8 @@ static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams
   GemmParams q = p;
   q.grid_y = grid_y;
   const long long tiles = static_cast<long long>((p.N + RT - 1) / RT) * grid_y;
-  return launch_pdl(kern, dim3(static_cast<unsigned>(tiles < resident ? tiles : resident)), dim3(192), C::SMEM, st, tw,
+  constexpr int threads = GROUPED ? 160 + 32 * C::GATHER_WARPS : 192;
+  return launch_pdl(kern, dim3(static_cast<unsigned>(tiles < resident ? tiles : resident)), dim3(threads), C::SMEM, st, tw,
                     tx, q) == cudaSuccess ? 0 : -4;
 }
 
@@ -865,7 +931,7 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
     p.gx = static_cast<const bf16*>(X);
     p.ldgx = ldx;
     if (make_map(&tx, X, K, bt, 0, ldx, 0, bt)) return -1;  // unused by the gathering producer, but a valid map
-  } else if (make_map(&tx, X, K, cap, 0, K, 0, bt)) return -1;
+  } else if (make_map(&tx, X, K, cap, 0, K, 0, bt == 128 ? VAR_BOX : bt)) return -1;  // 128: Cfg::VAR_N
   switch (epi) {
     case EPI_BF16: return dispatch_bt<EPI_BF16, true>(bt, tw, tx, p, max_tiles, st);
     case EPI_SILU_MUL: return dispatch_bt<EPI_SILU_MUL, true>(bt, tw, tx, p, max_tiles, st);

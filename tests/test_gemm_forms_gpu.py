@@ -47,3 +47,25 @@ def test_expert_block_of_a_few_rows_with_packed_weights(C, T, inter, H):
     got = C.moe_block(x, router, C.pack_weight(gu.clone(), gate_up=True), C.pack_weight(dn.clone()), E, k, True)
     C.check_errors(x.device)
     assert torch.equal(got, plain)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(600, 16, 4, 256, 128), (1100, 32, 8, 2048, 512), (515, 8, 2, 512, 192)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_wide_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, packed):
+    """Experts of every size around the tile: full tiles, last tiles of few rows, an expert without rows."""
+    x = _bf(T, H, seed=T)
+    router = _bf(E + 1, H, scale=0.3, seed=34)
+    router[3] = -4.0 * x.float().mean(0).bfloat16()  # rarely picked
+    wgu, wd = _bf(E + 1, 2 * I, H, scale=0.05, seed=35), _bf(E + 1, H, I, scale=0.05, seed=36)
+    if packed:
+        wgu, wd = C.pack_weight(wgu, gate_up=True), C.pack_weight(wd)
+    keep = C.GATHER_MAX_BT, C.WIDE_MIN_ROWS
+    try:
+        C.WIDE_MIN_ROWS = 1
+        wide = C.moe_block(x, router, wgu, wd, E, k, True)
+        C.GATHER_MAX_BT = 64
+        narrow = C.moe_block(x, router, wgu, wd, E, k, True)
+    finally:
+        C.GATHER_MAX_BT, C.WIDE_MIN_ROWS = keep
+    C.check_errors(x.device)
+    assert torch.equal(wide, narrow)
