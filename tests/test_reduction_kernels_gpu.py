@@ -81,3 +81,35 @@ def test_greedy_head_takes_the_lowest_id_among_equal_logits(C, T, V):
     first = torch.where(logits == top, torch.arange(V, device="cuda"), V).amin(1)
     idx, val = C.lm_head_argmax(x, w, return_value=True)
     assert torch.equal(idx, first) and torch.equal(val.double(), top[:, 0])
+
+
+@pytest.mark.parametrize("n_q,n_kv,D,rot", [(16, 2, 256, 64), (8, 1, 64, 16), (4, 2, 128, 128), (4, 1, 32, 8), (32, 4, 64, 20)])
+def test_attention_prep_heads_and_rotary_dims(C, n_q, n_kv, D, rot):
+    """More heads than warps of a CTA, rotary dims that end inside a lane's run, every row in a page of its own."""
+    from b200serve.ops import torch_ops as O
+
+    T, dev = 37, "cuda"
+    g = torch.Generator(device=dev).manual_seed(D + rot)
+    qkv = torch.randn(T, (2 * n_q + 2 * n_kv) * D + 8, device=dev, generator=g).bfloat16()[:, :-8]
+    qn, kn = (torch.randn(D, device=dev, generator=g).bfloat16() * 0.1 for _ in range(2))
+    positions = torch.randint(0, 4096, (T,), device=dev, generator=g)
+    tables = torch.zeros(T, 64, dtype=torch.int32, device=dev)
+    tables[torch.arange(T), positions // 64] = torch.arange(1, T + 1, dtype=torch.int32, device=dev)
+    seq = torch.arange(T, dtype=torch.int32, device=dev)
+    kv = torch.zeros(T + 1, 2, n_kv, 64, D, device=dev, dtype=torch.bfloat16)
+    q = torch.empty(T, n_q, D, device=dev, dtype=torch.bfloat16)
+    gate = torch.empty(T, n_q * D, device=dev, dtype=torch.bfloat16)
+    rc = C.lib().b200_attn_prep(qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), tables.data_ptr(), 64, seq.data_ptr(),
+                                qn.data_ptr(), kn.data_ptr(), q.data_ptr(), gate.data_ptr(), kv.data_ptr(), T, n_q, n_kv, D,
+                                rot, 1e7, 1e-6, T + 1, C.err_word(qkv.device).data_ptr(), C._stream())
+    assert rc == 0
+    C.check_errors(qkv.device)
+    rq, rg, rk, rv = O.attn_prep(qkv.float(), positions, qn.float(), kn.float(), n_q, n_kv, D, rot, 1e7, 1e-6)
+    rows = torch.arange(T, device=dev)
+    assert torch.equal(gate, rg.bfloat16()) and torch.equal(kv[rows + 1, 1, :, positions % 64], rv.bfloat16())
+    for got, ref in ((q, rq), (kv[rows + 1, 0, :, positions % 64], rk)):
+        size = ref.abs().clone()  # a rotated pair mixes two dims: four roundings to bf16 (2^-8 each) of up to their norm
+        half = rot // 2
+        pair = (ref[..., :half] ** 2 + ref[..., half:2 * half] ** 2).sqrt()
+        size[..., :half], size[..., half:2 * half] = pair, pair
+        assert ((got.float() - ref).abs() <= 2.0 ** -6 * size * 1.5 + 1e-3).all()
