@@ -6,15 +6,22 @@
 // M = BLOCK_R x GROUP rows the same way on MFMA). Per 64-key page:
 //
 //   S[128 x 64]  = Q[128 x D] K[64 x D]^T      tcgen05.mma, both operands K-major, S in TMEM
-//   softmax      : each of 128 threads owns one TMEM lane = one row, so row max / sum need no
-//                  shuffles; P = exp2(S - m) goes to shared memory as bf16 in the swizzled K-major
-//                  layout the next MMA reads; the O accumulator in TMEM is rescaled only when a
-//                  row maximum grew by more than 2^8 (exact: the final division uses the same m)
+//   softmax      : warps 0..3 take the even pages, warps 4..7 the odd ones, each thread one whole row (TMEM lane), so a
+//                  page's maximum, exponentials and sum need no other thread. What two pages share is the running row
+//                  maximum, which the thread of page i hands to the thread of page i + 1 as soon as it has seen its
+//                  scores: the exponentials of two pages run at the same time. P = exp2(S - m) goes to shared memory
+//                  as bf16 in the swizzled K-major layout the next MMA reads; the O accumulator in TMEM is rescaled only
+//                  when a row maximum grew by more than 2^8 (exact: the final division uses the same m)
 //   O[128 x D]  += P[128 x 64] V[64 x D]       V is read straight from its page layout as an
 //                                              MN-major B operand (no transpose)
 //
-// Warp 4 lane 0 drives TMA (Q once, K/V pages double-buffered) and issues all MMAs; warps 0..3
-// do the softmax and the epilogue (divide by the row sum, multiply by sigmoid(gate), store bf16).
+// Warp 8 issues the MMAs (Q K^T two pages ahead of P V), warps 9 and 10 drive TMA (Q once; K and V pages in rings of their own: a
+// K page is free when its scores are there, a V page after its P V). The epilogue divides by the row sum, multiplies by
+// sigmoid(gate) and stores bf16. Bound: shared memory, which per page and SM takes 64 KB of K and V in and gives the MMAs
+// 96 KB (Q K^T: N = 64, 48 cycles an MMA) and 48 KB (P V). With one thread for all loads and MMAs, which also read the page
+// table between a free stage and its load, and one page in the softmax at a time, a page took 3400 cycles; it takes about
+// 1800 now: 4 x 2048 rows behind 6.5k to 28.7k tokens 3.70 -> 1.94 ms (1.23 PFLOP/s at 30k), 8 x 1024 rows 249 -> 206 us,
+// decode of 256 x 2.2k tokens 282 -> 224 us, of four sequences of 50-90k 147 -> 118 us.
 // Chunked prefill: queries sit at positions pos0.. of their sequence, keys are 0..pos.
 // All waits are bounded (common.cuh). No cluster multicast.
 #include "common.cuh"
@@ -61,11 +68,12 @@ struct FlashCfg {
   // dynamic shared memory is declared 1024-byte aligned (checked at run time), so no alignment slack is budgeted:
   // with D = 256 the tiles, the barriers and the 2 KB of static exchange arrays fill the 227 KB of an SM
   static constexpr int SMEM = Q_BYTES + 2 * ST * KV_BYTES + 2 * P_BYTES + 256;
+  static constexpr int ROW_WARPS = DEC ? 1 : 4;  // softmax warps per page: the decode form's 8 rows are one warp's
   static constexpr int TMEM_COLS = (128 + D) <= 256 ? 256 : 512;  // two score tiles of 64 columns + the output
 };
 
 template <int D, int GROUP, bool DEC = false>
-__global__ void __launch_bounds__(288, 1)
+__global__ void __launch_bounds__(352, 1)
 flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, FlashParams p) {
   using C = FlashCfg<D, DEC>;
   constexpr int DB = C::DB;
@@ -84,13 +92,17 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint8_t* sV = sK + ST * C::KV_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + ST * C::KV_BYTES);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;                // [ST]
-  uint64_t* kv_empty = bars + 4;               // [ST]: completes when P.V of the page in that stage has finished
-  uint64_t* s_full = bars + 7;                 // [2]: one per score tile
-  uint64_t* p_full = bars + 9;
-  uint64_t* acc_done = bars + 10;
-  uint64_t* x_bar = bars + 11;                 // exchange point of the 256 softmax threads (bounded wait, unlike bar.sync)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* k_full = bars + 1;                 // [ST]
+  uint64_t* v_full = bars + 4;                 // [ST]
+  uint64_t* k_empty = bars + 7;                // [ST]: Q K^T of the page in that stage has finished
+  uint64_t* v_empty = bars + 10;               // [ST]: P V of the page in that stage has finished
+  uint64_t* s_full = bars + 13;                // [2]: one per score tile
+  uint64_t* p_full = bars + 15;                // [2]: one per probability tile
+  uint64_t* pv_done = bars + 17;               // [2]: P V of an even / odd page has finished
+  uint64_t* acc_done = bars + 19;
+  uint64_t* x_bar = bars + 20;                 // exchange point of the softmax threads (bounded wait, unlike bar.sync)
+  uint64_t* m_bar = bars + 21;                 // [2][4]: the row maxima up to an even / odd page, one per warp of rows
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 29);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -118,12 +130,11 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < ST; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 256);
+    for (int s = 0; s < ST; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 32 * C::ROW_WARPS); mbar_init(&pv_done[s], 1); }
+    for (int w = 0; w < 8; ++w) mbar_init(&m_bar[w], 1);
     mbar_init(acc_done, 1);
-    mbar_init(x_bar, 256);
+    mbar_init(x_bar, 64 * C::ROW_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -137,32 +148,39 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   pdl_launch();  // this CTA holds its TMEM columns: the next kernel's CTAs may queue behind it
   const uint32_t tmem_S = tmem, tmem_O = tmem + 128;  // score tile of page i at tmem_S + (i & 1) * 64
 
-  if (warp == 8) {
+  if (warp >= 9) {
+    // warp 9 brings Q and the K pages, warp 10 the V pages: K runs a page ahead of what frees V, and one thread for both
+    // would hold each back behind the other. The next page number is read before the wait for a free stage.
     if (elect_one()) {
-      auto load_page = [&](int i) {
+      const int which = warp - 9;
+      uint64_t* full = which ? v_full : k_full;
+      uint64_t* empty = which ? v_empty : k_empty;
+      uint8_t* stages = which ? sV : sK;
+      const int* table = p.tables + static_cast<size_t>(seg) * p.max_pages + first;
+      if (which == 0) {
+        mbar_expect_tx(q_full, DEC ? DB * GROUP * 128 : C::Q_BYTES);  // decode: GROUP rows of 128 bytes per block
+        for (int a = 0; a < DB; ++a) tma_load_4d(sQ + a * C::Q_BLOCK, &tmQ, q_full, a * 64, 0, kh, seg_row0 + p0);
+      }
+      int next = table[0];
+      for (int i = 0; i < np; ++i) {
         const int s = i % ST;
-        int page = p.tables[static_cast<size_t>(seg) * p.max_pages + first + i];
+        int page = next;
+        if (i + 1 < np) next = table[i + 1];
         if (page < 0 || page >= p.num_pages) { atomicCAS(p.err, 0, ERR_BAD_INDEX); page = 0; }
-        const int krow = ((page * 2 + 0) * p.n_kv + kh) * FP_PAGE;
-        const int vrow = ((page * 2 + 1) * p.n_kv + kh) * FP_PAGE;
-        mbar_expect_tx(&kv_full[s], 2 * C::KV_BYTES);
-        for (int a = 0; a < DB; ++a) {
-          tma_load_2d(sK + s * C::KV_BYTES + a * FP_PAGE * 128, &tmKV, &kv_full[s], a * 64, krow);
-          tma_load_2d(sV + s * C::KV_BYTES + a * FP_PAGE * 128, &tmKV, &kv_full[s], a * 64, vrow);
-        }
-      };
-      mbar_expect_tx(q_full, DEC ? DB * GROUP * 128 : C::Q_BYTES);  // decode: GROUP rows of 128 bytes per block
-      for (int a = 0; a < DB; ++a) tma_load_4d(sQ + a * C::Q_BLOCK, &tmQ, q_full, a * 64, 0, kh, seg_row0 + p0);
-      for (int i = 0; i < ST && i < np; ++i) load_page(i);
+        if (!mbar_wait(&empty[s], ((i / ST) & 1) ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) break;
+        mbar_expect_tx(&full[s], C::KV_BYTES);
+        const int row = ((page * 2 + which) * p.n_kv + kh) * FP_PAGE;
+        for (int a = 0; a < DB; ++a) tma_load_2d(stages + s * C::KV_BYTES + a * FP_PAGE * 128, &tmKV, &full[s], a * 64, row);
+      }
+    }
+  } else if (warp == 8) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 64);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, D) | (1u << 16);  // B operand MN-major
-      // Software pipeline: Q K^T of page i + 1 is issued before the wait for the probabilities of page i, into the
-      // other score tile, so the tensor pipe works on the next scores while the softmax threads are busy.
-      bool ok = mbar_wait(q_full, 0, p.err, ERR_WAIT_FULL, abort_flag);
       const uint32_t qa = smem_u32(sQ);
       auto issue_qk = [&](int i) {
         const int s = i % ST;
-        if (!mbar_wait(&kv_full[s], (i / ST) & 1, p.err, ERR_WAIT_FULL, abort_flag)) return false;
+        if (!mbar_wait(&k_full[s], (i / ST) & 1, p.err, ERR_WAIT_FULL, abort_flag)) return false;
         tc_fence_after();
         const uint32_t ka = smem_u32(sK + s * C::KV_BYTES);
 #pragma unroll
@@ -172,131 +190,127 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                     umma_smem_desc(ka + blk * FP_PAGE * 128 + koff), idesc_qk, kk != 0);
         }
         umma_commit(&s_full[i & 1]);
+        umma_commit(&k_empty[s]);
         return true;
       };
-      ok = ok && issue_qk(0);
-      // The stage of page i - 1 is free once its P.V has finished; it takes page i - 1 + ST. With two stages that is
-      // page i + 1, which Q K^T needs in this very iteration, so the refill comes first (and waits for the P.V just
-      // issued). With three stages page i + 1 is already there and the refill waits until the softmax of page i has
-      // run, by when P.V of page i - 1 is long done: two pages are loaded or on their way while page i is used.
-      auto refill = [&](int i) {
-        if (i < 1 || i - 1 + ST >= np) return true;
-        if (!mbar_wait(&kv_empty[(i - 1) % ST], ((i - 1) / ST) & 1, p.err, ERR_WAIT_EMPTY, abort_flag)) return false;
-        load_page(i - 1 + ST);
-        return true;
-      };
+      bool ok = mbar_wait(q_full, 0, p.err, ERR_WAIT_FULL, abort_flag);
+      ok = ok && issue_qk(0) && (np < 2 || issue_qk(1));
       for (int i = 0; i < np && ok; ++i) {
+        // the probabilities of page i are written, so its score tile has been read: Q K^T of page i + 2 goes first, the
+        // threads that just finished page i wait for it
+        ok = mbar_wait(&p_full[i & 1], (i >> 1) & 1, p.err, ERR_WAIT_FULL, abort_flag);
+        if (ok && i + 2 < np) ok = issue_qk(i + 2);
         const int s = i % ST;
-        if (ST == 2) { ok = refill(i); if (!ok) break; }
-        if (i + 1 < np) {
-          ok = issue_qk(i + 1);  // its score tile was last read by the softmax of page i - 1, which has arrived at p_full
-          if (!ok) break;
-        }
-        ok = mbar_wait(p_full, i & 1, p.err, ERR_WAIT_FULL, abort_flag);
+        ok = ok && mbar_wait(&v_full[s], (i / ST) & 1, p.err, ERR_WAIT_FULL, abort_flag);
         if (!ok) break;
-        if (ST > 2) { ok = refill(i); if (!ok) break; }
         tc_fence_after();
         const uint32_t pa = smem_u32(sP + (i & 1) * C::P_BYTES), va = smem_u32(sV + s * C::KV_BYTES);
 #pragma unroll
         for (int kk = 0; kk < FP_PAGE / 16; ++kk)
           umma_bf16(tmem_O, umma_smem_desc(pa + kk * 32), umma_smem_desc_mn(va + kk * 2048, FP_PAGE * 128), idesc_pv,
                     (i | kk) != 0);
-        umma_commit(&kv_empty[s]);
+        umma_commit(&pv_done[i & 1]);
+        umma_commit(&v_empty[s]);
       }
       umma_commit(acc_done);
     }
-  } else {
-    // ---------------- softmax + epilogue: 256 threads, two per TMEM lane. Thread (r = tid & 127, hf = tid >> 7) owns
-    // row r = one (position, head) and the half hf of everything indexed by a column: 32 of the page's 64 scores,
-    // half of the output columns. The two halves of a row agree on the row maximum through shared memory, so both
-    // take the same rescale decision; their partial row sums are added (half 0 + half 1) at the end.
-    __shared__ float s_mx[2][2][128];  // [page parity][half][row]; reused for the row sums at the end
-    const int r = threadIdx.x & 127, hf = threadIdx.x >> 7;
-    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  } else if ((warp & 3) < C::ROW_WARPS) {
+    // ---------------- softmax + epilogue: thread (r = tid & 127, hf = tid >> 7) owns row r = one (position, head) on the
+    // pages i with i & 1 == hf, and the half hf of the output columns at the end.
+    __shared__ float s_m[128];  // the running row maximum, in the hands of the page that is to see its scores next
+    const int r = threadIdx.x & 127, hf = threadIdx.x >> 7, rw = warp & 3;
+    const uint32_t lane_base = static_cast<uint32_t>(rw * 32) << 16;
     const int lp = r / GROUP, head = r % GROUP;
     const int qpos = pos0 + p0 + lp;
     const bool row_valid = lp < n_pos;
     constexpr int DH = D / 2;
-    float m_used = -INFINITY, l = 0.f;
+    float m_loc = -INFINITY, l = 0.f;  // the maximum and the sum of this thread's own pages, at that maximum
     bool ok = true;
-    for (int i = 0; i < np && ok; ++i) {
-      ok = mbar_wait(&s_full[i & 1], (i >> 1) & 1, p.err, ERR_WAIT_TMEM, abort_flag);
+    for (int i = hf; i < np && ok; i += 2) {
+      const uint32_t ph = (i >> 1) & 1;
+      ok = mbar_wait(&s_full[hf], ph, p.err, ERR_WAIT_TMEM, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      float sc[32];
+      float sc[64];
+      tmem_ld64(tmem_S + hf * 64 + lane_base, sc);
+      const int kbase = (first + i) * FP_PAGE;
+      if (DEC || kbase + FP_PAGE - 1 > pos0 + p0) {  // only pages that end behind the tile's first query hide keys
+        // decode: rows past the real ones hold whatever the MMA read behind the Q atom; masked, so that they never ask for
+        // a rescale of the output tile
 #pragma unroll
-      for (int c = 0; c < 32; c += 16) tmem_ld16(tmem_S + (i & 1) * 64 + hf * 32 + lane_base + c, sc + c);
-      float mx = -INFINITY;
-      const int kbase = (first + i) * FP_PAGE + hf * 32;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        // decode: rows past the real ones hold whatever the MMA read behind the Q atom; masked, so that they never
-        // ask for a rescale of the output tile
-        sc[j] = (kbase + j <= qpos && (!DEC || row_valid)) ? sc[j] * p.scale_log2 : -INFINITY;
-        mx = fmaxf(mx, sc[j]);
+        for (int j = 0; j < 64; ++j) sc[j] = (kbase + j <= qpos && (!DEC || row_valid)) ? sc[j] : -INFINITY;
       }
-      s_mx[i & 1][hf][r] = mx;
-      mbar_arrive(x_bar);
-      ok = mbar_wait(x_bar, i & 1, p.err, ERR_WAIT_FULL, abort_flag);
-      if (!ok) break;
-      mx = fmaxf(mx, s_mx[i & 1][hf ^ 1][r]);
-      const bool need = mx > m_used + 8.0f;
-      // The scores of this page were computed while P.V of the previous page may still be running. This page's
-      // probability tile was last read by P.V of page i - 2; the output tile may only be rescaled once P.V of page
-      // i - 1 has finished, which is waited for only in the (rare, after the first pages) case of a rescale.
-      if (i >= 2) {
-        ok = mbar_wait(&kv_empty[(i - 2) % ST], ((i - 2) / ST) & 1, p.err, ERR_WAIT_EMPTY, abort_flag);
+      float mx4[4] = {sc[0], sc[1], sc[2], sc[3]};
+#pragma unroll
+      for (int j = 4; j < 64; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], sc[j]);
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      float m_prev = -INFINITY;
+      if (i > 0) {
+        ok = mbar_wait(&m_bar[(hf ^ 1) * 4 + rw], ((i - 1) >> 1) & 1, p.err, ERR_WAIT_FULL, abort_flag);
         if (!ok) break;
+        m_prev = s_m[r];
       }
-      const bool any_need = __any_sync(0xffffffffu, need);
-      if (any_need && i > 0) {
-        ok = mbar_wait(&kv_empty[(i - 1) % ST], ((i - 1) / ST) & 1, p.err, ERR_WAIT_EMPTY, abort_flag);
+      const bool need = mx > m_prev + 8.0f;
+      const float m = need ? mx : m_prev;
+      s_m[r] = m;
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(&m_bar[hf * 4 + rw]);
+      // The output tile may only be rescaled once P V of page i - 1 has finished; P V of this page and the later ones wait
+      // for this page's probabilities.
+      if (__any_sync(0xffffffffu, need) && i > 0) {  // warp-uniform: TMEM loads/stores are warp-collective
+        ok = mbar_wait(&pv_done[hf ^ 1], ((i - 1) >> 1) & 1, p.err, ERR_WAIT_EMPTY, abort_flag);
         if (!ok) break;
         tc_fence_after();
-      }
-      if (any_need) {  // warp-uniform: TMEM loads/stores are warp-collective
-        const float factor = need ? exp2f(m_used - mx) : 1.0f;  // exp2(-inf) = 0 on the first page
-        if (need) { m_used = mx; l *= factor; }
-        if (i > 0) {
+        const float factor = need ? exp2_ftz(m_prev - m) : 1.0f;
 #pragma unroll 1
-          for (int c = 0; c < DH; c += 16) {
-            float o[16];
-            tmem_ld16(tmem_O + lane_base + hf * DH + c, o);
+        for (int c = 0; c < D; c += 16) {
+          float o[16];
+          tmem_ld16(tmem_O + lane_base + c, o);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] *= factor;
-            tmem_st16(tmem_O + lane_base + hf * DH + c, o);
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          for (int j = 0; j < 16; ++j) o[j] *= factor;
+          tmem_st16(tmem_O + lane_base + c, o);
         }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      float sum = 0.f;
-      uint8_t* prow = sP + (i & 1) * C::P_BYTES + r * 128;
+      if (m != m_loc) { l *= exp2_ftz(m_loc - m); m_loc = m; }  // exp2(-inf) = 0 on this thread's first page
+      if (i >= 2) {  // this page's probability tile was last read by P V of page i - 2
+        ok = mbar_wait(&pv_done[hf], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag);
+        if (!ok) break;
+      }
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      uint8_t* prow = sP + hf * C::P_BYTES + r * 128;
       if (!DEC || r < 8)  // decode: the probability tile holds one 8-row atom; the other rows' scores are not kept
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 8; ++c) {
         uint4 packed;
         __nv_bfloat162* pe = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float a = exp2f(sc[c * 8 + 2 * j] - m_used), b2 = exp2f(sc[c * 8 + 2 * j + 1] - m_used);
-          sum += a + b2;
+          const float a = exp2_ftz(fmaf(sc[c * 8 + 2 * j], p.scale_log2, -m)), b2 = exp2_ftz(fmaf(sc[c * 8 + 2 * j + 1], p.scale_log2, -m));
+          sum[(2 * j) & 3] += a;
+          sum[(2 * j + 1) & 3] += b2;
           pe[j] = __floats2bfloat162_rn(a, b2);
         }
-        *reinterpret_cast<uint4*>(prow + (((hf * 4 + c) ^ (r & 7)) * 16)) = packed;  // 128-byte swizzle of the K-major tile
+        *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) * 16)) = packed;  // 128-byte swizzle of the K-major tile
       }
-      l += sum;
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc_fence_before();
-      mbar_arrive(p_full);
+      mbar_arrive(&p_full[hf]);
     }
     ok = ok && mbar_wait(acc_done, 0, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
     tc_fence_after();
-    if (ok) {
-      // every thread has read its partner's last maximum (it arrived at p_full afterwards, and acc_done follows that)
-      s_mx[0][hf][r] = l;
+    float m_used = m_loc;
+    if (ok) {  // the probability tiles are free now: even and odd pages put their sums together, even + odd
+      float* ex = reinterpret_cast<float*>(sP);
+      constexpr int STRIDE = 32 * C::ROW_WARPS;
+      ex[(hf * STRIDE + r) * 2] = l;
+      ex[(hf * STRIDE + r) * 2 + 1] = m_loc;
       mbar_arrive(x_bar);
-      ok = mbar_wait(x_bar, np & 1, p.err, ERR_WAIT_FULL, abort_flag);
-      l = s_mx[0][0][r] + s_mx[0][1][r];
+      ok = mbar_wait(x_bar, 0, p.err, ERR_WAIT_FULL, abort_flag);
+      const float l0 = ex[r * 2], m0 = ex[r * 2 + 1], l1 = ex[(STRIDE + r) * 2], m1 = ex[(STRIDE + r) * 2 + 1];
+      m_used = fmaxf(m0, m1);  // a running maximum never falls: the larger one is the last page's
+      l = l0 * exp2_ftz(m0 - m_used) + l1 * exp2_ftz(m1 - m_used);
     }
     if (ok && p.split_pages > 0) {
       const size_t row = static_cast<size_t>(seg_row0 + p0 + lp);
@@ -385,7 +399,7 @@ int fp_launch(const CUtensorMap& tq, const CUtensorMap& tkv, const FlashParams& 
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashCfg<D, DEC>::SMEM) != cudaSuccess) return -3;
     configured[dev] = true;
   }
-  return launch_pdl(kern, dim3(n_tiles, p.n_kv, gz), dim3(288), FlashCfg<D, DEC>::SMEM, st, tq, tkv, p) == cudaSuccess ? 0 : -4;
+  return launch_pdl(kern, dim3(n_tiles, p.n_kv, gz), dim3(352), FlashCfg<D, DEC>::SMEM, st, tq, tkv, p) == cudaSuccess ? 0 : -4;
 }
 }  // namespace
 

@@ -113,3 +113,26 @@ def test_attention_prep_heads_and_rotary_dims(C, n_q, n_kv, D, rot):
         pair = (ref[..., :half] ** 2 + ref[..., half:2 * half] ** 2).sqrt()
         size[..., :half], size[..., half:2 * half] = pair, pair
         assert ((got.float() - ref).abs() <= 2.0 ** -6 * size * 1.5 + 1e-3).all()
+
+
+@pytest.mark.parametrize("n_q,n_kv,D", [(16, 2, 256), (4, 1, 128), (2, 2, 64)])
+@pytest.mark.parametrize("pos0,n", [(0, 1), (0, 64), (63, 2), (64, 65), (130, 40), (256, 193), (510, 300)])
+def test_flash_pages_of_growing_scores(C, n_q, n_kv, D, pos0, n):
+    """Even and odd page counts; scores that grow along the context, so that the running maximum of a row, which two groups
+    of threads pass to and fro, keeps moving and the output is rescaled on many pages."""
+    from b200serve.ops import torch_ops as O
+
+    g = torch.Generator(device="cuda").manual_seed(n + pos0)
+    pages = (pos0 + n + 63) // 64
+    kv = torch.randn(pages + 1, 2, n_kv, 64, D, device="cuda", generator=g)
+    table = (torch.randperm(pages, device="cuda", generator=g) + 1).int().view(1, -1)
+    for i, pg in enumerate(table[0].tolist()):
+        kv[pg, 0] *= 1.0 + 1.5 * i  # log2 of a row's largest score grows by about 8 per page
+    kv = kv.bfloat16()
+    q = torch.randn(n, n_q, D, device="cuda", generator=g).bfloat16()
+    gate = torch.randn(n, n_q * D, device="cuda", generator=g).bfloat16()
+    got = C.flash_prefill(q, gate, kv, table, [0, n], [pos0])
+    C.check_errors(q.device)
+    ref = O.paged_attention(q.float(), gate.float(), kv.float(), table, [0, n], [pos0])
+    # probabilities, output and gated output are rounded to bf16 (2^-8 each), on values of up to about four
+    assert (got.float() - ref).abs().max().item() <= 3 * 2.0 ** -8 * 5
