@@ -13,8 +13,9 @@
 //  gdn_scan_tc : one CTA per (sequence, value head), chunks in order. The transposed fp32 state S^T [dv, dk] lives
 //                in TMEM for the whole sequence, with a bf16 copy in shared memory as the MMA operand. Per chunk:
 //                v_new^T = u^T - S^T w^T and o^T = S^T (q e^g)^T (tcgen05, N = 64 tokens), v_new goes to shared memory
-//                as bf16, then o^T += v_new^T scores^T and S^T = S^T e^{g_last} + v_new^T (k e^{g_last-g})
-//                (reference: engine/fast/gdn_chunk.py:494-628). A TMA producer warp runs two chunks ahead.
+//                as bf16, then S^T = S^T e^{g_last} + v_new^T (k e^{g_last-g}) and o^T += v_new^T scores^T
+//                (reference: engine/fast/gdn_chunk.py:494-628). A TMA producer warp runs two chunks ahead, four warps
+//                store o while the next chunk is under way.
 //
 // Operands are rounded to bf16 where the reference's chunk kernels round them too (w, u, the decayed q / k, the
 // state as an MMA operand); accumulation and the resident state are fp32. Padding rows of a partial chunk have
@@ -419,60 +420,85 @@ struct ScanParams {
 };
 
 constexpr int SC_STAGE = 4 * 16384 + 8192;  // w | u | qg | kg | scores
-constexpr int SC_SMEM = 32768 + 16384 + 2 * SC_STAGE + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int SC_SMEM = 32768 + 16384 + 2 * SC_STAGE + 16384 + 1024 /*align*/ + 256 /*barriers*/;
 
-__global__ void __launch_bounds__(192, 1)
+// The chunks of a sequence are a serial chain, and with few sequences nothing else hides it: 148 -> 74 us for one
+// span of 2048 tokens x 32 heads (32 chunks, 8500 -> 3100 cycles each), 168 -> 89 us for 8 x 1024 (256 CTAs, 148 SMs).
+// What is kept out of the chain: the next chunk's u rows are read while the state MMAs run; the scaling by the next chunk's
+// decay rides on the pass that refreshes the bf16 copy of the state; two threads share a TMEM lane, each with half of the
+// columns; the state MMAs go before the rest of o's; and four warps of their own take o (two accumulators in turn) out of
+// TMEM, transpose it through shared memory and store 16-byte pieces (the chain's threads spent 2950 of 6000 cycles a chunk on
+// two-byte stores; the gated norm in these warps as well made them the bottleneck, 6700 cycles).
+__global__ void __launch_bounds__(448, 1)
 gdn_scan_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, ScanParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sS = smem;                 // bf16 S^T [128 dv][128 dk], two K atoms
   uint8_t* sVN = smem + 32768;        // bf16 v_new^T [128 dv][64 tokens]
   uint8_t* stages = smem + 49152;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stages + 2 * SC_STAGE);
-  uint64_t* full = bars;              // [2]
-  uint64_t* empty = bars + 2;         // [2]
-  uint64_t* vn_done = bars + 4;       // MMA -> threads: v_new and the state part of o are in TMEM
-  uint64_t* vn_ready = bars + 5;      // threads -> MMA: bf16 v_new in shared memory, state scaled (128 arrivals)
-  uint64_t* o_done = bars + 6;        // MMA -> threads: o complete, state updated
-  uint64_t* s_ready = bars + 7;       // threads -> MMA: bf16 state copy refreshed (128 arrivals)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint8_t* sO = stages + 2 * SC_STAGE;  // bf16 o [64 tokens][128 dv]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 16384);
+  uint64_t* full = bars;              // [3][2]: w and qg | u | kg and scores
+  uint64_t* empty = bars + 6;         // [3][2]
+  uint64_t* vn_done = bars + 12;      // MMA -> threads: S^T w^T is in TMEM
+  uint64_t* vn_ready = bars + 13;     // threads -> MMA: bf16 v_new in shared memory
+  uint64_t* s_done = bars + 14;       // MMA -> threads: state updated, its bf16 copy no longer read
+  uint64_t* s_ready = bars + 15;      // threads -> MMA: bf16 state copy refreshed, state scaled for the next chunk
+  uint64_t* o_done = bars + 16;       // [2] MMA -> output threads: o of an even / odd chunk is complete
+  uint64_t* o_free = bars + 18;       // [2] output threads -> MMA: it has been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int seg = blockIdx.x, h = blockIdx.y;
-  const int2 sc = p.seg_chunks[seg];
-  const int nc = sc.y;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < 6; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], s == 2 || s == 3 ? 256 : 1); }
     mbar_init(vn_done, 1);
-    mbar_init(vn_ready, 128);
-    mbar_init(o_done, 1);
-    mbar_init(s_ready, 128);
+    mbar_init(vn_ready, 256);
+    mbar_init(s_done, 1);
+    mbar_init(s_ready, 256);
+    mbar_init(&o_done[0], 1);
+    mbar_init(&o_done[1], 1);
+    mbar_init(&o_free[0], 128);
+    mbar_init(&o_free[1], 128);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const int2 sc = p.seg_chunks[seg];
+  const int nc = sc.y;
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tmem_S = tmem, tmem_VN = tmem + 128, tmem_O = tmem + 192;
+  const uint32_t tmem_S = tmem, tmem_VN = tmem + 128, tmem_O = tmem + 192;  // o of chunk i at tmem_O + (i & 1) * 64
 
   if (warp == 0) {
     if (elect_one()) {
       for (int i = 0; i < nc; ++i) {
+        // Three groups of operands with barriers of their own, so that each is asked for again as soon as it has been
+        // used, up to two chunks before its next use: one chunk's time does not cover the way from memory.
         const int s = i & 1;
-        if (!mbar_wait(&empty[s], ((i >> 1) & 1) ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) break;
+        const uint32_t ph = ((i >> 1) & 1) ^ 1;
         uint8_t* st = stages + s * SC_STAGE;
         const int ch = (sc.x + i) * p.HV + h;
-        mbar_expect_tx(&full[s], SC_STAGE);
-        for (int part = 0; part < 4; ++part)
-          for (int a = 0; a < 2; ++a)
-            tma_load_2d(st + part * 16384 + a * 8192, &tmA, &full[s], a * 64, ch * 256 + part * 64);
-        tma_load_2d(st + 65536, &tmB, &full[s], 0, ch * 64);
+        auto load = [&](int part, uint64_t* bar) {
+          for (int a = 0; a < 2; ++a) tma_load_2d(st + part * 16384 + a * 8192, &tmA, bar, a * 64, ch * 256 + part * 64);
+        };
+        if (!mbar_wait(&empty[s], ph, p.err, ERR_WAIT_EMPTY, abort_flag)) break;
+        mbar_expect_tx(&full[s], 32768);
+        load(0, &full[s]);
+        load(2, &full[s]);
+        if (!mbar_wait(&empty[2 + s], ph, p.err, ERR_WAIT_EMPTY, abort_flag)) break;
+        mbar_expect_tx(&full[2 + s], 16384);
+        load(1, &full[2 + s]);
+        if (!mbar_wait(&empty[4 + s], ph, p.err, ERR_WAIT_EMPTY, abort_flag)) break;
+        mbar_expect_tx(&full[4 + s], 16384 + 8192);
+        load(3, &full[4 + s]);
+        tma_load_2d(st + 65536, &tmB, &full[4 + s], 0, ch * 64);
       }
     }
   } else if (warp == 1) {
@@ -482,7 +508,7 @@ gdn_scan_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       const uint32_t sa = smem_u32(sS), vna = smem_u32(sVN);
       for (int i = 0; i < nc; ++i) {
         const int s = i & 1;
-        const uint32_t st = smem_u32(stages + s * SC_STAGE);
+        const uint32_t st = smem_u32(stages + s * SC_STAGE), o = tmem_O + (i & 1) * 64;
         if (!mbar_wait(&full[s], (i >> 1) & 1, p.err, ERR_WAIT_FULL, abort_flag)) break;
         if (!mbar_wait(s_ready, i & 1, p.err, ERR_WAIT_FULL, abort_flag)) break;
         tc_fence_after();
@@ -491,127 +517,157 @@ gdn_scan_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           const uint32_t aoff = (kk >> 2) * 16384 + (kk & 3) * 32, boff = (kk >> 2) * 8192 + (kk & 3) * 32;
           umma_bf16(tmem_VN, umma_smem_desc(sa + aoff), umma_smem_desc(st + boff), idesc64, kk != 0);
         }
+        umma_commit(vn_done);
+        if (!mbar_wait(&o_free[s], ((i >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag)) break;
+        tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {  // o^T = S^T (q e^g)^T
           const uint32_t aoff = (kk >> 2) * 16384 + (kk & 3) * 32, boff = (kk >> 2) * 8192 + (kk & 3) * 32;
-          umma_bf16(tmem_O, umma_smem_desc(sa + aoff), umma_smem_desc(st + 32768 + boff), idesc64, kk != 0);
+          umma_bf16(o, umma_smem_desc(sa + aoff), umma_smem_desc(st + 32768 + boff), idesc64, kk != 0);
         }
-        umma_commit(vn_done);
+        umma_commit(&empty[s]);
+        if (!mbar_wait(&full[4 + s], (i >> 1) & 1, p.err, ERR_WAIT_FULL, abort_flag)) break;
         if (!mbar_wait(vn_ready, i & 1, p.err, ERR_WAIT_FULL, abort_flag)) break;
         tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)    // o^T += v_new^T scores^T, contraction over the chunk's tokens
-          umma_bf16(tmem_O, umma_smem_desc(vna + kk * 32), umma_smem_desc(st + 65536 + kk * 32), idesc64, 1);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)    // S^T += v_new^T (k e^{g_last - g})
+        for (int kk = 0; kk < 4; ++kk)    // S^T += v_new^T (k e^{g_last - g}), contraction over the chunk's tokens
           umma_bf16(tmem_S, umma_smem_desc(vna + kk * 32), umma_smem_desc_mn(st + 49152 + kk * 2048, 8192), idesc_kg, 1);
-        umma_commit(&empty[s]);
-        umma_commit(o_done);
+        umma_commit(s_done);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)    // o^T += v_new^T scores^T
+          umma_bf16(o, umma_smem_desc(vna + kk * 32), umma_smem_desc(st + 65536 + kk * 32), idesc64, 1);
+        umma_commit(&empty[4 + s]);
+        umma_commit(&o_done[s]);
       }
     }
+  } else if (warp >= 10) {
+    // ---------------- output: thread dv reads TMEM lane dv; then 16 lanes share a token's 128 values, 16 bytes each
+    const int q = warp & 3, dv = q * 32 + lane;
+    const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
+    const int col = (lane & 15) * 8, t_own = (warp - 10) * 2 + (lane >> 4);  // tokens t_own + 8 j
+    bf16* so = reinterpret_cast<bf16*>(sO);
+    bool ok = true;
+    for (int i = 0; i < nc; ++i) {
+      const ChunkInfoTc ci = p.chunks[sc.x + i];
+      ok = mbar_wait(&o_done[i & 1], (i >> 1) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && ok;
+      tc_fence_after();
+#pragma unroll
+      for (int t0 = 0; t0 < 64; t0 += 16) {
+        float v[16];
+        tmem_ld16(tmem_O + (i & 1) * 64 + lane_base + t0, v);  // warp-collective: never predicated
+#pragma unroll
+        for (int j = 0; j < 16; ++j) so[(t0 + j) * 128 + dv] = __float2bfloat16(v[j]);
+      }
+      tc_fence_before();
+      mbar_arrive(&o_free[i & 1]);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int t = t_own + 8 * j;
+        const uint4 o = *reinterpret_cast<const uint4*>(so + t * 128 + col);
+        if (ok && t < ci.nrows)
+          *reinterpret_cast<uint4*>(p.o_out + (static_cast<size_t>(ci.row0 + t) * p.HV + h) * 128 + col) = o;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // the tile has been read
+    }
   } else {
-    // ---------------- thread dv owns TMEM lane dv: one row of S^T, v_new^T and o^T
-    const int q = warp & 3;
+    // ---------------- thread (dv, hf) works on TMEM lane dv, one row of S^T and v_new^T, and on half hf of the columns
+    const int q = warp & 3, hf = warp >= 6 ? 1 : 0;
     const int dv = q * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
     float* Sg = p.rec_state + (static_cast<size_t>(p.slots[seg]) * p.HV + h) * 128 * 128;
-    // initial state: S[k][dv] -> TMEM row dv and the bf16 copy
-#pragma unroll 1
-    for (int k0 = 0; k0 < 128; k0 += 16) {
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = Sg[static_cast<size_t>(k0 + j) * 128 + dv];
-      tmem_st16(tmem_S + lane_base + k0, v);
+    const float* glast = p.glast + static_cast<size_t>(sc.x) * p.HV + h;
+    uint8_t* s_copy = sS + hf * 16384;
+    const uint32_t s_row = tmem_S + lane_base + hf * 64;
+    // 16 state columns: the bf16 operand copy, and the state scaled by the next chunk's decay back into TMEM
+    auto keep = [&](int k0, float* v, float scale) {
       uint4 o[2];
       bf16* oe = reinterpret_cast<bf16*>(o);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) oe[j] = __float2bfloat16(v[j]);
-      uint8_t* atom = sS + (k0 >> 6) * 16384;
-      *reinterpret_cast<uint4*>(atom + swz(dv, (k0 & 63) >> 3)) = o[0];
-      *reinterpret_cast<uint4*>(atom + swz(dv, ((k0 & 63) >> 3) + 1)) = o[1];
+      for (int j = 0; j < 16; ++j) { oe[j] = __float2bfloat16(v[j]); v[j] *= scale; }
+      tmem_st16(s_row + k0, v);
+      *reinterpret_cast<uint4*>(s_copy + swz(dv, k0 >> 3)) = o[0];
+      *reinterpret_cast<uint4*>(s_copy + swz(dv, (k0 >> 3) + 1)) = o[1];
+    };
+    float g_next = nc > 0 ? glast[0] : 0.f;
+    {
+      const float eg = __expf(g_next);
+#pragma unroll
+      for (int k0 = 0; k0 < 64; k0 += 16) {  // initial state: S[k][dv] -> TMEM row dv and the bf16 copy
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = Sg[static_cast<size_t>(hf * 64 + k0 + j) * 128 + dv];
+        keep(k0, v, eg);
+      }
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     mbar_arrive(s_ready);
     bool ok = true;
-    for (int i = 0; i < nc && ok; ++i) {
+    bf16 u[32];
+    auto read_u = [&](int i) {  // chunk i's u rows: 32 tokens of this thread's dv
       const int s = i & 1;
-      const uint8_t* st = stages + s * SC_STAGE;
-      const int cidx = sc.x + i;
-      const ChunkInfoTc ci = p.chunks[cidx];
-      const float eg = __expf(p.glast[static_cast<size_t>(cidx) * p.HV + h]);
+      if (!mbar_wait(&full[2 + s], (i >> 1) & 1, p.err, ERR_WAIT_FULL, abort_flag)) return false;
+      const uint8_t* su = stages + s * SC_STAGE + 16384 + (dv >> 6) * 8192 + (dv & 7) * 2;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) u[j] = *reinterpret_cast<const bf16*>(su + swz(hf * 32 + j, (dv & 63) >> 3));
+      mbar_arrive(&empty[2 + s]);
+      return true;
+    };
+    if (nc > 0) ok = read_u(0);
+    for (int i = 0; i < nc && ok; ++i) {
+      const bool last = i + 1 == nc;
+      g_next = last ? 0.f : glast[static_cast<size_t>(i + 1) * p.HV];
       ok = mbar_wait(vn_done, i & 1, p.err, ERR_WAIT_TMEM, abort_flag);
       if (!ok) break;
       tc_fence_after();
       // v_new^T[dv][t] = u[t][dv] - (S^T w^T)[dv][t], as bf16 into the K-major operand tile (row dv, 64 tokens)
-      const uint8_t* su = st + 16384 + (dv >> 6) * 8192;
-      const uint32_t ucol = ((dv & 63) >> 3), ubyte = (dv & 7) * 2;
 #pragma unroll
-      for (int t0 = 0; t0 < 64; t0 += 16) {
+      for (int t0 = 0; t0 < 32; t0 += 16) {
         float v[16];
-        tmem_ld16(tmem_VN + lane_base + t0, v);
+        tmem_ld16(tmem_VN + lane_base + hf * 32 + t0, v);
         uint4 o[2];
         bf16* oe = reinterpret_cast<bf16*>(o);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float u = __bfloat162float(*reinterpret_cast<const bf16*>(su + swz(t0 + j, ucol) + ubyte));
-          oe[j] = __float2bfloat16(u - v[j]);
-        }
-        *reinterpret_cast<uint4*>(sVN + swz(dv, t0 >> 3)) = o[0];
-        *reinterpret_cast<uint4*>(sVN + swz(dv, (t0 >> 3) + 1)) = o[1];
+        for (int j = 0; j < 16; ++j) oe[j] = __float2bfloat16(__bfloat162float(u[t0 + j]) - v[j]);
+        const uint32_t c16 = (hf * 32 + t0) >> 3;
+        *reinterpret_cast<uint4*>(sVN + swz(dv, c16)) = o[0];
+        *reinterpret_cast<uint4*>(sVN + swz(dv, c16 + 1)) = o[1];
       }
-      // S^T *= e^{g_last} before the MMA adds this chunk's update
-#pragma unroll 1
-      for (int k0 = 0; k0 < 128; k0 += 16) {
-        float v[16];
-        tmem_ld16(tmem_S + lane_base + k0, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] *= eg;
-        tmem_st16(tmem_S + lane_base + k0, v);
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc_fence_before();
       mbar_arrive(vn_ready);
-      ok = mbar_wait(o_done, i & 1, p.err, ERR_WAIT_TMEM, abort_flag);
+      const float eg = __expf(g_next);
+      if (!last) ok = read_u(i + 1);
+      ok = ok && mbar_wait(s_done, i & 1, p.err, ERR_WAIT_TMEM, abort_flag);
       if (!ok) break;
       tc_fence_after();
+      if (last) {
 #pragma unroll
-      for (int t0 = 0; t0 < 64; t0 += 16) {
-        float v[16];
-        tmem_ld16(tmem_O + lane_base + t0, v);  // warp-collective: never predicated
+        for (int k0 = 0; k0 < 64; k0 += 16) {
+          float v[16];
+          tmem_ld16(s_row + k0, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (t0 + j < ci.nrows)
-            p.o_out[(static_cast<size_t>(ci.row0 + t0 + j) * p.HV + h) * 128 + dv] = __float2bfloat16(v[j]);
-      }
-      const bool last = i + 1 == nc;
-#pragma unroll 1
-      for (int k0 = 0; k0 < 128; k0 += 16) {
-        float v[16];
-        tmem_ld16(tmem_S + lane_base + k0, v);
-        if (last) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) Sg[static_cast<size_t>(k0 + j) * 128 + dv] = v[j];
-        } else {
-          uint4 o[2];
-          bf16* oe = reinterpret_cast<bf16*>(o);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) oe[j] = __float2bfloat16(v[j]);
-          uint8_t* atom = sS + (k0 >> 6) * 16384;
-          *reinterpret_cast<uint4*>(atom + swz(dv, (k0 & 63) >> 3)) = o[0];
-          *reinterpret_cast<uint4*>(atom + swz(dv, ((k0 & 63) >> 3) + 1)) = o[1];
+          for (int j = 0; j < 16; ++j) Sg[static_cast<size_t>(hf * 64 + k0 + j) * 128 + dv] = v[j];
         }
+      } else {
+#pragma unroll
+        for (int k0 = 0; k0 < 64; k0 += 16) {
+          float v[16];
+          tmem_ld16(s_row + k0, v);
+          keep(k0, v, eg);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tc_fence_before();
+        mbar_arrive(s_ready);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tc_fence_before();
-      mbar_arrive(s_ready);
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 256); }
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
 }  // namespace b200
@@ -680,6 +736,6 @@ extern "C" int b200_gdn_prefill_tc(const void* mixed, int ld, const void* conv_o
   ScanParams sp{static_cast<const ChunkInfoTc*>(chunks), static_cast<const int2*>(seg_chunks), slots, rec_state,
                 reinterpret_cast<const float*>(static_cast<uint8_t*>(work) + tc_region_g(nch)),
                 static_cast<bf16*>(o_tmp), HV, err};
-  gdn_scan_tc_kernel<<<dim3(n_seg, HV), 192, SC_SMEM, st>>>(ta, tb, sp);
+  gdn_scan_tc_kernel<<<dim3(n_seg, HV), 448, SC_SMEM, st>>>(ta, tb, sp);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
