@@ -56,16 +56,19 @@ constexpr int WY_SMEM = 3 * 32768 + 1024 /*align*/ + 5120 /*small arrays + barri
 __device__ long long g_wy_clocks[12];
 #define WY_STAMP(k) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) g_wy_clocks[k] = clock64(); } while (0)
 
+// Bound by shared memory: the substitution's reads of A (16 bytes for two lanes' four products each) and two CTAs per SM.
+// 230 -> 198 us at 8192 rows x 32 heads, 64 -> 54 at 2048, since the columns of T live in registers (the v rows then load at
+// the start and not behind the substitution) and w and u leave by TMA.
 // 256 threads. Row phases: thread (i = tid & 127, half = tid >> 7) works on token row i = TMEM lane i and on one
 // 64-column half of it. Substitution phase: thread (col = tid >> 1, part = tid & 1) owns column col of T together with
 // its neighbour lane; the pair splits every dot product and meets in one shuffle.
 __global__ void __launch_bounds__(256, 2)
-gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
+gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, const __grid_constant__ CUtensorMap tmA, WyParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;            // raw q, later the fp32 A blocks, later the bf16 block-diagonal T diag(beta)
-  uint8_t* sK = smem + 32768;    // raw k, later k e^g / |k|
-  uint8_t* sV = smem + 65536;    // the substitution's columns (fp32), later raw v
+  uint8_t* sQ = smem;            // raw q, later the fp32 A blocks, the bf16 block-diagonal T diag(beta), at last w
+  uint8_t* sK = smem + 32768;    // raw k, later k e^g / |k|, at last u
+  uint8_t* sV = smem + 65536;    // raw v
   float* sG = reinterpret_cast<float*>(smem + 98304);  // [128] cumulative log decay
   float* sRk = sG + 128;                               // [128] 1 / |k|
   float* sBeta = sRk + 128;                            // [128]
@@ -76,7 +79,8 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(sTot + 8);
   uint64_t* tma_bar = bars;
   uint64_t* mma_bar = bars + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+  uint64_t* v_bar = bars + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -86,15 +90,15 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   const int key_dim = p.HK * 128;
   const int chunk_idx = 2 * blockIdx.x + c;
   const bool present = chunk_idx < p.n_chunks;
-  const ChunkInfoTc ci = p.chunks[present ? chunk_idx : 2 * blockIdx.x];
-  const bool valid = present && r < ci.nrows;
 
   if (tid == 0) {
     mbar_init(tma_bar, 1);
     mbar_init(mma_bar, 1);
+    mbar_init(v_bar, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmConv);
+    tma_prefetch_desc(&tmA);
   }
   if (warp == 0) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
@@ -102,11 +106,15 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  pdl_wait();
+  pdl_launch();
+  const ChunkInfoTc ci = p.chunks[present ? chunk_idx : 2 * blockIdx.x];
+  const bool valid = present && r < ci.nrows;
 
   if (tid == 0) {
-    // q and k rows of both chunks (a missing second chunk re-reads the first: finite data, never written out);
-    // v arrives later: its region is scratch for the substitution first
+    // q and k rows of both chunks (a missing second chunk re-reads the first: finite data, never written out), then v
     mbar_expect_tx(tma_bar, 2 * 32768);
+    mbar_expect_tx(v_bar, 32768);
     for (int cc = 0; cc < 2; ++cc) {
       const int idx = 2 * blockIdx.x + cc;
       const int row0 = p.chunks[idx < p.n_chunks ? idx : 2 * blockIdx.x].row0;
@@ -114,6 +122,8 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
         tma_load_2d(sQ + a * 16384 + cc * 8192, &tmConv, tma_bar, hk * 128 + a * 64, row0);
         tma_load_2d(sK + a * 16384 + cc * 8192, &tmConv, tma_bar, key_dim + hk * 128 + a * 64, row0);
       }
+      for (int a = 0; a < 2; ++a)
+        tma_load_2d(sV + a * 16384 + cc * 8192, &tmConv, v_bar, 2 * key_dim + h * 128 + a * 64, row0);
     }
   }
   WY_STAMP(0);
@@ -186,7 +196,6 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
     sFk[i] = rk * __expf(glast - gs);
   }
   const size_t ch = static_cast<size_t>(present ? chunk_idx : 0) * p.HV + h;
-  bf16* regA = reinterpret_cast<bf16*>(p.work) + ch * 256 * 128;
   if (present && r == 63 && half == 0)
     *reinterpret_cast<float*>(p.work + tc_region_g(static_cast<size_t>(p.n_chunks) * p.HV) + ch * 4) = glast;
   __syncthreads();
@@ -267,42 +276,37 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   }
   __syncthreads();
   WY_STAMP(5);  // A built, k scaled
-  // T = (I + A)^-1 by forward substitution. Lanes (2m, 2m + 1) of a warp own column col = tid >> 1 of T: entry j of
-  // the column lives at sC[(j >> 2) * 512 + col * 4 + (j & 3)] (the v region, free until v is loaded); the pair
-  // splits the groups of four entries of every dot product by parity and adds the halves with one shuffle. A column
-  // is private to its pair and the reads of A are the same addresses across the warp, so only __syncwarp is needed.
+  // T = (I + A)^-1 by forward substitution. Lanes (2m, 2m + 1) of a warp own column col = tid >> 1 of T, each the groups of
+  // four entries of its own parity, in registers; the pair splits every dot product that way and adds the halves with
+  // one shuffle. The reads of A are the same two addresses across the warp.
   {
     const int col = tid >> 1, part = tid & 1;
     const int cc = col >> 6, rr = col & 63;
     const float* sAc = reinterpret_cast<const float*>(sQ + cc * 16384);
-    float* sC = reinterpret_cast<float*>(sV);
-    // Blocked by 16 rows so that a column entry is read from shared memory once per BLOCK, not once per row: for
-    // block b, first the panel acc[i] = sum over earlier blocks' entries j of A[16 b + i][j] T[j] (the pair splits
-    // the groups of four j by parity and meets in 16 shuffles), then the 16 x 16 triangle with the block's own
-    // entries in registers, then one store of the block's 16 entries. Blocks that lie entirely above every diagonal
-    // of the warp's columns are zero and skipped.
+    // Blocked by 16 rows: for block b, first the panel acc[i] = sum over earlier blocks' entries j of A[16 b + i][j] T[j],
+    // then the 16 x 16 triangle with the block's own entries. Blocks that lie entirely above every diagonal of the warp's
+    // columns are zero and skipped, as are zero groups.
     const int lo = (warp & 3) * 16;  // smallest column of this warp inside its chunk
-#pragma unroll 1
-    for (int blk = 0; blk < 4; ++blk) {
-      float t[16];
-      if (16 * blk + 15 < lo) {  // warp-uniform
-        if (part == 0) {
+    float tc[8][4];                  // entries 4 (2 gi + part) + x of the column
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<float4*>(sC + (4 * blk + q4) * 512 + col * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    for (int blk = 0; blk < 4; ++blk) {
+      if (16 * blk + 15 < lo) {  // warp-uniform
+#pragma unroll
+        for (int x = 0; x < 4; ++x) tc[2 * blk][x] = tc[2 * blk + 1][x] = 0.f;
         continue;
       }
-      float acc[16];
+      float t[16], acc[16];
 #pragma unroll
       for (int ii = 0; ii < 16; ++ii) acc[ii] = 0.f;
-#pragma unroll 1
-      for (int j4 = (lo >> 2) + part; j4 < 4 * blk; j4 += 2) {
-        const float4 c4 = *reinterpret_cast<const float4*>(sC + j4 * 512 + col * 4);
+#pragma unroll
+      for (int gi = 0; gi < 2 * blk; ++gi) {
+        if (8 * gi + 7 < lo) continue;  // warp-uniform
+        const int j4 = 2 * gi + part;
 #pragma unroll
         for (int ii = 0; ii < 16; ++ii) {
           const int row = 16 * blk + ii;
           const float4 a4 = *reinterpret_cast<const float4*>(sAc + row * 64 + (((j4 + row) & 15) << 2));
-          acc[ii] += (a4.x * c4.x + a4.y * c4.y) + (a4.z * c4.z + a4.w * c4.w);
+          acc[ii] += (a4.x * tc[gi][0] + a4.y * tc[gi][1]) + (a4.z * tc[gi][2] + a4.w * tc[gi][3]);
         }
       }
 #pragma unroll
@@ -324,23 +328,24 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
         }
         t[ii] = row > rr ? -a : (row == rr ? 1.f : 0.f);
       }
-      if (part == 0) {
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4)
-          *reinterpret_cast<float4*>(sC + (4 * blk + q4) * 512 + col * 4) = make_float4(t[4 * q4], t[4 * q4 + 1], t[4 * q4 + 2], t[4 * q4 + 3]);
+      for (int x = 0; x < 4; ++x) {
+        tc[2 * blk][x] = part ? t[4 + x] : t[x];
+        tc[2 * blk + 1][x] = part ? t[12 + x] : t[8 + x];
       }
-      __syncwarp();
     }
     WY_STAMP(6);  // substitution done (this warp)
     __syncthreads();  // every thread has finished reading A: the region becomes the bf16 operand tile
-    // T diag(beta), block-diagonal, as a K-major A operand: row (cc * 64 + ii), K index (cc * 64 + rr) -> atom cc;
-    // the pair writes alternate rows
+    // T diag(beta), block-diagonal, as a K-major A operand: row (cc * 64 + ii), K index (cc * 64 + rr) -> atom cc
     uint8_t* tile = sQ + cc * 16384;
     const float bcol = sBeta[col];
-#pragma unroll 8
-    for (int ii = part; ii < 64; ii += 2)
-      *reinterpret_cast<bf16*>(tile + swz(cc * 64 + ii, rr >> 3) + (rr & 7) * 2) =
-          __float2bfloat16(sC[(ii >> 2) * 512 + col * 4 + (ii & 3)] * bcol);
+#pragma unroll
+    for (int gi = 0; gi < 8; ++gi)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int ii = 4 * (2 * gi + part) + x;
+        *reinterpret_cast<bf16*>(tile + swz(cc * 64 + ii, rr >> 3) + (rr & 7) * 2) = __float2bfloat16(tc[gi][x] * bcol);
+      }
   }
   {  // the other atom's rows of this chunk are zero: w = (T diag(beta)) (k e^g), u = (T diag(beta)) v
     uint8_t* other = sQ + (1 - c) * 16384;
@@ -353,14 +358,6 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   __syncthreads();
   if (tid == 0 && ok) {
     tc_fence_after();
-    // the v rows of both chunks replace the scratch columns while the first MMA runs
-    mbar_expect_tx(tma_bar, 32768);
-    for (int cc = 0; cc < 2; ++cc) {
-      const int idx = 2 * blockIdx.x + cc;
-      const int row0 = p.chunks[idx < p.n_chunks ? idx : 2 * blockIdx.x].row0;
-      for (int a = 0; a < 2; ++a)
-        tma_load_2d(sV + a * 16384 + cc * 8192, &tmConv, tma_bar, 2 * key_dim + h * 128 + a * 64, row0);
-    }
     constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | (1u << 16);  // B operand MN-major: [token][feature]
     const uint32_t ta = smem_u32(sQ), ka = smem_u32(sK), va = smem_u32(sV);
 #pragma unroll
@@ -368,7 +365,7 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
       const uint32_t aoff = (kk >> 2) * 16384 + (kk & 3) * 32;
       umma_bf16(tmem, umma_smem_desc(ta + aoff), umma_smem_desc_mn(ka + kk * 2048, 16384), idesc, kk != 0);        // w
     }
-    if (!mbar_wait(tma_bar, 1, p.err, ERR_WAIT_FULL, abort_flag)) ok = false;
+    if (!mbar_wait(v_bar, 0, p.err, ERR_WAIT_FULL, abort_flag)) ok = false;
     tc_fence_after();
     if (ok) {
 #pragma unroll
@@ -383,9 +380,12 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
   ok = mbar_wait(mma_bar, 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
   tc_fence_after();
   WY_STAMP(9);  // w / u in TMEM
+  // w and u as bf16 into the tiles that the MMAs have read, and from there by TMA to rows [0, 64) and [64, 128) of the
+  // chunk's A-region (a workspace of whole chunks: there are no ragged edges). Stored by the threads, each its own row, the
+  // 16-byte pieces of 32 rows made 32 lines of every instruction.
 #pragma unroll 1
-  for (int which = 0; which < 2; ++which) {  // 0: w -> rows [0, 64), 1: u -> rows [64, 128) of the chunk's A-region
-    uint4* dst = reinterpret_cast<uint4*>(regA + (which * 64 + r) * 128) + half * 8;
+  for (int which = 0; which < 2; ++which) {
+    uint8_t* dst = (which ? sK : sQ) + half * 16384;
 #pragma unroll
     for (int c0 = 0; c0 < 64; c0 += 16) {
       float v[16];
@@ -394,8 +394,22 @@ gdn_wy_tc_kernel(const __grid_constant__ CUtensorMap tmConv, WyParams p) {
       bf16* oe = reinterpret_cast<bf16*>(o);
 #pragma unroll
       for (int j = 0; j < 16; ++j) oe[j] = __float2bfloat16(v[j]);
-      if (present && ok) { dst[c0 / 8] = o[0]; dst[c0 / 8 + 1] = o[1]; }
+      *reinterpret_cast<uint4*>(dst + swz(tile_row, c0 >> 3)) = o[0];
+      *reinterpret_cast<uint4*>(dst + swz(tile_row, (c0 >> 3) + 1)) = o[1];
     }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  if (tid == 0) {
+    for (int cc = 0; cc < 2 && ok; ++cc) {
+      const int idx = 2 * blockIdx.x + cc;
+      if (idx >= p.n_chunks) break;
+      for (int which = 0; which < 2; ++which)
+        for (int a = 0; a < 2; ++a)
+          tma_store_2d(&tmA, (which ? sK : sQ) + a * 16384 + cc * 8192, a * 64, (idx * p.HV + h) * 256 + which * 64);
+    }
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   WY_STAMP(10);  // w / u written
   tc_fence_before();
@@ -471,6 +485,8 @@ gdn_scan_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_launch();
   const int2 sc = p.seg_chunks[seg];
   const int nc = sc.y;
   const uint32_t tmem = *tmem_slot;
@@ -732,10 +748,9 @@ extern "C" int b200_gdn_prefill_tc(const void* mixed, int ld, const void* conv_o
   if (tc_map_2d(&tb, static_cast<uint8_t*>(work) + tc_region_b(nch), 64, nch * 64, 64)) return -1;
   WyParams wp{static_cast<const bf16*>(mixed), ld, C + value_dim, C + value_dim + HV,
               static_cast<const ChunkInfoTc*>(chunks), n_chunks, A_log, dt_bias, static_cast<uint8_t*>(work), HK, HV, err};
-  gdn_wy_tc_kernel<<<dim3((n_chunks + 1) / 2, HV), 256, WY_SMEM, st>>>(tc, wp);
+  if (launch_pdl(gdn_wy_tc_kernel, dim3((n_chunks + 1) / 2, HV), dim3(256), WY_SMEM, st, tc, ta, wp) != cudaSuccess) return -4;
   ScanParams sp{static_cast<const ChunkInfoTc*>(chunks), static_cast<const int2*>(seg_chunks), slots, rec_state,
                 reinterpret_cast<const float*>(static_cast<uint8_t*>(work) + tc_region_g(nch)),
                 static_cast<bf16*>(o_tmp), HV, err};
-  gdn_scan_tc_kernel<<<dim3(n_seg, HV), 448, SC_SMEM, st>>>(ta, tb, sp);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  return launch_pdl(gdn_scan_tc_kernel, dim3(n_seg, HV), dim3(448), SC_SMEM, st, ta, tb, sp) == cudaSuccess ? 0 : -4;
 }
