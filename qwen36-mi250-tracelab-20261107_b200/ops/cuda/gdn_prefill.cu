@@ -42,6 +42,8 @@ gdn_conv_prefill_kernel(const bf16* x, int ld, const int* seq_of_row, const int*
                         const bf16* conv_state, const bf16* conv_w, bf16* out, int T, int C) {
   constexpr int BATCH = 4;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  pdl_wait();
+  pdl_launch();
   if (c >= C) return;
   float w[8][4];
   {
@@ -112,6 +114,8 @@ __global__ void gdn_conv_state_update_kernel(const bf16* x, int ld, const int* s
                                              bf16* conv_state, int C) {
   const int seg = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_launch();
   if (c >= C) return;
   const int s0 = seg_start[seg], s1 = seg_start[seg + 1], n = s1 - s0;
   bf16* st = conv_state + (static_cast<size_t>(slots[seg]) * C + c) * 3;
@@ -399,6 +403,8 @@ gdn_gated_norm_kernel(const bf16* o, const bf16* mixed, int ld, int z_off, const
   static_assert(DV == 32 || DV == 64 || DV == 128, "head dim 32, 64 or 128");
   const int lane = threadIdx.x % LANES;
   const int n = rows * HV;
+  pdl_wait();
+  pdl_launch();
   const uint4 wv = *reinterpret_cast<const uint4*>(w + lane * 8);
   const bf16* we = reinterpret_cast<const bf16*>(&wv);
   uint4 ov[NORM_UNITS], zv[NORM_UNITS];
@@ -432,10 +438,11 @@ gdn_gated_norm_kernel(const bf16* o, const bf16* mixed, int ld, int z_off, const
 }
 
 template <int DV>
-static void launch_gated_norm(const bf16* o, const bf16* mixed, int ld, int z_off, const bf16* w, bf16* out, int rows,
+static cudaError_t launch_gated_norm(const bf16* o, const bf16* mixed, int ld, int z_off, const bf16* w, bf16* out, int rows,
                               int HV, float eps, cudaStream_t st) {
   const int per = 256 / (DV / 8) * NORM_UNITS;
-  gdn_gated_norm_kernel<DV><<<(rows * HV + per - 1) / per, 256, 0, st>>>(o, mixed, ld, z_off, w, out, rows, HV, eps);
+  return launch_pdl(gdn_gated_norm_kernel<DV>, dim3((rows * HV + per - 1) / per), dim3(256), 0, st, o, mixed, ld, z_off, w, out,
+                    rows, HV, eps);
 }
 
 }  // namespace b200
@@ -462,7 +469,7 @@ int gdn_prefill_launch(const bf16* mixed, int ld, const bf16* conv_out, const Ch
   }
   wy<<<dim3(n_chunks, HV), 256, wy_smem, st>>>(conv_out, mixed, ld, b_off, a_off, chunks, A_log, dt_bias, work, HK, HV);
   scan<<<dim3(n_seg, HV, DKV / 32), 256, scan_smem, st>>>(work, chunks, seg_chunks, slots, rec_state, o_tmp, HV);
-  launch_gated_norm<DKV>(o_tmp, mixed, ld, z_off, gnorm_w, out, T, HV, eps, st);
+  if (launch_gated_norm<DKV>(o_tmp, mixed, ld, z_off, gnorm_w, out, T, HV, eps, st) != cudaSuccess) return -4;
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 }  // namespace
@@ -491,14 +498,14 @@ extern "C" int b200_gdn_prefill(const void* mixed, int ld, const int* seq_of_row
   if (C % 8 || ld % 8) return -7;
   // Runs of 16 rows read three rows in sixteen twice; below 4096 rows runs of 8 put twice as many threads to work.
   const auto conv = [&](auto kern, int run) {
-    kern<<<dim3((C / 8 + 127) / 128, (T + run - 1) / run), 128, 0, st>>>(
-        static_cast<const bf16*>(mixed), ld, seq_of_row, seg_start, slots, static_cast<const bf16*>(conv_state),
-        static_cast<const bf16*>(conv_w), static_cast<bf16*>(conv_out), T, C);
+    return launch_pdl(kern, dim3((C / 8 + 127) / 128, (T + run - 1) / run), dim3(128), 0, st, static_cast<const bf16*>(mixed),
+                      ld, seq_of_row, seg_start, slots, static_cast<const bf16*>(conv_state),
+                      static_cast<const bf16*>(conv_w), static_cast<bf16*>(conv_out), T, C);
   };
-  if (T >= 4096) conv(gdn_conv_prefill_kernel<16>, 16);
-  else conv(gdn_conv_prefill_kernel<8>, 8);
-  gdn_conv_state_update_kernel<<<dim3((C + 127) / 128, n_seg), 128, 0, st>>>(
-      static_cast<const bf16*>(mixed), ld, seg_start, slots, static_cast<bf16*>(conv_state), C);
+  if ((T >= 4096 ? conv(gdn_conv_prefill_kernel<16>, 16) : conv(gdn_conv_prefill_kernel<8>, 8)) != cudaSuccess) return -4;
+  if (launch_pdl(gdn_conv_state_update_kernel, dim3((C + 127) / 128, n_seg), dim3(128), 0, st, static_cast<const bf16*>(mixed),
+                 ld, seg_start, slots, static_cast<bf16*>(conv_state), C) != cudaSuccess)
+    return -4;
 #define GP(DKV)                                                                                                      \
   return gdn_prefill_launch<DKV>(static_cast<const bf16*>(mixed), ld, static_cast<const bf16*>(conv_out),            \
                                  static_cast<const ChunkInfo*>(chunks), n_chunks, static_cast<const int2*>(seg_chunks), \
@@ -509,8 +516,9 @@ extern "C" int b200_gdn_prefill(const void* mixed, int ld, const int* seq_of_row
     const int rc = b200_gdn_prefill_tc(mixed, ld, conv_out, chunks, n_chunks, seg_chunks, n_seg, slots, rec_state, A_log,
                                        dt_bias, work, o_tmp, T, HK, HV, err, st);
     if (rc) return rc;
-    launch_gated_norm<128>(static_cast<const bf16*>(o_tmp), static_cast<const bf16*>(mixed), ld, C,
-                           static_cast<const bf16*>(gnorm_w), static_cast<bf16*>(out), T, HV, eps, st);
+    if (launch_gated_norm<128>(static_cast<const bf16*>(o_tmp), static_cast<const bf16*>(mixed), ld, C,
+                               static_cast<const bf16*>(gnorm_w), static_cast<bf16*>(out), T, HV, eps, st) != cudaSuccess)
+      return -4;
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }
   if (DK == 128) GP(128);
