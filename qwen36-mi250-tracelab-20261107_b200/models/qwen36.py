@@ -18,8 +18,10 @@ captured in a CUDA graph and replayed on refreshed input buffers.
 
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from ..config import PAGE_SIZE, ModelConfig
@@ -44,18 +46,40 @@ class PackedBatch:
 
     @classmethod
     def prefill(cls, token_lists, slots, pos0, block_tables, device) -> "PackedBatch":
-        lens = [len(t) for t in token_lists]
+        """The index tensors of a ragged pass. On a CUDA device they are views of ONE buffer that one asynchronous copy from
+        pinned memory fills: a copy per tensor from pageable memory, five of them, each waited for everything launched
+        before, so that the GPU stood still while the host built the next pass (a 61-row pass of 4 layers: 1.56 -> 1.42 ms).
+        The copy is ordered on the stream that is current here, which is the one to run the pass on."""
+        dev = torch.device(device)
         starts = [0]
-        for n in lens:
-            starts.append(starts[-1] + n)
-        tokens = torch.tensor([t for ts in token_lists for t in ts], dtype=torch.int64)
-        positions = torch.cat([torch.arange(p, p + n, dtype=torch.int64) for p, n in zip(pos0, lens)])
-        seq = torch.repeat_interleave(torch.arange(len(lens), dtype=torch.int32), torch.tensor(lens))
-        return cls(
-            tokens.to(device), positions.to(device), seq.to(device),
-            torch.tensor(slots, dtype=torch.int32, device=device), block_tables.to(device), 0,
-            starts, list(slots), list(pos0),
-        )
+        for t in token_lists:
+            starts.append(starts[-1] + len(t))
+        T, n = starts[-1], len(token_lists)
+        # a page table in host memory travels with the rest
+        with_table = block_tables.device.type == "cpu" and block_tables.dtype == torch.int32
+        sizes = (T * 8, T * 8, T * 4, len(slots) * 4, block_tables.numel() * 4 if with_table else 0)
+        offs = [0]
+        for nbytes in sizes:
+            offs.append(offs[-1] + (nbytes + 15) // 16 * 16)
+        host = torch.empty(offs[-1], dtype=torch.uint8, pin_memory=dev.type == "cuda")
+
+        def views(buf):
+            v = [buf[o : o + nbytes] for o, nbytes in zip(offs, sizes)]
+            return (v[0].view(torch.int64), v[1].view(torch.int64), v[2].view(torch.int32), v[3].view(torch.int32),
+                    v[4].view(torch.int32).view(block_tables.shape) if with_table else None)
+
+        h = views(host)
+        tokens, positions, seq = (t.numpy() for t in h[:3])
+        for i, (ts, p) in enumerate(zip(token_lists, pos0)):
+            a, b = starts[i], starts[i + 1]
+            tokens[a:b] = array("q", ts)
+            positions[a:b] = np.arange(p, p + b - a)
+            seq[a:b] = i
+        h[3].numpy()[:] = slots
+        if with_table:
+            h[4].copy_(block_tables)
+        d = views(host.to(dev, non_blocking=True))
+        return cls(d[0], d[1], d[2], d[3], d[4] if with_table else block_tables.to(dev), 0, starts, list(slots), list(pos0))
 
     @classmethod
     def uniform(cls, tokens, positions, slots, block_tables, G: int, device) -> "PackedBatch":

@@ -15,6 +15,7 @@ import ctypes
 import time
 from ctypes import c_float, c_int, c_void_p
 
+import numpy as np
 import torch
 
 from ..obs import buildlog
@@ -517,26 +518,33 @@ def _memo(key, make):
     return val
 
 
+def _to_device(table: np.ndarray, dev) -> torch.Tensor:
+    """An int32 table on the device, by one asynchronous copy from pinned memory."""
+    t = torch.from_numpy(table.astype(np.int32))
+    return t.pin_memory().to(dev, non_blocking=True) if dev.type == "cuda" else t
+
+
 def _gdn_prefill_meta(seg_starts, seg_slots, T: int, dev):
     def make():
         nseg = len(seg_slots)
-        chunks, seg_chunks, seq_of_row = [], [], []
-        for i in range(nseg):
-            a, b = seg_starts[i], seg_starts[i + 1]
-            first = len(chunks)
-            for r0 in range(a, b, 64):
-                chunks.append((i, r0, min(64, b - r0), int(r0 == a)))
-            seg_chunks.append((first, len(chunks) - first))
-            seq_of_row.extend([i] * (b - a))
-        meta = torch.tensor([c for ch in chunks for c in ch] + [c for sc in seg_chunks for c in sc] + seq_of_row
-                            + list(seg_starts) + list(seg_slots), dtype=torch.int32).to(dev, non_blocking=True)
+        starts = np.asarray(seg_starts, dtype=np.int64)
+        lens = np.diff(starts)
+        per_seg = (lens + 63) // 64
+        first = np.cumsum(per_seg) - per_seg
+        n_chunks = int(per_seg.sum())
+        seg = np.repeat(np.arange(nseg), per_seg)
+        nth = np.arange(n_chunks) - first[seg]
+        r0 = starts[seg] + 64 * nth
+        chunks = np.stack([seg, r0, np.minimum(64, starts[seg + 1] - r0), nth == 0], 1)
+        meta = _to_device(np.concatenate([chunks.reshape(-1), np.stack([first, per_seg], 1).reshape(-1),
+                                          np.repeat(np.arange(nseg), lens), starts, np.asarray(seg_slots)]), dev)
         o = 0
-        chunks_t = meta[o : o + 4 * len(chunks)]; o += 4 * len(chunks)
+        chunks_t = meta[o : o + 4 * n_chunks]; o += 4 * n_chunks
         segc_t = meta[o : o + 2 * nseg]; o += 2 * nseg
         sor_t = meta[o : o + T]; o += T
         start_t = meta[o : o + nseg + 1]; o += nseg + 1
         slots_t = meta[o : o + nseg]
-        return len(chunks), chunks_t, segc_t, sor_t, start_t, slots_t
+        return n_chunks, chunks_t, segc_t, sor_t, start_t, slots_t
 
     return _memo(("gdn", tuple(seg_starts), tuple(seg_slots), T, str(dev)), make)
 
@@ -626,12 +634,13 @@ def flash_prefill(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, b
     dev = q.device
 
     def make():
-        tiles = []
-        for i in range(len(seg_starts) - 1):
-            n = seg_starts[i + 1] - seg_starts[i]
-            tiles.extend((i, p0, seg_starts[i], n) for p0 in range(0, n, R))
-        return (len(tiles), torch.tensor(tiles, dtype=torch.int32).reshape(-1, 4).to(dev, non_blocking=True),
-                torch.tensor(seg_pos0, dtype=torch.int32).to(dev, non_blocking=True))
+        starts = np.asarray(seg_starts, dtype=np.int64)
+        lens = np.diff(starts)
+        per_seg = (lens + R - 1) // R
+        seg = np.repeat(np.arange(len(lens)), per_seg)
+        p0 = R * (np.arange(len(seg)) - (np.cumsum(per_seg) - per_seg)[seg])
+        table = _to_device(np.concatenate([np.stack([seg, p0, starts[seg], lens[seg]], 1).reshape(-1), np.asarray(seg_pos0)]), dev)
+        return len(seg), table[: 4 * len(seg)].view(-1, 4), table[4 * len(seg) :]
 
     if meta is not None:
         r_meta, n_tiles, tiles_t, pos0_t = meta

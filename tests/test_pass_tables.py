@@ -1,0 +1,30 @@
+"""The index tables of a ragged prefill pass against their definitions, on the CPU."""
+
+import pytest
+import torch
+
+from b200serve.models.qwen36 import PackedBatch
+from b200serve.ops import cuda_ops
+
+
+@pytest.mark.parametrize("lens", [[1], [64], [65, 1, 200], [3, 0, 130], [7, 64, 63, 128]])
+def test_batch_and_span_tables(lens):
+    n, dev = len(lens), torch.device("cpu")
+    toks = [list(range(10 * i, 10 * i + m)) for i, m in enumerate(lens)]
+    pos0 = [64 * i for i in range(n)]
+    table = torch.arange(n * 5, dtype=torch.int32).view(n, 5)
+    for tokens in (toks, [tuple(t) for t in toks]):
+        b = PackedBatch.prefill(tokens, [i + 3 for i in range(n)], pos0, table, "cpu")
+        assert b.tokens.dtype == b.positions.dtype == torch.int64 and b.seq_of_row.dtype == b.slots.dtype == torch.int32
+        assert b.tokens.tolist() == [t for ts in toks for t in ts]
+        assert b.positions.tolist() == [p + j for p, m in zip(pos0, lens) for j in range(m)]
+        assert b.seq_of_row.tolist() == [i for i, m in enumerate(lens) for _ in range(m)]
+        assert b.slots.tolist() == [i + 3 for i in range(n)] and torch.equal(b.block_tables, table) and b.G == 0
+    assert torch.equal(PackedBatch.prefill(toks, [0] * n, pos0, table.long(), "cpu").block_tables, table.long())
+    starts = b.seg_starts
+    T = starts[-1]
+    n_chunks, chunks, per_seg, seq, st, slots = cuda_ops._gdn_prefill_meta(starts, b.seg_slots, T, dev)
+    ref = [[i, r, min(64, starts[i + 1] - r), int(r == starts[i])] for i in range(n) for r in range(starts[i], starts[i + 1], 64)]
+    assert n_chunks == len(ref) and chunks.view(-1, 4).tolist() == ref
+    assert per_seg.view(-1, 2).tolist() == [[sum(-(-m // 64) for m in lens[:i]), -(-lens[i] // 64)] for i in range(n)]
+    assert seq.tolist() == b.seq_of_row.tolist() and st.tolist() == starts and slots.tolist() == b.seg_slots
