@@ -69,3 +69,31 @@ def test_wide_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, p
         C.GATHER_MAX_BT, C.WIDE_MIN_ROWS = keep
     C.check_errors(x.device)
     assert torch.equal(wide, narrow)
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (31, 64, 32), (32, 64, 32), (33, 64, 32), (32, 300, 7), (700, 40, 3)])
+def test_routing_and_plan_of_tied_rows(C, T, E, k):
+    """Quantised logits, so that ties are everywhere; the largest table that stays in shared memory, and one beyond it."""
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    logits = (torch.randn(T, E + 1, device="cuda", generator=g) * 3).round() / 2
+    P, dev = k + 1, "cuda"
+    wts = torch.empty(T, P, device=dev)
+    idx, perm, inv, src = (torch.full((T * P,), -7, dtype=torch.int32, device=dev) for _ in range(4))
+    offsets = torch.empty(E + 2, dtype=torch.int32, device=dev)
+    max_tiles = min(E + 1, T * P) + T * P // 16 + 1
+    tiles, n = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev), torch.empty(1, dtype=torch.int32, device=dev)
+    err = C.err_word(logits.device)
+    rc = C.lib().b200_moe_route_plan(logits.data_ptr(), E + 1, T, E, k, 1, wts.data_ptr(), idx.data_ptr(), None, E + 1, 16,
+                                     offsets.data_ptr(), tiles.data_ptr(), n.data_ptr(), max_tiles, perm.data_ptr(), inv.data_ptr(),
+                                     err.data_ptr(), src.data_ptr(), C._ticket(logits.device).data_ptr(), C._stream())
+    assert rc == 0
+    C.check_errors(logits.device)
+    # equal logits have equal probabilities: the lower expert id first
+    order = torch.sort(logits[:, :E], dim=1, descending=True, stable=True).indices[:, :k]
+    table = idx.view(T, P).long()
+    assert torch.equal(table[:, :k], order) and (table[:, k] == E).all()
+    pr = torch.softmax(logits[:, :E].double(), 1).gather(1, order)
+    assert torch.allclose(wts[:, :k].double(), pr / pr.sum(1, keepdim=True), rtol=2.0 ** -8 * 1.01, atol=1e-7)  # bf16 weights
+    assert torch.equal(offsets.long(), torch.nn.functional.pad(table.flatten().bincount(minlength=E + 1).cumsum(0), (1, 0)))
+    assert torch.equal(perm.long().sort().values, torch.arange(T * P, device=dev)) and torch.equal(perm[inv.long()].long(), torch.arange(T * P, device=dev))
+    assert torch.equal(table.flatten()[perm.long()], table.flatten().sort().values) and torch.equal(src, perm // P)
