@@ -152,9 +152,12 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   // Persistent tile loop: CTA b takes output tiles b, b + gridDim.x, ... (weight tile fastest, so CTAs that run
   // together share the activation tile). A split-K cluster takes the single tile its grid position names.
   const int tiles_n = (p.N + RT - 1) / RT;
+  // The role's first table entry is read beside the entry count, not behind it (the table has room for the whole grid).
+  const int tile0 = SPLIT ? static_cast<int>(blockIdx.y) * tiles_n + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
+  int4 t_next = make_int4(0, 0, 0, 0);
+  if (GROUPED) t_next = p.tiles[tile0 / tiles_n];
   const int tiles_y = GROUPED ? *p.n_tiles : p.grid_y;
   const int total = tiles_n * tiles_y;
-  const int tile0 = SPLIT ? static_cast<int>(blockIdx.y) * tiles_n + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
   const int tstep = SPLIT ? (1 << 30) : static_cast<int>(gridDim.x);
   constexpr int ACC = SPLIT ? 1 : C::ACC_STAGES;
   if (SPLIT && tile0 >= total) return;  // the whole cluster leaves together, before any barrier or TMEM use
@@ -184,8 +187,6 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   // geometry of output tile `tile`
   // (the table entry of the role's next tile is requested one tile ahead: its latency would otherwise open every tile)
-  int4 t_next = make_int4(0, 0, 0, 0);
-  if (GROUPED && tile0 < total) t_next = p.tiles[tile0 / tiles_n];
   auto tile_geom = [&](int tile, int& n0, int& by, int& expert, int& row0, int& nrows) {
     const int nx = tile % tiles_n, byr = tile / tiles_n;
     n0 = nx * RT;
