@@ -606,13 +606,16 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, C::TMEM_COLS); }
 }
 
-// Reduce the LM-head partials of each row over the vocabulary tiles, first maximum wins.
+// Reduce the LM-head partials of each row over the vocabulary tiles, first maximum wins. Bound by the latency of a thread's
+// loads: while there are no more rows than SMs a row gets 1024 threads (two loads each at 1940 tiles, not eight): 6.4 -> 4.6 us
+// at one to twelve rows, 8.0 -> 6.9 at 128.
 __global__ void argmax_finish_kernel(const float* part_max, const int* part_idx, int n_tiles, int T, int64_t* out,
                                      float* out_val) {
   pdl_wait();
   pdl_launch();
   const int t = blockIdx.x;
   float m = -INFINITY; int idx = 0x7fffffff;
+#pragma unroll 2
   for (int i = threadIdx.x; i < n_tiles; i += blockDim.x) {
     const float om = part_max[static_cast<size_t>(i) * T + t]; const int oi = part_idx[static_cast<size_t>(i) * T + t];
     if (om > m || (om == m && oi < idx)) { m = om; idx = oi; }
@@ -1021,7 +1024,8 @@ extern "C" int b200_gemm_gathered(const void* X, const void* W, void* out, int T
 extern "C" int b200_argmax_finish(const float* part_max, const int* part_idx, int n_tiles, int T, int64_t* out,
                                   float* out_val, cudaStream_t st) {
   if (T <= 0) return 0;
-  return launch_pdl(argmax_finish_kernel, dim3(T), dim3(256), 0, st, part_max, part_idx, n_tiles, T, out, out_val) ==
+  const int threads = T <= sm_count() && n_tiles > 512 ? 1024 : 256;
+  return launch_pdl(argmax_finish_kernel, dim3(T), dim3(threads), 0, st, part_max, part_idx, n_tiles, T, out, out_val) ==
                  cudaSuccess ? 0 : -4;
 }
 

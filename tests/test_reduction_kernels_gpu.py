@@ -69,7 +69,7 @@ def test_expert_outputs_of_a_row(C, T, P, H):
     assert torch.equal(new, ref_new) and torch.equal(y, ref_y)
 
 
-@pytest.mark.parametrize("T,V", [(1, 128), (2, 1000), (17, 129), (64, 4096), (200, 777), (256, 1280), (300, 2500)])
+@pytest.mark.parametrize("T,V", [(1, 128), (2, 1000), (17, 129), (64, 4096), (200, 777), (256, 1280), (300, 2500), (3, 70001), (150, 70001)])
 def test_greedy_head_takes_the_lowest_id_among_equal_logits(C, T, V):
     """Small whole numbers: every logit is exact, and a row has many columns with the same largest one."""
     g = torch.Generator(device="cuda").manual_seed(T * 7 + V)
