@@ -294,9 +294,21 @@ __device__ __forceinline__ float exp2_ftz(float x) {
   return y;
 }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
-// The same with the reciprocal unit's quotient (2 ulp instead of a correctly rounded one, far below the bf16 rounding that
-// follows it in every use): the exact division alone was a third of the instructions of the elementwise prefill kernels.
-__device__ __forceinline__ float silu_fast_f(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+// silu_f by the reciprocal unit's quotient, for values that are rounded to bf16 next. __fdividef is off by 2 units in the last
+// place at most, and gives 0 for a denominator above 2^126. So where no quotient is that small and none lies within 4 units of
+// a tie between two bf16 numbers, all of them round to the bf16 numbers that silu_f's do; where `settled` says no (one
+// value in 7000, and the far ends of the range), the caller takes silu_f. (A NaN is one in both.)
+struct SiluCheck {
+  uint32_t tie = 0xffffffffu;  // smallest distance above "4 units below a tie", in the upper half of the word
+  float least = INFINITY;
+  __device__ __forceinline__ float quotient(float x) {
+    const float q = __fdividef(x, 1.0f + __expf(-x));
+    tie = min(tie, (__float_as_uint(q) << 16) - 0x7ffc0000u);
+    least = fminf(least, fabsf(q));
+    return q;
+  }
+  __device__ __forceinline__ bool settled() const { return tie > 0x00080000u && least >= 0x1p-110f; }
+};
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(__expf(x)); }
 

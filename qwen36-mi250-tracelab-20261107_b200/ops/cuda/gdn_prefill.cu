@@ -34,8 +34,10 @@ struct ChunkInfo {  // one per (sequence chunk)
 // A thread owns 8 consecutive channels (16-byte loads) over ROWS rows and slides a 3-row window down them; the window is
 // rebuilt from the three rows above at the start of a run (they are in L2: the neighbouring run reads them too), or from
 // the slot's conv state where a span starts. The loads of four rows are issued together, and a run looks its span up once
-// and not row by row. 134 -> 68 us at 8192 rows x 8192 channels (268 MB, 4 TB/s; two rows per batch 75 us), 30 -> 5.5 us at
-// 61 rows, where a thread's 32 rows used to be one chain of dependent loads.
+// and not row by row. 134 -> 91 us at 8192 rows x 8192 channels (268 MB, 2.9 TB/s), 30 -> 7.5 us at 61 rows, where a thread's
+// 32 rows used to be one chain of dependent loads. The rest is arithmetic, of which the quotient of the SiLU is the largest
+// part: 120 us with silu_f for every value, 72 with the reciprocal unit's quotient unchecked, which rounds some values to
+// other bf16 numbers than the decode step does and loses results below 2^-125.
 template <int ROWS>
 __global__ void __launch_bounds__(128, 5)
 gdn_conv_prefill_kernel(const bf16* x, int ld, const int* seq_of_row, const int* seg_start, const int* slots,
@@ -93,14 +95,21 @@ gdn_conv_prefill_kernel(const bf16* x, int ld, const int* seq_of_row, const int*
         const bf16* xe = reinterpret_cast<const bf16*>(&xv[b]);
         uint4 ov;
         bf16* oe = reinterpret_cast<bf16*>(&ov);
+        const auto conv = [&](int ch) {
+          return w[ch][0] * win[0][ch] + w[ch][1] * win[1][ch] + w[ch][2] * win[2][ch] + w[ch][3] * __bfloat162float(xe[ch]);
+        };
+        SiluCheck check;
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch) oe[ch] = __float2bfloat16(check.quotient(conv(ch)));
+        if (!check.settled()) {
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch) oe[ch] = __float2bfloat16(silu_f(conv(ch)));
+        }
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch) {
-          const float cur = __bfloat162float(xe[ch]);
-          const float acc = w[ch][0] * win[0][ch] + w[ch][1] * win[1][ch] + w[ch][2] * win[2][ch] + w[ch][3] * cur;
-          oe[ch] = __float2bfloat16(silu_fast_f(acc));
           win[0][ch] = win[1][ch];
           win[1][ch] = win[2][ch];
-          win[2][ch] = cur;
+          win[2][ch] = __bfloat162float(xe[ch]);
         }
         *reinterpret_cast<uint4*>(out + static_cast<size_t>(r + b) * C + c) = ov;
       }
@@ -392,8 +401,8 @@ gdn_chunk_scan_kernel(const float* work, const ChunkInfo* chunks, const int2* se
 }
 
 // out[row, h, :] = bf16(w * bf16(o * rsqrt(mean(o^2) + eps)) * silu(z)). DV / 8 lanes share one (row, head), 16 bytes of
-// each tensor per lane, and a thread works on NORM_UNITS of them so that their loads are in flight together: 63 -> 37 us at
-// 8192 rows x 32 heads (201 MB, 5.4 TB/s).
+// each tensor per lane, and a thread works on NORM_UNITS of them so that their loads are in flight together: 63 -> 47 us at
+// 8192 rows x 32 heads (201 MB, 4.3 TB/s).
 constexpr int NORM_UNITS = 2;
 template <int DV>
 __global__ void __launch_bounds__(256)
@@ -430,7 +439,7 @@ gdn_gated_norm_kernel(const bf16* o, const bf16* mixed, int ld, int z_off, const
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float nb = __bfloat162float(__float2bfloat16(v[j] * inv));
-      re[j] = __float2bfloat16(__bfloat162float(we[j]) * nb * silu_fast_f(__bfloat162float(ze[j])));
+      re[j] = __float2bfloat16(__bfloat162float(we[j]) * nb * silu_f(__bfloat162float(ze[j])));
     }
     const int u = u0 + i * PER_CTA;
     if (u < n) *reinterpret_cast<uint4*>(out + static_cast<size_t>(u) * DV + lane * 8) = rv;
