@@ -287,12 +287,6 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-// 2^x by the special function unit, results below 2^-126 flushed to zero (exp2f spends three more instructions on those).
-__device__ __forceinline__ float exp2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 // silu_f by the reciprocal unit's quotient, for values that are rounded to bf16 next. __fdividef is off by 2 units in the last
 // place at most, and gives 0 for a denominator above 2^126. So where no quotient is that small and none lies within 4 units of

@@ -21,7 +21,9 @@
 // 96 KB (Q K^T: N = 64, 48 cycles an MMA) and 48 KB (P V). With one thread for all loads and MMAs, which also read the page
 // table between a free stage and its load, and one page in the softmax at a time, a page took 3400 cycles; it takes about
 // 1800 now: 4 x 2048 rows behind 6.5k to 28.7k tokens 3.70 -> 1.94 ms (1.23 PFLOP/s at 30k), 8 x 1024 rows 249 -> 206 us,
-// decode of 256 x 2.2k tokens 282 -> 224 us, of four sequences of 50-90k 147 -> 118 us.
+// decode of 256 x 2.2k tokens 282 -> 230 us, of four sequences of 50-90k 147 -> 120 us. The exponentials keep results below
+// 2^-126, which count where the value beside them is large; the unit's flushing form would save 1 to 2 % in decode (224 and
+// 118 us) and nothing in prefill.
 // Chunked prefill: queries sit at positions pos0.. of their sequence, keys are 0..pos.
 // All waits are bounded (common.cuh). No cluster multicast.
 #include "common.cuh"
@@ -261,7 +263,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         ok = mbar_wait(&pv_done[hf ^ 1], ((i - 1) >> 1) & 1, p.err, ERR_WAIT_EMPTY, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const float factor = need ? exp2_ftz(m_prev - m) : 1.0f;
+        const float factor = need ? exp2f(m_prev - m) : 1.0f;
 #pragma unroll 1
         for (int c = 0; c < D; c += 16) {
           float o[16];
@@ -272,7 +274,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      if (m != m_loc) { l *= exp2_ftz(m_loc - m); m_loc = m; }  // exp2(-inf) = 0 on this thread's first page
+      if (m != m_loc) { l *= exp2f(m_loc - m); m_loc = m; }  // exp2(-inf) = 0 on this thread's first page
       if (i >= 2) {  // this page's probability tile was last read by P V of page i - 2
         ok = mbar_wait(&pv_done[hf], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag);
         if (!ok) break;
@@ -286,7 +288,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         __nv_bfloat162* pe = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float a = exp2_ftz(fmaf(sc[c * 8 + 2 * j], p.scale_log2, -m)), b2 = exp2_ftz(fmaf(sc[c * 8 + 2 * j + 1], p.scale_log2, -m));
+          const float a = exp2f(fmaf(sc[c * 8 + 2 * j], p.scale_log2, -m)), b2 = exp2f(fmaf(sc[c * 8 + 2 * j + 1], p.scale_log2, -m));
           sum[(2 * j) & 3] += a;
           sum[(2 * j + 1) & 3] += b2;
           pe[j] = __floats2bfloat162_rn(a, b2);
@@ -310,7 +312,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       ok = mbar_wait(x_bar, 0, p.err, ERR_WAIT_FULL, abort_flag);
       const float l0 = ex[r * 2], m0 = ex[r * 2 + 1], l1 = ex[(STRIDE + r) * 2], m1 = ex[(STRIDE + r) * 2 + 1];
       m_used = fmaxf(m0, m1);  // a running maximum never falls: the larger one is the last page's
-      l = l0 * exp2_ftz(m0 - m_used) + l1 * exp2_ftz(m1 - m_used);
+      l = l0 * exp2f(m0 - m_used) + l1 * exp2f(m1 - m_used);
     }
     if (ok && p.split_pages > 0) {
       const size_t row = static_cast<size_t>(seg_row0 + p0 + lp);

@@ -1,0 +1,41 @@
+"""Attention over the whole range of its numbers: far probabilities beside large values, sums of partials in one chain."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def C():
+    from b200serve.ops import cuda_ops
+
+    cuda_ops.lib()
+    return cuda_ops
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_probability_below_the_normal_range_beside_a_large_value(C, D, decode):
+    """Key 0 has log-2 score 130 above the others, and four of them have values of 2^127: each adds about 2^-130 * 2^127 to
+    an output of 1."""
+    n_q, n_kv, n = 8, 1, 100  # two pages
+    q = torch.zeros(n, n_q, D, dtype=torch.bfloat16, device="cuda")
+    kv = torch.zeros(3, 2, n_kv, 64, D, dtype=torch.bfloat16, device="cuda")
+    q[:, :, 0] = 32.0
+    kv[1, 0, 0, 0, 0] = torch.tensor(90.0 * D ** 0.5 / 32.0).bfloat16()
+    kv[1, 1, 0, 0] = 1.0
+    kv[1, 1, 0, 3:7] = 2.0 ** 127
+    gate = torch.full((n, n_q * D), 30.0, dtype=torch.bfloat16, device="cuda")  # sigmoid rounds to 1
+    table = torch.tensor([[1, 2]], dtype=torch.int32, device="cuda")
+    if decode:
+        got = C.flash_decode(q[-1:].contiguous(), gate[-1:].contiguous(), kv, table, torch.tensor([n - 1], device="cuda"), 1)
+    else:
+        got = C.flash_prefill(q, gate, kv, table, [0, n], [0])[-1:]
+    C.check_errors(q.device)
+    score = 32.0 * kv[1, 0, 0, 0, 0].double().item() * D ** -0.5
+    p = torch.exp(torch.tensor(-score, dtype=torch.float64)).item()
+    far = p * 4 * 2.0 ** 127
+    assert 0.2 < far < 1.0
+    # a probability of 2^-130 is a multiple of 2^-133 as bf16: off by a sixteenth at most; the sum is rounded to bf16
+    assert ((got.double() - (1.0 + far)).abs() <= far / 16 + 2.0 ** -7).all()
