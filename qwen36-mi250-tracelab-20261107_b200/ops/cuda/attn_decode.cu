@@ -8,7 +8,8 @@
 //                CTA z walks pages z, z+Z, z+2Z, ... with one running online softmax, so the
 //                reduction order of a sequence depends only on its own length, never on the batch
 //                (reference: engine/fast/kernels.py:377-443 splits the context the same way).
-//  attn_combine: merge the Z partials in order, multiply by sigmoid(gate), store bf16
+//  attn_combine: merge the Z partials in an order that the splits with keys fix (up to 16 of them one after the other,
+//                more as sixteen running sums), multiply by sigmoid(gate), store bf16
 //                (reference: engine/fast/fused.py:530-551).
 //
 // KV layout: kv[page][2][n_kv][PAGE][D] bf16; page tables int32 [B, max_pages]; page 0 is scratch.
@@ -254,17 +255,22 @@ paged_attn_kernel(const bf16* q, const bf16* kv, const int* tables, int max_page
   }
 }
 
-// Merge the Z partials of one (row, head). The partials are dealt to COMBINE_GROUPS running sums, partial z to sum
-// z % COMBINE_GROUPS, which are added in order at the end: the order depends on the number of finite partials only,
-// never on the table width behind Z or on the launch. A thread owns four columns and GPT of the sums, so GPT partial
-// rows are in flight at once (one thread per column walking all partials was bound by their latency: 58 us for four
-// sequences of 50-90k tokens in a 512-partial table, 7.4 us now).
 constexpr int COMBINE_GROUPS = 16;
+__device__ __forceinline__ bf16 gated(float o, bf16 gate) {
+  return __float2bfloat16(__bfloat162float(__float2bfloat16(o)) * sigmoid_f(__bfloat162float(gate)));
+}
+
+// Merge the Z partials of one (row, head). Up to COMBINE_GROUPS splits are added in order, each sum one chain of fused
+// multiply-adds (a product that is rounded before it is added costs the sum bits where partials cancel). Of more splits,
+// partial z goes to running sum z % COMBINE_GROUPS, and the sums are added in order at the end. Which of the two, and the
+// order, depends on the splits that hold keys only, never on the table width behind them or on the launch. A thread owns
+// four columns and GPT of the sums, so GPT partial rows are in flight at once (one thread per column walking all
+// partials was bound by their latency: 58 us for four sequences of 50-90k tokens in a 512-partial table, 7.4 us now).
 template <int D, int GPT>
 __global__ void __launch_bounds__(D / 4 * COMBINE_GROUPS / GPT)
 attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gate, bf16* out, int n_q, int Z) {
   constexpr int QUADS = D / 4, THREADS = QUADS * COMBINE_GROUPS / GPT, WARPS = THREADS / 32;
-  __shared__ float s_max[WARPS], s_l[COMBINE_GROUPS];
+  __shared__ float s_max[WARPS], s_l[COMBINE_GROUPS], s_f[COMBINE_GROUPS];
   __shared__ int s_last[WARPS];
   __shared__ __align__(16) float s_acc[COMBINE_GROUPS][D];
   const int row = blockIdx.x, qh = blockIdx.y;
@@ -286,6 +292,7 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < WARPS; ++w) { m = fmaxf(m, s_max[w]); last = max(last, s_last[w]); }
+  const bool few = last <= COMBINE_GROUPS;
   const float4* pa = reinterpret_cast<const float4*>(part_acc + head * Z * D) + quad;
   float l[GPT];
   float4 acc[GPT];
@@ -304,7 +311,7 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
 #pragma unroll
     for (int u = 0; u < GPT; ++u) {
       if (pm[u].x == -INFINITY) continue;
-      const float sc = __expf(pm[u].x - m);
+      const float sc = few ? 1.f : __expf(pm[u].x - m);  // few: one partial per sum, scaled when it is added
       l[u] += pm[u].y * sc;
       acc[u].x += v[u].x * sc; acc[u].y += v[u].y * sc; acc[u].z += v[u].z * sc; acc[u].w += v[u].w * sc;
     }
@@ -312,20 +319,21 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
 #pragma unroll
   for (int u = 0; u < GPT; ++u) {
     *reinterpret_cast<float4*>(&s_acc[g0 + u][quad * 4]) = acc[u];
-    if (quad == 0) s_l[g0 + u] = l[u];
+    if (quad == 0) {
+      s_l[g0 + u] = l[u];
+      s_f[g0 + u] = !few ? 1.f : g0 + u < last ? __expf(ml[g0 + u].x - m) : 0.f;
+    }
   }
   __syncthreads();
   for (int d = threadIdx.x; d < D; d += THREADS) {
     float ls = 0.f, o = 0.f;
 #pragma unroll
-    for (int g = 0; g < COMBINE_GROUPS; ++g) { ls += s_l[g]; o += s_acc[g][d]; }
-    const float ob = __bfloat162float(__float2bfloat16(o / ls));
-    out[head * D + d] = __float2bfloat16(ob * sigmoid_f(__bfloat162float(gate[head * D + d])));
+    for (int g = 0; g < COMBINE_GROUPS; ++g) { ls = fmaf(s_l[g], s_f[g], ls); o = fmaf(s_acc[g][d], s_f[g], o); }
+    out[head * D + d] = gated(o / ls, gate[head * D + d]);
   }
 }
 
-// At most COMBINE_GROUPS partials: every running sum has one term, so the same result (product rounded, then added in
-// order) needs neither the shared-memory exchange nor a barrier. D / 4 threads per (row, head).
+// At most COMBINE_GROUPS partials: neither an exchange between threads nor a barrier. D / 4 threads per (row, head).
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_combine_few_kernel(const float* part_acc, const float* part_ml, const bf16* gate, bf16* out, int heads, int Z) {
@@ -355,19 +363,18 @@ attn_combine_few_kernel(const float* part_acc, const float* part_ml, const bf16*
     for (int u = 0; u < BATCH; ++u) {
       if (pm[z0 + u].x == -INFINITY) continue;
       const float sc = __expf(pm[z0 + u].x - m);
-      ls = __fadd_rn(ls, __fmul_rn(pm[z0 + u].y, sc));
-      o[0] = __fadd_rn(o[0], __fmul_rn(v[u].x, sc));
-      o[1] = __fadd_rn(o[1], __fmul_rn(v[u].y, sc));
-      o[2] = __fadd_rn(o[2], __fmul_rn(v[u].z, sc));
-      o[3] = __fadd_rn(o[3], __fmul_rn(v[u].w, sc));
+      ls = fmaf(pm[z0 + u].y, sc, ls);
+      o[0] = fmaf(v[u].x, sc, o[0]);
+      o[1] = fmaf(v[u].y, sc, o[1]);
+      o[2] = fmaf(v[u].z, sc, o[2]);
+      o[3] = fmaf(v[u].w, sc, o[3]);
     }
   }
   const bf16* ge = reinterpret_cast<const bf16*>(&graw);
   uint2 raw;
   bf16* oe = reinterpret_cast<bf16*>(&raw);
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    oe[j] = __float2bfloat16(__bfloat162float(__float2bfloat16(o[j] / ls)) * sigmoid_f(__bfloat162float(ge[j])));
+  for (int j = 0; j < 4; ++j) oe[j] = gated(o[j] / ls, ge[j]);
   reinterpret_cast<uint2*>(out + head * D)[quad] = raw;
 }
 
@@ -458,7 +465,7 @@ extern "C" int b200_paged_attn(const void* q, const void* gate, const void* kv, 
   return rc == cudaSuccess ? 0 : -4;
 }
 
-// Merge split partials [rows, n_q, Z, D] / [rows, n_q, Z, 2] in split order, apply sigmoid(gate), store bf16.
+// Merge split partials [rows, n_q, Z, D] / [rows, n_q, Z, 2] (the order: attn_combine_kernel), apply sigmoid(gate), store bf16.
 extern "C" int b200_attn_combine(const float* part_acc, const float* part_ml, const void* gate, void* out, int rows,
                                  int n_q, int D, int Z, cudaStream_t st) {
   if (rows <= 0) return 0;

@@ -668,7 +668,7 @@ def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, bl
 
     Each sequence is one query tile (its ``G`` positions x the GQA group fill the first rows of the 128-row
     MMA tile); the context is cut into runs of ``SPLIT_PAGES`` pages handled by separate CTAs whose partial
-    results are merged in order. Only device tensors are touched, so the call can be captured in a CUDA graph."""
+    results are merged in an order that the context's length fixes. Only device tensors are touched, so the call can be captured in a CUDA graph."""
     rows, n_q, D = q.shape
     n_kv = kv_layer.shape[2]
     B = rows // G

@@ -39,3 +39,23 @@ def test_probability_below_the_normal_range_beside_a_large_value(C, D, decode):
     assert 0.2 < far < 1.0
     # a probability of 2^-130 is a multiple of 2^-133 as bf16: off by a sixteenth at most; the sum is rounded to bf16
     assert ((got.double() - (1.0 + far)).abs() <= far / 16 + 2.0 ** -7).all()
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("Z", [4, 16, 17, 64, 512])
+def test_partials_of_up_to_16_splits_are_added_in_one_fused_chain(C, D, Z):
+    """Partials -4 s, 3 s and s with s = e^-x: 3 s is not a float, but a chain of fused multiply-adds never forms it (-4 s, -s,
+    0). Products that are rounded before they are added leave a remainder."""
+    rows, n_q = 64, 2
+    acc = torch.full((rows, n_q, Z, D), float("nan"), device="cuda")
+    ml = torch.zeros(rows, n_q, Z, 2, device="cuda")
+    ml[..., 0] = float("-inf")
+    acc[:, :, 0], ml[:, :, 0, 0], ml[:, :, 0, 1] = 0.0, 0.0, 1.0
+    x = torch.linspace(0.01, 5.0, rows, device="cuda")[:, None]
+    for z, v in ((1, -4.0), (2, 3.0), (3, 1.0)):
+        acc[:, :, z], ml[:, :, z, 0], ml[:, :, z, 1] = v, -x, 1.0
+    gate = torch.full((rows, n_q * D), 30.0, dtype=torch.bfloat16, device="cuda")
+    out = torch.empty(rows, n_q * D, dtype=torch.bfloat16, device="cuda")
+    C._check(C.lib().b200_attn_combine(acc.data_ptr(), ml.data_ptr(), gate.data_ptr(), out.data_ptr(), rows, n_q, D, Z, C._stream()),
+             "attn_combine")
+    assert (out == 0).all()
