@@ -62,8 +62,8 @@ gdn_conv_prefill_kernel(const bf16* x, int ld, const int* seq_of_row, const int*
   const int r1 = min(T, r + ROWS);
   while (r < r1) {
     const int seg = seq_of_row[r];
-    const int s0 = seg_start[seg], e = min(r1, seg_start[seg + 1]);
-    if (e <= r) return;  // not a table of consecutive spans
+    // a row behind the end that the table gives its span is a run of its own: no row is left out
+    const int s0 = seg_start[seg], e = max(r + 1, min(r1, seg_start[seg + 1]));
     float win[3][8];  // inputs of rows r-3, r-2, r-1
     {
       uint4 sv[3];

@@ -96,3 +96,14 @@ def test_silu_of_far_negative_arguments(C, d):
     ref = par[3].double() * normed * silu[:, None, None]
     # the normed value may round to its other bf16 neighbour (2^-7); below 2^-126 a result has an absolute step of 2^-133
     assert ((out.double().view(T, n_v, d) - ref).abs() <= (2.0 ** -7 + tol) * 1.01 * ref.abs() + 2.0 ** -133).all()
+
+
+@pytest.mark.parametrize("T,end", [(24, 16), (40, 3), (700, 699), (4100, 4090)])
+def test_rows_behind_the_end_that_the_table_gives_their_span(C, T, end):
+    """The conv of such a row still takes the rows above it: nothing is left unwritten."""
+    n_k, n_v, d = 2, 4, 32
+    par, ch = _params(n_k, n_v, d), 2 * n_k * d + n_v * d
+    mixed, state = _bf(T, ch + n_v * d + 2 * n_v, seed=6), _bf(2, ch, 3, seed=7)
+    whole, _, _ = _prefill(C, mixed, [0, T], par, n_k, n_v, d, state.clone())
+    got, _, _ = _prefill(C, mixed, [0, T], par, n_k, n_v, d, state.clone(), seg_start=_i32([0, end]))
+    assert torch.equal(got, whole)
