@@ -379,15 +379,18 @@ attn_combine_few_kernel(const float* part_acc, const float* part_ml, const bf16*
 }
 
 // Up to 16 partials (contexts up to 8192 tokens, or short tables): no exchange between threads (128 rows of 8 partials:
-// 4.3 us, 11.7 us with the exchange; 256 rows 12.9 -> 8.7 us). Below 64 partials (512 pages of table) four sums per thread fill a CTA of 256
-// threads (D = 256) and rows and heads fill the GPU; beyond, few sequences share the GPU and one sum per thread keeps
+// 4.3 us, 11.7 us with the exchange; 256 rows 12.9 -> 8.7 us). Below 64 partials (512 pages of table) four sums per thread
+// fill a CTA of 256 threads (D = 256) and rows and heads fill the GPU; beyond, few sequences share the GPU and one sum per thread keeps
 // four times as many rows in flight per CTA.
 template <int D>
 static cudaError_t launch_combine(const float* part_acc, const float* part_ml, const bf16* gate, bf16* out, int rows,
                                   int n_q, int Z, cudaStream_t st) {
   constexpr int T4 = D / 4 * COMBINE_GROUPS / 4;
   const dim3 grid(rows, n_q);
-  if (Z <= COMBINE_GROUPS) {
+  const auto at = [](const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+  if (!at(part_acc, 16) || !at(part_ml, 8)) return cudaErrorInvalidValue;
+  // (the gate may be a view that starts at any element: the other kernels read it and write `out` element by element)
+  if (Z <= COMBINE_GROUPS && at(gate, 8) && at(out, 8)) {
     const int per = 256 / (D / 4), heads = rows * n_q;
     return launch_pdl(attn_combine_few_kernel<D>, dim3((heads + per - 1) / per), dim3(256), 0, st, part_acc, part_ml, gate,
                       out, heads, Z);

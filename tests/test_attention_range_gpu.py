@@ -59,3 +59,19 @@ def test_partials_of_up_to_16_splits_are_added_in_one_fused_chain(C, D, Z):
     C._check(C.lib().b200_attn_combine(acc.data_ptr(), ml.data_ptr(), gate.data_ptr(), out.data_ptr(), rows, n_q, D, Z, C._stream()),
              "attn_combine")
     assert (out == 0).all()
+
+
+@pytest.mark.parametrize("width", [64, 200])
+@pytest.mark.parametrize("n_q,n_kv,D", [(16, 2, 256), (4, 1, 64)])
+def test_gate_that_starts_at_an_odd_element(C, width, n_q, n_kv, D):
+    g = torch.Generator(device="cuda").manual_seed(D + width)
+    pos = torch.tensor([700, 63, 1500], device="cuda")
+    kv = torch.randn(60, 2, n_kv, 64, D, device="cuda", generator=g).bfloat16()
+    table = torch.randint(1, 60, (3, width), device="cuda", generator=g).int()
+    q = torch.randn(3, n_q, D, device="cuda", generator=g).bfloat16()
+    flat = torch.randn(3 * n_q * D + 8, device="cuda", generator=g).bfloat16()
+    for off in (1, 2, 3):
+        gate = flat[off:off + 3 * n_q * D].view(3, n_q * D)
+        got = C.flash_decode(q, gate, kv, table, pos, 1)
+        C.check_errors(q.device)
+        assert torch.equal(got, C.flash_decode(q, gate.clone(), kv, table, pos, 1))
