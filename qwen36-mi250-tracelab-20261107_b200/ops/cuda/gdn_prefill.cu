@@ -414,8 +414,13 @@ gdn_gated_norm_kernel(const bf16* o, const bf16* mixed, int ld, int z_off, const
   const int n = rows * HV;
   pdl_wait();
   pdl_launch();
-  const uint4 wv = *reinterpret_cast<const uint4*>(w + lane * 8);
-  const bf16* we = reinterpret_cast<const bf16*>(&wv);
+  __align__(16) bf16 we[8];
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {  // the weights may be a view that starts at any element
+    *reinterpret_cast<uint4*>(we) = *reinterpret_cast<const uint4*>(w + lane * 8);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) we[j] = w[lane * 8 + j];
+  }
   uint4 ov[NORM_UNITS], zv[NORM_UNITS];
   const int u0 = blockIdx.x * (PER_CTA * NORM_UNITS) + threadIdx.x / LANES;
 #pragma unroll
@@ -505,6 +510,10 @@ extern "C" int b200_gdn_prefill(const void* mixed, int ld, const int* seq_of_row
   if (DK != DV) return -7;
   const int C = 2 * HK * DK + HV * DV;
   if (C % 8 || ld % 8) return -7;
+  // the kernels move 16 bytes at a time between these (the norm's weights may start anywhere)
+  for (const void* b : {mixed, static_cast<const void*>(conv_state), conv_w, static_cast<const void*>(conv_out),
+                        static_cast<const void*>(o_tmp), static_cast<const void*>(out)})
+    if (reinterpret_cast<uintptr_t>(b) & 15) return -7;
   // Runs of 16 rows read three rows in sixteen twice; below 4096 rows runs of 8 put twice as many threads to work.
   const auto conv = [&](auto kern, int run) {
     return launch_pdl(kern, dim3((C / 8 + 127) / 128, (T + run - 1) / run), dim3(128), 0, st, static_cast<const bf16*>(mixed),

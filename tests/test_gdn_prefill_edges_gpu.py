@@ -107,3 +107,15 @@ def test_rows_behind_the_end_that_the_table_gives_their_span(C, T, end):
     whole, _, _ = _prefill(C, mixed, [0, T], par, n_k, n_v, d, state.clone())
     got, _, _ = _prefill(C, mixed, [0, T], par, n_k, n_v, d, state.clone(), seg_start=_i32([0, end]))
     assert torch.equal(got, whole)
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_norm_weights_that_start_at_any_element(C, d):
+    n_k, n_v, T = 2, 4, 70
+    par, ch = _params(n_k, n_v, d), 2 * n_k * d + n_v * d
+    mixed, state = _bf(T, ch + n_v * d + 2 * n_v, seed=8), torch.zeros(2, ch, 3, dtype=torch.bfloat16, device="cuda")
+    want = _prefill(C, mixed, [0, T], par, n_k, n_v, d, state.clone())[2]
+    for off in (1, 2, 4, 8):
+        flat = torch.zeros(d + 8, dtype=torch.bfloat16, device="cuda")
+        flat[off:off + d] = par[3]
+        assert torch.equal(_prefill(C, mixed, [0, T], (*par[:3], flat[off:off + d]), n_k, n_v, d, state.clone())[2], want)
