@@ -111,12 +111,12 @@ __global__ void moe_gather_kernel(const bf16* x, const int* perm, const int* n_v
 // With NORM the same launch also does what add_rmsnorm would do next: res' = bf16(res + out[t]) and
 // y = bf16(res' * rsqrt(mean(res'^2) + eps) * (1 + w)) (zero-centred weight), with the same rounding points.
 //
-// Bound by the latency of the gathered rows at decode sizes and by memory at prefill sizes. The weights and positions
-// of a row are fetched by its first threads before the dependency wait (the routing kernel that wrote them is at least
-// two launches back, and the launch before this one released its dependents only after its own wait), and the rows of
-// COMBINE_U pairs are requested together instead of one behind the other: 8.4 -> 3.7 us at 128 rows of 9 pairs, 79 -> 71 us
-// at 8192 rows (402 MB, 5.6 TB/s). All nine in flight take 75 registers and lose more in resident CTAs at the large
-// size (85 us) than they gain at the small one (3.5 us).
+// Bound by the latency of the gathered rows at decode sizes and by memory at prefill sizes. The first threads of a row fetch
+// its weights and positions for all of them, and the rows of COMBINE_U pairs are requested together instead of one behind
+// the other: 8.4 -> 4.1 us at 128 rows of 9 pairs, 79 -> 71 us at 8192 rows (402 MB, 5.6 TB/s). All nine in flight take 75
+// registers and lose more in resident CTAs at the large size (85 us) than they gain at the small one (0.2 us). (Weights and
+// positions fetched before the dependency wait save 0.4 us of a launch, but hold only while the kernel that writes them
+// is two launches back.)
 constexpr int COMBINE_U = 5;
 constexpr int COMBINE_P = 33;  // most pairs per row (top_k <= 32, checked by the routing launcher, plus the shared expert)
 template <bool NORM>
@@ -128,12 +128,12 @@ moe_combine_kernel(const bf16* pair_out, const float* wts, const int* inv, int P
   __shared__ float s_w[COMBINE_P];
   __shared__ int s_pos[COMBINE_P];
   const int t = blockIdx.x;
-  if (threadIdx.x < P) {
-    s_w[threadIdx.x] = __ldcg(wts + static_cast<size_t>(t) * P + threadIdx.x);
-    s_pos[threadIdx.x] = __ldcg(inv + static_cast<size_t>(t) * P + threadIdx.x);
-  }
   pdl_wait();
   pdl_launch();
+  if (threadIdx.x < P) {
+    s_w[threadIdx.x] = wts[static_cast<size_t>(t) * P + threadIdx.x];
+    s_pos[threadIdx.x] = inv[static_cast<size_t>(t) * P + threadIdx.x];
+  }
   __syncthreads();
   float ss = 0.f;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
