@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 from ..obs import buildlog
+from ..utils.upload import to_device
 from . import torch_ops
 from .build import lib_path
 
@@ -519,9 +520,9 @@ def _memo(key, make):
 
 
 def _to_device(table: np.ndarray, dev) -> torch.Tensor:
-    """An int32 table on the device, by one asynchronous copy from pinned memory."""
+    """An int32 table on the device, by one copy from pinned memory that is complete on return."""
     t = torch.from_numpy(table.astype(np.int32))
-    return t.pin_memory().to(dev, non_blocking=True) if dev.type == "cuda" else t
+    return to_device(t.pin_memory(), dev) if dev.type == "cuda" else t
 
 
 def _gdn_prefill_meta(seg_starts, seg_slots, T: int, dev):
