@@ -73,10 +73,10 @@ class PackedBatch:
         tokens, positions, seq = (t.numpy() for t in h[:3])
         for i, (ts, p) in enumerate(zip(token_lists, pos0)):
             a, b = starts[i], starts[i + 1]
-            tokens[a:b] = array("q", ts)
+            tokens[a:b] = array("q", list(ts) if isinstance(ts, (bytes, bytearray)) else ts)  # bytes: one token each
             positions[a:b] = np.arange(p, p + b - a)
             seq[a:b] = i
-        h[3].numpy()[:] = slots
+        h[3].copy_(torch.as_tensor(slots, dtype=torch.int32))
         if with_table:
             h[4].copy_(block_tables)
         d = views(to_device(host, dev))

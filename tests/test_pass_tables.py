@@ -28,3 +28,12 @@ def test_batch_and_span_tables(lens):
     assert n_chunks == len(ref) and chunks.view(-1, 4).tolist() == ref
     assert per_seg.view(-1, 2).tolist() == [[sum(-(-m // 64) for m in lens[:i]), -(-lens[i] // 64)] for i in range(n)]
     assert seq.tolist() == b.seq_of_row.tolist() and st.tolist() == starts and slots.tolist() == b.seg_slots
+
+
+def test_batch_from_other_kinds_of_sequences():
+    """Tokens and slots in any container of whole numbers, bytes among them: one token per byte."""
+    table = torch.zeros(2, 4, dtype=torch.int32)
+    for toks in ([b"abcdefgh", bytearray(b"xyz")], [torch.arange(97, 105), (120, 121, 122)], [range(97, 105), [120, 121, 122]]):
+        for slots in ([4, 9], (4, 9), torch.tensor([4, 9])):
+            b = PackedBatch.prefill(toks, slots, [0, 64], table, "cpu")
+            assert b.tokens.tolist() == list(range(97, 105)) + [120, 121, 122] and b.slots.tolist() == [4, 9]
