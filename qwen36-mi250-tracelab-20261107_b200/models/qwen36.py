@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from ..config import PAGE_SIZE, ModelConfig
-from ..ops import torch_ops
+from ..ops import spans, torch_ops
 from ..utils.upload import to_device
 from .checkpoint import LayerWeights, Weights
 
@@ -44,43 +44,48 @@ class PackedBatch:
     seg_slots: list[int] | None = None
     seg_pos0: list[int] | None = None
     meta: object | None = None  # ragged prefill from fixed-shape device tables (``sched/graphs.py`` ``PrefillTables``)
+    tables: spans.SpanTables | None = None  # ragged prefill on a GPU: the span tables of the lists above, made with the batch
+
+    TILE_ROWS = 16  # positions per query tile of the attention kernel at eight query heads per key head
 
     @classmethod
     def prefill(cls, token_lists, slots, pos0, block_tables, device) -> "PackedBatch":
         """The index tensors of a ragged pass. On a CUDA device they are views of ONE buffer that one copy from pinned memory
         fills. A copy per tensor from pageable memory, five of them, each waited for everything launched before, so that the
         GPU stood still while the host built the next pass (a 61-row pass of 4 layers: 1.56 -> 1.42 ms). This one waits for
-        itself only (``utils.upload``): the batch may be run on any stream."""
+        itself only (``utils.upload``): the batch may be run on any stream. On a GPU the span tables travel with it."""
         dev = torch.device(device)
+        slots, pos0 = [int(s) for s in slots], [int(p) for p in pos0]
         starts = [0]
         for t in token_lists:
             starts.append(starts[-1] + len(t))
-        T, n = starts[-1], len(token_lists)
+        T, n = starts[-1], len(slots)
+        on_gpu = dev.type == "cuda"
         # a page table in host memory travels with the rest
         with_table = block_tables.device.type == "cpu" and block_tables.dtype == torch.int32
-        sizes = (T * 8, T * 8, T * 4, len(slots) * 4, block_tables.numel() * 4 if with_table else 0)
-        offs = [0]
-        for nbytes in sizes:
-            offs.append(offs[-1] + (nbytes + 15) // 16 * 16)
-        host = torch.empty(offs[-1], dtype=torch.uint8, pin_memory=dev.type == "cuda")
-
-        def views(buf):
-            v = [buf[o : o + nbytes] for o, nbytes in zip(offs, sizes)]
-            return (v[0].view(torch.int64), v[1].view(torch.int64), v[2].view(torch.int32), v[3].view(torch.int32),
-                    v[4].view(torch.int32).view(block_tables.shape) if with_table else None)
-
-        h = views(host)
-        tokens, positions, seq = (t.numpy() for t in h[:3])
+        # int32 words; whatever is read in larger pieces comes first
+        sizes = [2 * T, 2 * T, *(spans.words(starts, cls.TILE_ROWS) if on_gpu else [0] * 6), T, n,
+                 block_tables.numel() if with_table else 0]
+        host = torch.empty(sum(sizes), dtype=torch.int32, pin_memory=on_gpu)
+        h, at = [], 0
+        for k in sizes:
+            h.append(host.numpy()[at : at + k])
+            at += k
+        tokens, positions, seq = h[0].view(np.int64), h[1].view(np.int64), h[8]
         for i, (ts, p) in enumerate(zip(token_lists, pos0)):
             a, b = starts[i], starts[i + 1]
             tokens[a:b] = array("q", list(ts) if isinstance(ts, (bytes, bytearray)) else ts)  # bytes: one token each
             positions[a:b] = np.arange(p, p + b - a)
             seq[a:b] = i
-        h[3].copy_(torch.as_tensor(slots, dtype=torch.int32))
+        h[9][:] = slots
         if with_table:
-            h[4].copy_(block_tables)
-        d = views(to_device(host, dev))
-        return cls(d[0], d[1], d[2], d[3], d[4] if with_table else block_tables.to(dev), 0, starts, list(slots), list(pos0))
+            h[10][:] = block_tables.numpy().reshape(-1)
+        if on_gpu:
+            spans.write(h[2:8], starts, slots, pos0, cls.TILE_ROWS)
+        d = to_device(host, dev).split(sizes)
+        return cls(d[0].view(torch.int64), d[1].view(torch.int64), d[8], d[9],
+                   d[10].view(block_tables.shape) if with_table else block_tables.to(dev), 0, starts, slots, pos0,
+                   tables=spans.tables(d[2:8], d[8], starts, slots, pos0, cls.TILE_ROWS) if on_gpu else None)
 
     @classmethod
     def uniform(cls, tokens, positions, slots, block_tables, G: int, device) -> "PackedBatch":
@@ -179,6 +184,19 @@ class Model:
         sg = torch.sigmoid(ops.linear(x, lw.shared_gate, out_dtype=torch.float32))
         return out + (sg * shared.float()).to(x.dtype)
 
+    def _span_meta(self, batch: PackedBatch, kind: str) -> dict:
+        """The ``meta`` argument of a ragged pass's kernels: the captured pass's tables, or the ones that every layer of
+        this pass shares, built here for a batch that came without them (or whose lists have changed since)."""
+        if batch.G or (batch.meta is None and not getattr(self.ops, "SPAN_TABLES", False)):
+            return {}
+        if batch.meta is not None:
+            return {"meta": getattr(batch.meta, kind)}
+        group = self.cfg.num_attention_heads // self.cfg.num_key_value_heads
+        tile_rows = 128 // group if group in (1, 2, 4, 8) else None
+        if batch.tables is None or not batch.tables.of(batch.seg_starts, batch.seg_slots, batch.seg_pos0, tile_rows):
+            batch.tables = spans.span_tables(batch.seg_starts, batch.seg_slots, batch.seg_pos0, tile_rows, self.device)
+        return {"meta": getattr(batch.tables, kind)}
+
     def _attention(self, lw, kv_layer, h, batch: PackedBatch) -> torch.Tensor:
         cfg, ops = self.cfg, self.ops
         qkv = ops.linear(h, lw.in_proj)
@@ -186,7 +204,7 @@ class Model:
             qkv, batch.positions, batch.seq_of_row, batch.block_tables, kv_layer, lw.q_norm, lw.k_norm,
             cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.rotary_dim, cfg.rope_theta,
             cfg.rms_norm_eps, batch.G, batch.seg_starts, batch.seg_pos0,
-            **({} if batch.meta is None else {"meta": batch.meta.flash}),
+            **self._span_meta(batch, "flash"),
         )
         return self._out_proj(core, lw.out_proj)
 
@@ -199,8 +217,7 @@ class Model:
         )
         conv, rec = self.conv_state[gi], self.rec_state[gi]
         if batch.G == 0:
-            core = ops.gdn_prefill(mixed, batch.seg_starts, batch.seg_slots, conv, rec, *args,
-                                   **({} if batch.meta is None else {"meta": batch.meta.gdn}))
+            core = ops.gdn_prefill(mixed, batch.seg_starts, batch.seg_slots, conv, rec, *args, **self._span_meta(batch, "gdn"))
         else:
             r = None if ring is None else (ring[0][gi], ring[1][gi])
             core = ops.gdn_decode(mixed, batch.slots, conv, rec, *args, G=batch.G, ring=r)
@@ -293,12 +310,13 @@ class Model:
                 gi = self._gdn_index[i]
                 core = ops.gdn_prefill(mixed[:T], batch.seg_starts, batch.seg_slots, self.conv_state[gi], self.rec_state[gi],
                                        lw.conv_w, lw.A_log, lw.dt_bias, lw.gnorm_w, cfg.linear_num_key_heads,
-                                       cfg.linear_num_value_heads, cfg.linear_key_head_dim, cfg.linear_value_head_dim, eps)
+                                       cfg.linear_num_value_heads, cfg.linear_key_head_dim, cfg.linear_value_head_dim, eps,
+                                       **self._span_meta(batch, "gdn"))
             else:
                 core = ops.attention(mixed[:T], batch.positions, batch.seq_of_row, batch.block_tables,
                                      self.kv[self._kv_index[i]], lw.q_norm, lw.k_norm, cfg.num_attention_heads,
                                      cfg.num_key_value_heads, cfg.head_dim, cfg.rotary_dim, cfg.rope_theta, eps, 0,
-                                     batch.seg_starts, batch.seg_pos0)
+                                     batch.seg_starts, batch.seg_pos0, **self._span_meta(batch, "flash"))
             sp.gemm_reduce_scatter(pad(core), lw.out_proj)
             res, full = sp.reduce_norm_allgather(rpr, res, lw.post_norm, eps)
             logits = sp.gemm_gathered(full, lw.router, out_dtype=torch.float32)

@@ -15,13 +15,12 @@ import ctypes
 import time
 from ctypes import c_float, c_int, c_void_p
 
-import numpy as np
 import torch
 
 from ..obs import buildlog
-from ..utils.upload import to_device
 from . import torch_ops
 from .build import lib_path
+from .spans import span_tables
 
 _lib = None
 ATTN_Z = 32  # context lanes of the decode attention (fixed: part of the numerics contract)
@@ -154,6 +153,7 @@ SPLIT_K_ENABLED = __import__("os").environ.get("ENGINE_SPLIT_K", "0") == "1"
 # Gated DeltaNet prefill with head dims of 128: tcgen05 WY transform and state pass (ENGINE_GDN_TC=0 selects the fp32
 # CUDA-core kernels, which other head dims always use)
 GDN_PREFILL_TC = __import__("os").environ.get("ENGINE_GDN_TC", "1") == "1"
+SPAN_TABLES = True  # gdn_prefill and attention take the span tables of a ragged pass as `meta`
 
 
 def split_k(N: int, K: int, grouped: bool = False) -> int:
@@ -506,56 +506,16 @@ def ring_commit(conv_state, rec_state, ring, slots: torch.Tensor, keep_rows: tor
     _check(rc, "ring_commit")
 
 
-_meta_memo: dict = {}  # the span tables of the pass being run: every layer of a pass asks for the same ones
-
-
-def _memo(key, make):
-    """Single-entry memo per kind of table: the 40 layers of a prefill pass share one host build and one copy."""
-    hit = _meta_memo.get(key[0])
-    if hit is not None and hit[0] == key:
-        return hit[1]
-    val = make()
-    _meta_memo[key[0]] = (key, val)
-    return val
-
-
-def _to_device(table: np.ndarray, dev) -> torch.Tensor:
-    """An int32 table on the device, by one copy from pinned memory that is complete on return."""
-    t = torch.from_numpy(table.astype(np.int32))
-    return to_device(t.pin_memory(), dev) if dev.type == "cuda" else t
-
-
 def _gdn_prefill_meta(seg_starts, seg_slots, T: int, dev):
-    def make():
-        nseg = len(seg_slots)
-        starts = np.asarray(seg_starts, dtype=np.int64)
-        lens = np.diff(starts)
-        per_seg = (lens + 63) // 64
-        first = np.cumsum(per_seg) - per_seg
-        n_chunks = int(per_seg.sum())
-        seg = np.repeat(np.arange(nseg), per_seg)
-        nth = np.arange(n_chunks) - first[seg]
-        r0 = starts[seg] + 64 * nth
-        chunks = np.stack([seg, r0, np.minimum(64, starts[seg + 1] - r0), nth == 0], 1)
-        meta = _to_device(np.concatenate([chunks.reshape(-1), np.stack([first, per_seg], 1).reshape(-1),
-                                          np.repeat(np.arange(nseg), lens), starts, np.asarray(seg_slots)]), dev)
-        o = 0
-        chunks_t = meta[o : o + 4 * n_chunks]; o += 4 * n_chunks
-        segc_t = meta[o : o + 2 * nseg]; o += 2 * nseg
-        sor_t = meta[o : o + T]; o += T
-        start_t = meta[o : o + nseg + 1]; o += nseg + 1
-        slots_t = meta[o : o + nseg]
-        return n_chunks, chunks_t, segc_t, sor_t, start_t, slots_t
-
-    return _memo(("gdn", tuple(seg_starts), tuple(seg_slots), T, str(dev)), make)
+    return span_tables(seg_starts, seg_slots, [0] * len(seg_slots), None, dev).gdn[1:]
 
 
 def gdn_prefill(mixed, seg_starts, seg_slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnorm_w, n_k, n_v, dk,
                 dv, eps, meta=None) -> torch.Tensor:
     """Chunked prefill of the gated delta rule over packed spans (conv, WY transform, state scan, gated norm).
 
-    ``meta``: the span tables as device tensors that the caller keeps up to date (``PrefillTables.gdn``); the host
-    lists are then not read, which lets the call be captured in a CUDA graph."""
+    ``meta``: the span tables as device tensors that the caller keeps (``SpanTables.gdn``, ``PrefillTables.gdn``); the host
+    lists are then not read, which lets the call be captured in a CUDA graph. Without it every call builds them."""
     if dk != dv or dk not in (32, 64, 128) or conv_w.shape[1] != 4 or mixed.stride(0) % 8 or (n_k * dk) % 4:
         return torch_ops.gdn_prefill_batched(
             mixed, seg_starts, seg_slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnorm_w, n_k, n_v, dk, dv, eps
@@ -627,28 +587,20 @@ def flash_prefill(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, b
     """Causal gated attention of ragged prefill spans over the paged cache (tcgen05 flash kernel).
 
     ``q [T, n_q, D]`` normed and rotated; the spans' K/V are already in their pages. ``meta``: ``(rows per tile,
-    n_tiles, tiles [n_tiles, 4], pos0 [nseg])`` kept on the device by the caller (``PrefillTables.flash``; entries
-    with a span length of 0 are fillers that their CTAs skip); the host lists are then not read."""
+    n_tiles, tiles of 4 words each, pos0 [nseg])`` kept on the device by the caller (``SpanTables.flash``,
+    ``PrefillTables.flash``; entries with a span length of 0 are fillers that their CTAs skip); the host lists are then not
+    read. Without it every call builds them."""
     T, n_q, D = q.shape
     n_kv = kv_layer.shape[2]
     R = 128 // (n_q // n_kv)
     dev = q.device
-
-    def make():
-        starts = np.asarray(seg_starts, dtype=np.int64)
-        lens = np.diff(starts)
-        per_seg = (lens + R - 1) // R
-        seg = np.repeat(np.arange(len(lens)), per_seg)
-        p0 = R * (np.arange(len(seg)) - (np.cumsum(per_seg) - per_seg)[seg])
-        table = _to_device(np.concatenate([np.stack([seg, p0, starts[seg], lens[seg]], 1).reshape(-1), np.asarray(seg_pos0)]), dev)
-        return len(seg), table[: 4 * len(seg)].view(-1, 4), table[4 * len(seg) :]
 
     if meta is not None:
         r_meta, n_tiles, tiles_t, pos0_t = meta
         if r_meta != R:
             raise ValueError(f"flash_prefill: the tile table was built for {r_meta} positions per tile, the kernel takes {R}")
     else:
-        n_tiles, tiles_t, pos0_t = _memo(("flash", tuple(seg_starts), tuple(seg_pos0), R, str(dev)), make)
+        _, n_tiles, tiles_t, pos0_t = span_tables(seg_starts, [0] * len(seg_pos0), seg_pos0, R, dev).flash
     out = torch.empty(T, n_q * D, dtype=q.dtype, device=dev)
     rc = lib().b200_flash_prefill(
         _ptr(q), _ptr(gate), _ptr(kv_layer), _ptr(out), _ptr(tiles_t), n_tiles, _ptr(pos0_t), _ptr(block_tables),

@@ -13,16 +13,18 @@ def to_device(host: torch.Tensor, device: torch.device) -> torch.Tensor:
     with. Refused inside a graph capture: a replay would copy from host memory that has been given away since."""
     if device.type != "cuda":
         return host.to(device)
-    current = torch.cuda.current_stream(device)
-    with torch.cuda.stream(current):
+    with torch.cuda.device(device):
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("host tables cannot be copied inside a graph capture: make them before it")
-    index = current.device_index
-    copy = _streams.get(index)
-    if copy is None:
-        copy = _streams[index] = torch.cuda.Stream(device=current.device)
-    with torch.cuda.stream(copy):
-        out = host.to(current.device, non_blocking=True)
-    copy.synchronize()
-    out.record_stream(current)  # the memory is the copy stream's: not reused before the current stream is done with it
+        current = torch.cuda.current_stream()
+        copy = _streams.get(current.device_index)
+        if copy is None:
+            copy = _streams[current.device_index] = torch.cuda.Stream()
+        torch.cuda.set_stream(copy)
+        try:
+            out = host.to(copy.device, non_blocking=True)
+        finally:
+            torch.cuda.set_stream(current)
+        copy.synchronize()
+        out.record_stream(current)  # the memory is the copy stream's: not reused before the current stream is done with it
     return out

@@ -64,3 +64,45 @@ def test_batch_under_capture_is_refused():
             _batch(2)
     graph.replay()
     assert x.tolist() == [1.0] * 4
+
+
+@pytest.mark.parametrize("heads", [8, 4])  # query heads of the one key head: the batch's own tile table, and one built on demand
+def test_captured_pass_keeps_its_tables_while_other_passes_run(heads):
+    from b200serve.config import ModelConfig
+    from b200serve.models.checkpoint import random_weights
+    from b200serve.models.qwen36 import Model, PackedBatch
+    from b200serve.ops import cuda_ops
+
+    cfg = ModelConfig.tiny(num_attention_heads=heads, head_dim=64)
+    model = Model(random_weights(cfg, seed=0, device="cuda", dtype=torch.bfloat16, std=0.05), 40, 6, ops=cuda_ops)
+    toks = torch.randint(0, cfg.vocab_size, (400,), generator=torch.Generator().manual_seed(3)).tolist()
+    table = torch.arange(1, 29, dtype=torch.int32).view(4, 7)
+
+    def run(spans, batch=None):
+        model.conv_state.zero_()
+        model.rec_state.zero_()
+        model.kv.zero_()
+        batch = batch or PackedBatch.prefill([toks[a:b] for a, b in spans], list(range(1, len(spans) + 1)), [0] * len(spans),
+                                             table[: len(spans)], "cuda")
+        return model.forward(batch), batch
+
+    spans, others = [(0, 70), (10, 11), (5, 135)], [[(0, 300)], [(0, 20), (20, 150)], [(3, 9), (9, 100), (0, 1), (7, 77)]]
+    want, batch = run(spans)
+    want = want.clone()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got, _ = run(spans, batch)
+    alone = [run(s)[0].clone() for s in others]
+    graph.replay()
+    assert torch.equal(got, want)
+    for s, h in zip(others, alone):  # and two passes in turn on two streams
+        a = torch.cuda.Stream()
+        a.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(a):
+            again, _ = run(s)
+        torch.cuda.current_stream().wait_stream(a)
+        assert torch.equal(again, h)
+    graph.replay()
+    assert torch.equal(got, want)
+    cuda_ops.check_errors(got.device)
