@@ -45,20 +45,11 @@ __device__ __forceinline__ void route_row(const float* row, int E, int top_k, in
       const int e = i * 32 + lane;
       if (v[i] > bm) { bm = v[i]; be = e; }  // ascending e within a lane: first maximum kept
     }
-#ifdef B200_EMU
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float om = __shfl_xor_sync(0xffffffffu, bm, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-      if (om > bm || (om == bm && oe < be)) { bm = om; be = oe; }
-    }
-#else
     // Largest value, then lowest id among the lanes that hold it, as two warp reductions: the values are -1 or not negative
     // and never NaN here (a NaN loses every comparison above), so they order like their bits.
     const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bm));
     be = __reduce_min_sync(0xffffffffu, __float_as_int(bm) == top ? be : 0x7fffffff);
     bm = __int_as_float(top);
-#endif
 #pragma unroll
     for (int i = 0; i < PER_LANE; ++i)
       if (i * 32 + lane == be) v[i] = -1.0f;  // remove the winner (static indexing keeps v in registers)

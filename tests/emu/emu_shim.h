@@ -109,6 +109,16 @@ inline T __shfl_up_sync(unsigned, T v, int delta) {
   std::memcpy(&v, &f, sizeof f);
   return v;
 }
+inline int __float_as_int(float v) { int i; std::memcpy(&i, &v, sizeof i); return i; }
+inline float __int_as_float(int v) { float f; std::memcpy(&f, &v, sizeof f); return f; }
+inline int __reduce_max_sync(unsigned mask, int v) {
+  for (int o = 16; o > 0; o >>= 1) v = std::max(v, __shfl_xor_sync(mask, v, o));
+  return v;
+}
+inline int __reduce_min_sync(unsigned mask, int v) {
+  for (int o = 16; o > 0; o >>= 1) v = std::min(v, __shfl_xor_sync(mask, v, o));
+  return v;
+}
 inline int atomicAdd(int* p, int v) { return std::atomic_ref<int>(*p).fetch_add(v); }
 inline unsigned atomicAdd(unsigned* p, unsigned v) { return std::atomic_ref<unsigned>(*p).fetch_add(v); }
 inline int atomicCAS(int* p, int expect, int v) {

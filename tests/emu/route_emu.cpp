@@ -79,6 +79,32 @@ int main() {
     for (int k = 0; k < K; ++k)
       if (idx[1 * (K + 1) + k] != (use_map ? map[k] : k)) { std::printf("tied row picked %d at %d\n", idx[1 * (K + 1) + k], k); ++bad; }
   }
+  // Infinities and NaN: an expert whose probability is NaN is never picked, ties among zeros go to the lower id, and a row
+  // without any probability names no expert (an index that the plan refuses).
+  {
+    const float inf = INFINITY, nan = std::nanf("");
+    struct Row { const char* what; std::function<float(int)> logit; std::vector<int> want; bool weights; };
+    const std::vector<Row> rows = {
+        {"one NaN", [&](int e) { return e == 40 ? nan : static_cast<float>(E - e) * 0.01f; }, {0, 1, 2, 3, 4, 5, 6, 7}, true},
+        {"NaN in front", [&](int e) { return e < 3 ? nan : static_cast<float>(E - e) * 0.01f; }, {3, 4, 5, 6, 7, 8, 9, 10}, true},
+        {"ten finite", [&](int e) { return e % 25 == 7 ? static_cast<float>(e) * 0.01f : -inf; }, {232, 207, 182, 157, 132, 107, 82, 57}, true},
+        {"three finite", [&](int e) { return e == 9 || e == 70 || e == 200 ? 1.f : -inf; }, {9, 70, 200, 0, 1, 2, 3, 4}, true},
+        {"one infinite", [&](int e) { return e == 2 ? inf : 0.f; }, {0, 1, 3, 4, 5, 6, 7, 8}, false},
+        {"all -infinite", [&](int) { return -inf; }, std::vector<int>(K, 0x7fffffff), false},
+        {"all NaN", [&](int) { return nan; }, std::vector<int>(K, 0x7fffffff), false}};
+    for (const Row& r : rows) {
+      std::vector<float> row(E + 1, 0.f), wts(K + 1, -1.f);
+      std::vector<int> idx(K + 1, -7);
+      for (int e = 0; e < E; ++e) row[e] = r.logit(e);
+      run_cta(32, 0, 0, [&] { route_row<PER_LANE>(row.data(), E, K, 1, wts.data(), idx.data(), nullptr, nullptr, static_cast<int>(threadIdx.x)); });
+      float tot = 0.f;
+      for (int k = 0; k < K; ++k) {
+        tot += wts[k];
+        if (idx[k] != r.want[k]) { std::printf("%s: pick %d is %d, want %d\n", r.what, k, idx[k], r.want[k]); ++bad; }
+      }
+      if (r.weights && !(std::fabs(tot - 1.f) < K / 256.f)) { std::printf("%s: the weights add up to %f\n", r.what, tot); ++bad; }
+    }
+  }
   if (bad) return 1;
   std::printf("OK route_row: %d rows x top-%d of %d experts, with and without a local expert map\n", ROWS, K, E);
   return 0;
