@@ -426,7 +426,7 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
     if bt == 64 and not _MOE_BT_FIXED and GATHER_MAX_BT >= 128 and T * top_k >= WIDE_MIN_ROWS * n_experts:
         bt = 128
     # the gate/up GEMM fetches each activation row by index, so no expert-sorted copy of x is made
-    gather = bt <= GATHER_MAX_BT and x.stride(0) % 8 == 0 and x.stride(1) == 1
+    gather = bt <= GATHER_MAX_BT and x.stride(0) % 8 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0
     src_rows = ints[Et + 2 + 2 * n_pairs :] if gather else None
     max_tiles = min(Et, n_pairs) + n_pairs // bt + 1
     tiles = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
@@ -447,6 +447,8 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
                                    EPI_SILU_MUL, inter, bt, _ptr(tiles), _ptr(n_tiles), max_tiles, _ptr(err), 1,
                                    is_packed(w_gate_up), _ptr(src_rows), x.stride(0), st), "gemm_grouped(gate_up, gather)")
     else:
+        if not x.is_contiguous() or x.data_ptr() % 16:  # the copy kernel takes whole rows, 16 bytes at a time
+            x = x.clone(memory_format=torch.contiguous_format)
         xs = torch.empty(n_pairs, H, dtype=x.dtype, device=dev)
         _check(L.b200_moe_gather(_ptr(x), _ptr(perm), _ptr(offsets[Et:]), n_pairs, T, Pn, H, _ptr(xs), st), "moe_gather")
         _check(L.b200_gemm_grouped(_ptr(xs), _ptr(w_gate_up), _ptr(act), n_pairs, Et, inter, 2 * inter, H, inter,

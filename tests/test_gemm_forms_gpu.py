@@ -97,3 +97,17 @@ def test_routing_and_plan_of_tied_rows(C, T, E, k):
     assert torch.equal(offsets.long(), torch.nn.functional.pad(table.flatten().bincount(minlength=E + 1).cumsum(0), (1, 0)))
     assert torch.equal(perm.long().sort().values, torch.arange(T * P, device=dev)) and torch.equal(perm[inv.long()].long(), torch.arange(T * P, device=dev))
     assert torch.equal(table.flatten()[perm.long()], table.flatten().sort().values) and torch.equal(src, perm // P)
+
+
+@pytest.mark.parametrize("T", [5, 300, 700])
+def test_expert_block_of_rows_that_are_further_apart(C, T):
+    """Row strides and starts that the in-GEMM row fetch does not take: the same rows, copied first."""
+    E, k, H, I = 16, 4, 256, 128
+    router, gu, dn = _bf(E + 1, H, scale=0.3, seed=2), _bf(E + 1, 2 * I, H, scale=0.05, seed=3), _bf(E + 1, H, I, scale=0.05, seed=4)
+    wide = _bf(T * (H + 16) + 8, seed=T)
+    for stride, start in ((H, 0), (H + 8, 0), (H + 4, 0), (H + 1, 0), (H + 8, 1), (H, 3)):
+        x = wide[start:].as_strided((T, H), (stride, 1))
+        rows = x.clone(memory_format=torch.contiguous_format)
+        want, logits = C.moe_block(rows, router, gu, dn, E, k, True), C.linear(rows, router, out_dtype=torch.float32)
+        assert torch.equal(C.moe_block(x, router, gu, dn, E, k, True, logits=logits), want), (stride, start)
+    C.check_errors(wide.device)
