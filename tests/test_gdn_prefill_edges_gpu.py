@@ -119,3 +119,22 @@ def test_norm_weights_that_start_at_any_element(C, d):
         flat = torch.zeros(d + 8, dtype=torch.bfloat16, device="cuda")
         flat[off:off + d] = par[3]
         assert torch.equal(_prefill(C, mixed, [0, T], (*par[:3], flat[off:off + d]), n_k, n_v, d, state.clone())[2], want)
+
+
+@pytest.mark.parametrize("d", [32, 128])
+def test_conv_of_large_passes_has_the_bits_of_small_ones(C, d):
+    """From 4096 rows on the conv runs over 16 rows, below over 8: spans that start and end inside such a run, a last run that
+    is not full, a span that leaves a state of its own rows and one that is shorter than the window."""
+    n_k, n_v, lens = 2, 4, [1, 3, 17, 2, 4070, 5, 64, 9]
+    par, ch = _params(n_k, n_v, d), 2 * n_k * d + n_v * d
+    starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    T = starts[-1]
+    assert T > 4096 and T % 16
+    mixed, state = _bf(T, ch + n_v * d + 2 * n_v, seed=9), _bf(len(lens) + 1, ch, 3, seed=10)
+    whole_state = state.clone()
+    whole, _, _ = _prefill(C, mixed, starts, par, n_k, n_v, d, whole_state)
+    for i, (a, b) in enumerate(zip(starts, starts[1:])):
+        own = torch.stack([state[0], state[1 + i]])
+        part, _, _ = _prefill(C, mixed[a:b].clone(), [0, b - a], par, n_k, n_v, d, own)
+        assert torch.equal(whole[a:b], part), i
+        assert torch.equal(whole_state[1 + i], own[1]), i

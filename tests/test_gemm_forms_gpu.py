@@ -111,3 +111,20 @@ def test_expert_block_of_rows_that_are_further_apart(C, T):
         want, logits = C.moe_block(rows, router, gu, dn, E, k, True), C.linear(rows, router, out_dtype=torch.float32)
         assert torch.equal(C.moe_block(x, router, gu, dn, E, k, True, logits=logits), want), (stride, start)
     C.check_errors(wide.device)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(600, 16, 4, 256, 128), (515, 8, 2, 512, 192), (3, 8, 2, 512, 128)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_wide_expert_tiles_through_the_tensor_map(C, T, E, k, H, I, packed, monkeypatch):
+    """128-row tiles whose rows come from the expert-sorted copy (the second row-fetching warp has nothing to do)."""
+    x = _bf(T, H, seed=T)
+    router = _bf(E + 1, H, scale=0.3, seed=34)
+    wgu, wd = _bf(E + 1, 2 * I, H, scale=0.05, seed=35), _bf(E + 1, H, I, scale=0.05, seed=36)
+    if packed:
+        wgu, wd = C.pack_weight(wgu, gate_up=True), C.pack_weight(wd)
+    want = C.moe_block(x, router, wgu, wd, E, k, True)
+    monkeypatch.setattr(C, "_MOE_BT_FIXED", 128)
+    assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)  # rows by index
+    monkeypatch.setattr(C, "GATHER_MAX_BT", 64)
+    assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
+    C.check_errors(x.device)

@@ -136,3 +136,32 @@ def test_flash_pages_of_growing_scores(C, n_q, n_kv, D, pos0, n):
     ref = O.paged_attention(q.float(), gate.float(), kv.float(), table, [0, n], [pos0])
     # probabilities, output and gated output are rounded to bf16 (2^-8 each), on values of up to about four
     assert (got.float() - ref).abs().max().item() <= 3 * 2.0 ** -8 * 5
+
+
+@pytest.mark.parametrize("T", [1, 16, 17, 130, 256])
+@pytest.mark.parametrize("V", [200, 1000, 66000])
+def test_greedy_head_with_infinite_and_undefined_logits(C, T, V):
+    """Rows whose largest logit is infinite, rows of minus infinity but for one id, and rows of NaN beside ordinary ones."""
+    w = _whole(V, 64, seed=V)
+    w[:, 0] = 0.0
+    high = torch.tensor([5, 127, 128, V - 1], device="cuda") % V
+    w[high, 0] = float("inf")
+    x = _whole(T, 64, seed=T)
+    x[:, 0] = torch.tensor([1.0, -1.0, 2.0], device="cuda").repeat(T // 3 + 1)[:T]  # +inf or -inf at `high`
+    if T > 2:
+        x[T // 2] = float("nan")
+    logits = x.double() @ w.double().t()
+    top = logits.amax(1, keepdim=True)
+    first = torch.where(logits == top, torch.arange(V, device="cuda"), V).amin(1)
+    idx, val = C.lm_head_argmax(x, w, return_value=True)
+    ok = ~torch.isnan(x).any(1)
+    assert torch.equal(idx[ok], first[ok]) and torch.equal(val[ok].double(), top[ok, 0])
+    assert (idx[~ok] >= V).all()  # no id: the embedding of such a row sets the error word
+    w[:, 0] = float("inf")  # every logit minus infinity: the lowest id
+    x[:, 0] = -1.0
+    assert (C.lm_head_argmax(x[: max(1, T // 2)], w) == 0).all()
+
+
+def _whole(rows, cols, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randint(-2, 3, (rows, cols), device="cuda", generator=g).bfloat16()
