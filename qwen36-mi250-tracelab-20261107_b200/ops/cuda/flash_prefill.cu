@@ -68,7 +68,7 @@ struct FlashCfg {
   static constexpr int P_BYTES = DEC ? 1024 : 128 * 128;  // one probability tile; two are kept
   static constexpr int ST = DEC ? 3 : 2;        // K/V stages
   // dynamic shared memory is declared 1024-byte aligned (checked at run time), so no alignment slack is budgeted:
-  // with D = 256 the tiles, the barriers and the 2 KB of static exchange arrays fill the 227 KB of an SM
+  // with D = 256 the tiles, the barriers and 512 bytes of static arrays fill the 227 KB of an SM
   static constexpr int SMEM = Q_BYTES + 2 * ST * KV_BYTES + 2 * P_BYTES + 256;
   static constexpr int ROW_WARPS = DEC ? 1 : 4;  // softmax warps per page: the decode form's 8 rows are one warp's
   static constexpr int TMEM_COLS = (128 + D) <= 256 ? 256 : 512;  // two score tiles of 64 columns + the output

@@ -153,7 +153,7 @@ __device__ __forceinline__ void bulk_prefetch(const void* gsrc, uint32_t bytes) 
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 #endif
 
-constexpr int STEP_AHEAD = 148;
+constexpr int STEP_AHEAD = 148;  // the SMs of the one chip that this is built for
 template <int DK, int DV>
 __global__ void __launch_bounds__(4 * DV, 3)
 gdn_step_kernel(const bf16* conv_out,   // [B*G, C]  q | k | v after conv+silu

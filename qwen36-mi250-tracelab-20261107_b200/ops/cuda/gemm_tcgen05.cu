@@ -10,7 +10,8 @@
 // reference gets the same property from fixed GEMV tiles, engine/fast/mfma.py:6-11, 60-71).
 //
 // Pipeline per CTA (192 threads): warp 0 = TMA producer, warp 1 = tcgen05.mma issuer and TMEM
-// owner, warps 2..5 = epilogue (one TMEM lane quarter each). Operand tiles are 64 bf16 wide
+// owner, warps 2..5 = epilogue (one TMEM lane quarter each); the 128-row gate/up tiles have a seventh warp that
+// fetches half of the rows by index. Operand tiles are 64 bf16 wide
 // (128 bytes, TMA 128B swizzle), STAGES deep, guarded by full/empty mbarriers; tcgen05.commit
 // releases a stage when the MMAs that read it have finished. No cluster multicast is used.
 //
@@ -55,7 +56,7 @@ struct GemmParams {
   int y_rot;         // dense sequence-parallel GEMMs: token tile = (blockIdx.y + y_rot) % gridDim.y, so that each rank
                      // starts with the tiles whose data (or whose consumer) is furthest from being the bottleneck
   int grid_y;        // dense: number of token tiles (set by the launcher)
-  const int* gather_rows;  // grouped, token tiles <= 64 rows: sorted position -> row of `gx`; the producer warp then
+  const int* gather_rows;  // grouped, token tiles <= GATHER_BT_MAX rows: sorted position -> row of `gx`; the producer warp then
                      // fetches each activation row by index (16-byte async copies into the swizzled operand layout)
                      // instead of reading an expert-sorted copy through the tensor map
   const bf16* gx;    // gather source [rows, ldgx]
@@ -828,7 +829,7 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   return {T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256, BM, 1};
 }
 
-// Thin dense launch; 1 when the form is the plain one.
+// Launch of a thin dense form; -5 where there is no such form.
 template <int EPI>
 static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, GemmParams p, int ldx, cudaStream_t st) {
   CUtensorMap tw, tx;
@@ -885,8 +886,9 @@ extern "C" int b200_pick_bt(int T) {
   return 256;
 }
 
-// Dense: out[T, N] = X[T, K] W[N, K]^T. bt <= 0: the launcher picks the form, otherwise the token tile is `bt` rows.   epi: 0 bf16, 1 fp32, 2 silu(gate)*up (N = rows of each half, W has 2N rows
-// with the up half at row `up_offset`), 3 argmax partials (part_max/part_idx sized [ceil(N/128), T]).
+// Dense: out[T, N] = X[T, K] W[N, K]^T. bt <= 0: the launcher picks the form, otherwise the token tile is `bt` rows.
+// epi: 0 bf16, 1 fp32, 2 silu(gate)*up (N = rows of each half, W has 2N rows with the up half at row `up_offset`),
+// 3 argmax partials (part_max/part_idx sized [ceil(N/128), T]).
 extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, int N, int K, int ldx, int ldw, int ldo,
                                int epi, int up_offset, int bt, float* part_max, int* part_idx, int* err,
                                int splits, int packed, cudaStream_t st) {
@@ -923,7 +925,7 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
                                  int ldo, int epi, int up_offset, int bt, const void* tiles, const int* n_tiles,
                                  int max_tiles, int* err, int splits, int packed, const int* gather_rows, int ldx,
                                  cudaStream_t st) {
-  // gather_rows != null (token tiles of at most 64 rows): X is [any rows, ldx] and sorted position i reads row
+  // gather_rows != null (token tiles of at most GATHER_BT_MAX rows): X is [any rows, ldx] and sorted position i reads row
   // gather_rows[i] of it; otherwise X is the expert-sorted buffer [cap, K] itself.
   if (max_tiles <= 0) return 0;
   if (gather_rows != nullptr && (bt > GATHER_BT_MAX || splits > 1 || ldx % 8)) return -7;

@@ -376,18 +376,29 @@ def moe_bt(T: int, pairs_per_row: int, n_experts: int) -> int:
     for bt in (16, 32, 64):
         if per <= bt:
             return bt
-    # many rows per expert (prefill): 64-row tiles waste less on each expert's last tile than 128-row ones and run two
-    # CTAs per SM (measured at 8192 rows, ~256 per expert: 970 us for the block against 1002 us with 128-row tiles)
+    # many rows per expert (prefill): 64-row tiles waste less on each expert's last tile than 128-row ones whose MMAs take
+    # all 128 columns, and run two CTAs per SM (8192 rows, ~256 per expert: 970 us for the block against 1002 us)
     return 64
 
 
 # widest token tile whose rows the gate/up GEMM fetches by index (0 turns the in-GEMM row gather off): no expert-sorted copy
 # of x at any size (8 x 1024 tokens, 4 layers: 7.52 -> 7.29 ms per pass)
 GATHER_MAX_BT = int(__import__("os").environ.get("ENGINE_MOE_GATHER_BT", "128"))
-# expected rows per routed expert from which the expert GEMMs take 128-row tiles, whose MMAs cover the rows they have: two
-# such tiles replace four of 64 rows (8192 rows, 256 per expert: gate/up 496 -> 365 us, down 239 -> 246). At 64 rows per
-# expert both forms need about one tile (207 and 204 us, 99 and 101 us).
+# expected rows per routed expert from which the expert GEMMs of ``moe_block`` take 128-row tiles, whose MMAs cover the rows
+# they have: two such tiles replace four of 64 rows (8192 rows, 256 per expert: gate/up 496 -> 365 us; down 239 -> 246, but
+# both GEMMs walk one tile table). At 64 rows per expert both forms need about one tile (207 and 204 us, 99 and 101 us).
 WIDE_MIN_ROWS = 96
+
+
+def block_bt(T: int, top_k: int, pairs_per_row: int, n_experts: int) -> int:
+    """Token-tile width of ``moe_block``: ``moe_bt``'s, or 128 rows where the rows are enough and fetched by index. (The
+    expert-parallel block keeps ``moe_bt``: its scatter epilogue has no MMAs that follow the row count.)"""
+    bt = moe_bt(T, pairs_per_row, n_experts)
+    if bt == 64 and not _MOE_BT_FIXED and GATHER_MAX_BT >= 128 and T * top_k >= WIDE_MIN_ROWS * n_experts:
+        return 128
+    return bt
+
+
 FUSED_MOE_NORM = True  # Model._moe_norm: combine + residual add + next RMSNorm as one kernel
 ROUTE_PLAN_SPLIT = __import__("os").environ.get("ENGINE_ROUTE_PLAN_SPLIT", "0") == "1"  # routing and plan as two launches
 ROUTE_PLAN_MAX_ROWS = 32  # up to one row per warp of a single CTA, routing and the expert plan run as one launch
@@ -422,9 +433,7 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
     ints = torch.empty(Et + 2 + 3 * n_pairs, dtype=torch.int32, device=dev)
     offsets, n_tiles = ints[: Et + 1], ints[Et + 1 : Et + 2]
     perm, inv = ints[Et + 2 : Et + 2 + n_pairs], ints[Et + 2 + n_pairs : Et + 2 + 2 * n_pairs]
-    bt = moe_bt(T, Pn, n_experts)
-    if bt == 64 and not _MOE_BT_FIXED and GATHER_MAX_BT >= 128 and T * top_k >= WIDE_MIN_ROWS * n_experts:
-        bt = 128
+    bt = block_bt(T, top_k, Pn, n_experts)
     # the gate/up GEMM fetches each activation row by index, so no expert-sorted copy of x is made
     gather = bt <= GATHER_MAX_BT and x.stride(0) % 8 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0
     src_rows = ints[Et + 2 + 2 * n_pairs :] if gather else None

@@ -61,7 +61,7 @@ def _lib():
 
 class EpMoE:
     # widest token tile whose rows the gate/up GEMM fetches by index from the receive buffer; wider tiles (prefill-size
-    # blocks) are compacted into expert order first. The local block gathers up to 64 rows; here the 32-row form is the
+    # blocks) are compacted into expert order first. The local block gathers up to 128 rows; here the 32-row form is the
     # one measured on 2 and 4 GPUs.
     GATHER_MAX_BT = 32
 
