@@ -294,10 +294,10 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
   for (int w = 0; w < WARPS; ++w) { m = fmaxf(m, s_max[w]); last = max(last, s_last[w]); }
   const bool few = last <= COMBINE_GROUPS;
   const float4* pa = reinterpret_cast<const float4*>(part_acc + head * Z * D) + quad;
-  float l[GPT];
+  float l[GPT], f[GPT];  // f, few: the factor of the sum's one partial, applied when it is added
   float4 acc[GPT];
 #pragma unroll
-  for (int u = 0; u < GPT; ++u) { l[u] = 0.f; acc[u] = make_float4(0.f, 0.f, 0.f, 0.f); }
+  for (int u = 0; u < GPT; ++u) { l[u] = f[u] = 0.f; acc[u] = make_float4(0.f, 0.f, 0.f, 0.f); }
 #pragma unroll 2
   for (int z0 = g0; z0 < last; z0 += COMBINE_GROUPS) {
     float2 pm[GPT];
@@ -311,7 +311,8 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
 #pragma unroll
     for (int u = 0; u < GPT; ++u) {
       if (pm[u].x == -INFINITY) continue;
-      const float sc = few ? 1.f : __expf(pm[u].x - m);  // few: one partial per sum, scaled when it is added
+      f[u] = __expf(pm[u].x - m);
+      const float sc = few ? 1.f : f[u];
       l[u] += pm[u].y * sc;
       acc[u].x += v[u].x * sc; acc[u].y += v[u].y * sc; acc[u].z += v[u].z * sc; acc[u].w += v[u].w * sc;
     }
@@ -319,16 +320,18 @@ attn_combine_kernel(const float* part_acc, const float* part_ml, const bf16* gat
 #pragma unroll
   for (int u = 0; u < GPT; ++u) {
     *reinterpret_cast<float4*>(&s_acc[g0 + u][quad * 4]) = acc[u];
-    if (quad == 0) {
-      s_l[g0 + u] = l[u];
-      s_f[g0 + u] = !few ? 1.f : g0 + u < last ? __expf(ml[g0 + u].x - m) : 0.f;
-    }
+    if (quad == 0) { s_l[g0 + u] = l[u]; s_f[g0 + u] = f[u]; }
   }
   __syncthreads();
   for (int d = threadIdx.x; d < D; d += THREADS) {
     float ls = 0.f, o = 0.f;
+    if (few) {
 #pragma unroll
-    for (int g = 0; g < COMBINE_GROUPS; ++g) { ls = fmaf(s_l[g], s_f[g], ls); o = fmaf(s_acc[g][d], s_f[g], o); }
+      for (int g = 0; g < COMBINE_GROUPS; ++g) { ls = fmaf(s_l[g], s_f[g], ls); o = fmaf(s_acc[g][d], s_f[g], o); }
+    } else {
+#pragma unroll
+      for (int g = 0; g < COMBINE_GROUPS; ++g) { ls += s_l[g]; o += s_acc[g][d]; }
+    }
     out[head * D + d] = gated(o / ls, gate[head * D + d]);
   }
 }
