@@ -67,9 +67,9 @@ class PackedBatch:
         sizes = [2 * T, 2 * T, *(spans.words(starts, cls.TILE_ROWS) if on_gpu else [0] * 6), T, n,
                  block_tables.numel() if with_table else 0]
         host = torch.empty(sum(sizes), dtype=torch.int32, pin_memory=on_gpu)
-        h, at = [], 0
+        words, h, at = host.numpy(), [], 0
         for k in sizes:
-            h.append(host.numpy()[at : at + k])
+            h.append(words[at : at + k])
             at += k
         tokens, positions, seq = h[0].view(np.int64), h[1].view(np.int64), h[8]
         for i, (ts, p) in enumerate(zip(token_lists, pos0)):
