@@ -66,6 +66,7 @@ struct GemmParams {
   int w_tiles;       // packed: weight tiles per expert
   int x_rows;        // dense, not thin: rows per activation box (0: the token tile). With a single token tile it is the row
                      // count rounded up to 16: the MMA covers and shared memory takes no more columns than there are rows
+  int pair_bt;       // gemm_pair_kernel, dense: token rows per tile
 };
 
 // RT: weight rows per tile. 128 fills the MMA's M; the thin forms (64, 32) load that many rows into the first rows of the
@@ -637,6 +638,10 @@ __global__ void argmax_finish_kernel(const float* part_max, const int* part_idx,
   }
 }
 
+}  // namespace b200
+#include "gemm_pair.cuh"
+namespace b200 {
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -829,6 +834,83 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   return {T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256, BM, 1};
 }
 
+constexpr int PAIR_FORM = -256;  // token tile of up to 256 rows on two SMs, in the `bt` argument of the launchers
+
+// Two SMs per tile (gemm_pair.cuh). A cluster's CTAs sit on one SM each; the persistent grid is one cluster per pair of SMs.
+template <int EPI, bool GROUPED>
+static int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, GemmParams p, int grid_y, cudaStream_t st) {
+  auto kern = gemm_pair_kernel<EPI, GROUPED>;
+  static bool configured[MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return -3;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) return -3;
+    configured[dev] = true;
+  }
+  p.grid_y = grid_y;
+  const int rows = EPI == EPI_SILU_MUL ? BM : 2 * BM;
+  const long long tiles = static_cast<long long>((p.N + rows - 1) / rows) * grid_y, pairs = sm_count() / 2;
+  return launch_clusters(2, kern, dim3(2 * static_cast<unsigned>(tiles < pairs ? tiles : pairs)), dim3(pair_threads(EPI)), PAIR_SMEM,
+                         st, tw, tx, p) == cudaSuccess ? 0 : -4;
+}
+
+// What the pair form asks of a launch: whole k-blocks, and output rows that leave in 16-byte pieces.
+static bool pair_takes(const GemmParams& p) {
+  return p.K % BK == 0 && p.N % 8 == 0 && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+}
+
+// Token rows per tile of a dense launch: the fewest cycles over the waves of the persistent grid. A k-block of bt rows takes an
+// SM 2 bt cycles of MMA, and its 16 KB of weights and 64 bt bytes of rows 256 + bt cycles out of L2.
+static int pair_rows(int T, int N) {
+  const long long n = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count() / 2;
+  int best = PAIR_BT;
+  long long least = -1;
+  for (int bt = PAIR_BT; bt >= PAIR_N_STEP; bt -= PAIR_N_STEP) {
+    const long long waves = (n * ((T + bt - 1) / bt) + pairs - 1) / pairs, cost = waves * (2 * BM + bt);
+    if (least < 0 || cost < least) { least = cost; best = bt; }
+  }
+  return best;
+}
+
+// Whether a dense launch is better off with two SMs per tile, us, best other form -> pair, weights not in L2 (about 10 us of
+// each is the measurement's own):
+//   rows    129           256           257           512           1024          2048          8192
+//   12352   26.7 -> 22.5  26.6 -> 24.6  34.8 -> 29.4  40.9 -> 32.8  53.3 -> 47.1  88.1 -> 75.8  277 -> 253
+//   9216    24.6 -> 21.3  26.7 -> 23.6  27.6 -> 23.6  27.5 -> 25.3  41.0 -> 36.9  63.5 -> 57.3  203 -> 186
+//   2048    20.5 -> 22.5  23.5 -> 22.6  35.8 -> 22.6  35.5 -> 23.3  36.9 -> 24.6  36.9 -> 32.8  113 -> 86
+// (12352 and 9216 x 2048, 2048 x 4096). A single pair of weight tiles would leave half of one idle below 256 columns.
+static bool pair_pays(int T, int N) { return N >= 2 * BM && (T > 256 || (T > 128 && N > 32 * BM)); }
+
+// Dense bf16 GEMM with two SMs per tile.
+static int launch_pair_dense(const void* X, const void* W, GemmParams p, int ldx, int ldw, int packed, cudaStream_t st) {
+  CUtensorMap tw, tx;
+  p.pair_bt = pair_rows(p.T, p.N);
+  if (weight_map(&tw, W, 0, p.N, p.N, p.K, ldw, false, packed, &p)) return -1;
+  if (make_map(&tx, X, p.K, p.T, 0, ldx, 0, p.pair_bt / 2)) return -1;
+  return launch_pair<EPI_BF16, false>(tw, tx, p, (p.T + p.pair_bt - 1) / p.pair_bt, st);
+}
+
+// Grouped GEMMs with two SMs per tile of up to 256 rows: gate/up with rows by index, or a bf16 projection of sorted rows.
+// Tile-packed weights only.
+static int launch_pair_grouped(const void* X, const void* W, GemmParams p, int E, int w_rows, int epi, const int* gather_rows,
+                               int ldx, int max_tiles, cudaStream_t st) {
+  CUtensorMap tw, tx;
+  const bool silu = epi == EPI_SILU_MUL;
+  if (weight_map(&tw, W, E, p.N, w_rows, p.K, p.K, silu, 1, &p)) return -1;
+  if (!silu) {
+    if (make_map(&tx, X, p.K, p.T, 0, p.K, 0, VAR_BOX)) return -1;
+    return launch_pair<EPI_BF16, true>(tw, tx, p, max_tiles, st);
+  }
+  // a CTA's half of a k-block of a tile: 64 gate rows, then 64 up rows
+  const uint64_t nk = p.K / BK;
+  if (make_map_packed(&tw, W, static_cast<uint64_t>(E) * p.w_tiles * nk * BM * 2, BM / 2)) return -1;
+  p.gather_rows = gather_rows;
+  p.gx = static_cast<const bf16*>(X);
+  p.ldgx = ldx;
+  if (make_map(&tx, X, p.K, 1, 0, ldx, 0, 1)) return -1;  // never read through, but a valid map
+  return launch_pair<EPI_SILU_MUL, true>(tw, tx, p, max_tiles, st);
+}
+
 // Launch of a thin dense form; -5 where there is no such form.
 template <int EPI>
 static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, GemmParams p, int ldx, cudaStream_t st) {
@@ -886,7 +968,8 @@ extern "C" int b200_pick_bt(int T) {
   return 256;
 }
 
-// Dense: out[T, N] = X[T, K] W[N, K]^T. bt <= 0: the launcher picks the form, otherwise the token tile is `bt` rows.
+// Dense: out[T, N] = X[T, K] W[N, K]^T. bt <= 0: the launcher picks the form, otherwise the token tile is `bt` rows; PAIR_FORM
+// asks for two SMs per tile.
 // epi: 0 bf16, 1 fp32, 2 silu(gate)*up (N = rows of each half, W has 2N rows with the up half at row `up_offset`),
 // 3 argmax partials (part_max/part_idx sized [ceil(N/128), T]).
 extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, int N, int K, int ldx, int ldw, int ldo,
@@ -896,6 +979,9 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   const int w_rows = (epi == EPI_SILU_MUL) ? up_offset + N : N;
   GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
+  if (bt == PAIR_FORM && (epi != EPI_BF16 || splits > 1 || !pair_takes(p))) return -7;
+  if (bt == PAIR_FORM || (bt <= 0 && epi == EPI_BF16 && splits == 1 && pair_takes(p) && pair_pays(T, N)))
+    return launch_pair_dense(X, W, p, ldx, ldw, packed, st);
   if (bt <= 0 && (epi == EPI_BF16 || epi == EPI_F32)) {
     const DenseForm f = dense_form(T, N, K, packed && splits == 1);
     if (f.rt < BM || f.kps > 1)
@@ -928,6 +1014,12 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   // gather_rows != null (token tiles of at most GATHER_BT_MAX rows): X is [any rows, ldx] and sorted position i reads row
   // gather_rows[i] of it; otherwise X is the expert-sorted buffer [cap, K] itself.
   if (max_tiles <= 0) return 0;
+  if (bt == PAIR_FORM) {
+    GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, 1, nullptr, {}};
+    if (!packed || splits > 1 || !pair_takes(p) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) || (epi == EPI_SILU_MUL) != (gather_rows != nullptr) ||
+        (epi != EPI_SILU_MUL && epi != EPI_BF16)) return -7;
+    return launch_pair_grouped(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st);
+  }
   if (gather_rows != nullptr && (bt > GATHER_BT_MAX || splits > 1 || ldx % 8)) return -7;
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   CUtensorMap tw, tx;

@@ -14,6 +14,13 @@
 
 namespace b200 {
 
+// Rows per tile of an expert with c rows in t tiles. Tiles of 256 rows share an expert's rows evenly, in the steps of 32 that
+// their MMAs take: 272 rows as 160 + 112 and not 256 + 16, whose second tile waits for its weights only (gate/up of 8192
+// rows, about 256 per expert: 336 -> 324 us).
+__device__ __forceinline__ int tile_rows(int c, int t, int bt) {
+  return bt < 256 || t < 2 ? bt : ((c + t - 1) / t + 31) / 32 * 32;
+}
+
 // One CTA of 1024 threads turns the (row, pair) -> expert table into everything the grouped GEMMs need, without
 // global atomics or a zeroed workspace: rows per expert (shared-memory histogram), exclusive offsets (experts laid
 // out in id order, rows of one expert contiguous), the token-tile table (expert, row0, nrows) and its length, and
@@ -59,8 +66,9 @@ __device__ void plan_scatter(const int* idx, int n_pairs, int Et, int bt, int* o
   s_off[e] = row0;
   if (e < Et) {
     offsets[e] = row0;
-    for (int i = 0, ti = tile0; i * bt < c && ti < max_tiles; ++i, ++ti)
-      tiles[ti] = make_int4(e, row0 + i * bt, min(bt, c - i * bt), 0);
+    const int rows = tile_rows(c, t, bt);
+    for (int i = 0, ti = tile0; i * rows < c && ti < max_tiles; ++i, ++ti)
+      tiles[ti] = make_int4(e, row0 + i * rows, min(rows, c - i * rows), 0);
   }
   if (e == Et - 1) {
     offsets[Et] = row0 + c;
@@ -188,8 +196,9 @@ moe_route_plan_grid_kernel(const float* logits, int ldl, int T, int E, int top_k
   const int tile0 = stl - t + (w ? w_tiles[w - 1] : 0);
   if (e < Et) {
     offsets[e] = row0;
-    for (int i = 0, ti = tile0; i * bt < c && ti < max_tiles; ++i, ++ti)
-      tiles[ti] = make_int4(e, row0 + i * bt, min(bt, c - i * bt), 0);
+    const int rows = tile_rows(c, t, bt);
+    for (int i = 0, ti = tile0; i * rows < c && ti < max_tiles; ++i, ++ti)
+      tiles[ti] = make_int4(e, row0 + i * rows, min(rows, c - i * rows), 0);
   }
   if (e == Et - 1) {
     offsets[Et] = row0 + c;

@@ -388,6 +388,11 @@ GATHER_MAX_BT = int(__import__("os").environ.get("ENGINE_MOE_GATHER_BT", "128"))
 # they have: two such tiles replace four of 64 rows (8192 rows, 256 per expert: gate/up 496 -> 365 us; down 239 -> 246, but
 # both GEMMs walk one tile table). At 64 rows per expert both forms need about one tile (207 and 204 us, 99 and 101 us).
 WIDE_MIN_ROWS = 96
+# Expected rows per routed expert from which the expert GEMMs of ``moe_block`` take tiles of up to 256 rows on two SMs each
+# (tile-packed weights; 128-row tiles remain for plain ones). Block of 257 experts, us, without -> with: 48 rows per expert
+# 323 -> 333, 56: 339 -> 337, 64: 353 -> 347, 80: 396 -> 357, 128: 439 -> 401, 156: 527 -> 429, 256: 699 -> 601.
+PAIR_MIN_ROWS = 64
+PAIR_FORM = -256  # the launchers' token tile of up to 256 rows on two SMs
 
 
 def block_bt(T: int, top_k: int, pairs_per_row: int, n_experts: int) -> int:
@@ -436,6 +441,11 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
     bt = block_bt(T, top_k, Pn, n_experts)
     # the gate/up GEMM fetches each activation row by index, so no expert-sorted copy of x is made
     gather = bt <= GATHER_MAX_BT and x.stride(0) % 8 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0
+    pair = (gather and bt >= 64 and not _MOE_BT_FIXED and T * top_k >= PAIR_MIN_ROWS * n_experts and is_packed(w_gate_up)
+            and is_packed(w_down) and H % 256 == 0)
+    if pair:
+        bt = 256
+    form = PAIR_FORM if pair else bt
     src_rows = ints[Et + 2 + 2 * n_pairs :] if gather else None
     max_tiles = min(Et, n_pairs) + n_pairs // bt + 1
     tiles = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
@@ -453,7 +463,7 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
     act = torch.empty(n_pairs, inter, dtype=x.dtype, device=dev)
     if gather:
         _check(L.b200_gemm_grouped(_ptr(x), _ptr(w_gate_up), _ptr(act), n_pairs, Et, inter, 2 * inter, H, inter,
-                                   EPI_SILU_MUL, inter, bt, _ptr(tiles), _ptr(n_tiles), max_tiles, _ptr(err), 1,
+                                   EPI_SILU_MUL, inter, form, _ptr(tiles), _ptr(n_tiles), max_tiles, _ptr(err), 1,
                                    is_packed(w_gate_up), _ptr(src_rows), x.stride(0), st), "gemm_grouped(gate_up, gather)")
     else:
         if not x.is_contiguous() or x.data_ptr() % 16:  # the copy kernel takes whole rows, 16 bytes at a time
@@ -465,8 +475,8 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
                                    split_k(inter, H, grouped=True), is_packed(w_gate_up), None, 0, st),
                "gemm_grouped(gate_up)")
     pair_out = torch.empty(n_pairs, H, dtype=x.dtype, device=dev)
-    _check(L.b200_gemm_grouped(_ptr(act), _ptr(w_down), _ptr(pair_out), n_pairs, Et, H, H, inter, H, EPI_BF16, 0, bt,
-                               _ptr(tiles), _ptr(n_tiles), max_tiles, _ptr(err), split_k(H, inter, grouped=True),
+    _check(L.b200_gemm_grouped(_ptr(act), _ptr(w_down), _ptr(pair_out), n_pairs, Et, H, H, inter, H, EPI_BF16, 0, form,
+                               _ptr(tiles), _ptr(n_tiles), max_tiles, _ptr(err), 1 if pair else split_k(H, inter, grouped=True),
                                is_packed(w_down), None, 0, st),
            "gemm_grouped(down)")
     if norm_w is not None and not partial_f32:

@@ -128,3 +128,34 @@ def test_wide_expert_tiles_through_the_tensor_map(C, T, E, k, H, I, packed, monk
     monkeypatch.setattr(C, "GATHER_MAX_BT", 64)
     assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("N,K", [(256, 64), (392, 448), (2048, 4096), (1160, 128)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_two_sm_tiles_give_the_bits_of_the_plain_tile(C, N, K, packed):
+    """Fewer k-blocks than stages, a last tile without a second half or with part of one, token tiles of every width."""
+    w = _bf(N, K, scale=0.05, seed=1)
+    ww = C.pack_weight(w.clone()) if packed else w
+    for T in (1, 31, 32, 33, 255, 257, 300, 1000, 2500):
+        x = _bf(T, K + 64, seed=T)[:, 32:32 + K]
+        want = C.linear(x, w, bt=16)
+        assert torch.equal(C.linear(x, ww, bt=C.PAIR_FORM)[:, :N], want), T
+        assert torch.equal(C.linear(x, ww)[:, :N], want), T
+    C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(600, 16, 4, 256, 128), (1100, 32, 8, 2048, 512), (515, 8, 2, 512, 256), (3, 8, 2, 512, 128),
+                                       (4103, 12, 2, 256, 384)])
+def test_two_sm_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, monkeypatch):
+    """Experts with none, one and several tiles, tiles of 1 to 256 rows; the shared expert has T rows."""
+    x = _bf(T, H + 8, seed=T)[:, :H]
+    router = _bf(E + 1, H, scale=0.3, seed=34)
+    router[3] = -4.0 * x.float().mean(0).bfloat16()  # rarely picked
+    wgu = C.pack_weight(_bf(E + 1, 2 * I, H, scale=0.05, seed=35), gate_up=True)
+    wd = C.pack_weight(_bf(E + 1, H, I, scale=0.05, seed=36))
+    monkeypatch.setattr(C, "PAIR_MIN_ROWS", 1 << 30)
+    want = C.moe_block(x, router, wgu, wd, E, k, True)
+    monkeypatch.setattr(C, "PAIR_MIN_ROWS", 0)
+    monkeypatch.setattr(C, "moe_bt", lambda *a: 64)
+    assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
+    C.check_errors(x.device)
