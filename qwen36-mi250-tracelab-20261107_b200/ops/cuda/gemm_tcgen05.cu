@@ -831,6 +831,14 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   if (by2 && T <= 64 && tiles(64, 64) <= 2 * sms) return {T <= 32 ? 32 : 64, 64, 2};
   if (by2 && T <= 128 && tiles(64, 64) <= 2 * sms) return {64, 64, 2};
   if (by2 && T > 128 && T <= 256 && tiles(BM, 64) <= 2 * sms) return {64, BM, 2};
+  if (T > 256) {
+    // few weight tiles and many rows (the router): the narrowest token tile whose CTAs are resident together, as long as the
+    // K loop of a CTA and not the rows it reads sets the time. Router, 257 x 2048, us, 256-row tiles -> these: 300 rows
+    // 16.4 -> 7.6, 1531: 16.6 -> 8.8 (16 rows); 2048: 16.6 -> 9.6 (64; 16: 14.1); 4096: 17.0 -> 10.9 (128); 8192: 17.8
+    if (tiles(BM, 16) <= 2 * sms) return {16, BM, 1};
+    if (tiles(BM, 64) <= sms) return {64, BM, 1};
+    if (tiles(BM, 128) <= sms) return {128, BM, 1};
+  }
   return {T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256, BM, 1};
 }
 

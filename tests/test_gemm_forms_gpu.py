@@ -159,3 +159,10 @@ def test_two_sm_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I,
     monkeypatch.setattr(C, "moe_bt", lambda *a: 64)
     assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T", [257, 1531, 1600, 3000, 4100, 6400])
+def test_forms_of_few_weight_tiles_and_many_rows(C, T):
+    w, x = _bf(257, 256, scale=0.05, seed=1), _bf(T, 256, seed=T)
+    assert torch.equal(C.linear(x, C.pack_weight(w.clone()), out_dtype=torch.float32)[:, :257], C.linear(x, w, out_dtype=torch.float32, bt=256))
+    C.check_errors(x.device)
