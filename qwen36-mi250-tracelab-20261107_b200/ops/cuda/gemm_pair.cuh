@@ -61,13 +61,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
-  if (GROUPED) pdl_wait();  // the tile table was written by the kernel just before this one
   const int tiles_n = (p.N + PAIR_ROWS - 1) / PAIR_ROWS;
   const int tile0 = static_cast<int>(blockIdx.x >> 1), tstep = static_cast<int>(gridDim.x >> 1);
   const int bt = p.pair_bt;
-  int4 t_next = make_int4(0, 0, 0, 0);
-  if (GROUPED) t_next = p.tiles[tile0 / tiles_n];
-  const int total = tiles_n * (GROUPED ? *p.n_tiles : p.grid_y);
   const int num_k = p.K / BK;
 
   if (threadIdx.x == 0) {
@@ -87,6 +83,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   cluster_sync();  // both CTAs' barriers are ready before anything arrives at them from the other side
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (GROUPED) {  // the tile table was written by the kernel just before this one
+    pdl_wait();
+    if (warp == 0) pdl_launch();
+  }
+  int4 t_next = make_int4(0, 0, 0, 0);
+  if (GROUPED) t_next = p.tiles[tile0 / tiles_n];
+  const int total = tiles_n * (GROUPED ? *p.n_tiles : p.grid_y);
 
   // tile -> weight tile, expert, first token row, token rows; the next table entry is requested one tile ahead
   auto tile_geom = [&](int tile, int& nx, int& expert, int& row0, int& nrows) {
@@ -126,7 +129,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     int first = gw;  // the warp's first k-block of the tile
     int it = gw;     // stages of this warp and all others before it
     bool live = true;
-    if (warp == 0) pdl_launch();
     for (int tile = tile0; tile < total && live; tile += tstep) {
       int nx, expert, row0, nrows;
       tile_geom(tile, nx, expert, row0, nrows);
@@ -182,7 +184,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
       }
       pdl_wait();
-      pdl_launch();
+      if (!GROUPED) pdl_launch();
       for (int tile = tile0; tile < total && live; tile += tstep) {
         int nx, expert, row0, nrows;
         tile_geom(tile, nx, expert, row0, nrows);

@@ -150,21 +150,15 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __shared__ int red_idx[4][RED];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // The grouped tile table is written by the kernel just before this one: wait for it before the first read.
-  // Dense launches wait later (the producer streams the first weight stages before it waits).
-  if (GROUPED) pdl_wait();
+  if (SPLIT) pdl_wait();
   // Persistent tile loop: CTA b takes output tiles b, b + gridDim.x, ... (weight tile fastest, so CTAs that run
   // together share the activation tile). A split-K cluster takes the single tile its grid position names.
   const int tiles_n = (p.N + RT - 1) / RT;
-  // The role's first table entry is read beside the entry count, not behind it (the table has room for the whole grid).
   const int tile0 = SPLIT ? static_cast<int>(blockIdx.y) * tiles_n + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
-  int4 t_next = make_int4(0, 0, 0, 0);
-  if (GROUPED) t_next = p.tiles[tile0 / tiles_n];
-  const int tiles_y = GROUPED ? *p.n_tiles : p.grid_y;
-  const int total = tiles_n * tiles_y;
   const int tstep = SPLIT ? (1 << 30) : static_cast<int>(gridDim.x);
   constexpr int ACC = SPLIT ? 1 : C::ACC_STAGES;
-  if (SPLIT && tile0 >= total) return;  // the whole cluster leaves together, before any barrier or TMEM use
+  // the whole cluster leaves together, before any barrier or TMEM use
+  if (SPLIT && tile0 >= tiles_n * (GROUPED ? *p.n_tiles : p.grid_y)) return;
   const int num_k_all = (p.K + BK * KPS - 1) / (BK * KPS);  // in stages
   // split-K: the cluster's CTAs (blockIdx.z = rank in the cluster) take consecutive runs of k-blocks; their fp32
   // partial tiles meet in the leader through distributed shared memory, added in rank order
@@ -188,6 +182,17 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // The grouped tile table is written by the kernel just before this one: wait for it before the first read, with the
+  // set-up above behind it. Dense launches wait later (the producer streams the first weight stages before it waits).
+  if (GROUPED) {
+    pdl_wait();
+    if (!SPLIT && warp == 0) pdl_launch();
+  }
+  // The role's first table entry is read beside the entry count, not behind it (the table has room for the whole grid).
+  int4 t_next = make_int4(0, 0, 0, 0);
+  if (GROUPED) t_next = p.tiles[tile0 / tiles_n];
+  const int tiles_y = GROUPED ? *p.n_tiles : p.grid_y;
+  const int total = tiles_n * tiles_y;
 
   // geometry of output tile `tile`
   // (the table entry of the role's next tile is requested one tile ahead: its latency would otherwise open every tile)
@@ -292,7 +297,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         }
       }
       pdl_wait();
-      pdl_launch();
+      if (!GROUPED) pdl_launch();
       for (int tile = tile0; tile < total && live; tile += tstep) {
       int n0, by, expert, row0, nrows;
       tile_geom(tile, n0, by, expert, row0, nrows);
