@@ -149,7 +149,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __shared__ float red_max[4][RED];
   __shared__ int red_idx[4][RED];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (SPLIT) pdl_wait();
   // Persistent tile loop: CTA b takes output tiles b, b + gridDim.x, ... (weight tile fastest, so CTAs that run
   // together share the activation tile). A split-K cluster takes the single tile its grid position names.
@@ -323,7 +323,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
     if (SPLIT) { __syncwarp(); cluster_sync(); }
   } else if (warp == 1) {
-    if (elect_one()) {
+    const uint32_t issue = elect_one();
+    {
       uint32_t idesc = umma_idesc_bf16(BM, !GROUPED && !C::THIN && p.x_rows > 0 ? p.x_rows : BT);
       bool ok = true;
       int it = 0, lt = 0;  // k-blocks and tiles consumed so far
@@ -336,12 +337,12 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int acc = lt % ACC;
       const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
       // the epilogue must have drained this accumulator stage (two tiles ago) before it is overwritten
-      ok = mbar_wait(&acc_empty[acc], ((lt / ACC) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
+      ok = mbar_wait_warp(&acc_empty[acc], ((lt / ACC) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
       if (ok) tc_fence_after();
       for (int kb = 0; kb < num_k && ok; ++kb, ++it) {
         const int s = it % C::STAGES;
         const uint32_t ph = (it / C::STAGES) & 1;
-        ok = mbar_wait(&full[s], ph, p.err, ERR_WAIT_FULL, abort_flag);
+        ok = mbar_wait_warp(&full[s], ph, p.err, ERR_WAIT_FULL, abort_flag);
         if (!ok) break;
         // rows that the gathering producer wrote through the generic proxy must be visible to the tensor core's reads
         if (GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -353,13 +354,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           const uint32_t koff = (k % (BK / UMMA_K)) * UMMA_K * 2;  // bytes inside the 128-byte swizzled row
           const uint32_t aoff = k / (BK / UMMA_K) * C::A_STEP + koff;
           const uint64_t db = umma_smem_desc(b_addr + k / (BK / UMMA_K) * C::B_BYTES + koff);
-          umma_bf16(tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
+          umma_bf16_if(issue, tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
           if (EPI == EPI_SILU_MUL)
-            umma_bf16(tmem + BT, umma_smem_desc(a_addr + C::UP_OFF + aoff), db, idesc, (kb | k) != 0);
+            umma_bf16_if(issue, tmem + BT, umma_smem_desc(a_addr + C::UP_OFF + aoff), db, idesc, (kb | k) != 0);
         }
-        umma_commit(&empty[s]);  // stage reusable once these MMAs have read it
+        umma_commit_if(issue, &empty[s]);  // stage reusable once these MMAs have read it
       }
-      umma_commit(&acc_full[acc]);  // always arrive so that the epilogue is released
+      umma_commit_if(issue, &acc_full[acc]);  // always arrive so that the epilogue is released
       }
     }
     if (SPLIT) { __syncwarp(); cluster_sync(); }
