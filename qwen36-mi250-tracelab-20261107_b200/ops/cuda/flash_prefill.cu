@@ -48,12 +48,6 @@ struct FlashParams {
   float* part_ml;         // [T, n_q, gridDim.z, 2] (row maximum in natural-log units, row sum)
 };
 
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z, int w) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
 // DEC (decode: one query position per tile, so GROUP <= 8 real rows): the Q and P operands keep only their first
 // 8-row swizzle atom per 128-byte block (1 KB instead of 16 KB); the MMA still reads 128 rows from those bases, the
 // other 120 come from whatever shared memory follows (the K/V stages) and land in accumulator rows nobody reads: an

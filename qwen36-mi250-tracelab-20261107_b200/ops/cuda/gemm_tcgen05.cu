@@ -69,23 +69,26 @@ struct GemmParams {
   int pair_bt;       // gemm_pair_kernel, dense: token rows per tile
 };
 
-// RT: weight rows per tile. 128 fills the MMA's M; the thin forms (64, 32) load that many rows into the first rows of the
-// operand tile and let the MMA read whatever shared memory holds behind them: an accumulator row depends on its own operand
-// row only, the surplus rows are never read back, and the instruction shape, and with it every bit of the result, stay
-// those of RT = 128. They exist for launches whose 128-row tiles would leave most SMs without work.
+// RT: weight rows per tile. 128 fills the MMA's M; the thin forms (64, 32) exist for launches whose 128-row tiles would leave
+// most SMs without work. Their MMA has 64 rows where the tile has no more: it reads half as much shared memory (27 cycles per
+// instruction of 16 columns, not 42). An accumulator row depends on its own operand row only and is the same in both
+// instructions; rows that a 32-row tile does not have are whatever shared memory holds behind it, and are never read back.
+// A thin gate/up tile is one operand: RT gate rows and the RT up rows behind them, one MMA for both.
 // KPS: k-blocks per pipeline stage. One trip through the pipeline (wait, expect, TMA, wait, MMAs, commit) costs a CTA about
 // 0.2 us however little it moves, and at decode sizes a CTA's time is the sum of its trips; a stage of KPS k-blocks comes
-// with one TMA instruction per operand. Tile-packed weights only.
+// with one TMA instruction per operand. Thin tiles of tile-packed weights only.
 template <int BT, int EPI, int RT = BM, int KPS = 1>
 struct Cfg {
   static constexpr int A_TILES = (EPI == EPI_SILU_MUL) ? 2 : 1;
   static constexpr int A_BYTES = RT * BK * 2;
   static constexpr int B_BYTES = BT * BK * 2;
   static constexpr int STAGE_BYTES = KPS * (A_TILES * A_BYTES + B_BYTES);
-  static constexpr int A_STEP = (RT == BM ? A_TILES : 1) * A_BYTES;  // bytes between the k-blocks of a stage
-  static constexpr int UP_OFF = RT == BM ? A_BYTES : KPS * A_BYTES;  // from a gate tile to its up tile
+  static constexpr int A_STEP = A_TILES * A_BYTES;  // bytes between the k-blocks of a stage
   static constexpr int B_OFF = KPS * A_TILES * A_BYTES;
-  static constexpr bool THIN = RT < BM || KPS > 1;
+  static constexpr bool THIN = RT < BM;
+  static constexpr bool MERGED = THIN && EPI == EPI_SILU_MUL;  // gate and up rows in one accumulator
+  static constexpr int A_ROWS = MERGED ? 2 * RT : RT;          // operand rows of an MMA
+  static constexpr int MMA_M = A_ROWS <= 64 ? 64 : 128;        // accumulator row r: TMEM lane r, or 32 (r / 16) + r % 16 of 64
   // Wide expert tiles (prefill): the MMA's N follows the tile's row count (a 128-row tile with 40 rows costs 48 columns and
   // loads 64 rows), and two producer warps fetch the rows by index. Grouped launches only. What bounds the expert GEMMs is
   // shared memory: each k-block is written once and its weight half is read again for every MMA, so a wider tile moves
@@ -105,17 +108,23 @@ struct Cfg {
   // The fused gate/up GEMM at 16-row token tiles runs three CTAs per SM with two deep stages each: the same bytes in
   // flight per SM, but a decode step's ~1300 tiles then fill 2.9 waves of 444 CTAs instead of 4.4 waves of 296, and
   // the partial last wave is what the weight-streaming time loses.
-  static constexpr int CTAS_PER_SM = THIN ? 2 : (BT <= 16 && EPI == EPI_SILU_MUL) ? 3 : BT <= 64 ? 2 : 1;
-  static constexpr int BUDGET = THIN ? (RT < BM ? 96 * 1024 : 108 * 1024) : CTAS_PER_SM == 3 ? 72 * 1024 : BT <= 64 ? 108 * 1024 : 200 * 1024;
+  // Thin tiles of four k-blocks per stage run alone on their SM, with all of its shared memory: more bytes on their way, and
+  // one commit for two stages.
+  static constexpr bool SOLO = THIN && KPS == 4;
+  static constexpr int CTAS_PER_SM = SOLO ? 1 : THIN ? 2 : (BT <= 16 && EPI == EPI_SILU_MUL) ? 3 : BT <= 64 ? 2 : 1;
+  static constexpr int BUDGET = SOLO ? 200 * 1024 : MERGED ? 108 * 1024 : THIN ? 96 * 1024 : CTAS_PER_SM == 3 ? 72 * 1024 : BT <= 64 ? 108 * 1024 : 200 * 1024;
   static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
-  static constexpr int ACC_COLS = A_TILES * BT;  // one accumulator stage
+  // Stages that are released together, by one commit. A commit drains the tensor core: n MMAs and their commit take F + n e
+  // cycles, with (F, e) = (281, 42) for 128 x 16, (332, 27) for 64 x 16, (192, 66) for 128 x 128; at 128 x 256 F is hidden.
+  static constexpr int GROUP = SOLO ? 2 : 1;
+  static constexpr int STAGES = (STAGES_RAW > 8 ? 8 : STAGES_RAW) / GROUP * GROUP;
+  static constexpr int ACC_COLS = (MERGED ? 1 : A_TILES) * BT;  // one accumulator stage
   // two accumulator stages whenever they fit (512 columns per SM shared by the resident CTAs): the epilogue of
   // one tile then overlaps the main loop of the CTA's next tile
   static constexpr int ACC_STAGES = (2 * ACC_COLS * CTAS_PER_SM <= 512) ? 2 : 1;
   static constexpr int TMEM_COLS_RAW = ACC_COLS * ACC_STAGES;
   static constexpr int TMEM_COLS = TMEM_COLS_RAW <= 32 ? 32 : TMEM_COLS_RAW <= 64 ? 64 : TMEM_COLS_RAW <= 128 ? 128 : TMEM_COLS_RAW <= 256 ? 256 : 512;
-  static constexpr int OVERREAD = (BM - RT) * BK * 2;  // bytes behind the last stage that a thin tile's MMA may read
+  static constexpr int OVERREAD = (MMA_M - A_ROWS) * BK * 2;  // bytes behind the last stage that a thin tile's MMA may read
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + (OVERREAD > 256 ? OVERREAD : 256) /*barriers first*/ + OUT_BYTES;
 };
 
@@ -148,6 +157,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   constexpr int RED = EPI == EPI_ARGMAX ? BT : 1;
   __shared__ float red_max[4][RED];
   __shared__ int red_idx[4][RED];
+  __shared__ uint4 exchange[C::MERGED ? 128 : 1];
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (SPLIT) pdl_wait();
@@ -215,8 +225,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   auto load_weights = [&](uint8_t* st, uint64_t* bar, int n0, int expert, int kb) {
     if constexpr (C::THIN) {  // packed only: [expert, tile, k-block][rows of the tile][64], KPS k-blocks per box
       const int z = ((expert * p.w_tiles + n0 / BM) * num_k_all + kb) * KPS;
-      tma_load_3d(st, &tmW, bar, 0, n0 % BM, z);  // RT = 128: gate and up rows are one box
-      if (RT < BM && EPI == EPI_SILU_MUL) tma_load_3d(st + C::UP_OFF, &tmW, bar, 0, BM + n0 % BM, z);
+      if constexpr (C::MERGED) tma_load_4d(st, &tmW, bar, 0, n0 % BM, 0, z);  // [k-block][gate, up][rows][64]
+      else tma_load_3d(st, &tmW, bar, 0, n0 % BM, z);
     } else if (p.packed) {
       tma_load_2d(st, &tmW, bar, 0, ((expert * p.w_tiles + n0 / BM) * num_k_all + kb) * (BM * C::A_TILES));
     } else if (GROUPED) {
@@ -226,6 +236,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       tma_load_2d(st, &tmW, bar, kb * BK, n0);
       if (EPI == EPI_SILU_MUL) tma_load_2d(st + C::A_BYTES, &tmW, bar, kb * BK, p.up_offset + n0);
     }
+  };
+
+  // the stage of step `it` may be filled (a group's first stage stands for all of them)
+  auto wait_free = [&](int it) {
+    constexpr int NG = C::STAGES / C::GROUP;
+    const int g = it / C::GROUP;
+    return it % C::GROUP != 0 || mbar_wait(&empty[g % NG], ((g / NG) & 1) ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag);
   };
 
   constexpr int GW = GROUPED ? C::GATHER_WARPS : 1;
@@ -253,8 +270,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
       for (int kb = 0; kb < num_k; ++kb, ++it) {
         const int s = it % C::STAGES;
-        const uint32_t ph = (it / C::STAGES) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
+        if (!wait_free(it)) { live = false; break; }
         uint8_t* st = smem + s * C::STAGE_BYTES;
         if (lane == 0 && (GW == 1 || warp == 0)) {
           mbar_expect_tx(&full[s], C::B_OFF);
@@ -306,10 +322,9 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (p.x_flags != nullptr && !wait_flag(p.x_flags + row0 / p.rows_per_rank, *p.x_epoch, p.err)) *abort_flag = 1;
       for (int kb = 0; kb < num_k; ++kb, ++it) {
         const int s = it % C::STAGES;
-        const uint32_t ph = (it / C::STAGES) & 1;
         uint8_t* st = smem + s * C::STAGE_BYTES;
         if (it >= pre) {
-        if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
+        if (!wait_free(it)) { live = false; break; }
         mbar_expect_tx(&full[s], !GROUPED ? x_stage : C::VAR_N ? C::B_OFF + (nrows + VAR_BOX - 1) / VAR_BOX * (VAR_BOX * BK * 2) : C::STAGE_BYTES);
         load_weights(st, &full[s], n0, expert, kb0 + kb);
         }
@@ -325,7 +340,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   } else if (warp == 1) {
     const uint32_t issue = elect_one();
     {
-      uint32_t idesc = umma_idesc_bf16(BM, !GROUPED && !C::THIN && p.x_rows > 0 ? p.x_rows : BT);
+      uint32_t idesc = umma_idesc_bf16(C::MMA_M, !GROUPED && !C::THIN && p.x_rows > 0 ? p.x_rows : BT);
       bool ok = true;
       int it = 0, lt = 0;  // k-blocks and tiles consumed so far
       for (int tile = tile0; tile < total && ok; tile += tstep, ++lt) {
@@ -355,10 +370,11 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           const uint32_t aoff = k / (BK / UMMA_K) * C::A_STEP + koff;
           const uint64_t db = umma_smem_desc(b_addr + k / (BK / UMMA_K) * C::B_BYTES + koff);
           umma_bf16_if(issue, tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
-          if (EPI == EPI_SILU_MUL)
-            umma_bf16_if(issue, tmem + BT, umma_smem_desc(a_addr + C::UP_OFF + aoff), db, idesc, (kb | k) != 0);
+          if (EPI == EPI_SILU_MUL && !C::MERGED)
+            umma_bf16_if(issue, tmem + BT, umma_smem_desc(a_addr + C::A_BYTES + aoff), db, idesc, (kb | k) != 0);
         }
-        umma_commit_if(issue, &empty[s]);  // stage reusable once these MMAs have read it
+        // the group's stages are reusable once these MMAs have read them
+        if (it % C::GROUP == C::GROUP - 1) umma_commit_if(issue, &empty[it / C::GROUP % (C::STAGES / C::GROUP)]);
       }
       umma_commit_if(issue, &acc_full[acc]);  // always arrive so that the epilogue is released
       }
@@ -379,10 +395,12 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const int acc = lt % ACC;
     const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
     bool ok = mbar_wait(&acc_full[acc], (lt / ACC) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag;
-    if (C::STAGED && staged) ok = epilogue_all(ok);  // the batches below hold barriers: all four warps take them, or none
+    // batches that hold barriers: all four warps take them, or none
+    if (C::MERGED || (C::STAGED && staged)) ok = epilogue_all(ok);
     tc_fence_after();
-    const int n = n0 + q * 32 + lane;
-    const bool n_ok = n < p.N && (RT == BM || q * 32 + lane < RT);
+    const int arow = C::MMA_M == 64 ? q * 16 + lane : q * 32 + lane;  // accumulator row of this thread
+    const int n = n0 + (C::MERGED ? arow % RT : arow);
+    const bool n_ok = n < p.N && (C::MMA_M == 128 || lane < 16) && arow < C::A_ROWS;
     if (EPI == EPI_ALLREDUCE) {
       // Fused GEMM -> one-shot all-reduce: this tile's fp32 partial goes straight from TMEM into every
       // rank's receive slot over NVLink; when all R partials of the tile have arrived they are added in
@@ -479,7 +497,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       cluster_sync();  // first cluster barrier (every thread of the cluster takes part exactly once)
     } else {
     if (SPLIT) cluster_sync();  // first cluster barrier: the followers' partial tiles are in place
-    if (ok && q * 32 < RT) {
+    if (ok && q * (C::MMA_M / 4) < C::A_ROWS) {
       const uint32_t red_local = smem_u32(smem);
 #pragma unroll 1
       for (int c = 0; c < BT; c += 16) {
@@ -492,6 +510,33 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] += ld_dsmem_f32(remote + ((c + j) * BM + q * 32 + lane) * 4);
           }
+        }
+        if constexpr (C::MERGED) {
+          // the threads of an output's gate and up row swap half of their columns, rounded to bf16 as the unfused sequence
+          // of ops rounds them, and finish eight each
+          const bool up = q >= 2;
+          const int tid = q * 32 + lane;
+          uint4 mine, theirs;
+          bf16* me = reinterpret_cast<bf16*>(&mine);
+          const bf16* te = reinterpret_cast<const bf16*>(&theirs);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) me[j] = __float2bfloat16(up ? v[j] : v[8 + j]);
+          exchange[tid] = mine;
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          theirs = exchange[tid ^ 64];
+          asm volatile("bar.sync 2, 128;" ::: "memory");
+          const int c0 = c + (up ? 8 : 0);
+          if (n_ok) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float own = __bfloat162float(__float2bfloat16(up ? v[8 + j] : v[j])), other = __bfloat162float(te[j]);
+              const float gate = up ? other : own, lin = up ? own : other;
+              if (c0 + j < nrows)
+                reinterpret_cast<bf16*>(p.out)[static_cast<size_t>(row0 + c0 + j) * p.ldo + n] =
+                    __float2bfloat16(__bfloat162float(__float2bfloat16(silu_f(gate))) * lin);
+            }
+          }
+          continue;
         }
         if (EPI == EPI_SILU_MUL) {
           float u[16];
@@ -709,6 +754,20 @@ static int make_map_kblocks(CUtensorMap* m, const void* base, uint64_t rows, uin
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// The same for thin gate/up tiles: [tile, k-block][gate, up][BM rows][64], `rows` rows of either half and `kps` k-blocks per box.
+static int make_map_gate_up(CUtensorMap* m, const void* base, uint64_t blocks, uint32_t rows, uint32_t kps) {
+  EncodeFn fn = encode_fn();
+  if (!fn) return -1;
+  cuuint64_t dims[4] = {BK, BM, 2, blocks};
+  cuuint64_t strides[3] = {BK * 2, BM * BK * 2, 2 * BM * BK * 2};
+  cuuint32_t box[4] = {BK, rows, 2, kps};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -2;
+}
+
 // Weight map of a launch: `packed` selects the tile-packed layout (N padded to a multiple of 128 per expert, K a
 // multiple of 64; with the SiLU-mul epilogue the gate and up tiles of a k-block are stored back to back).
 static int weight_map(CUtensorMap* m, const void* W, int E, int N, int w_rows, int K, int ldw, bool silu, int packed,
@@ -808,7 +867,8 @@ struct DenseForm {
 // The form of a dense bf16 / fp32 GEMM. It never changes a row's bits (every element sees the same k order in the same
 // instruction shape), so it may follow the number of rows. Measured in chains of launches on weights that are not in L2, us,
 // plain form -> chosen form; 12352 x 2048 is a GDN layer's input projection, 9216 x 2048 an attention layer's, 2048 x 4096
-// the output projection, 257 x 2048 the router:
+// the output projection, 257 x 2048 the router (taken before thin tiles had MMAs of 64 rows and SMs of their own, which
+// brought 2048 x 4096 of one row from 9.3 to 7.9 us, 257 x 2048 from 5.7 to 4.9, 9216 x 2048 from 8.4 to 7.4 in a step):
 //   up to 16 rows     12352: 13.0 -> 12.0   9216: 11.6 -> 10.4   2048: 15.4 -> 10.9   257: 8.5 -> 6.3
 //   32 rows           12352: 14.5 -> 13.0   9216: 13.3 -> 12.1   2048: 15.2 -> 11.1   257: 8.5 -> 6.3
 //   61 rows           12352: 16.6 -> 15.4   9216: 15.5 -> 14.2   2048: 14.7 -> 12.5   257: 8.4 -> 6.5
@@ -819,9 +879,11 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   const auto tiles = [&](int rt, int bt) { return static_cast<long long>((N + rt - 1) / rt) * ((T + bt - 1) / bt); };
   const bool by2 = packed && K % (2 * BK) == 0, by4 = packed && K % (4 * BK) == 0;
   if (T <= 16) {
-    // one token tile: the weights are streamed once whatever the tile, so the thinnest tile whose CTAs (two per SM) are
-    // all resident wins; beyond that the second wave costs more (386 CTAs of 32 rows: 14.2 us for the 12352 rows)
-    if (by4 && tiles(32, 16) <= 2 * sms) return {16, 32, 4};
+    // one token tile: the weights are streamed once whatever the tile, so the thinnest tile whose CTAs have an SM each wins
+    // (9216 rows as 288 CTAs of 32 rows, two per SM: 8.4 us, as 144 of 64: 7.4), then the thinnest whose CTAs, two per SM, are
+    // all resident; beyond that the second wave costs more (386 CTAs of 32 rows: 14.2 us for the 12352 rows)
+    if (by4 && tiles(32, 16) <= sms) return {16, 32, 4};
+    if (by4 && tiles(64, 16) <= sms) return {16, 64, 4};
     if (by2 && tiles(64, 16) <= 2 * sms) return {16, 64, 2};
     return {16, BM, 1};
   }
@@ -836,7 +898,6 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   }
   if (by2 && T <= 64 && tiles(64, 64) <= 2 * sms) return {T <= 32 ? 32 : 64, 64, 2};
   if (by2 && T <= 128 && tiles(64, 64) <= 2 * sms) return {64, 64, 2};
-  if (by2 && T > 128 && T <= 256 && tiles(BM, 64) <= 2 * sms) return {64, BM, 2};
   if (T > 256) {
     // few weight tiles and many rows (the router): the narrowest token tile whose CTAs are resident together, as long as the
     // K loop of a CTA and not the rows it reads sets the time. Router, 257 x 2048, us, 256-row tiles -> these: 300 rows
@@ -936,35 +997,37 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
   if (make_map_kblocks(&tx, X, p.T, static_cast<uint64_t>(ldx) * 2, nk, BK * 2, f.bt, f.kps)) return -1;
   const int gy = (p.T + f.bt - 1) / f.bt;
   if (f.bt == 16 && f.rt == 32 && f.kps == 4) return launch<16, EPI, false, 32, 4>(tw, tx, p, gy, st);
+  if (f.bt == 16 && f.rt == 64 && f.kps == 4) return launch<16, EPI, false, 64, 4>(tw, tx, p, gy, st);
   if (f.bt == 16 && f.rt == 64 && f.kps == 2) return launch<16, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 64 && f.rt == 64 && f.kps == 2) return launch<64, EPI, false, 64, 2>(tw, tx, p, gy, st);
-  if (f.bt == 64 && f.rt == BM && f.kps == 2) return launch<64, EPI, false, BM, 2>(tw, tx, p, gy, st);
   return -5;
 }
 
 // Gate/up GEMM of the experts of a few rows (16-row token tiles, at most one per pair, tile-packed weights): each 128-row
-// tile becomes four when that still leaves at most one CTA per SM, two when at most two. Whole block, us: 1 row 41.5 ->
+// tile becomes four when that still leaves at most one CTA per SM, two when at most two. This GEMM in a decode step, us: 1 row
+// 14.7 as two operands of 128-row MMAs -> 9.2 as one. Whole block with the two operands against plain tiles: 1 row 41.5 ->
 // 30.7, 2 rows 46.1 -> 39.4, 4 rows 54.8 -> 52.7; at 8 rows the plain tiles are as good (77.3, thin 78.9). The down
 // projection (16 weight tiles per expert) has CTAs enough at one row. Returns 1 when the plain form is to run.
 static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
                                int max_tiles, cudaStream_t st) {
   const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
   const int sms = sm_count(), rt = 4 * tiles <= sms ? 32 : 2 * tiles <= 2 * sms ? 64 : BM;
-  if (rt == BM || p.K % (2 * BK) || p.N % BM) return 1;
+  const int kps = rt == 32 ? 4 : 2;
+  if (rt == BM || p.K % (kps * BK) || p.N % BM) return 1;
   CUtensorMap tw, tx;
   const uint64_t nk = p.K / BK;
   p.packed = 1;
   p.w_tiles = p.N / BM;
-  if (make_map_kblocks(&tw, W, 2 * BM, BK * 2, static_cast<uint64_t>(E) * p.w_tiles * nk, 2 * BM * BK * 2, rt, 2)) return -1;
+  if (make_map_gate_up(&tw, W, static_cast<uint64_t>(E) * p.w_tiles * nk, rt, kps)) return -1;
   if (gather_rows != nullptr) {
     p.gather_rows = gather_rows;
     p.gx = static_cast<const bf16*>(X);
     p.ldgx = ldx;
   }
   // with row indices the producer never reads through this map, but it has to be a valid one
-  if (make_map_kblocks(&tx, X, gather_rows ? 16 : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, 16, 2)) return -1;
-  if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 2>(tw, tx, p, max_tiles, st);
+  if (make_map_kblocks(&tx, X, gather_rows ? 16 : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, 16, kps)) return -1;
+  if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 4>(tw, tx, p, max_tiles, st);
   return launch<16, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
 }
 
@@ -998,7 +1061,7 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
     return launch_pair_dense(X, W, p, ldx, ldw, packed, st);
   if (bt <= 0 && (epi == EPI_BF16 || epi == EPI_F32)) {
     const DenseForm f = dense_form(T, N, K, packed && splits == 1);
-    if (f.rt < BM || f.kps > 1)
+    if (f.rt < BM)
       return epi == EPI_F32 ? launch_thin_dense<EPI_F32>(f, X, W, p, ldx, st) : launch_thin_dense<EPI_BF16>(f, X, W, p, ldx, st);
     bt = f.bt;
   }
