@@ -116,7 +116,7 @@ struct Cfg {
   static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
   // Stages that are released together, by one commit. A commit drains the tensor core: n MMAs and their commit take F + n e
   // cycles, with (F, e) = (281, 42) for 128 x 16, (332, 27) for 64 x 16, (192, 66) for 128 x 128; at 128 x 256 F is hidden.
-  static constexpr int GROUP = SOLO ? 2 : 1;
+  static constexpr int GROUP = SOLO && STAGES_RAW >= 4 ? 2 : 1;
   static constexpr int STAGES = (STAGES_RAW > 8 ? 8 : STAGES_RAW) / GROUP * GROUP;
   static constexpr int ACC_COLS = (MERGED ? 1 : A_TILES) * BT;  // one accumulator stage
   // two accumulator stages whenever they fit (512 columns per SM shared by the resident CTAs): the epilogue of
@@ -889,11 +889,14 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
   }
   if (T <= 256 && N <= 32 * BM) {
     // few weight tiles: 16-row token tiles put 8x more CTAs on the K loop. Several token tiles re-read the weights, so
-    // thin tiles pay only while the CTAs have an SM each, with a little room (144 CTAs already share some)
+    // thin tiles pay only while the CTAs have an SM each, with a little room (144 CTAs already share some). Output projection
+    // of 128 rows in a step 13.1 us with two 32-row tiles' stages per SM, 11 with all of an SM's shared memory; 256 rows 16 as
+    // 256 CTAs of 16 x 128, 14 as 128 of 64 x 64
     const int lim = sms * 7 / 8;
     if (by4 && tiles(32, 16) <= lim) return {16, 32, 4};
-    if (by2 && tiles(64, 16) <= lim) return {16, 64, 2};
-    if (by2 && tiles(64, 32) <= lim) return {32, 64, 2};
+    if (by4 && tiles(64, 16) <= lim) return {16, 64, 4};
+    if (by4 && tiles(64, 32) <= lim) return {32, 64, 4};
+    if (by4 && tiles(64, 64) <= lim) return {64, 64, 4};
     return {16, BM, 1};
   }
   if (by2 && T <= 64 && tiles(64, 64) <= 2 * sms) return {T <= 32 ? 32 : 64, 64, 2};
@@ -999,6 +1002,8 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
   if (f.bt == 16 && f.rt == 32 && f.kps == 4) return launch<16, EPI, false, 32, 4>(tw, tx, p, gy, st);
   if (f.bt == 16 && f.rt == 64 && f.kps == 4) return launch<16, EPI, false, 64, 4>(tw, tx, p, gy, st);
   if (f.bt == 16 && f.rt == 64 && f.kps == 2) return launch<16, EPI, false, 64, 2>(tw, tx, p, gy, st);
+  if (f.bt == 32 && f.rt == 64 && f.kps == 4) return launch<32, EPI, false, 64, 4>(tw, tx, p, gy, st);
+  if (f.bt == 64 && f.rt == 64 && f.kps == 4) return launch<64, EPI, false, 64, 4>(tw, tx, p, gy, st);
   if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 64 && f.rt == 64 && f.kps == 2) return launch<64, EPI, false, 64, 2>(tw, tx, p, gy, st);
   return -5;
