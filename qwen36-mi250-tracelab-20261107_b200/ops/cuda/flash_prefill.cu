@@ -35,6 +35,8 @@ constexpr int FP_PAGE = 64;
 struct FlashParams {
   const int4* tiles;      // (segment, first local position, segment start row, segment length)
   const int* seg_pos0;    // position of each segment's first row
+  const int64_t* positions;  // instead of seg_pos0: position of every row (decode passes have these; a conversion kernel in
+                             // front cost a step about 2 us per attention layer)
   const int* tables;      // [segments, max_pages]
   int max_pages;
   int num_pages;
@@ -106,7 +108,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int4 tile = p.tiles[blockIdx.x];
   const int seg = tile.x, p0 = tile.y, seg_row0 = tile.z, seg_len = tile.w;
   const int kh = blockIdx.y;
-  const int pos0 = p.seg_pos0[seg];
+  const int pos0 = p.positions ? static_cast<int>(p.positions[seg_row0]) : p.seg_pos0[seg];
   const int n_pos = min(R, seg_len - p0);
   if (n_pos <= 0) return;  // filler entry: a captured prefill pass keeps its tile table at a fixed length
   const int np_all = (pos0 + p0 + n_pos - 1) / FP_PAGE + 1;  // pages that hold visible keys
@@ -403,9 +405,9 @@ int fp_launch(const CUtensorMap& tq, const CUtensorMap& tkv, const FlashParams& 
 
 // q: [T, n_q, D] bf16 (already normed and rotated), gate/out: [T, n_q * D], kv: one layer of the paged pool
 // [num_pages, 2, n_kv, 64, D]; tiles: int4 (segment, first local position, segment start row, segment length) with
-// 128 / (n_q / n_kv) positions per tile; seg_pos0 / tables per segment. The span's K/V must already be in the pages.
+// 128 / (n_q / n_kv) positions per tile; seg_pos0 (or `positions`, one per row) and tables per segment. The span's K/V must already be in the pages.
 extern "C" int b200_flash_prefill(const void* q, const void* gate, const void* kv, void* out, const void* tiles,
-                                  int n_tiles, const int* seg_pos0, const int* tables, int max_pages, int num_pages,
+                                  int n_tiles, const int* seg_pos0, const int64_t* positions, const int* tables, int max_pages, int num_pages,
                                   int T, int n_q, int n_kv, int D, int split_pages, int n_splits, float* part_acc,
                                   float* part_ml, int one_position, int* err, cudaStream_t st) {
   // one_position != 0: every tile holds a single query position (plain decode): the form with small Q / P tiles
@@ -428,7 +430,7 @@ extern "C" int b200_flash_prefill(const void* q, const void* gate, const void* k
     cuuint32_t box[2] = {64, FP_PAGE};
     if (fp_make_map(&tkv, kv, 2, dims, strides, box)) return -1;
   }
-  FlashParams p{static_cast<const int4*>(tiles), seg_pos0, tables, max_pages, num_pages, static_cast<const bf16*>(gate),
+  FlashParams p{static_cast<const int4*>(tiles), seg_pos0, positions, tables, max_pages, num_pages, static_cast<const bf16*>(gate),
                 static_cast<bf16*>(out), n_q, n_kv, 1.4426950408889634f / sqrtf(static_cast<float>(D)), err,
                 split_pages, part_acc, part_ml};
   const int gz = split_pages > 0 ? n_splits : 1;

@@ -78,7 +78,7 @@ class _Sig:
     b200_gdn_prefill = [P, I, P, P, P, P, P, P, P, P, P, P, P, I, P, I, P, P, P, I, I, I, I, I, F, I, P, P]
     b200_gdn_prefill_work_stride = [I]
     b200_ring_commit = [P, P, P, P, P, P, I, I, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
-    b200_flash_prefill = [P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P]
+    b200_flash_prefill = [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P]
     b200_attn_combine = [P, P, P, P, I, I, I, I, P]
 
 
@@ -624,7 +624,7 @@ def flash_prefill(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, b
         _, n_tiles, tiles_t, pos0_t = span_tables(seg_starts, [0] * len(seg_pos0), seg_pos0, R, dev).flash
     out = torch.empty(T, n_q * D, dtype=q.dtype, device=dev)
     rc = lib().b200_flash_prefill(
-        _ptr(q), _ptr(gate), _ptr(kv_layer), _ptr(out), _ptr(tiles_t), n_tiles, _ptr(pos0_t), _ptr(block_tables),
+        _ptr(q), _ptr(gate), _ptr(kv_layer), _ptr(out), _ptr(tiles_t), n_tiles, _ptr(pos0_t), None, _ptr(block_tables),
         block_tables.stride(0), kv_layer.shape[0], T, n_q, n_kv, D, 0, 1, None, None, 0, _ptr(err_word(dev)), _stream(),
     )
     _check(rc, "flash_prefill")
@@ -653,13 +653,14 @@ def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, bl
         _decode_tiles[key] = torch.stack([b, torch.zeros_like(b), b * G, torch.full_like(b, G)], 1).contiguous().to(dev)
     tiles = _decode_tiles[key]
     n_splits = max(1, (block_tables.shape[1] + SPLIT_PAGES - 1) // SPLIT_PAGES)
-    pos0 = positions[::G].to(torch.int32)
+    if positions.dtype != torch.int64 or not positions.is_contiguous():
+        positions = positions.to(torch.int64).contiguous()
     part_acc = torch.empty(rows, n_q, n_splits, D, dtype=torch.float32, device=dev)
     part_ml = torch.empty(rows, n_q, n_splits, 2, dtype=torch.float32, device=dev)
     out = torch.empty(rows, n_q * D, dtype=q.dtype, device=dev)
     L = lib()
     rc = L.b200_flash_prefill(
-        _ptr(q), _ptr(gate), _ptr(kv_layer), None, _ptr(tiles), B, _ptr(pos0), _ptr(block_tables),
+        _ptr(q), _ptr(gate), _ptr(kv_layer), None, _ptr(tiles), B, None, _ptr(positions), _ptr(block_tables),
         block_tables.stride(0), kv_layer.shape[0], rows, n_q, n_kv, D, SPLIT_PAGES, n_splits, _ptr(part_acc),
         _ptr(part_ml), 1 if (G == 1 and DECODE_ATTN_SMALL_TILES and n_q // n_kv <= 8) else 0, _ptr(err_word(dev)), _stream(),
     )
