@@ -343,8 +343,10 @@ class Model:
         if pp is not None and not pp.is_first:
             res, h = pp.recv(batch.tokens.shape[0], cfg.hidden_size, self.dtype, self.device)
         else:
-            x = ops.embed(batch.tokens, self.w.embed)
-            res, h = ops.add_rmsnorm(x, None, layers[0].input_norm, cfg.rms_norm_eps)
+            if hasattr(ops, "embed_rmsnorm"):
+                res, h = ops.embed_rmsnorm(batch.tokens, self.w.embed, layers[0].input_norm, cfg.rms_norm_eps)
+            else:
+                res, h = ops.add_rmsnorm(ops.embed(batch.tokens, self.w.embed), None, layers[0].input_norm, cfg.rms_norm_eps)
         for i, lw in enumerate(layers):
             nxt = layers[i + 1].input_norm if i + 1 < len(layers) else self.w.final_norm
             if lw.kind == "linear_attention":

@@ -26,17 +26,24 @@ __global__ void embed_kernel(const int64_t* tokens, const bf16* table, bf16* out
 
 // ------------------------------------------------------------------ (add +) RMSNorm
 // res' = bf16(res + x) (or x when res == nullptr); y = bf16(res' * rsqrt(mean(res'^2)+eps) * (1 + w)).
-// One CTA per row, 8 elements per thread per step. `res_out` may alias `res` or `x`.
-template <bool ZERO_CENTRED>
+// One CTA per row, 8 elements per thread per step. `res_out` may alias `res` or `x`. EMBED: row t of x is x[tokens[t]] (row 0
+// for a token outside the vocabulary): the pass's first two launches as one, 8.0 -> 4.9 us of a decode step, 35 -> 25 us at
+// 8192 rows.
+template <bool ZERO_CENTRED, bool EMBED = false>
 __global__ void add_rmsnorm_kernel(const bf16* x, const bf16* res, const bf16* w, bf16* res_out, bf16* y, int H,
-                                   float eps) {
+                                   float eps, const int64_t* tokens, int vocab) {
   pdl_wait();
   pdl_launch();
   const size_t row = static_cast<size_t>(blockIdx.x) * H;
+  size_t x_row = row;
+  if (EMBED) {
+    const int64_t tok = tokens[blockIdx.x];
+    x_row = tok < 0 || tok >= vocab ? 0 : static_cast<size_t>(tok) * H;
+  }
   extern __shared__ float vals[];  // H floats
   float ss = 0.f;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    uint4 xv = *reinterpret_cast<const uint4*>(x + row + i);
+    uint4 xv = *reinterpret_cast<const uint4*>(x + x_row + i);
     const bf16* xe = reinterpret_cast<const bf16*>(&xv);
     uint4 rv;
     const bf16* re = reinterpret_cast<const bf16*>(&rv);
@@ -294,7 +301,17 @@ extern "C" int b200_add_rmsnorm(const void* x, const void* res, const void* w, v
   auto k = zero_centred ? add_rmsnorm_kernel<true> : add_rmsnorm_kernel<false>;
   LAUNCHED(launch_pdl(k, dim3(T), dim3(threads), H * sizeof(float), st, static_cast<const bf16*>(x),
                       static_cast<const bf16*>(res), static_cast<const bf16*>(w), static_cast<bf16*>(res_out),
-                      static_cast<bf16*>(y), H, eps));
+                      static_cast<bf16*>(y), H, eps, static_cast<const int64_t*>(nullptr), 0));
+}
+
+// x [T, H] = table[tokens], y = its zero-centred RMSNorm.
+extern "C" int b200_embed_rmsnorm(const int64_t* tokens, const void* table, const void* w, void* x, void* y, int T, int H,
+                                  int vocab, float eps, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if (H % 8) return -7;
+  LAUNCHED(launch_pdl(add_rmsnorm_kernel<true, true>, dim3(T), dim3(H >= 2048 ? 256 : 128), H * sizeof(float), st,
+                      static_cast<const bf16*>(table), static_cast<const bf16*>(nullptr), static_cast<const bf16*>(w),
+                      static_cast<bf16*>(x), static_cast<bf16*>(y), H, eps, tokens, vocab));
 }
 
 // Routing only (any number of rows). `counts` may be null; when given it is zeroed here and receives rows per expert.

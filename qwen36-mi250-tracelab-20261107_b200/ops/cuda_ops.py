@@ -63,6 +63,7 @@ class _Sig:
     b200_argmax_finish = [P, P, I, I, P, P, P]
     b200_ivf_pick = [P, I, P, I, I, I, P, I, P, P, I, I, P, P, I, P, P]
     b200_embed = [P, P, P, I, I, I, P]
+    b200_embed_rmsnorm = [P, P, P, P, P, I, I, I, F, P]
     b200_add_rmsnorm = [P, P, P, P, P, I, I, F, I, P]
     b200_moe_route = [P, I, I, I, I, I, P, P, P, I, P, P]
     b200_moe_plan = [P, I, I, I, P, P, P, I, P, P, P, I, P, P]
@@ -362,6 +363,16 @@ def embed(tokens: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     out = torch.empty(T, table.shape[1], dtype=table.dtype, device=table.device)
     _check(lib().b200_embed(_ptr(tokens), _ptr(table), _ptr(out), T, table.shape[1], table.shape[0], _stream()), "embed")
     return out
+
+
+def embed_rmsnorm(tokens: torch.Tensor, table: torch.Tensor, w: torch.Tensor, eps: float):
+    """``(embed(tokens), add_rmsnorm(embed(tokens), None, w, eps)[1])`` in one launch."""
+    T, H = tokens.shape[0], table.shape[1]
+    x = torch.empty(T, H, dtype=table.dtype, device=table.device)
+    y = torch.empty_like(x)
+    _check(lib().b200_embed_rmsnorm(_ptr(tokens), _ptr(table), _ptr(w), _ptr(x), _ptr(y), T, H, table.shape[0], eps, _stream()),
+           "embed_rmsnorm")
+    return x, y
 
 
 # --------------------------------------------------------------------------- MoE

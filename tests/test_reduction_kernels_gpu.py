@@ -165,3 +165,16 @@ def test_greedy_head_with_infinite_and_undefined_logits(C, T, V):
 def _whole(rows, cols, seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
     return torch.randint(-2, 3, (rows, cols), device="cuda", generator=g).bfloat16()
+
+
+@pytest.mark.parametrize("H", [64, 2048, 2056])
+def test_embedding_with_the_first_norm_is_the_two_ops(H):
+    from b200serve.ops import cuda_ops as C
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    table = torch.randn(50, H, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(H, device="cuda", generator=g) * 0.1).bfloat16()
+    tokens = torch.tensor([0, 49, 7, 7, -1, 50, 31], device="cuda")  # two outside the table
+    x, y = C.embed_rmsnorm(tokens, table, w, 1e-6)
+    want = C.embed(tokens, table)
+    assert torch.equal(x, want) and torch.equal(y, C.add_rmsnorm(want, None, w, 1e-6)[1])
