@@ -325,6 +325,17 @@ __global__ void ring_commit_kernel(uint4* conv_state, uint4* rec_state, const ui
   for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < conv_row; i += static_cast<size_t>(gridDim.x) * blockDim.x)
     dst_c[i] = src_c[i];
 }
+
+// One slot of every layer's states to zero. Grid (chunks, layers). Bound by its launch: 6.3 MB of three layers in 2 us, where a
+// strided fill per tensor took 6.4.
+__global__ void reset_slot_kernel(uint4* conv_state, uint4* rec_state, int slot, int n_slots, size_t conv_row, size_t rec_row) {
+  pdl_wait();
+  pdl_launch();
+  const size_t at = static_cast<size_t>(blockIdx.y) * n_slots + slot;
+  const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<size_t>(gridDim.x) * blockDim.x;
+  for (size_t i = first; i < rec_row; i += step) rec_state[at * rec_row + i] = make_uint4(0, 0, 0, 0);
+  for (size_t i = first; i < conv_row; i += step) conv_state[at * conv_row + i] = make_uint4(0, 0, 0, 0);
+}
 }  // namespace b200
 
 using namespace b200;
@@ -341,6 +352,16 @@ extern "C" int b200_ring_commit(void* conv_state, void* rec_state, const void* r
       static_cast<uint4*>(conv_state), static_cast<uint4*>(rec_state), static_cast<const uint4*>(ring_conv),
       static_cast<const uint4*>(ring_rec), slots, keep, B, G, n_slots, conv_bytes / 16, rec_bytes / 16);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// conv_state [layers, n_slots, conv_bytes], rec_state [layers, n_slots, rec_bytes]; row sizes in bytes, multiples of 16.
+extern "C" int b200_reset_slot(void* conv_state, void* rec_state, int slot, int layers, int n_slots,
+                               unsigned long long conv_bytes, unsigned long long rec_bytes, cudaStream_t st) {
+  if (layers <= 0) return 0;
+  if (slot < 0 || slot >= n_slots || conv_bytes % 16 || rec_bytes % 16) return -7;
+  return launch_pdl(reset_slot_kernel, dim3(128, layers), dim3(256), 0, st, static_cast<uint4*>(conv_state),
+                    static_cast<uint4*>(rec_state), slot, n_slots, static_cast<size_t>(conv_bytes / 16),
+                    static_cast<size_t>(rec_bytes / 16)) == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int b200_gdn_decode(const void* mixed, int ld, const int* slots, void* conv_state, void* rec_state,

@@ -78,6 +78,7 @@ class _Sig:
     b200_paged_attn = [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, P]
     b200_gdn_prefill = [P, I, P, P, P, P, P, P, P, P, P, P, P, I, P, I, P, P, P, I, I, I, I, I, F, I, P, P]
     b200_gdn_prefill_work_stride = [I]
+    b200_reset_slot = [P, P, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
     b200_ring_commit = [P, P, P, P, P, P, I, I, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
     b200_flash_prefill = [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P]
     b200_attn_combine = [P, P, P, P, I, I, I, I, P]
@@ -520,6 +521,19 @@ def gdn_decode(mixed, slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnor
     )
     _check(rc, "gdn_decode")
     return out
+
+
+def reset_slot(conv_state: torch.Tensor, rec_state: torch.Tensor, slot: int) -> None:
+    """Zero one slot of the states ``[layers, slots, ...]`` of all layers in one launch; rows of multiples of 16 bytes."""
+    layers, n = rec_state.shape[:2]
+    assert conv_state.is_contiguous() and rec_state.is_contiguous() and conv_state.shape[:2] == (layers, n)
+    if not -n <= slot < n:
+        raise IndexError(f"slot {slot} of {n}")
+    with torch.cuda.device(rec_state.device):  # as a fill would, whatever the calling thread's current device is
+        rc = lib().b200_reset_slot(_ptr(conv_state), _ptr(rec_state), slot % n, layers, n,
+                                   conv_state[0, 0].numel() * conv_state.element_size(),
+                                   rec_state[0, 0].numel() * rec_state.element_size(), _stream())
+    _check(rc, "reset_slot")
 
 
 def ring_commit(conv_state, rec_state, ring, slots: torch.Tensor, keep_rows: torch.Tensor) -> None:

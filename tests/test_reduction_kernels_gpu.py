@@ -178,3 +178,17 @@ def test_embedding_with_the_first_norm_is_the_two_ops(H):
     x, y = C.embed_rmsnorm(tokens, table, w, 1e-6)
     want = C.embed(tokens, table)
     assert torch.equal(x, want) and torch.equal(y, C.add_rmsnorm(want, None, w, 1e-6)[1])
+
+
+@pytest.mark.parametrize("slot", [0, 3, -1])
+def test_reset_slot_zeroes_one_slot_of_every_layer(slot):
+    from b200serve.ops import cuda_ops as C
+
+    conv = torch.randn(3, 5, 264, 3, device="cuda").bfloat16()
+    rec = torch.randn(3, 5, 2, 32, 33, device="cuda")[:, :, :, :, :32].contiguous()
+    want_c, want_r = conv.clone(), rec.clone()
+    want_c[:, slot], want_r[:, slot] = 0.0, 0.0
+    C.reset_slot(conv, rec, slot)
+    assert torch.equal(conv, want_c) and torch.equal(rec, want_r)
+    with pytest.raises(IndexError):
+        C.reset_slot(conv, rec, 5)
