@@ -36,9 +36,13 @@ __device__ void plan_scatter(const int* idx, int n_pairs, int Et, int bt, int* o
   s_count[e] = 0;
   s_cur[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
+  int mine[2] = {-1, -1};  // the thread's first pairs: the second walk over the table need not fetch them again
+  int turn = 0;
+  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x, ++turn) {
     const int x = s_idx ? s_idx[i] : __ldcg(idx + i);  // through L2: other CTAs of the same launch may have written it
     if (x >= 0 && x < Et) atomicAdd(&s_count[x], 1);
+    if (turn == 0) mine[0] = x;
+    else if (turn == 1) mine[1] = x;
   }
   __syncthreads();
   const int c = e < Et ? s_count[e] : 0;
@@ -76,8 +80,9 @@ __device__ void plan_scatter(const int* idx, int n_pairs, int Et, int bt, int* o
     *n_tiles = total < max_tiles ? total : max_tiles;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int x = s_idx ? s_idx[i] : __ldcg(idx + i);
+  turn = 0;
+  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x, ++turn) {
+    const int x = turn == 0 ? mine[0] : turn == 1 ? mine[1] : s_idx ? s_idx[i] : __ldcg(idx + i);
     if (x < 0) { inv[i] = -1; continue; }  // pair served by another rank
     if (x >= Et) { atomicCAS(err, 0, ERR_BAD_INDEX); inv[i] = -1; continue; }
     const int pos = s_off[x] + atomicAdd(&s_cur[x], 1);
@@ -119,7 +124,8 @@ moe_route_plan_kernel(const float* logits, int ldl, int T, int E, int top_k, int
   plan_scatter(idx, T * P, Et, bt, offsets, tiles, n_tiles, max_tiles, perm, inv, err, P, src_rows, fits ? s_idx : nullptr);
 }
 
-// Any number of rows, still one launch: a grid of 1024-thread CTAs routes 32 rows each; the CTA that finishes last
+// Any number of rows, still one launch: a grid of 1024-thread CTAs routes up to 32 rows each, shared evenly (a row is one warp's
+// 500 instructions, and 32 of them on one SM wait for each other); the CTA that finishes last
 // (a ticket counter in global memory, which it puts back to zero for the next launch) builds the plan from the whole
 // index table. Everything the other CTAs wrote is visible to it: they fence before taking their ticket.
 // `work` (optional): 2 * 1024 ints kept zero between launches (per-expert counts, per-expert cursors). With it the
@@ -138,15 +144,15 @@ moe_route_plan_grid_kernel(const float* logits, int ldl, int T, int E, int top_k
   __shared__ int s_hist[1024];
   const int P = top_k + (shared ? 1 : 0);
   const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 32 + (threadIdx.x >> 5);
+  const int rows = (T + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);  // at most 32
+  const int row0 = blockIdx.x * rows, r = row0 + (threadIdx.x >> 5);
   if (work) s_hist[threadIdx.x] = 0;
-  if (r < T)
+  if (r < min(T, row0 + rows))
     route_row<PER_LANE>(logits + static_cast<size_t>(r) * ldl, E, top_k, shared, wts + static_cast<size_t>(r) * P,
                         idx + static_cast<size_t>(r) * P, expert_map, nullptr, lane);
   if (work) {
     __syncthreads();  // this CTA's 32 rows of idx are written (and visible to the CTA)
-    const int row0 = blockIdx.x * 32;
-    const int n_here = min(32, T - row0) * P;
+    const int n_here = max(0, min(rows, T - row0)) * P;
     for (int i = threadIdx.x; i < n_here; i += blockDim.x) {
       const int x = idx[static_cast<size_t>(row0) * P + i];
       if (x >= 0 && x < Et) atomicAdd(&s_hist[x], 1);
@@ -192,16 +198,16 @@ moe_route_plan_grid_kernel(const float* logits, int ldl, int T, int E, int top_k
     w_rows[lane] = a; w_tiles[lane] = b2;
   }
   __syncthreads();
-  const int row0 = sc - c + (w ? w_rows[w - 1] : 0);
+  const int at = sc - c + (w ? w_rows[w - 1] : 0);
   const int tile0 = stl - t + (w ? w_tiles[w - 1] : 0);
   if (e < Et) {
-    offsets[e] = row0;
-    const int rows = tile_rows(c, t, bt);
-    for (int i = 0, ti = tile0; i * rows < c && ti < max_tiles; ++i, ++ti)
-      tiles[ti] = make_int4(e, row0 + i * rows, min(rows, c - i * rows), 0);
+    offsets[e] = at;
+    const int step = tile_rows(c, t, bt);
+    for (int i = 0, ti = tile0; i * step < c && ti < max_tiles; ++i, ++ti)
+      tiles[ti] = make_int4(e, at + i * step, min(step, c - i * step), 0);
   }
   if (e == Et - 1) {
-    offsets[Et] = row0 + c;
+    offsets[Et] = at + c;
     const int total = tile0 + t;
     *n_tiles = total < max_tiles ? total : max_tiles;
   }
