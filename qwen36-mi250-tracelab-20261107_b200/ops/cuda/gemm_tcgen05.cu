@@ -957,7 +957,13 @@ static int pair_rows(int T, int N) {
 //   9216    24.6 -> 21.3  26.7 -> 23.6  27.6 -> 23.6  27.5 -> 25.3  41.0 -> 36.9  63.5 -> 57.3  203 -> 186
 //   2048    20.5 -> 22.5  23.5 -> 22.6  35.8 -> 22.6  35.5 -> 23.3  36.9 -> 24.6  36.9 -> 32.8  113 -> 86
 // (12352 and 9216 x 2048, 2048 x 4096). A single pair of weight tiles would leave half of one idle below 256 columns.
-static bool pair_pays(int T, int N) { return N >= 2 * BM && (T > 256 || (T > 128 && N > 32 * BM)); }
+// Many weight tiles and 33 to 128 rows, in chains of norm and projection: 12352 x 2048 at 64 rows 15.7 -> 14.0, 9216 x 2048
+// at 64 14.6 -> 13.5, at 128 15.1 -> 13.9; but 12352 at 80 13.6 -> 14.3: above 64 rows 128-row tiles stay while more than half
+// of the SMs get one.
+static bool pair_pays(int T, int N) {
+  const int n = (N + BM - 1) / BM;
+  return N >= 2 * BM && (T > 256 || (N > 32 * BM && (T > 128 || (T > 32 && (T <= 64 || 2 * n <= sm_count())))));
+}
 
 // Dense bf16 GEMM with two SMs per tile.
 static int launch_pair_dense(const void* X, const void* W, GemmParams p, int ldx, int ldw, int packed, cudaStream_t st) {
