@@ -1015,17 +1015,18 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
   return -5;
 }
 
-// Gate/up GEMM of the experts of a few rows (16-row token tiles, at most one per pair, tile-packed weights): each 128-row
-// tile becomes four when that still leaves at most one CTA per SM, two when at most two. This GEMM in a decode step, us: 1 row
-// 14.7 as two operands of 128-row MMAs -> 9.2 as one. Whole block with the two operands against plain tiles: 1 row 41.5 ->
-// 30.7, 2 rows 46.1 -> 39.4, 4 rows 54.8 -> 52.7; at 8 rows the plain tiles are as good (77.3, thin 78.9). The down
-// projection (16 weight tiles per expert) has CTAs enough at one row. Returns 1 when the plain form is to run.
+// Gate/up GEMM of the experts with token tiles of 16 or 32 rows and tile-packed weights: tiles of 64 gate and 64 up rows, or of
+// 32 and 32 while that leaves at most one CTA per SM (16-row token tiles, at most one per pair). A tile is one operand and not
+// two of 128 rows, and twice as many tiles spread more evenly over the SMs. This GEMM, us, 128-row tiles -> these: 1 row of 9
+// pairs 14.7 -> 9.2, 5 rows 40.5 -> 34.8, 13: 75.3 -> 71.7, 40: 140 -> 132, 128: 176.6 -> 170.2, 256: 179.5 -> 179; 32-row
+// token tiles, 700 rows: 183 -> 180, 1024: 209 -> 191. (Tiles of 32 and 32 for all: 13 rows 73.7, 128: 175; 64-row token tiles
+// are as good with 128 rows: 1300 rows 186 and 190.) The down projection has 16 weight tiles per expert and CTAs enough at
+// one row. Returns 1 when the plain form is to run.
 static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
-                               int max_tiles, cudaStream_t st) {
+                               int max_tiles, int bt, cudaStream_t st) {
   const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
-  const int sms = sm_count(), rt = 4 * tiles <= sms ? 32 : 2 * tiles <= 2 * sms ? 64 : BM;
-  const int kps = rt == 32 ? 4 : 2;
-  if (rt == BM || p.K % (kps * BK) || p.N % BM) return 1;
+  const int rt = bt == 16 && 4 * tiles <= sm_count() ? 32 : 64, kps = rt == 32 ? 4 : 2;
+  if (p.K % (kps * BK) || p.N % BM) return 1;
   CUtensorMap tw, tx;
   const uint64_t nk = p.K / BK;
   p.packed = 1;
@@ -1037,7 +1038,8 @@ static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E
     p.ldgx = ldx;
   }
   // with row indices the producer never reads through this map, but it has to be a valid one
-  if (make_map_kblocks(&tx, X, gather_rows ? 16 : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, 16, kps)) return -1;
+  if (make_map_kblocks(&tx, X, gather_rows ? bt : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, bt, kps)) return -1;
+  if (bt == 32) return launch<32, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
   if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 4>(tw, tx, p, max_tiles, st);
   return launch<16, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
 }
@@ -1112,8 +1114,8 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   CUtensorMap tw, tx;
   GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
-  if (packed && splits == 1 && bt == 16 && epi == EPI_SILU_MUL) {
-    const int rc = launch_thin_grouped(X, W, p, E, gather_rows, ldx, max_tiles, st);
+  if (packed && splits == 1 && bt <= 32 && epi == EPI_SILU_MUL) {
+    const int rc = launch_thin_grouped(X, W, p, E, gather_rows, ldx, max_tiles, bt, st);
     if (rc <= 0) return rc;
   }
   if (weight_map(&tw, W, E, N, w_rows, K, K, epi == EPI_SILU_MUL, packed, &p)) return -1;
