@@ -360,7 +360,7 @@ extern "C" int b200_moe_route_plan(const float* logits, int ldl, int T, int E, i
     return -4;
   if (work == nullptr) return 0;
   const int n_pairs = T * (top_k + (shared ? 1 : 0));
-  LAUNCHED(launch_pdl(moe_scatter_kernel, dim3(min((n_pairs + 255) / 256, 592)), dim3(256), 0, st,
+  LAUNCHED(launch_pdl(moe_scatter_kernel, dim3(min((n_pairs + 256 * SCATTER_PER - 1) / (256 * SCATTER_PER), 592)), dim3(256), 0, st,
                       static_cast<const int*>(idx), n_pairs, Et, static_cast<const int*>(offsets), work + 1024, perm, inv,
                       err, top_k + (shared ? 1 : 0), src_rows));
 }

@@ -36,14 +36,28 @@ __device__ void plan_scatter(const int* idx, int n_pairs, int Et, int bt, int* o
   s_count[e] = 0;
   s_cur[e] = 0;
   __syncthreads();
-  int mine[2] = {-1, -1};  // the thread's first pairs: the second walk over the table need not fetch them again
-  int turn = 0;
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x, ++turn) {
-    const int x = s_idx ? s_idx[i] : __ldcg(idx + i);  // through L2: other CTAs of the same launch may have written it
-    if (x >= 0 && x < Et) atomicAdd(&s_count[x], 1);
-    if (turn == 0) mine[0] = x;
-    else if (turn == 1) mine[1] = x;
+  const auto fetch = [&](int i) {
+    return s_idx ? s_idx[i] : __ldcg(idx + i);  // through L2: other CTAs of the same launch may have written it
+  };
+  // A thread keeps its first pairs and the places that counting them gave them among their expert's, so that they need no second
+  // fetch and no second counter (every row counts at the shared expert: its counter is what such a walk waits for). The pairs
+  // behind those are counted first and take the first places by a second walk.
+  constexpr int KEEP = 5;
+  if (n_pairs > KEEP * 1024) {
+    for (int i = KEEP * 1024 + threadIdx.x; i < n_pairs; i += blockDim.x) {
+      const int x = fetch(i);
+      if (x >= 0 && x < Et) atomicAdd(&s_count[x], 1);
+    }
+    __syncthreads();
   }
+  int mine[KEEP], place[KEEP];
+#pragma unroll
+  for (int u = 0; u < KEEP; ++u) {
+    const int i = u * 1024 + threadIdx.x;
+    mine[u] = i < n_pairs ? fetch(i) : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < KEEP; ++u) place[u] = mine[u] >= 0 && mine[u] < Et ? atomicAdd(&s_count[mine[u]], 1) : 0;
   __syncthreads();
   const int c = e < Et ? s_count[e] : 0;
   const int t = (c + bt - 1) / bt;
@@ -80,15 +94,22 @@ __device__ void plan_scatter(const int* idx, int n_pairs, int Et, int bt, int* o
     *n_tiles = total < max_tiles ? total : max_tiles;
   }
   __syncthreads();
-  turn = 0;
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x, ++turn) {
-    const int x = turn == 0 ? mine[0] : turn == 1 ? mine[1] : s_idx ? s_idx[i] : __ldcg(idx + i);
-    if (x < 0) { inv[i] = -1; continue; }  // pair served by another rank
-    if (x >= Et) { atomicCAS(err, 0, ERR_BAD_INDEX); inv[i] = -1; continue; }
-    const int pos = s_off[x] + atomicAdd(&s_cur[x], 1);
+  const auto put = [&](int i, int x, int at) {
+    if (x < 0) { inv[i] = -1; return; }  // pair served by another rank
+    if (x >= Et) { atomicCAS(err, 0, ERR_BAD_INDEX); inv[i] = -1; return; }
+    const int pos = s_off[x] + at;
     perm[pos] = i;
     inv[i] = pos;
     if (src_rows) src_rows[pos] = i / P;  // the activation row behind sorted position pos (for a gathering GEMM)
+  };
+#pragma unroll
+  for (int u = 0; u < KEEP; ++u) {
+    const int i = u * 1024 + threadIdx.x;
+    if (i < n_pairs) put(i, mine[u], place[u]);
+  }
+  for (int i = KEEP * 1024 + threadIdx.x; i < n_pairs; i += blockDim.x) {
+    const int x = fetch(i);
+    put(i, x, x >= 0 && x < Et ? atomicAdd(&s_cur[x], 1) : 0);
   }
 }
 
@@ -213,20 +234,44 @@ moe_route_plan_grid_kernel(const float* logits, int ldl, int T, int E, int top_k
   }
 }
 
-// Second half of the plan at prefill sizes: every pair takes the next free position of its expert's run
-// (a global cursor per expert, zero before the launch; the order inside an expert does not influence any output).
-__global__ void moe_scatter_kernel(const int* idx, int n_pairs, int Et, const int* offsets, int* cursors, int* perm,
-                                   int* inv, int* err, int P, int* src_rows) {
+// Second half of the plan at prefill sizes: every pair takes a free position of its expert's run (the order inside an expert
+// does not influence any output). A CTA counts the pairs of SCATTER_PAIRS in shared memory, takes that many places of each
+// expert at once (a global cursor per expert, zero before the launch) and hands them out. One global atomic per pair made
+// the launch wait for the shared expert's cursor, which every row takes a place of: 8192 rows 16.2 -> 4.9 us, 2048: 5.4 -> 4.1.
+constexpr int SCATTER_PER = 4;  // pairs per thread
+__global__ void __launch_bounds__(256)
+moe_scatter_kernel(const int* idx, int n_pairs, int Et, const int* offsets, int* cursors, int* perm, int* inv, int* err, int P,
+                   int* src_rows) {
+  __shared__ int s_count[1024], s_base[1024];
   pdl_wait();
   pdl_launch();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pairs; i += gridDim.x * blockDim.x) {
-    const int x = idx[i];
-    if (x < 0) { inv[i] = -1; continue; }  // pair served by another rank
-    if (x >= Et) { atomicCAS(err, 0, ERR_BAD_INDEX); inv[i] = -1; continue; }
-    const int pos = offsets[x] + atomicAdd(&cursors[x], 1);
-    perm[pos] = i;
-    inv[i] = pos;
-    if (src_rows) src_rows[pos] = i / P;
+  for (int first = blockIdx.x * blockDim.x * SCATTER_PER; first < n_pairs; first += gridDim.x * blockDim.x * SCATTER_PER) {
+    for (int e = threadIdx.x; e < Et; e += blockDim.x) s_count[e] = 0;
+    __syncthreads();
+    int x[SCATTER_PER], place[SCATTER_PER];
+#pragma unroll
+    for (int u = 0; u < SCATTER_PER; ++u) {
+      const int i = first + u * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x);
+      x[u] = i < n_pairs ? idx[i] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < SCATTER_PER; ++u) place[u] = x[u] >= 0 && x[u] < Et ? atomicAdd(&s_count[x[u]], 1) : 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < Et; e += blockDim.x)
+      if (s_count[e]) s_base[e] = offsets[e] + atomicAdd(&cursors[e], s_count[e]);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < SCATTER_PER; ++u) {
+      const int i = first + u * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x);
+      if (i >= n_pairs) continue;
+      if (x[u] < 0) { inv[i] = -1; continue; }  // pair served by another rank
+      if (x[u] >= Et) { atomicCAS(err, 0, ERR_BAD_INDEX); inv[i] = -1; continue; }
+      const int pos = s_base[x[u]] + place[u];
+      perm[pos] = i;
+      inv[i] = pos;
+      if (src_rows) src_rows[pos] = i / P;
+    }
+    __syncthreads();  // the counters are cleared again
   }
 }
 
