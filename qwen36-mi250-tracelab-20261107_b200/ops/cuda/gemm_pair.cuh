@@ -14,16 +14,22 @@ namespace b200 {
 
 constexpr int PAIR_BT = 256;      // most token rows of a tile
 constexpr int PAIR_N_STEP = 32;   // the MMA's column count is a multiple of this when it has 256 rows
-constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_A_BYTES = BM * BK * 2;
-constexpr int PAIR_B_BYTES = PAIR_BT / 2 * BK * 2;
-constexpr int PAIR_STAGE_BYTES = PAIR_A_BYTES + PAIR_B_BYTES;
 constexpr int PAIR_GROUPS = 2;    // epilogue warpgroups: they take alternate batches of 16 token columns
 constexpr int PAIR_GATHER_WARP = 2 + 4 * PAIR_GROUPS;  // the row-fetching warps: warp 0 and three behind the epilogue's
 constexpr int PAIR_GATHER_WARPS = 4;
 constexpr int pair_threads(int epi) { return 32 * (epi == EPI_SILU_MUL ? PAIR_GATHER_WARP + PAIR_GATHER_WARPS - 1 : PAIR_GATHER_WARP); }
 constexpr int PAIR_OUT_BYTES = 2 * 16 * BM * 2;  // per group: two staging buffers (SiLU: the exchange and one buffer)
-constexpr int PAIR_SMEM = 1024 + PAIR_STAGES * PAIR_STAGE_BYTES + 256 + PAIR_GROUPS * PAIR_OUT_BYTES;
+
+// PBT: most token rows of a tile, 256 or 128. Tiles of up to 128 rows leave room for eight stages instead of six, which is 128 KB
+// of weights on their way to an SM and not 96: expert block of 64 rows per expert, gate/up 202 -> 193 us, down 99 -> 96.
+template <int PBT>
+struct PairCfg {
+  static constexpr int B_BYTES = PBT / 2 * BK * 2;
+  static constexpr int STAGE_BYTES = PAIR_A_BYTES + B_BYTES;
+  static constexpr int STAGES = PBT == 256 ? 6 : 8;
+  static constexpr int SMEM = 1024 + STAGES * STAGE_BYTES + 256 + PAIR_GROUPS * PAIR_OUT_BYTES;
+};
 
 // Whether `ok` holds in all 128 threads of epilogue group `id - 2`.
 __device__ __forceinline__ bool group_all(bool ok, int id) {
@@ -41,23 +47,25 @@ __device__ __forceinline__ void group_sync(int id) { asm volatile("barrier.cta.s
 // EPI_BF16 (dense, or grouped with rows that are sorted already) or EPI_SILU_MUL (grouped, rows fetched by index,
 // tile-packed weights). In a SiLU tile a CTA's 128 accumulator rows are 64 gate rows and the 64 up rows
 // that go with them.
-template <int EPI, bool GROUPED>
+template <int EPI, bool GROUPED, int PBT>
 __global__ void __launch_bounds__(pair_threads(EPI), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, GemmParams p) {
   constexpr bool SILU = EPI == EPI_SILU_MUL;
   constexpr int PAIR_ROWS = SILU ? BM : 2 * BM;  // output columns of a tile
   constexpr int CTA_ROWS = PAIR_ROWS / 2;
+  constexpr int STAGES = PairCfg<PBT>::STAGES, STAGE_BYTES = PairCfg<PBT>::STAGE_BYTES;
+  constexpr int LANE_ROWS = PBT / 8;  // of a CTA's half of the rows, fetched by a group of eight lanes
   static_assert(EPI == EPI_BF16 || (SILU && GROUPED), "epilogues of the pair form");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + PAIR_STAGES * PAIR_STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full = bars;                         // used in the first CTA: both CTAs' loads are counted there
-  uint64_t* empty = bars + PAIR_STAGES;          // one in each CTA, the MMAs' commits arrive at both
-  uint64_t* acc_full = bars + 2 * PAIR_STAGES;   // [2], both CTAs
+  uint64_t* empty = bars + STAGES;          // one in each CTA, the MMAs' commits arrive at both
+  uint64_t* acc_full = bars + 2 * STAGES;   // [2], both CTAs
   uint64_t* acc_empty = acc_full + 2;            // [2], used in the first CTA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* out_stage = smem + PAIR_STAGES * PAIR_STAGE_BYTES + 256;
+  uint8_t* out_stage = smem + STAGES * STAGE_BYTES + 256;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -67,7 +75,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   const int num_k = p.K / BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < PAIR_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], SILU ? 3 : 1);  // the announcement of bytes, and of each CTA's rows
       mbar_init(&empty[s], 1);
     }
@@ -133,18 +141,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       int nx, expert, row0, nrows;
       tile_geom(tile, nx, expert, row0, nrows);
       const int cols = columns(nrows), half = cols / 2, t0 = static_cast<int>(rank) * half;
-      int g[32];
+      int g[LANE_ROWS];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {  // (columns behind the last row keep what they hold: nobody reads their results)
+      for (int i = 0; i < LANE_ROWS; ++i) {  // (columns behind the last row keep what they hold: nobody reads their results)
         const int r = (lane >> 3) + 4 * i;
         g[i] = r < half && t0 + r < nrows ? p.gather_rows[row0 + t0 + r] : -1;
       }
       int kb = first;
       for (; kb < num_k; kb += PAIR_GATHER_WARPS, it += PAIR_GATHER_WARPS) {
-        const int s = it % PAIR_STAGES;
-        const uint32_t ph = (it / PAIR_STAGES) & 1;
+        const int s = it % STAGES;
+        const uint32_t ph = (it / STAGES) & 1;
         if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
-        uint8_t* st = smem + s * PAIR_STAGE_BYTES;
+        uint8_t* st = smem + s * STAGE_BYTES;
         const uint32_t bar = dsmem_addr(smem_u32(&full[s]), 0);
         if (lane == 0) {
           if (rank == 0) mbar_expect_tx(&full[s], 2 * PAIR_A_BYTES);
@@ -153,7 +161,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const uint32_t xb = smem_u32(st + PAIR_A_BYTES);
         const bf16* gx = p.gx + kb * BK + j * 8;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < LANE_ROWS; ++i) {
           const int r = (lane >> 3) + 4 * i;
           if (g[i] >= 0)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
@@ -177,10 +185,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       if (!GROUPED && tile0 < total) {
         int nx, expert, row0, nrows;
         tile_geom(tile0, nx, expert, row0, nrows);
-        pre = num_k < PAIR_STAGES ? num_k : PAIR_STAGES;
+        pre = num_k < STAGES ? num_k : STAGES;
         for (int kb = 0; kb < pre; ++kb) {
           if (rank == 0) mbar_expect_tx(&full[kb], dense_bytes);
-          load_weights(smem + kb * PAIR_STAGE_BYTES, dsmem_addr(smem_u32(&full[kb]), 0), nx, 0, kb);
+          load_weights(smem + kb * STAGE_BYTES, dsmem_addr(smem_u32(&full[kb]), 0), nx, 0, kb);
         }
       }
       pdl_wait();
@@ -192,9 +200,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         // grouped: boxes of VAR_BOX rows, as many as cover the half
         const int boxes = (half + VAR_BOX - 1) / VAR_BOX;
         for (int kb = 0; kb < num_k; ++kb, ++it) {
-          const int s = it % PAIR_STAGES;
-          const uint32_t ph = (it / PAIR_STAGES) & 1;
-          uint8_t* st = smem + s * PAIR_STAGE_BYTES;
+          const int s = it % STAGES;
+          const uint32_t ph = (it / STAGES) & 1;
+          uint8_t* st = smem + s * STAGE_BYTES;
           const uint32_t bar = dsmem_addr(smem_u32(&full[s]), 0);
           if (it >= pre) {
             if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
@@ -225,11 +233,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         ok = mbar_wait(&acc_empty[acc], ((lt >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
         if (ok) tc_fence_after();
         for (int kb = 0; kb < num_k && ok; ++kb, ++it) {
-          const int s = it % PAIR_STAGES;
-          ok = mbar_wait(&full[s], (it / PAIR_STAGES) & 1, p.err, ERR_WAIT_FULL, abort_flag);
+          const int s = it % STAGES;
+          ok = mbar_wait(&full[s], (it / STAGES) & 1, p.err, ERR_WAIT_FULL, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * PAIR_STAGE_BYTES);
+          const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_bf16_pair(tmem, umma_smem_desc(a_addr + k * UMMA_K * 2), umma_smem_desc(a_addr + PAIR_A_BYTES + k * UMMA_K * 2),

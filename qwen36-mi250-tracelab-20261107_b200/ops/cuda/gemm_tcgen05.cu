@@ -864,16 +864,14 @@ struct DenseForm {
   int bt, rt, kps;  // token rows per tile, weight rows per tile, k-blocks per stage
 };
 
-// The form of a dense bf16 / fp32 GEMM. It never changes a row's bits (every element sees the same k order in the same
-// instruction shape), so it may follow the number of rows. Measured in chains of launches on weights that are not in L2, us,
-// plain form -> chosen form; 12352 x 2048 is a GDN layer's input projection, 9216 x 2048 an attention layer's, 2048 x 4096
-// the output projection, 257 x 2048 the router (taken before thin tiles had MMAs of 64 rows and SMs of their own, which
-// brought 2048 x 4096 of one row from 9.3 to 7.9 us, 257 x 2048 from 5.7 to 4.9, 9216 x 2048 from 8.4 to 7.4 in a step):
-//   up to 16 rows     12352: 13.0 -> 12.0   9216: 11.6 -> 10.4   2048: 15.4 -> 10.9   257: 8.5 -> 6.3
-//   32 rows           12352: 14.5 -> 13.0   9216: 13.3 -> 12.1   2048: 15.2 -> 11.1   257: 8.5 -> 6.3
-//   61 rows           12352: 16.6 -> 15.4   9216: 15.5 -> 14.2   2048: 14.7 -> 12.5   257: 8.4 -> 6.5
-//   128 rows          12352: 16.9           9216: 16.2 -> 14.5   2048: 15.0 -> 13.8   257: 8.4 -> 6.5
-//   256 rows          12352: 25.1           9216: 24.2 -> 17.6   2048: 16.1           257: 8.4 -> 7.0
+// The form of a dense bf16 / fp32 GEMM with one SM per tile. It never changes a row's bits (every element sees the same k order
+// in the same products), so it may follow the number of rows. Measured in chains of launches on weights that are not in L2, us,
+// 128-row tiles with one k-block per stage -> chosen form; 12352 x 2048 is a GDN layer's input projection, 9216 x 2048 an
+// attention layer's, 2048 x 4096 the output projection, 257 x 2048 the router (in a decode step):
+//   up to 16 rows     12352: 13.0 -> 12.0   9216: 11.6 -> 7.4   2048: 15.4 -> 7.9   257: 8.5 -> 4.9
+//   61 rows           2048: 14.7 -> 11.5   257: 8.4 -> 5.0
+//   128 rows          2048: 15.0 -> 10.3   257: 8.4 -> 5.3
+//   256 rows          2048: 16.1 -> 13.0   257: 8.4 -> 5.3
 static DenseForm dense_form(int T, int N, int K, bool packed) {
   const int sms = sm_count();
   const auto tiles = [&](int rt, int bt) { return static_cast<long long>((N + rt - 1) / rt) * ((T + bt - 1) / bt); };
@@ -899,8 +897,6 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
     if (by4 && tiles(64, 64) <= lim) return {64, 64, 4};
     return {16, BM, 1};
   }
-  if (by2 && T <= 64 && tiles(64, 64) <= 2 * sms) return {T <= 32 ? 32 : 64, 64, 2};
-  if (by2 && T <= 128 && tiles(64, 64) <= 2 * sms) return {64, 64, 2};
   if (T > 256) {
     // few weight tiles and many rows (the router): the narrowest token tile whose CTAs are resident together, as long as the
     // K loop of a CTA and not the rows it reads sets the time. Router, 257 x 2048, us, 256-row tiles -> these: 300 rows
@@ -913,22 +909,23 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
 }
 
 constexpr int PAIR_FORM = -256;  // token tile of up to 256 rows on two SMs, in the `bt` argument of the launchers
+constexpr int PAIR_FORM_128 = -128;  // of up to 128 rows
 
 // Two SMs per tile (gemm_pair.cuh). A cluster's CTAs sit on one SM each; the persistent grid is one cluster per pair of SMs.
-template <int EPI, bool GROUPED>
+template <int EPI, bool GROUPED, int PBT>
 static int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, GemmParams p, int grid_y, cudaStream_t st) {
-  auto kern = gemm_pair_kernel<EPI, GROUPED>;
+  auto kern = gemm_pair_kernel<EPI, GROUPED, PBT>;
   static bool configured[MAX_DEVICES] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return -3;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<PBT>::SMEM) != cudaSuccess) return -3;
     configured[dev] = true;
   }
   p.grid_y = grid_y;
   const int rows = EPI == EPI_SILU_MUL ? BM : 2 * BM;
   const long long tiles = static_cast<long long>((p.N + rows - 1) / rows) * grid_y, pairs = sm_count() / 2;
-  return launch_clusters(2, kern, dim3(2 * static_cast<unsigned>(tiles < pairs ? tiles : pairs)), dim3(pair_threads(EPI)), PAIR_SMEM,
+  return launch_clusters(2, kern, dim3(2 * static_cast<unsigned>(tiles < pairs ? tiles : pairs)), dim3(pair_threads(EPI)), PairCfg<PBT>::SMEM,
                          st, tw, tx, p) == cudaSuccess ? 0 : -4;
 }
 
@@ -957,13 +954,10 @@ static int pair_rows(int T, int N) {
 //   9216    24.6 -> 21.3  26.7 -> 23.6  27.6 -> 23.6  27.5 -> 25.3  41.0 -> 36.9  63.5 -> 57.3  203 -> 186
 //   2048    20.5 -> 22.5  23.5 -> 22.6  35.8 -> 22.6  35.5 -> 23.3  36.9 -> 24.6  36.9 -> 32.8  113 -> 86
 // (12352 and 9216 x 2048, 2048 x 4096). A single pair of weight tiles would leave half of one idle below 256 columns.
-// Many weight tiles and 33 to 128 rows, in chains of norm and projection: 12352 x 2048 at 64 rows 15.7 -> 14.0, 9216 x 2048
-// at 64 14.6 -> 13.5, at 128 15.1 -> 13.9; but 12352 at 80 13.6 -> 14.3: above 64 rows 128-row tiles stay while more than half
-// of the SMs get one.
-static bool pair_pays(int T, int N) {
-  const int n = (N + BM - 1) / BM;
-  return N >= 2 * BM && (T > 256 || (N > 32 * BM && (T > 128 || (T > 32 && (T <= 64 || 2 * n <= sm_count())))));
-}
+// Many weight tiles and 17 to 128 rows, in chains of norm and projection, 64- or 128-row tiles of one SM -> pair: 12352 x 2048 at
+// 24 rows 13.0 -> 13.0, at 64 15.7 -> 13.4, at 128 15.0 -> 14.4; 9216 x 2048 at 24 rows 11.4 -> 11.6, at 64 14.6 -> 12.9, at 128
+// 15.1 -> 13.2.
+static bool pair_pays(int T, int N) { return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM)); }
 
 // Dense bf16 GEMM with two SMs per tile.
 static int launch_pair_dense(const void* X, const void* W, GemmParams p, int ldx, int ldw, int packed, cudaStream_t st) {
@@ -971,11 +965,13 @@ static int launch_pair_dense(const void* X, const void* W, GemmParams p, int ldx
   p.pair_bt = pair_rows(p.T, p.N);
   if (weight_map(&tw, W, 0, p.N, p.N, p.K, ldw, false, packed, &p)) return -1;
   if (make_map(&tx, X, p.K, p.T, 0, ldx, 0, p.pair_bt / 2)) return -1;
-  return launch_pair<EPI_BF16, false>(tw, tx, p, (p.T + p.pair_bt - 1) / p.pair_bt, st);
+  const int gy = (p.T + p.pair_bt - 1) / p.pair_bt;
+  return p.pair_bt <= 128 ? launch_pair<EPI_BF16, false, 128>(tw, tx, p, gy, st) : launch_pair<EPI_BF16, false, PAIR_BT>(tw, tx, p, gy, st);
 }
 
-// Grouped GEMMs with two SMs per tile of up to 256 rows: gate/up with rows by index, or a bf16 projection of sorted rows.
+// Grouped GEMMs with two SMs per tile of up to PBT rows: gate/up with rows by index, or a bf16 projection of sorted rows.
 // Tile-packed weights only.
+template <int PBT>
 static int launch_pair_grouped(const void* X, const void* W, GemmParams p, int E, int w_rows, int epi, const int* gather_rows,
                                int ldx, int max_tiles, cudaStream_t st) {
   CUtensorMap tw, tx;
@@ -983,7 +979,7 @@ static int launch_pair_grouped(const void* X, const void* W, GemmParams p, int E
   if (weight_map(&tw, W, E, p.N, w_rows, p.K, p.K, silu, 1, &p)) return -1;
   if (!silu) {
     if (make_map(&tx, X, p.K, p.T, 0, p.K, 0, VAR_BOX)) return -1;
-    return launch_pair<EPI_BF16, true>(tw, tx, p, max_tiles, st);
+    return launch_pair<EPI_BF16, true, PBT>(tw, tx, p, max_tiles, st);
   }
   // a CTA's half of a k-block of a tile: 64 gate rows, then 64 up rows
   const uint64_t nk = p.K / BK;
@@ -992,7 +988,7 @@ static int launch_pair_grouped(const void* X, const void* W, GemmParams p, int E
   p.gx = static_cast<const bf16*>(X);
   p.ldgx = ldx;
   if (make_map(&tx, X, p.K, 1, 0, ldx, 0, 1)) return -1;  // never read through, but a valid map
-  return launch_pair<EPI_SILU_MUL, true>(tw, tx, p, max_tiles, st);
+  return launch_pair<EPI_SILU_MUL, true, PBT>(tw, tx, p, max_tiles, st);
 }
 
 // Launch of a thin dense form; -5 where there is no such form.
@@ -1010,8 +1006,6 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
   if (f.bt == 16 && f.rt == 64 && f.kps == 2) return launch<16, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 32 && f.rt == 64 && f.kps == 4) return launch<32, EPI, false, 64, 4>(tw, tx, p, gy, st);
   if (f.bt == 64 && f.rt == 64 && f.kps == 4) return launch<64, EPI, false, 64, 4>(tw, tx, p, gy, st);
-  if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
-  if (f.bt == 64 && f.rt == 64 && f.kps == 2) return launch<64, EPI, false, 64, 2>(tw, tx, p, gy, st);
   return -5;
 }
 
@@ -1104,11 +1098,12 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   // gather_rows != null (token tiles of at most GATHER_BT_MAX rows): X is [any rows, ldx] and sorted position i reads row
   // gather_rows[i] of it; otherwise X is the expert-sorted buffer [cap, K] itself.
   if (max_tiles <= 0) return 0;
-  if (bt == PAIR_FORM) {
+  if (bt == PAIR_FORM || bt == PAIR_FORM_128) {
     GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, 1, nullptr, {}};
     if (!packed || splits > 1 || !pair_takes(p) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) || (epi == EPI_SILU_MUL) != (gather_rows != nullptr) ||
         (epi != EPI_SILU_MUL && epi != EPI_BF16)) return -7;
-    return launch_pair_grouped(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st);
+    return bt == PAIR_FORM ? launch_pair_grouped<PAIR_BT>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st)
+                           : launch_pair_grouped<128>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st);
   }
   if (gather_rows != nullptr && (bt > GATHER_BT_MAX || splits > 1 || ldx % 8)) return -7;
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;

@@ -400,11 +400,15 @@ GATHER_MAX_BT = int(__import__("os").environ.get("ENGINE_MOE_GATHER_BT", "128"))
 # they have: two such tiles replace four of 64 rows (8192 rows, 256 per expert: gate/up 496 -> 365 us; down 239 -> 246, but
 # both GEMMs walk one tile table). At 64 rows per expert both forms need about one tile (207 and 204 us, 99 and 101 us).
 WIDE_MIN_ROWS = 96
-# Expected rows per routed expert from which the expert GEMMs of ``moe_block`` take tiles of up to 256 rows on two SMs each
-# (tile-packed weights; 128-row tiles remain for plain ones). Block of 257 experts, us, without -> with: 48 rows per expert
-# 323 -> 333, 56: 339 -> 337, 64: 353 -> 347, 80: 396 -> 357, 128: 439 -> 401, 156: 527 -> 429, 256: 699 -> 601.
-PAIR_MIN_ROWS = 64
-PAIR_FORM = -256  # the launchers' token tile of up to 256 rows on two SMs
+# Expected rows per routed expert from which the expert GEMMs of ``moe_block`` run with two SMs per tile (tile-packed weights;
+# 64- and 128-row tiles on one SM remain below it and for plain weights), and from which those tiles have up to 256 rows and
+# not 128. Block of 257 experts without the GEMMs' neighbours, gate/up + down in us, one SM per tile, 128 rows, 256 rows: 48 rows
+# per expert 188 + 95, 190 + 95, 198 + 96; 56: 199 + 98, 191 + 99, 200 + 97; 64: 204 + 98, 194 + 99, 203 + 98; 80: 236 + 109, 197 +
+# 102, 206 + 103; 104: -, 210 + 109, 214 + 110; 128: 236 + 135, 237 + 134, 219 + 115;
+# 256: 356 + 230, -, 324 + 171.
+PAIR_MIN_ROWS = 50
+PAIR_256_MIN_ROWS = 108
+PAIR_FORM, PAIR_FORM_128 = -256, -128  # the launchers' token tiles of up to 256 and 128 rows on two SMs
 
 
 def block_bt(T: int, top_k: int, pairs_per_row: int, n_experts: int) -> int:
@@ -455,9 +459,9 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
     gather = bt <= GATHER_MAX_BT and x.stride(0) % 8 == 0 and x.stride(1) == 1 and x.data_ptr() % 16 == 0
     pair = (gather and bt >= 64 and not _MOE_BT_FIXED and T * top_k >= PAIR_MIN_ROWS * n_experts and is_packed(w_gate_up)
             and is_packed(w_down) and H % 256 == 0)
+    form = bt
     if pair:
-        bt = 256
-    form = PAIR_FORM if pair else bt
+        bt, form = (256, PAIR_FORM) if T * top_k >= PAIR_256_MIN_ROWS * n_experts else (128, PAIR_FORM_128)
     src_rows = ints[Et + 2 + 2 * n_pairs :] if gather else None
     max_tiles = min(Et, n_pairs) + n_pairs // bt + 1
     tiles = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
