@@ -44,7 +44,7 @@ __device__ __forceinline__ bool group_all(bool ok, int id) {
 }
 __device__ __forceinline__ void group_sync(int id) { asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(id) : "memory"); }
 
-// EPI_BF16 (dense, or grouped with rows that are sorted already) or EPI_SILU_MUL (grouped, rows fetched by index,
+// EPI_BF16 (dense, or grouped with rows that are sorted already), EPI_F32 or EPI_ARGMAX (dense) or EPI_SILU_MUL (grouped, rows fetched by index,
 // tile-packed weights). In a SiLU tile a CTA's 128 accumulator rows are 64 gate rows and the 64 up rows
 // that go with them.
 template <int EPI, bool GROUPED, int PBT>
@@ -55,7 +55,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   constexpr int CTA_ROWS = PAIR_ROWS / 2;
   constexpr int STAGES = PairCfg<PBT>::STAGES, STAGE_BYTES = PairCfg<PBT>::STAGE_BYTES;
   constexpr int LANE_ROWS = PBT / 8;  // of a CTA's half of the rows, fetched by a group of eight lanes
-  static_assert(EPI == EPI_BF16 || (SILU && GROUPED), "epilogues of the pair form");
+  static_assert(EPI == EPI_BF16 || (!GROUPED && (EPI == EPI_F32 || EPI == EPI_ARGMAX)) || (SILU && GROUPED), "epilogues of the pair form");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -293,6 +293,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             const uint4 o = *reinterpret_cast<const uint4*>(stage + 128 * 16 + (r * CTA_ROWS + col) * 2);
             if (c + r < nrows && n0 + col < p.N)
               *reinterpret_cast<uint4*>(static_cast<bf16*>(p.out) + static_cast<size_t>(row0 + c + r) * p.ldo + n0 + col) = o;
+          } else if (EPI == EPI_F32) {
+            if (n0 + tid < p.N) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (c + j < nrows) static_cast<float*>(p.out)[static_cast<size_t>(row0 + c + j) * p.ldo + n0 + tid] = v[j];
+            }
+          } else if (EPI == EPI_ARGMAX) {
+            // the warps' picks of 16 columns meet in one of two buffers (as below: read ahead of the reader's next barrier)
+            float2* red = reinterpret_cast<float2*>(stage) + out_buf * (4 * 16);
+            out_buf ^= 1;
+            float best;
+            int at;
+            argmax_columns(v, n0 + tid, n0 + tid < p.N, lane, best, at);
+            if ((lane & 1) == 0) red[q * 16 + argmax_column(lane)] = make_float2(best, __int_as_float(at));
+            group_sync(bar_id);
+            const int wt = 2 * nx + static_cast<int>(rank);
+            if (tid < 16 && c + tid < nrows && wt * BM < p.N) {
+              float2 m = red[tid];
+#pragma unroll
+              for (int w = 1; w < 4; ++w) {
+                const float2 o = red[w * 16 + tid];
+                if (o.x > m.x || (o.x == m.x && __float_as_int(o.y) < __float_as_int(m.y))) m = o;
+              }
+              const size_t o = static_cast<size_t>(wt) * p.T + row0 + c + tid;
+              p.part_max[o] = m.x;
+              p.part_idx[o] = __float_as_int(m.y);
+            }
           } else {
             // [16 rows][128 weight rows] bf16, two buffers: a thread's reads of one precede its next barrier, behind which
             // it is written again

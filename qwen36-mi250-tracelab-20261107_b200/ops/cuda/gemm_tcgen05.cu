@@ -140,6 +140,42 @@ __device__ __forceinline__ bool epilogue_all(bool ok) {
   return r != 0;
 }
 
+// Largest of a warp's 32 weight rows (lanes; row n of this lane's column values v, left out where !n_ok) for each of 16 token
+// columns, lowest row on ties. Lanes with bit 0 clear end with one column each, named by their bits 4..1 (argmax_column).
+// Halves the columns a lane carries at every exchange instead of reducing each column over the whole warp (24 shuffles for 16
+// columns instead of 160). This epilogue, not the weight stream, set the LM head's time: 321 -> 202 us for 256 rows x 248320 x
+// 2048, 171 -> 154 us for 128.
+__device__ __forceinline__ void argmax_columns(const float* v, int n, bool n_ok, int lane, float& best, int& at) {
+  float m[16];
+  int id[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) { m[j] = n_ok ? v[j] : -INFINITY; id[j] = n; }
+#pragma unroll
+  for (int w = 8; w >= 1; w >>= 1) {
+    const int o = 2 * w;
+    const bool hi = lane & o;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float sm = hi ? m[j] : m[j + w];
+      const int si = hi ? id[j] : id[j + w];
+      float km = hi ? m[j + w] : m[j];
+      int ki = hi ? id[j + w] : id[j];
+      const float om = __shfl_xor_sync(0xffffffffu, sm, o);
+      const int oi = w == 8 ? (n ^ 16) : __shfl_xor_sync(0xffffffffu, si, o);
+      if (om > km || (om == km && oi < ki)) { km = om; ki = oi; }
+      m[j] = km; id[j] = ki;
+    }
+  }
+  const float om = __shfl_xor_sync(0xffffffffu, m[0], 1);
+  const int oi = __shfl_xor_sync(0xffffffffu, id[0], 1);
+  if (om > m[0] || (om == m[0] && oi < id[0])) { m[0] = om; id[0] = oi; }
+  best = m[0];
+  at = id[0];
+}
+__device__ __forceinline__ int argmax_column(int lane) {
+  return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+}
+
 template <int BT, int EPI, bool GROUPED, bool SPLIT = false, int RT = BM, int KPS = 1>
 __global__ void __launch_bounds__(GROUPED ? 160 + 32 * Cfg<BT, EPI, RT, KPS>::GATHER_WARPS : 192, Cfg<BT, EPI, RT, KPS>::CTAS_PER_SM)
 gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, GemmParams p) {
@@ -557,36 +593,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           }
         }
         if (EPI == EPI_ARGMAX) {
-          // 32 weight rows (lanes) x 16 token columns: halve the columns a lane carries at every exchange instead of
-          // reducing each column over the whole warp (24 shuffles for 16 columns instead of 160). This epilogue, not the
-          // weight stream, set the kernel's time: 321 -> 202 us for 256 rows x 248320 x 2048, 171 -> 154 us for 128.
-          float m[16];
-          int id[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) { m[j] = n_ok ? v[j] : -INFINITY; id[j] = n; }
-#pragma unroll
-          for (int w = 8; w >= 1; w >>= 1) {
-            const int o = 2 * w;
-            const bool hi = lane & o;
-#pragma unroll
-            for (int j = 0; j < w; ++j) {
-              const float sm = hi ? m[j] : m[j + w];
-              const int si = hi ? id[j] : id[j + w];
-              float km = hi ? m[j + w] : m[j];
-              int ki = hi ? id[j + w] : id[j];
-              const float om = __shfl_xor_sync(0xffffffffu, sm, o);
-              const int oi = w == 8 ? (n ^ 16) : __shfl_xor_sync(0xffffffffu, si, o);
-              if (om > km || (om == km && oi < ki)) { km = om; ki = oi; }
-              m[j] = km; id[j] = ki;
-            }
-          }
-          const float om = __shfl_xor_sync(0xffffffffu, m[0], 1);
-          const int oi = __shfl_xor_sync(0xffffffffu, id[0], 1);
-          if (om > m[0] || (om == m[0] && oi < id[0])) { m[0] = om; id[0] = oi; }
-          if ((lane & 1) == 0) {  // lane bits 4..1 name the column
-            const int col = c + ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-            red_max[q][col] = m[0];
-            red_idx[q][col] = id[0];
+          float best;
+          int at;
+          argmax_columns(v, n, n_ok, lane, best, at);
+          if ((lane & 1) == 0) {
+            const int col = c + argmax_column(lane);
+            red_max[q][col] = best;
+            red_idx[q][col] = at;
           }
         } else if (EPI == EPI_SCATTER) {
           // expert-parallel combine: each output row goes straight to the rank that owns the token,
@@ -929,9 +942,10 @@ static int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, GemmParams 
                          st, tw, tx, p) == cudaSuccess ? 0 : -4;
 }
 
-// What the pair form asks of a launch: whole k-blocks, and output rows that leave in 16-byte pieces.
-static bool pair_takes(const GemmParams& p) {
-  return p.K % BK == 0 && p.N % 8 == 0 && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+// What the pair form asks of a launch: whole k-blocks, and bf16 output rows that leave in 16-byte pieces.
+static bool pair_takes(const GemmParams& p, int epi) {
+  if (p.K % BK || epi == EPI_ARGMAX || epi == EPI_F32) return p.K % BK == 0;
+  return epi != EPI_ALLREDUCE && p.N % 8 == 0 && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
 // Token rows per tile of a dense launch: the fewest cycles over the waves of the persistent grid. A k-block of bt rows takes an
@@ -957,16 +971,22 @@ static int pair_rows(int T, int N) {
 // Many weight tiles and 17 to 128 rows, in chains of norm and projection, 64- or 128-row tiles of one SM -> pair: 12352 x 2048 at
 // 24 rows 13.0 -> 13.0, at 64 15.7 -> 13.4, at 128 15.0 -> 14.4; 9216 x 2048 at 24 rows 11.4 -> 11.6, at 64 14.6 -> 12.9, at 128
 // 15.1 -> 13.2.
-static bool pair_pays(int T, int N) { return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM)); }
+// The LM head (argmax or fp32 logits of 248320 x 2048) is bound by its weights up to 128 rows and by shared memory beyond:
+// picks of 160 rows 192 -> 172 us, of 256 226 -> 206; logits of 160 rows 221 -> 199, of 256 275 -> 240.
+static bool pair_pays(int T, int N, int epi) {
+  if (epi != EPI_BF16) return T > 128 && N > 32 * BM;
+  return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM));
+}
 
-// Dense bf16 GEMM with two SMs per tile.
+// Dense GEMM with two SMs per tile.
+template <int EPI>
 static int launch_pair_dense(const void* X, const void* W, GemmParams p, int ldx, int ldw, int packed, cudaStream_t st) {
   CUtensorMap tw, tx;
   p.pair_bt = pair_rows(p.T, p.N);
   if (weight_map(&tw, W, 0, p.N, p.N, p.K, ldw, false, packed, &p)) return -1;
   if (make_map(&tx, X, p.K, p.T, 0, ldx, 0, p.pair_bt / 2)) return -1;
   const int gy = (p.T + p.pair_bt - 1) / p.pair_bt;
-  return p.pair_bt <= 128 ? launch_pair<EPI_BF16, false, 128>(tw, tx, p, gy, st) : launch_pair<EPI_BF16, false, PAIR_BT>(tw, tx, p, gy, st);
+  return p.pair_bt <= 128 ? launch_pair<EPI, false, 128>(tw, tx, p, gy, st) : launch_pair<EPI, false, PAIR_BT>(tw, tx, p, gy, st);
 }
 
 // Grouped GEMMs with two SMs per tile of up to PBT rows: gate/up with rows by index, or a bf16 projection of sorted rows.
@@ -1063,9 +1083,13 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   const int w_rows = (epi == EPI_SILU_MUL) ? up_offset + N : N;
   GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
-  if (bt == PAIR_FORM && (epi != EPI_BF16 || splits > 1 || !pair_takes(p))) return -7;
-  if (bt == PAIR_FORM || (bt <= 0 && epi == EPI_BF16 && splits == 1 && pair_takes(p) && pair_pays(T, N)))
-    return launch_pair_dense(X, W, p, ldx, ldw, packed, st);
+  const bool pair_ok = splits == 1 && pair_takes(p, epi);
+  if (bt == PAIR_FORM && !pair_ok) return -7;
+  if (bt == PAIR_FORM || (bt <= 0 && pair_ok && pair_pays(T, N, epi))) {
+    if (epi == EPI_ARGMAX) return launch_pair_dense<EPI_ARGMAX>(X, W, p, ldx, ldw, packed, st);
+    if (epi == EPI_F32) return launch_pair_dense<EPI_F32>(X, W, p, ldx, ldw, packed, st);
+    return launch_pair_dense<EPI_BF16>(X, W, p, ldx, ldw, packed, st);
+  }
   if (bt <= 0 && (epi == EPI_BF16 || epi == EPI_F32)) {
     const DenseForm f = dense_form(T, N, K, packed && splits == 1);
     if (f.rt < BM)
@@ -1100,7 +1124,7 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   if (max_tiles <= 0) return 0;
   if (bt == PAIR_FORM || bt == PAIR_FORM_128) {
     GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, 1, nullptr, {}};
-    if (!packed || splits > 1 || !pair_takes(p) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) || (epi == EPI_SILU_MUL) != (gather_rows != nullptr) ||
+    if (!packed || splits > 1 || !pair_takes(p, epi) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) || (epi == EPI_SILU_MUL) != (gather_rows != nullptr) ||
         (epi != EPI_SILU_MUL && epi != EPI_BF16)) return -7;
     return bt == PAIR_FORM ? launch_pair_grouped<PAIR_BT>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st)
                            : launch_pair_grouped<128>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st);

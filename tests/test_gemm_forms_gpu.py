@@ -166,3 +166,22 @@ def test_forms_of_few_weight_tiles_and_many_rows(C, T):
     w, x = _bf(257, 256, scale=0.05, seed=1), _bf(T, 256, seed=T)
     assert torch.equal(C.linear(x, C.pack_weight(w.clone()), out_dtype=torch.float32)[:, :257], C.linear(x, w, out_dtype=torch.float32, bt=256))
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("N,K", [(4352, 64), (4163, 256), (9000, 448)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_two_sm_head_gives_the_logits_and_picks_of_the_plain_tile(C, N, K, packed):
+    """fp32 and argmax epilogues beyond 128 rows: a last pair without a second half, ties, more than one token tile."""
+    w = _bf(N, K, scale=0.05, seed=1)
+    w[N // 2:N // 2 + 300] = w[:300]  # equal rows: the first one is picked
+    ww = C.pack_weight(w.clone()) if packed else w
+    for T in (129, 160, 255, 257, 600):
+        x = _bf(T, K, seed=T)
+        want = C.linear(x, w, out_dtype=torch.float32, bt=16)
+        assert torch.equal(C.linear(x, ww, out_dtype=torch.float32)[:, :N], want), T
+        if packed and N % 128:
+            continue  # (a packed head has zero rows behind its vocabulary)
+        picks, val = C.lm_head_argmax(x, ww, return_value=True)
+        top = want.max(1, keepdim=True).values
+        assert torch.equal(val, top[:, 0]) and torch.equal(picks, (want == top).int().argmax(1)), T
+    C.check_errors(x.device)
