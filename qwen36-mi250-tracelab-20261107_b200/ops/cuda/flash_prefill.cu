@@ -20,10 +20,9 @@
 // sigmoid(gate) and stores bf16. Bound: shared memory, which per page and SM takes 64 KB of K and V in and gives the MMAs
 // 96 KB (Q K^T: N = 64, 48 cycles an MMA) and 48 KB (P V). With one thread for all loads and MMAs, which also read the page
 // table between a free stage and its load, and one page in the softmax at a time, a page took 3400 cycles; it takes about
-// 1800 now: 4 x 2048 rows behind 6.5k to 28.7k tokens 3.70 -> 1.94 ms (1.23 PFLOP/s at 30k), 8 x 1024 rows 249 -> 206 us,
-// decode of 256 x 2.2k tokens 282 -> 230 us, of four sequences of 50-90k 147 -> 120 us. The exponentials keep results below
-// 2^-126, which count where the value beside them is large; the unit's flushing form would save 1 to 2 % in decode (224 and
-// 118 us) and nothing in prefill.
+// 1800 now: 4 x 2048 rows behind 6.5k to 28.7k tokens 3.70 -> 1.94 ms (1.23 PFLOP/s at 30k), 8 x 1024 rows 249 -> 206 us.
+// The exponentials keep results below 2^-126, which count where the value beside them is large; the unit's flushing form
+// would save nothing. Passes of one position per sequence take flash_decode.cu.
 // Chunked prefill: queries sit at positions pos0.. of their sequence, keys are 0..pos.
 // All waits are bounded (common.cuh). No cluster multicast.
 #include "common.cuh"
@@ -50,42 +49,36 @@ struct FlashParams {
   float* part_ml;         // [T, n_q, gridDim.z, 2] (row maximum in natural-log units, row sum)
 };
 
-// DEC (decode: one query position per tile, so GROUP <= 8 real rows): the Q and P operands keep only their first
-// 8-row swizzle atom per 128-byte block (1 KB instead of 16 KB); the MMA still reads 64 rows from those bases, the
-// other 56 come from whatever shared memory follows (the K/V stages) and land in accumulator rows nobody reads: an
-// output row of an MMA depends on its own A row only. The 106 KB this frees hold a third K/V stage, so two pages
-// are on their way while one is being used.
-template <int D, bool DEC = false>
+template <int D>
 struct FlashCfg {
   static constexpr int DB = D / 64;             // 64-element (128-byte) blocks along the head dim
-  static constexpr int Q_BLOCK = DEC ? 1024 : 128 * 128;  // bytes between the 64-element blocks of the Q tile
+  static constexpr int Q_BLOCK = 128 * 128;     // bytes between the 64-element blocks of the Q tile
   static constexpr int Q_BYTES = DB * Q_BLOCK;
   static constexpr int KV_BYTES = DB * FP_PAGE * 128;  // one of K or V, one stage
-  static constexpr int P_BYTES = DEC ? 1024 : 128 * 128;  // one probability tile; two are kept
-  static constexpr int ST = DEC ? 3 : 2;        // K/V stages
+  static constexpr int P_BYTES = 128 * 128;     // one probability tile; two are kept
+  static constexpr int ST = 2;                  // K/V stages
   // dynamic shared memory is declared 1024-byte aligned (checked at run time), so no alignment slack is budgeted:
   // with D = 256 the tiles, the barriers and 512 bytes of static arrays fill the 227 KB of an SM
   static constexpr int SMEM = Q_BYTES + 2 * ST * KV_BYTES + 2 * P_BYTES + 256;
-  static constexpr int ROW_WARPS = DEC ? 1 : 4;  // softmax warps per page: the decode form's 8 rows are one warp's
+  static constexpr int ROW_WARPS = 4;           // softmax warps per page
   static constexpr int TMEM_COLS = (128 + D) <= 256 ? 256 : 512;  // two score tiles of 64 columns + the output
 };
 
-template <int D, int GROUP, bool DEC = false>
+template <int D, int GROUP>
 __global__ void __launch_bounds__(352, 1)
 flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, FlashParams p) {
-  using C = FlashCfg<D, DEC>;
+  using C = FlashCfg<D>;
   constexpr int DB = C::DB;
   constexpr int ST = C::ST;
-  constexpr int R = DEC ? 1 : 128 / GROUP;  // query positions per tile
+  constexpr int R = 128 / GROUP;  // query positions per tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need this alignment; leave with a status rather than compute garbage
     if (threadIdx.x == 0) atomicCAS(p.err, 0, ERR_BAD_INDEX);
     return;
   }
-  // Q and P first: in the decode form the MMAs read past their real rows into the K/V stages that follow
   uint8_t* sQ = smem;
-  uint8_t* sP = sQ + C::Q_BYTES;               // [2][128 x 128 B] (decode: [2][8 x 128 B]): page i uses tile i & 1
+  uint8_t* sP = sQ + C::Q_BYTES;               // [2][128 x 128 B]: page i uses tile i & 1
   uint8_t* sK = sP + 2 * C::P_BYTES;           // [ST stages][DB][64 x 128 B]
   uint8_t* sV = sK + ST * C::KV_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + ST * C::KV_BYTES);
@@ -156,7 +149,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       uint8_t* stages = which ? sV : sK;
       const int* table = p.tables + static_cast<size_t>(seg) * p.max_pages + first;
       if (which == 0) {
-        mbar_expect_tx(q_full, DEC ? DB * GROUP * 128 : C::Q_BYTES);  // decode: GROUP rows of 128 bytes per block
+        mbar_expect_tx(q_full, C::Q_BYTES);
         for (int a = 0; a < DB; ++a) tma_load_4d(sQ + a * C::Q_BLOCK, &tmQ, q_full, a * 64, 0, kh, seg_row0 + p0);
       }
       int next = table[0];
@@ -173,10 +166,8 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
   } else if (warp == 8) {
     if (elect_one()) {
-      // decode: the instructions of 64 rows read half as much of shared memory and keep rows 0-15 in lanes 0-15 (256 sequences of
-      // 2,300 tokens: 250 -> 226 us; four of 50,000 to 90,000: 121 -> 117)
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(DEC ? 64 : 128, 64);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(DEC ? 64 : 128, D) | (1u << 16);  // B operand MN-major
+      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 64);
+      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, D) | (1u << 16);  // B operand MN-major
       const uint32_t qa = smem_u32(sQ);
       auto issue_qk = [&](int i) {
         const int s = i % ST;
@@ -234,11 +225,9 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       float sc[64];
       tmem_ld64(tmem_S + hf * 64 + lane_base, sc);
       const int kbase = (first + i) * FP_PAGE;
-      if (DEC || kbase + FP_PAGE - 1 > pos0 + p0) {  // only pages that end behind the tile's first query hide keys
-        // decode: rows past the real ones hold whatever the MMA read behind the Q atom; masked, so that they never ask for
-        // a rescale of the output tile
+      if (kbase + FP_PAGE - 1 > pos0 + p0) {  // only pages that end behind the tile's first query hide keys
 #pragma unroll
-        for (int j = 0; j < 64; ++j) sc[j] = (kbase + j <= qpos && (!DEC || row_valid)) ? sc[j] : -INFINITY;
+        for (int j = 0; j < 64; ++j) sc[j] = kbase + j <= qpos ? sc[j] : -INFINITY;
       }
       float mx4[4] = {sc[0], sc[1], sc[2], sc[3]};
 #pragma unroll
@@ -279,7 +268,6 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
       uint8_t* prow = sP + hf * C::P_BYTES + r * 128;
-      if (!DEC || r < 8)  // decode: the probability tile holds one 8-row atom; the other rows' scores are not kept
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         uint4 packed;
@@ -389,17 +377,17 @@ int fp_make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* di
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
-template <int D, int GROUP, bool DEC>
+template <int D, int GROUP>
 int fp_launch(const CUtensorMap& tq, const CUtensorMap& tkv, const FlashParams& p, int n_tiles, int gz, cudaStream_t st) {
-  auto kern = flash_prefill_kernel<D, GROUP, DEC>;
+  auto kern = flash_prefill_kernel<D, GROUP>;
   static bool configured[64] = {};  // a function attribute is set per device
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashCfg<D, DEC>::SMEM) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashCfg<D>::SMEM) != cudaSuccess) return -3;
     configured[dev] = true;
   }
-  return launch_pdl(kern, dim3(n_tiles, p.n_kv, gz), dim3(352), FlashCfg<D, DEC>::SMEM, st, tq, tkv, p) == cudaSuccess ? 0 : -4;
+  return launch_pdl(kern, dim3(n_tiles, p.n_kv, gz), dim3(352), FlashCfg<D>::SMEM, st, tq, tkv, p) == cudaSuccess ? 0 : -4;
 }
 }  // namespace
 
@@ -409,9 +397,7 @@ int fp_launch(const CUtensorMap& tq, const CUtensorMap& tkv, const FlashParams& 
 extern "C" int b200_flash_prefill(const void* q, const void* gate, const void* kv, void* out, const void* tiles,
                                   int n_tiles, const int* seg_pos0, const int64_t* positions, const int* tables, int max_pages, int num_pages,
                                   int T, int n_q, int n_kv, int D, int split_pages, int n_splits, float* part_acc,
-                                  float* part_ml, int one_position, int* err, cudaStream_t st) {
-  // one_position != 0: every tile holds a single query position (plain decode): the form with small Q / P tiles
-  // and three K/V stages is used
+                                  float* part_ml, int* err, cudaStream_t st) {
   if (n_tiles <= 0) return 0;
   const int group = n_q / n_kv;
   if (group * n_kv != n_q || (D != 64 && D != 128 && D != 256) || 128 % group) return -7;
@@ -421,7 +407,7 @@ extern "C" int b200_flash_prefill(const void* q, const void* gate, const void* k
                           static_cast<cuuint64_t>(T)};
     cuuint64_t strides[3] = {static_cast<cuuint64_t>(D) * 2, static_cast<cuuint64_t>(group) * D * 2,
                              static_cast<cuuint64_t>(n_q) * D * 2};
-    cuuint32_t box[4] = {64, static_cast<cuuint32_t>(group), 1, static_cast<cuuint32_t>(one_position ? 1 : 128 / group)};
+    cuuint32_t box[4] = {64, static_cast<cuuint32_t>(group), 1, static_cast<cuuint32_t>(128 / group)};
     if (fp_make_map(&tq, q, 4, dims, strides, box)) return -1;
   }
   {
@@ -435,18 +421,11 @@ extern "C" int b200_flash_prefill(const void* q, const void* gate, const void* k
                 split_pages, part_acc, part_ml};
   const int gz = split_pages > 0 ? n_splits : 1;
 #define FP_GROUPS(DD)                                                         \
-  if (one_position) switch (group) {                                          \
-    case 1: return fp_launch<DD, 1, true>(tq, tkv, p, n_tiles, gz, st);           \
-    case 2: return fp_launch<DD, 2, true>(tq, tkv, p, n_tiles, gz, st);           \
-    case 4: return fp_launch<DD, 4, true>(tq, tkv, p, n_tiles, gz, st);           \
-    case 8: return fp_launch<DD, 8, true>(tq, tkv, p, n_tiles, gz, st);           \
-    default: return -7;                                                       \
-  }                                                                           \
   switch (group) {                                                            \
-    case 1: return fp_launch<DD, 1, false>(tq, tkv, p, n_tiles, gz, st);          \
-    case 2: return fp_launch<DD, 2, false>(tq, tkv, p, n_tiles, gz, st);          \
-    case 4: return fp_launch<DD, 4, false>(tq, tkv, p, n_tiles, gz, st);          \
-    case 8: return fp_launch<DD, 8, false>(tq, tkv, p, n_tiles, gz, st);          \
+    case 1: return fp_launch<DD, 1>(tq, tkv, p, n_tiles, gz, st);          \
+    case 2: return fp_launch<DD, 2>(tq, tkv, p, n_tiles, gz, st);          \
+    case 4: return fp_launch<DD, 4>(tq, tkv, p, n_tiles, gz, st);          \
+    case 8: return fp_launch<DD, 8>(tq, tkv, p, n_tiles, gz, st);          \
     default: return -7;                                                       \
   }
   if (D == 256) { FP_GROUPS(256) }

@@ -80,7 +80,8 @@ class _Sig:
     b200_gdn_prefill_work_stride = [I]
     b200_reset_slot = [P, P, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
     b200_ring_commit = [P, P, P, P, P, P, I, I, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
-    b200_flash_prefill = [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P]
+    b200_flash_prefill = [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, P, P]
+    b200_flash_decode = [P, P, P, P, I, I, I, I, I, I, I, I, P, P, P, P]
     b200_attn_combine = [P, P, P, P, I, I, I, I, P]
 
 
@@ -654,33 +655,36 @@ def flash_prefill(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, b
     out = torch.empty(T, n_q * D, dtype=q.dtype, device=dev)
     rc = lib().b200_flash_prefill(
         _ptr(q), _ptr(gate), _ptr(kv_layer), _ptr(out), _ptr(tiles_t), n_tiles, _ptr(pos0_t), None, _ptr(block_tables),
-        block_tables.stride(0), kv_layer.shape[0], T, n_q, n_kv, D, 0, 1, None, None, 0, _ptr(err_word(dev)), _stream(),
+        block_tables.stride(0), kv_layer.shape[0], T, n_q, n_kv, D, 0, 1, None, None, _ptr(err_word(dev)), _stream(),
     )
     _check(rc, "flash_prefill")
     return out
 
 
-DECODE_ATTN_SMALL_TILES = __import__("os").environ.get("ENGINE_ATTN_DECODE_FORM", "1") == "1"  # 8-row Q / P atoms, 3 K/V stages
+DECODE_ATTN_SMALL_TILES = __import__("os").environ.get("ENGINE_ATTN_DECODE_FORM", "1") == "1"  # one row per sequence: flash_decode.cu, not the split form of flash_prefill.cu
 SPLIT_PAGES = int(__import__("os").environ.get("ENGINE_ATTN_SPLIT_PAGES", "8"))  # pages (64 tokens each) of context per decode-attention CTA: fixed for a server's lifetime, part of the numerics contract
 _decode_tiles: dict = {}
 
 
-def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, block_tables: torch.Tensor,
-                 positions: torch.Tensor, G: int) -> torch.Tensor:
-    """Decode / verify attention (``G`` rows per sequence) on the tcgen05 flash kernel with split context.
-
-    Each sequence is one query tile (its ``G`` positions x the GQA group fill the first rows of the 128-row
-    MMA tile); the context is cut into runs of ``SPLIT_PAGES`` pages handled by separate CTAs whose partial
-    results are merged in an order that the context's length fixes. Only device tensors are touched, so the call can be captured in a CUDA graph."""
-    rows, n_q, D = q.shape
-    n_kv = kv_layer.shape[2]
-    B = rows // G
-    dev = q.device
+def _query_tiles(B: int, G: int, dev: torch.device) -> torch.Tensor:
     key = (B, G, dev.index)
     if key not in _decode_tiles:
         b = torch.arange(B, dtype=torch.int32)
         _decode_tiles[key] = torch.stack([b, torch.zeros_like(b), b * G, torch.full_like(b, G)], 1).contiguous().to(dev)
-    tiles = _decode_tiles[key]
+    return _decode_tiles[key]
+
+
+def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, block_tables: torch.Tensor,
+                 positions: torch.Tensor, G: int) -> torch.Tensor:
+    """Decode / verify attention (``G`` rows per sequence) on the tcgen05 flash kernels with split context.
+
+    Each sequence is one query tile (its ``G`` positions x the GQA group fill the first rows of the MMA tile); the context is
+    cut into runs of ``SPLIT_PAGES`` pages, each handled by a CTA of its own (``G > 1``) or by persistent CTAs that walk the
+    runs with keys (one row per sequence, with the same bits), whose partial results are merged in an order that the context's length fixes. Only device tensors are touched, so the call can be captured in a CUDA graph."""
+    rows, n_q, D = q.shape
+    n_kv = kv_layer.shape[2]
+    B = rows // G
+    dev = q.device
     n_splits = max(1, (block_tables.shape[1] + SPLIT_PAGES - 1) // SPLIT_PAGES)
     if positions.dtype != torch.int64 or not positions.is_contiguous():
         positions = positions.to(torch.int64).contiguous()
@@ -688,11 +692,17 @@ def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, bl
     part_ml = torch.empty(rows, n_q, n_splits, 2, dtype=torch.float32, device=dev)
     out = torch.empty(rows, n_q * D, dtype=q.dtype, device=dev)
     L = lib()
-    rc = L.b200_flash_prefill(
-        _ptr(q), _ptr(gate), _ptr(kv_layer), None, _ptr(tiles), B, None, _ptr(positions), _ptr(block_tables),
-        block_tables.stride(0), kv_layer.shape[0], rows, n_q, n_kv, D, SPLIT_PAGES, n_splits, _ptr(part_acc),
-        _ptr(part_ml), 1 if (G == 1 and DECODE_ATTN_SMALL_TILES and n_q // n_kv <= 8) else 0, _ptr(err_word(dev)), _stream(),
-    )
+    if G == 1 and DECODE_ATTN_SMALL_TILES:
+        rc = L.b200_flash_decode(
+            _ptr(q), _ptr(kv_layer), _ptr(positions), _ptr(block_tables), block_tables.stride(0), kv_layer.shape[0], B, n_q, n_kv, D,
+            SPLIT_PAGES, n_splits, _ptr(part_acc), _ptr(part_ml), _ptr(err_word(dev)), _stream(),
+        )
+    else:
+        rc = L.b200_flash_prefill(
+            _ptr(q), _ptr(gate), _ptr(kv_layer), None, _ptr(_query_tiles(B, G, dev)), B, None, _ptr(positions), _ptr(block_tables),
+            block_tables.stride(0), kv_layer.shape[0], rows, n_q, n_kv, D, SPLIT_PAGES, n_splits, _ptr(part_acc),
+            _ptr(part_ml), _ptr(err_word(dev)), _stream(),
+        )
     _check(rc, "flash_decode")
     _check(L.b200_attn_combine(_ptr(part_acc), _ptr(part_ml), _ptr(gate), _ptr(out), rows, n_q, D, n_splits, _stream()),
            "attn_combine")

@@ -75,3 +75,27 @@ def test_gate_that_starts_at_an_odd_element(C, width, n_q, n_kv, D):
         got = C.flash_decode(q, gate, kv, table, pos, 1)
         C.check_errors(q.device)
         assert torch.equal(got, C.flash_decode(q, gate.clone(), kv, table, pos, 1))
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(256, 16, 2), (128, 4, 1), (64, 8, 8), (128, 6, 3)])
+@pytest.mark.parametrize("B,longest", [(1, 1), (1, 64), (2, 513), (5, 5000), (150, 1100), (1030, 130)])
+def test_decode_walk_over_the_runs_gives_the_bits_of_a_cta_per_run(D, n_q, n_kv, B, longest, monkeypatch):
+    """Contexts of one key to many runs, more runs than CTAs, more sequences than one launch takes, a table wider than any of them."""
+    from b200serve.ops import cuda_ops as C
+
+    g = torch.Generator().manual_seed(B + D)
+    lens = torch.randint(1, longest + 1, (B,), generator=g)
+    lens[0] = longest
+    pages = [(int(n) + 63) // 64 for n in lens]
+    kv = torch.randn(sum(pages) + 1, 2, n_kv, 64, D, device="cuda").bfloat16()
+    table = torch.zeros(B, max(pages) + 9, dtype=torch.int32)
+    at = 1
+    for b, k in enumerate(pages):
+        table[b, :k] = torch.arange(at, at + k)
+        at += k
+    table, pos = table.cuda(), (lens - 1).cuda()
+    q, gate = torch.randn(B, n_q, D, device="cuda").bfloat16(), torch.randn(B, n_q * D, device="cuda").bfloat16()
+    got = C.flash_decode(q, gate, kv, table, pos, 1)
+    monkeypatch.setattr(C, "DECODE_ATTN_SMALL_TILES", False)
+    assert torch.equal(got, C.flash_decode(q, gate, kv, table, pos, 1))
+    C.check_errors(q.device)
