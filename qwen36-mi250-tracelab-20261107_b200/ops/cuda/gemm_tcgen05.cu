@@ -93,7 +93,7 @@ struct Cfg {
   // loads 64 rows), and two producer warps fetch the rows by index. Grouped launches only. What bounds the expert GEMMs is
   // shared memory: each k-block is written once and its weight half is read again for every MMA, so a wider tile moves
   // fewer bytes per product. Gate/up at 8192 rows of 9 pairs: 496 us with 64-row tiles, 365 with these (L2 prefetches of
-  // the weights 4 to 16 k-blocks ahead made it 388 to 419).
+  // the weights 4 to 16 k-blocks ahead made it 388 to 419). Plain weights only: packed ones take two SMs (gemm_pair.cuh).
   static constexpr bool VAR_N = BT == 128 && (EPI == EPI_SILU_MUL || EPI == EPI_BF16);
   static constexpr int GATHER_WARPS = (BT == 128 && EPI == EPI_SILU_MUL) ? 2 : 1;
   // Staged stores: 16 token rows at a time go through shared memory and leave as 16-byte pieces of 256-byte rows, instead of
@@ -105,9 +105,9 @@ struct Cfg {
   static constexpr int OUT_BYTES = OUT_BUFS * 16 * BM * 2;
   // small token tiles (decode) leave room for two CTAs per SM: one CTA's pipeline fill and epilogue
   // overlap the other's main loop, which matters when K is short (the MoE down projection has 8 k-blocks)
-  // The fused gate/up GEMM at 16-row token tiles runs three CTAs per SM with two deep stages each: the same bytes in
-  // flight per SM, but a decode step's ~1300 tiles then fill 2.9 waves of 444 CTAs instead of 4.4 waves of 296, and
-  // the partial last wave is what the weight-streaming time loses.
+  // The fused gate/up GEMM at 16-row token tiles and plain weights (packed ones take thin tiles) runs three CTAs per SM with
+  // two deep stages each: the same bytes in flight per SM, but a decode step's ~1300 tiles then fill 2.9 waves of 444 CTAs
+  // instead of 4.4 waves of 296, and the partial last wave is what the weight-streaming time loses.
   // Thin tiles of four k-blocks per stage run alone on their SM, with all of its shared memory: more bytes on their way, and
   // one commit for two stages.
   static constexpr bool SOLO = THIN && KPS == 4;
