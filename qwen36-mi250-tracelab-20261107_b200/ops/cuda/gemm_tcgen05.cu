@@ -942,10 +942,13 @@ static int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, GemmParams 
                          st, tw, tx, p) == cudaSuccess ? 0 : -4;
 }
 
-// What the pair form asks of a launch: whole k-blocks, and bf16 output rows that leave in 16-byte pieces.
-static bool pair_takes(const GemmParams& p, int epi) {
-  if (p.K % BK || epi == EPI_ARGMAX || epi == EPI_F32) return p.K % BK == 0;
-  return epi != EPI_ALLREDUCE && p.N % 8 == 0 && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+// What the pair form asks of a launch: an epilogue that it has (gate/up grouped only), whole k-blocks, and bf16 output rows that
+// leave in 16-byte pieces.
+static bool pair_takes(const GemmParams& p, int epi, bool grouped) {
+  if (p.K % BK) return false;
+  if (epi == EPI_ARGMAX || epi == EPI_F32) return !grouped;
+  if (epi != EPI_BF16 && !(epi == EPI_SILU_MUL && grouped)) return false;
+  return p.N % 8 == 0 && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
 // Token rows per tile of a dense launch: the fewest cycles over the waves of the persistent grid. A k-block of bt rows takes an
@@ -974,7 +977,7 @@ static int pair_rows(int T, int N) {
 // The LM head (argmax or fp32 logits of 248320 x 2048) is bound by its weights up to 128 rows and by shared memory beyond:
 // picks of 160 rows 192 -> 172 us, of 256 226 -> 206; logits of 160 rows 221 -> 199, of 256 275 -> 240.
 static bool pair_pays(int T, int N, int epi) {
-  if (epi != EPI_BF16) return T > 128 && N > 32 * BM;
+  if (epi == EPI_ARGMAX || epi == EPI_F32) return T > 128 && N > 32 * BM;
   return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM));
 }
 
@@ -1083,12 +1086,15 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   const int w_rows = (epi == EPI_SILU_MUL) ? up_offset + N : N;
   GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
-  const bool pair_ok = splits == 1 && pair_takes(p, epi);
+  const bool pair_ok = splits == 1 && pair_takes(p, epi, false);
   if (bt == PAIR_FORM && !pair_ok) return -7;
   if (bt == PAIR_FORM || (bt <= 0 && pair_ok && pair_pays(T, N, epi))) {
-    if (epi == EPI_ARGMAX) return launch_pair_dense<EPI_ARGMAX>(X, W, p, ldx, ldw, packed, st);
-    if (epi == EPI_F32) return launch_pair_dense<EPI_F32>(X, W, p, ldx, ldw, packed, st);
-    return launch_pair_dense<EPI_BF16>(X, W, p, ldx, ldw, packed, st);
+    switch (epi) {
+      case EPI_BF16: return launch_pair_dense<EPI_BF16>(X, W, p, ldx, ldw, packed, st);
+      case EPI_F32: return launch_pair_dense<EPI_F32>(X, W, p, ldx, ldw, packed, st);
+      case EPI_ARGMAX: return launch_pair_dense<EPI_ARGMAX>(X, W, p, ldx, ldw, packed, st);
+    }
+    return -7;
   }
   if (bt <= 0 && (epi == EPI_BF16 || epi == EPI_F32)) {
     const DenseForm f = dense_form(T, N, K, packed && splits == 1);
@@ -1124,8 +1130,8 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   if (max_tiles <= 0) return 0;
   if (bt == PAIR_FORM || bt == PAIR_FORM_128) {
     GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, 1, nullptr, {}};
-    if (!packed || splits > 1 || !pair_takes(p, epi) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) || (epi == EPI_SILU_MUL) != (gather_rows != nullptr) ||
-        (epi != EPI_SILU_MUL && epi != EPI_BF16)) return -7;
+    if (!packed || splits > 1 || !pair_takes(p, epi, true) || N % (epi == EPI_SILU_MUL ? BM : 2 * BM) ||
+        (epi == EPI_SILU_MUL) != (gather_rows != nullptr)) return -7;
     return bt == PAIR_FORM ? launch_pair_grouped<PAIR_BT>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st)
                            : launch_pair_grouped<128>(X, W, p, E, w_rows, epi, gather_rows, ldx, max_tiles, st);
   }

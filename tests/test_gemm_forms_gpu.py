@@ -185,3 +185,28 @@ def test_two_sm_head_gives_the_logits_and_picks_of_the_plain_tile(C, N, K, packe
         top = want.max(1, keepdim=True).values
         assert torch.equal(val, top[:, 0]) and torch.equal(picks, (want == top).int().argmax(1)), T
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T", [128, 129, 300])
+@pytest.mark.parametrize("I,K", [(4096, 128), (4104, 128), (8192, 192), (4160, 320)])
+def test_dense_gate_up_of_many_rows_and_outputs(C, T, I, K):
+    """Beyond the sizes from which other epilogues take two SMs per tile, which this one does not have."""
+    x, w = _bf(T, K, seed=T), _bf(2 * I, K, scale=0.05, seed=I)
+    got = C.linear_silu_mul(x, w)
+
+    def tile(bt):
+        out = torch.full((T, I), 7.0, dtype=torch.bfloat16, device="cuda")
+        rc = C.lib().b200_gemm_dense(x.data_ptr(), w.data_ptr(), out.data_ptr(), T, I, K, K, K, I, C.EPI_SILU_MUL, I, bt, None, None,
+                                     C.err_word(x.device).data_ptr(), 1, 0, C._stream())
+        return rc, out
+
+    rc, plain = tile(16)
+    assert rc == 0 and torch.equal(got, plain)
+    # the rounded halves are the unfused ops'; then silu and the product are rounded to bf16 (2^-8 each), silu from fp32
+    gate, up = C.linear(x, w[:I], bt=16).double(), C.linear(x, w[I:], bt=16).double()
+    ref = gate * torch.sigmoid(gate) * up
+    assert ((got.double() - ref).abs() <= 2.01 * 2.0 ** -8 * ref.abs() + 1e-30).all()
+    rc, out = tile(C.PAIR_FORM)
+    torch.cuda.synchronize()
+    assert rc == -7 and (out == 7.0).all()
+    C.check_errors(x.device)
