@@ -22,8 +22,8 @@ constexpr int FD_MAX_SEQS = 1024;  // of one launch
 
 struct FlashDecodeParams {
   const int64_t* positions;  // [B] position of each sequence's row
-  const int* tables;         // [B, max_pages]
-  int B, max_pages, num_pages, n_q, n_kv, n_splits, split_pages;
+  const int* tables;         // [B] rows of `width` pages, max_pages apart
+  int B, max_pages, width, num_pages, n_q, n_kv, n_splits, split_pages;
   float scale_log2;          // D^-0.5 * log2(e)
   float* part_acc;           // [B, n_q, n_splits, D]
   float* part_ml;            // [B, n_q, n_splits, 2]
@@ -106,7 +106,7 @@ flash_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == 8) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
   pdl_wait();  // positions and Q / K / V come from kernels earlier in the stream
   for (int b = threadIdx.x; b < p.B; b += blockDim.x)
-    s_np[b] = max(0, min(static_cast<int>(p.positions[b]) / FD_PAGE + 1, min(p.max_pages, p.n_splits * p.split_pages)));
+    s_np[b] = max(0, min(static_cast<int>(p.positions[b]) / FD_PAGE + 1, min(p.width, p.n_splits * p.split_pages)));
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -406,10 +406,11 @@ int fd_launch(const CUtensorMap& tq, const CUtensorMap& tkv, const FlashDecodePa
 }  // namespace
 
 // q: [B, n_q, D] bf16 (normed and rotated), one row per sequence; kv: one layer of the paged pool [num_pages, 2, n_kv, 64, D] that
-// holds the rows' own K / V already; positions [B], tables [B, max_pages]. Every partial of [B, n_q, n_splits] is written:
-// n_splits runs of split_pages pages cover the table.
+// holds the rows' own K / V already; positions [B], tables [B] rows of `width` pages, max_pages apart (any distance, 0 too).
+// n_splits runs of split_pages pages cover a row. part_ml is written for all of [B, n_q, n_splits], part_acc only where a run
+// holds keys: the combine passes over the others.
 extern "C" int b200_flash_decode(const void* q, const void* kv, const int64_t* positions, const int* tables, int max_pages,
-                                 int num_pages, int B, int n_q, int n_kv, int D, int split_pages, int n_splits, float* part_acc,
+                                 int width, int num_pages, int B, int n_q, int n_kv, int D, int split_pages, int n_splits, float* part_acc,
                                  float* part_ml, int* err, cudaStream_t st) {
   const int group = n_kv > 0 ? n_q / n_kv : 0;
   if (group * n_kv != n_q || (D != 64 && D != 128 && D != 256) || split_pages <= 0 || n_splits <= 0) return -7;
@@ -430,7 +431,7 @@ extern "C" int b200_flash_decode(const void* q, const void* kv, const int64_t* p
                              static_cast<cuuint64_t>(n_q) * D * 2};
     cuuint32_t box[4] = {64, static_cast<cuuint32_t>(group), 1, 1};
     if (fd_make_map(&tq, static_cast<const bf16*>(q) + heads * D, 4, dims, strides, box)) return -1;
-    const FlashDecodeParams p{positions + b0, tables + static_cast<size_t>(b0) * max_pages, n, max_pages, num_pages, n_q, n_kv,
+    const FlashDecodeParams p{positions + b0, tables + static_cast<size_t>(b0) * max_pages, n, max_pages, width, num_pages, n_q, n_kv,
                               n_splits, split_pages, 1.4426950408889634f / sqrtf(static_cast<float>(D)),
                               part_acc + heads * n_splits * D, part_ml + heads * n_splits * 2, err};
     int rc = -7;

@@ -81,7 +81,7 @@ class _Sig:
     b200_reset_slot = [P, P, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
     b200_ring_commit = [P, P, P, P, P, P, I, I, I, I, I, ctypes.c_ulonglong, ctypes.c_ulonglong, P]
     b200_flash_prefill = [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, P, P]
-    b200_flash_decode = [P, P, P, P, I, I, I, I, I, I, I, I, P, P, P, P]
+    b200_flash_decode = [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P, P, P]
     b200_attn_combine = [P, P, P, P, I, I, I, I, P]
 
 
@@ -694,8 +694,8 @@ def flash_decode(q: torch.Tensor, gate: torch.Tensor, kv_layer: torch.Tensor, bl
     L = lib()
     if G == 1 and DECODE_ATTN_SMALL_TILES:
         rc = L.b200_flash_decode(
-            _ptr(q), _ptr(kv_layer), _ptr(positions), _ptr(block_tables), block_tables.stride(0), kv_layer.shape[0], B, n_q, n_kv, D,
-            SPLIT_PAGES, n_splits, _ptr(part_acc), _ptr(part_ml), _ptr(err_word(dev)), _stream(),
+            _ptr(q), _ptr(kv_layer), _ptr(positions), _ptr(block_tables), block_tables.stride(0), block_tables.shape[1],
+            kv_layer.shape[0], B, n_q, n_kv, D, SPLIT_PAGES, n_splits, _ptr(part_acc), _ptr(part_ml), _ptr(err_word(dev)), _stream(),
         )
     else:
         rc = L.b200_flash_prefill(

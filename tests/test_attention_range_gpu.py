@@ -99,3 +99,21 @@ def test_decode_walk_over_the_runs_gives_the_bits_of_a_cta_per_run(D, n_q, n_kv,
     monkeypatch.setattr(C, "DECODE_ATTN_SMALL_TILES", False)
     assert torch.equal(got, C.flash_decode(q, gate, kv, table, pos, 1))
     C.check_errors(q.device)
+
+
+@pytest.mark.parametrize("G", [1, 2])
+def test_decode_with_rows_of_the_page_table_at_any_distance(G):
+    """One table for all sequences (distance 0), rows closer together than they are wide, a view of a wider table."""
+    from b200serve.ops import cuda_ops as C
+
+    n_q, n_kv, D, B, W = 8, 2, 128, 3, 20
+    kv = torch.randn(W + 3, 2, n_kv, 64, D, device="cuda").bfloat16()
+    row = torch.arange(W + 2, dtype=torch.int32, device="cuda") + 1
+    wide = torch.zeros(B, W + 12, dtype=torch.int32, device="cuda")
+    wide[:, :W] = row[:W]
+    pos = torch.tensor([[64 * W - G, 700, 40][b] + j for b in range(B) for j in range(G)], device="cuda")
+    q, gate = torch.randn(B * G, n_q, D, device="cuda").bfloat16(), torch.randn(B * G, n_q * D, device="cuda").bfloat16()
+    for table in (row[None, :W].expand(B, W), row.as_strided((B, W), (1, 1)), wide[:, :W], wide[:1, :W].expand(B, W)):
+        want = C.flash_decode(q, gate, kv, table.contiguous(), pos, G)
+        assert torch.equal(C.flash_decode(q, gate, kv, table, pos, G), want) and torch.isfinite(want.float()).all()
+    C.check_errors(q.device)
