@@ -224,7 +224,8 @@ class Model:
             core = ops.gdn_prefill(mixed, batch.seg_starts, batch.seg_slots, conv, rec, *args, **self._span_meta(batch, "gdn"))
         else:
             r = None if ring is None else (ring[0][gi], ring[1][gi])
-            core = ops.gdn_decode(mixed, batch.slots, conv, rec, *args, G=batch.G, ring=r)
+            behind = {"behind_projection": True} if getattr(ops, "GDN_BEHIND_PROJECTION", False) else {}
+            core = ops.gdn_decode(mixed, batch.slots, conv, rec, *args, G=batch.G, ring=r, **behind)
         return self._out_proj(core, lw.out_proj)
 
     def _out_proj(self, core: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

@@ -48,7 +48,9 @@ __device__ __forceinline__ uint32_t elect_one() {
 // descriptor prefetch, loads of weights nobody writes) overlap the predecessor's tail. The contract every such kernel
 // keeps: `pdl_wait()` before the first read of anything an earlier kernel wrote and before the first global write
 // (it returns once every earlier kernel has completed and its writes are visible), `pdl_launch()` once the CTA holds
-// all the resources it will ever ask for (after any TMEM allocation), which lets the next kernel's CTAs queue up.
+// all the resources it will ever ask for (after any TMEM allocation), which lets the next kernel's CTAs queue up. A kernel
+// that reads ahead of its wait what an earlier kernel wrote (gdn_decode.cu) is launched only where the kernel in front is
+// known, keeps this contract and does not write it: everything before that one is complete when this one starts.
 // Both are no-ops in a kernel launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -23,12 +23,13 @@ namespace b200 {
 // mixed: [B*G, ld] rows (row b*G + j), conv input at columns [0, C). conv_state: [slots, C, KW-1].
 // out: [B*G, C] = silu(sum_k w[c,k] * window[k]). The slot's state ends as the last KW-1 inputs;
 // with G > 1 the state after each row is also kept in ring_conv [B, G, C, KW-1] when given.
-// Bound by the latency of its loads and by how many of its CTAs an SM holds. The windows and weights are asked for ahead of the
-// dependency wait: like the step kernel's states they were last written by an earlier step or pass, never by the kernel just
-// before this one, whose output `mixed` is (and every kernel of this library releases its successor behind its own wait, so
-// whatever came before that one is complete). 72 registers hold the 2048 CTAs of 128 sequences of 8192 channels in one wave.
-// In a step, us: one sequence 3.4 -> 1.8, 128: 10.4 -> 6.5, 256: 13.8 -> 12.0.
-template <int KW>
+// Bound by the latency of its loads and by how many of its CTAs an SM holds. AHEAD: the slots, windows and weights are asked for
+// ahead of the dependency wait. The caller then says that the kernel just before this one is a projection of this library
+// that wrote `mixed` and none of them: it released this kernel behind its own wait, so whatever came before it is complete
+// (a fill, a copy, a slot reset, a ring commit or a prefill right in front would still be writing). 72 registers hold the
+// 2048 CTAs of 128 sequences of 8192 channels in one wave. In a step, us, in order -> AHEAD: one sequence 3.4 -> 1.8, 128:
+// 10.4 -> 6.5, 256: 13.8 -> 12.0.
+template <int KW, bool AHEAD = false>
 __global__ void __launch_bounds__(64, 14)
 gdn_conv_step_kernel(const bf16* mixed, int ld, const int* slots, bf16* conv_state, const bf16* conv_w, bf16* out,
                      bf16* ring_conv, int C, int G) {
@@ -36,6 +37,7 @@ gdn_conv_step_kernel(const bf16* mixed, int ld, const int* slots, bf16* conv_sta
   const int b = blockIdx.y;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   const bool live = c < C;
+  if (!AHEAD) { pdl_wait(); pdl_launch(); }
   bf16* st = conv_state;
   uint4 sq[KW - 1], wq[KW];
   if (live) {
@@ -45,8 +47,7 @@ gdn_conv_step_kernel(const bf16* mixed, int ld, const int* slots, bf16* conv_sta
 #pragma unroll
     for (int i = 0; i < KW; ++i) wq[i] = reinterpret_cast<const uint4*>(conv_w + static_cast<size_t>(c) * KW)[i];
   }
-  pdl_wait();
-  pdl_launch();
+  if (AHEAD) { pdl_wait(); pdl_launch(); }
   if (!live) return;
   bf16* sv = reinterpret_cast<bf16*>(sq);  // windows, oldest value of a channel first
   const bf16* wv = reinterpret_cast<const bf16*>(wq);
@@ -364,10 +365,9 @@ extern "C" int b200_reset_slot(void* conv_state, void* rec_state, int slot, int 
                     static_cast<size_t>(rec_bytes / 16)) == cudaSuccess ? 0 : -4;
 }
 
-extern "C" int b200_gdn_decode(const void* mixed, int ld, const int* slots, void* conv_state, void* rec_state,
-                               const void* conv_w, const float* A_log, const float* dt_bias, const void* gnorm_w,
-                               void* conv_out, void* out, void* ring_conv, float* ring_rec, int B, int G, int HK, int HV,
-                               int DK, int DV, int KW, float eps, int* err, cudaStream_t st) {
+static int gdn_decode(bool ahead, const void* mixed, int ld, const int* slots, void* conv_state, void* rec_state, const void* conv_w,
+                      const float* A_log, const float* dt_bias, const void* gnorm_w, void* conv_out, void* out, void* ring_conv,
+                      float* ring_rec, int B, int G, int HK, int HV, int DK, int DV, int KW, float eps, int* err, cudaStream_t st) {
   if (B <= 0) return 0;
   const int key_dim = HK * DK, value_dim = HV * DV, C = 2 * key_dim + value_dim;
   if (KW != 4) return -7;
@@ -377,7 +377,8 @@ extern "C" int b200_gdn_decode(const void* mixed, int ld, const int* slots, void
                    static_cast<const bf16*>(conv_w), static_cast<bf16*>(conv_out), static_cast<bf16*>(ring_conv), C,
                    G) != cudaSuccess) return -4;
   } else {
-    if (launch_pdl(gdn_conv_step_kernel<4>, dim3((C / 8 + 63) / 64, B), dim3(64), 0, st,
+    auto kern = ahead ? gdn_conv_step_kernel<4, true> : gdn_conv_step_kernel<4, false>;
+    if (launch_pdl(kern, dim3((C / 8 + 63) / 64, B), dim3(64), 0, st,
                    static_cast<const bf16*>(mixed), ld, slots, static_cast<bf16*>(conv_state),
                    static_cast<const bf16*>(conv_w), static_cast<bf16*>(conv_out), static_cast<bf16*>(ring_conv), C,
                    G) != cudaSuccess) return -4;
@@ -406,5 +407,22 @@ extern "C" int b200_gdn_decode(const void* mixed, int ld, const int* slots, void
   else return -7;
 #undef LAUNCH_STEP
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+extern "C" int b200_gdn_decode(const void* mixed, int ld, const int* slots, void* conv_state, void* rec_state,
+                               const void* conv_w, const float* A_log, const float* dt_bias, const void* gnorm_w,
+                               void* conv_out, void* out, void* ring_conv, float* ring_rec, int B, int G, int HK, int HV,
+                               int DK, int DV, int KW, float eps, int* err, cudaStream_t st) {
+  return gdn_decode(false, mixed, ld, slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnorm_w, conv_out, out, ring_conv,
+                    ring_rec, B, G, HK, HV, DK, DV, KW, eps, err, st);
+}
+
+// The same right behind the projection that wrote `mixed` (AHEAD above): slots and states have been written before that.
+extern "C" int b200_gdn_decode_behind_projection(const void* mixed, int ld, const int* slots, void* conv_state, void* rec_state,
+                                                 const void* conv_w, const float* A_log, const float* dt_bias, const void* gnorm_w,
+                                                 void* conv_out, void* out, void* ring_conv, float* ring_rec, int B, int G, int HK,
+                                                 int HV, int DK, int DV, int KW, float eps, int* err, cudaStream_t st) {
+  return gdn_decode(true, mixed, ld, slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnorm_w, conv_out, out, ring_conv,
+                    ring_rec, B, G, HK, HV, DK, DV, KW, eps, err, st);
 }
 #endif  // B200_EMU

@@ -74,6 +74,7 @@ class _Sig:
     b200_moe_gather = [P, P, P, I, I, I, I, P, P]
     b200_moe_combine = [P, P, P, I, I, I, P, P, P]
     b200_gdn_decode = [P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P, P]
+    b200_gdn_decode_behind_projection = b200_gdn_decode
     b200_attn_prep = [P, I, P, P, I, P, P, P, P, P, P, I, I, I, I, I, F, F, I, P, P]
     b200_paged_attn = [P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, P]
     b200_gdn_prefill = [P, I, P, P, P, P, P, P, P, P, P, P, P, I, P, I, P, P, P, I, I, I, I, I, F, I, P, P]
@@ -156,6 +157,7 @@ SPLIT_K_ENABLED = __import__("os").environ.get("ENGINE_SPLIT_K", "0") == "1"
 # Gated DeltaNet prefill with head dims of 128: tcgen05 WY transform and state pass (ENGINE_GDN_TC=0 selects the fp32
 # CUDA-core kernels, which other head dims always use)
 GDN_PREFILL_TC = __import__("os").environ.get("ENGINE_GDN_TC", "1") == "1"
+GDN_BEHIND_PROJECTION = True  # gdn_decode can be told that the projection is right in front of it
 SPAN_TABLES = True  # gdn_prefill and attention take the span tables of a ragged pass as `meta`
 
 
@@ -510,15 +512,20 @@ def moe_block(x: torch.Tensor, router: torch.Tensor, w_gate_up: torch.Tensor, w_
 
 # --------------------------------------------------------------------------- GDN
 def gdn_decode(mixed, slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnorm_w, n_k, n_v, dk, dv, eps,
-               G: int = 1, ring=None) -> torch.Tensor:
-    """Conv step + delta rule + gated norm for ``B*G`` rows (``G`` consecutive rows per slot)."""
+               G: int = 1, ring=None, behind_projection: bool = False) -> torch.Tensor:
+    """Conv step + delta rule + gated norm for ``B*G`` rows (``G`` consecutive rows per slot).
+
+    ``behind_projection``: the last kernel in the stream is the ``linear`` that wrote ``mixed``, so slots and states, written
+    before it, may be read while it still runs."""
     rows = mixed.shape[0]
     B = rows // G
     C = 2 * n_k * dk + n_v * dv
     conv_out = torch.empty(rows, C, dtype=mixed.dtype, device=mixed.device)
     out = torch.empty(rows, n_v * dv, dtype=mixed.dtype, device=mixed.device)
     slots32 = slots if slots.dtype == torch.int32 else slots.to(torch.int32)
-    rc = lib().b200_gdn_decode(
+    # (a conversion of the slots is the last kernel in the stream)
+    op = lib().b200_gdn_decode_behind_projection if behind_projection and slots32 is slots else lib().b200_gdn_decode
+    rc = op(
         _ptr(mixed), mixed.stride(0), _ptr(slots32), _ptr(conv_state), _ptr(rec_state), _ptr(conv_w), _ptr(A_log),
         _ptr(dt_bias), _ptr(gnorm_w), _ptr(conv_out), _ptr(out), _ptr(ring[0]) if ring else None,
         _ptr(ring[1]) if ring else None, B, G, n_k, n_v, dk, dv, conv_w.shape[1], eps, _ptr(err_word(mixed.device)),
