@@ -130,9 +130,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     // ---------------- row-fetching producers: warp w of PAIR_GATHER_WARPS fills every PAIR_GATHER_WARPS-th stage, the weights
     // by TMA, this CTA's half of the token rows by index as 16-byte asynchronous copies into the swizzled operand layout (as
     // in gemm_swapab_kernel), and announces the rows when they have landed.
-    // A whole stage per warp, because the announcement has to be a release for the cluster (the MMA is issued by the other
-    // SM), which takes 1400 cycles with copies of the warp in flight: four warps that each fetched a quarter of every stage
-    // made a k-block 1.2 us long. (Four-row TMA gathers take 70 cycles each: 1.26 us for the 32 of a stage.)
+    // The announcement is a release for the cluster (the first CTA issues the MMA that reads the second one's rows, and acquires
+    // at that scope), of shared memory only, which is all that the copies wrote and costs nothing that shows: passes of 8 x 1024
+    // and 2048 rows 6.21 and 2.59 ms with and without it. A release of everything waits for the SM's other traffic: 6.38 ->
+    // 6.78 and 2.67 -> 2.80, and 7.88 and 3.92 where one thread of the second CTA passes its warps' announcements on. A whole
+    // stage per warp, so that one lane announces it. (Four-row TMA gathers take 70 cycles each: 1.26 us for the 32 of a stage.)
     const int gw = warp == 0 ? 0 : warp - PAIR_GATHER_WARP + 1, j = lane & 7;
     int first = gw;  // the warp's first k-block of the tile
     int it = gw;     // stages of this warp and all others before it
@@ -151,7 +153,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       for (; kb < num_k; kb += PAIR_GATHER_WARPS, it += PAIR_GATHER_WARPS) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
+        if (!mbar_wait<true>(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
         uint8_t* st = smem + s * STAGE_BYTES;
         const uint32_t bar = dsmem_addr(smem_u32(&full[s]), 0);
         if (lane == 0) {
@@ -171,7 +173,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         asm volatile("cp.async.wait_all;" ::: "memory");  // (also: no copy of this lane may outlive the CTA's shared memory)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // for the tensor core's reads
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(bar);
+        if (lane == 0) mbar_arrive_release_shared(bar);
       }
       first = kb - num_k;
     }
@@ -205,7 +207,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           uint8_t* st = smem + s * STAGE_BYTES;
           const uint32_t bar = dsmem_addr(smem_u32(&full[s]), 0);
           if (it >= pre) {
-            if (!mbar_wait(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
+            if (!mbar_wait<true>(&empty[s], ph ^ 1, p.err, ERR_WAIT_EMPTY, abort_flag)) { live = false; break; }
             if (rank == 0) mbar_expect_tx(&full[s], GROUPED ? 2 * (PAIR_A_BYTES + boxes * (VAR_BOX * BK * 2)) : dense_bytes);
             load_weights(st, bar, nx, expert, kb);
           }
@@ -230,11 +232,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const uint32_t idesc = umma_idesc_bf16(2 * BM, columns(nrows));
         const int acc = lt & 1;
         const uint32_t tmem = tmem_base + acc * PAIR_BT;
-        ok = mbar_wait(&acc_empty[acc], ((lt >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
+        ok = mbar_wait<true>(&acc_empty[acc], ((lt >> 1) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
         if (ok) tc_fence_after();
         for (int kb = 0; kb < num_k && ok; ++kb, ++it) {
           const int s = it % STAGES;
-          ok = mbar_wait(&full[s], (it / STAGES) & 1, p.err, ERR_WAIT_FULL, abort_flag);
+          ok = mbar_wait<true>(&full[s], (it / STAGES) & 1, p.err, ERR_WAIT_FULL, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
@@ -262,7 +264,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       const uint32_t tmem = tmem_base + acc * PAIR_BT + (static_cast<uint32_t>(q * 32) << 16);
       const int n0 = nx * PAIR_ROWS + static_cast<int>(rank) * CTA_ROWS;
       // the batches below hold barriers: all four warps of the group take them, or none
-      const bool ok = group_all(mbar_wait(&acc_full[acc], (lt >> 1) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag, bar_id);
+      const bool ok = group_all(mbar_wait<true>(&acc_full[acc], (lt >> 1) & 1, p.err, ERR_WAIT_TMEM, abort_flag) && !*abort_flag, bar_id);
       tc_fence_after();
       if (ok) {
 #pragma unroll 1

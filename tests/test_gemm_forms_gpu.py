@@ -210,3 +210,20 @@ def test_dense_gate_up_of_many_rows_and_outputs(C, T, I, K):
     torch.cuda.synchronize()
     assert rc == -7 and (out == 7.0).all()
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T", [300, 600])
+def test_two_sm_expert_tiles_read_the_rows_of_their_own_pass(C, T):
+    """Two inputs in turn: rows of the pass before, which the same stages held, would show in either CTA's half."""
+    E, k, H, I = 32, 8, 2048, 512
+    wgu = C.pack_weight(_bf(E + 1, 2 * I, H, scale=0.05, seed=35), gate_up=True)
+    wd = C.pack_weight(_bf(E + 1, H, I, scale=0.05, seed=36))
+    router, xs = _bf(E + 1, H, scale=0.3, seed=34), (_bf(T, H, seed=1), _bf(T, H, seed=2))
+    assert C.PAIR_MIN_ROWS * E <= T * k
+    want = [C.moe_block(x, router, wgu, wd, E, k, True) for x in xs]
+    for x, w in zip(xs, want):
+        halves = torch.cat([C.moe_block(x[i:i + 100], router, wgu, wd, E, k, True) for i in range(0, T, 100)])  # one SM per tile
+        assert torch.equal(w, halves)
+    got = [C.moe_block(xs[i % 2], router, wgu, wd, E, k, True) for i in range(64)]
+    assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+    C.check_errors(xs[0].device)
