@@ -374,8 +374,15 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
     if (SPLIT) { __syncwarp(); cluster_sync(); }
   } else if (warp == 1) {
+    // The warp runs this loop as a whole, which keeps descriptors in uniform registers, and one lane issues. In dense gate/up
+    // launches, of two MMAs per step, that lane runs it alone but for 64-row tiles; us, warp -> lane (x 512 x 2048): 17 rows 17.2 ->
+    // 16.3, 128: 25.2 -> 23.0, 2048: 26.2 -> 23.8 (64: 21.2 -> 21.9; grouped launches show no difference).
+    constexpr bool LONE = EPI == EPI_SILU_MUL && !GROUPED && BT != 64;
     const uint32_t issue = elect_one();
-    {
+    const auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+      return LONE ? mbar_wait(bar, parity, p.err, code, abort_flag) : mbar_wait_warp(bar, parity, p.err, code, abort_flag);
+    };
+    if (!LONE || issue) {
       uint32_t idesc = umma_idesc_bf16(C::MMA_M, !GROUPED && !C::THIN && p.x_rows > 0 ? p.x_rows : BT);
       bool ok = true;
       int it = 0, lt = 0;  // k-blocks and tiles consumed so far
@@ -388,12 +395,12 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int acc = lt % ACC;
       const uint32_t tmem = tmem_base + acc * C::ACC_COLS;
       // the epilogue must have drained this accumulator stage (two tiles ago) before it is overwritten
-      ok = mbar_wait_warp(&acc_empty[acc], ((lt / ACC) & 1) ^ 1, p.err, ERR_WAIT_TMEM, abort_flag);
+      ok = wait(&acc_empty[acc], ((lt / ACC) & 1) ^ 1, ERR_WAIT_TMEM);
       if (ok) tc_fence_after();
       for (int kb = 0; kb < num_k && ok; ++kb, ++it) {
         const int s = it % C::STAGES;
         const uint32_t ph = (it / C::STAGES) & 1;
-        ok = mbar_wait_warp(&full[s], ph, p.err, ERR_WAIT_FULL, abort_flag);
+        ok = wait(&full[s], ph, ERR_WAIT_FULL);
         if (!ok) break;
         // rows that the gathering producer wrote through the generic proxy must be visible to the tensor core's reads
         if (GROUPED && BT <= GATHER_BT_MAX && p.gather_rows != nullptr) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -405,14 +412,14 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           const uint32_t koff = (k % (BK / UMMA_K)) * UMMA_K * 2;  // bytes inside the 128-byte swizzled row
           const uint32_t aoff = k / (BK / UMMA_K) * C::A_STEP + koff;
           const uint64_t db = umma_smem_desc(b_addr + k / (BK / UMMA_K) * C::B_BYTES + koff);
-          umma_bf16_if(issue, tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
+          umma_bf16_if(LONE ? 1u : issue, tmem, umma_smem_desc(a_addr + aoff), db, idesc, (kb | k) != 0);
           if (EPI == EPI_SILU_MUL && !C::MERGED)
-            umma_bf16_if(issue, tmem + BT, umma_smem_desc(a_addr + C::A_BYTES + aoff), db, idesc, (kb | k) != 0);
+            umma_bf16_if(LONE ? 1u : issue, tmem + BT, umma_smem_desc(a_addr + C::A_BYTES + aoff), db, idesc, (kb | k) != 0);
         }
         // the group's stages are reusable once these MMAs have read them
-        if (it % C::GROUP == C::GROUP - 1) umma_commit_if(issue, &empty[it / C::GROUP % (C::STAGES / C::GROUP)]);
+        if (it % C::GROUP == C::GROUP - 1) umma_commit_if(LONE ? 1u : issue, &empty[it / C::GROUP % (C::STAGES / C::GROUP)]);
       }
-      umma_commit_if(issue, &acc_full[acc]);  // always arrive so that the epilogue is released
+      umma_commit_if(LONE ? 1u : issue, &acc_full[acc]);  // always arrive so that the epilogue is released
       }
     }
     if (SPLIT) { __syncwarp(); cluster_sync(); }
