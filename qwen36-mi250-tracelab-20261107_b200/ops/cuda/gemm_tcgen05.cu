@@ -982,9 +982,12 @@ static int pair_rows(int T, int N) {
 // 24 rows 13.0 -> 13.0, at 64 15.7 -> 13.4, at 128 15.0 -> 14.4; 9216 x 2048 at 24 rows 11.4 -> 11.6, at 64 14.6 -> 12.9, at 128
 // 15.1 -> 13.2.
 // The LM head (argmax or fp32 logits of 248320 x 2048) is bound by its weights up to 128 rows and by shared memory beyond:
-// picks of 160 rows 192 -> 172 us, of 256 226 -> 206; logits of 160 rows 221 -> 199, of 256 275 -> 240.
+// picks of 160 rows 192 -> 172 us, of 256 226 -> 206; logits of 160 rows 221 -> 199, of 256 275 -> 240. fp32 rows of fewer
+// weight tiles than SMs are better off from 17 on, x 2048: 16384 at 48 rows 16.1 -> 14.5, at 128 16.3 -> 15.4; 18944 at 17 rows
+// 16.9 -> 15.4, at 64 18.7 -> 16.3 (31104 at 64 rows 24.6 -> 24.9; 62080 at 17 41.7 -> 45.0).
 static bool pair_pays(int T, int N, int epi) {
-  if (epi == EPI_ARGMAX || epi == EPI_F32) return T > 128 && N > 32 * BM;
+  if (epi == EPI_ARGMAX || epi == EPI_F32)
+    return N > 32 * BM && (T > 128 || (epi == EPI_F32 && T > 16 && N <= BM * sm_count()));
   return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM));
 }
 
