@@ -196,7 +196,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __shared__ uint4 exchange[C::MERGED ? 128 : 1];
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  if (SPLIT) pdl_wait();
+  // The grouped tile table is written by the kernel just before this one: wait for it before the first read, with the set-up
+  // below behind it. 128-row gate/up tiles, whose launches fill the SMs with three CTAs each, wait ahead of the set-up (block of
+  // 8 to 32 rows, plain weights, us, behind -> ahead: 87.2 -> 85.6, 116.4 -> 114.9, 159.5 -> 157.7, 198.3 -> 196.8; 128: 291.9
+  // -> 289.5; thin tiles of one row 28.5 -> 29.0). Dense launches wait later (the producer streams the first weight stages
+  // before it waits).
+  constexpr bool WAIT_FIRST = SPLIT || (GROUPED && EPI == EPI_SILU_MUL && !C::THIN);
+  if (WAIT_FIRST) pdl_wait();
   // Persistent tile loop: CTA b takes output tiles b, b + gridDim.x, ... (weight tile fastest, so CTAs that run
   // together share the activation tile). A split-K cluster takes the single tile its grid position names.
   const int tiles_n = (p.N + RT - 1) / RT;
@@ -228,10 +234,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // The grouped tile table is written by the kernel just before this one: wait for it before the first read, with the
-  // set-up above behind it. Dense launches wait later (the producer streams the first weight stages before it waits).
   if (GROUPED) {
-    pdl_wait();
+    if (!WAIT_FIRST) pdl_wait();
     if (!SPLIT && warp == 0) pdl_launch();
   }
   // The role's first table entry is read beside the entry count, not behind it (the table has room for the whole grid).
