@@ -1153,7 +1153,7 @@ extern "C" int b200_gemm_grouped(const void* X, const void* W, void* out, int ca
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) splits = 1;
   CUtensorMap tw, tx;
   GemmParams p{N, K, cap, ldo, out, reinterpret_cast<const int4*>(tiles), n_tiles, up_offset, nullptr, nullptr, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
-  if (packed && splits == 1 && bt <= 32 && epi == EPI_SILU_MUL) {
+  if (packed && splits == 1 && (bt == 16 || bt == 32) && epi == EPI_SILU_MUL) {
     const int rc = launch_thin_grouped(X, W, p, E, gather_rows, ldx, max_tiles, bt, st);
     if (rc <= 0) return rc;
   }

@@ -227,3 +227,18 @@ def test_two_sm_expert_tiles_read_the_rows_of_their_own_pass(C, T):
     got = [C.moe_block(xs[i % 2], router, wgu, wd, E, k, True) for i in range(64)]
     assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
     C.check_errors(xs[0].device)
+
+
+def test_grouped_launches_refuse_token_tiles_that_no_kernel_has(C):
+    E, H, I = 2, 128, 128
+    wgu, x = C.pack_weight(_bf(E, 2 * I, H, seed=1), gate_up=True), _bf(24, H, seed=2)
+    out = torch.full((24, I), 7.0, dtype=torch.bfloat16, device="cuda")
+    tiles = torch.tensor([[0, 0, 24, 0]], dtype=torch.int32, device="cuda")
+    n = torch.ones(1, dtype=torch.int32, device="cuda")
+    for bt in (24, 8, 1, 0, -1, 48):
+        assert C.lib().b200_gemm_grouped(x.data_ptr(), wgu.data_ptr(), out.data_ptr(), 24, E, I, 2 * I, H, I, C.EPI_SILU_MUL, I, bt,
+                                         tiles.data_ptr(), n.data_ptr(), 1, C.err_word(x.device).data_ptr(), 1, 1, None, 0,
+                                         C._stream()) != 0, bt
+    torch.cuda.synchronize()
+    assert (out == 7.0).all()
+    C.check_errors(x.device)
