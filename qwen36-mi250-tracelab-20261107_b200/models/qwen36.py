@@ -138,8 +138,7 @@ class Model:
 
     # ------------------------------------------------------------------ state management
     def reset_slot(self, slot: int) -> None:
-        if hasattr(self.ops, "reset_slot") and self.device.type == "cuda" and isinstance(slot, int) and self.conv_state.numel() \
-                and self.conv_state[0, 0].numel() * self.conv_state.element_size() % 16 == 0 and self.rec_state[0, 0].numel() % 4 == 0:
+        if hasattr(self.ops, "reset_slot") and self.device.type == "cuda" and isinstance(slot, int):
             self.ops.reset_slot(self.conv_state, self.rec_state, slot)
             return
         self.conv_state[:, slot].zero_()

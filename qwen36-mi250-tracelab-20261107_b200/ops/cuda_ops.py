@@ -536,11 +536,17 @@ def gdn_decode(mixed, slots, conv_state, rec_state, conv_w, A_log, dt_bias, gnor
 
 
 def reset_slot(conv_state: torch.Tensor, rec_state: torch.Tensor, slot: int) -> None:
-    """Zero one slot of the states ``[layers, slots, ...]`` of all layers in one launch; rows of multiples of 16 bytes."""
+    """Zero one slot of the states ``[layers, slots, ...]`` of all layers: one launch where they are contiguous, with rows of
+    multiples of 16 bytes, otherwise a fill of each."""
     layers, n = rec_state.shape[:2]
-    assert conv_state.is_contiguous() and rec_state.is_contiguous() and conv_state.shape[:2] == (layers, n)
     if not -n <= slot < n:
         raise IndexError(f"slot {slot} of {n}")
+    if conv_state.shape[:2] != (layers, n) or not all(
+            s.numel() and s.is_contiguous() and s.data_ptr() % 16 == 0 and s[0, 0].numel() * s.element_size() % 16 == 0
+            for s in (conv_state, rec_state)):
+        conv_state[:, slot].zero_()
+        rec_state[:, slot].zero_()
+        return
     with torch.cuda.device(rec_state.device):  # as a fill would, whatever the calling thread's current device is
         rc = lib().b200_reset_slot(_ptr(conv_state), _ptr(rec_state), slot % n, layers, n,
                                    conv_state[0, 0].numel() * conv_state.element_size(),

@@ -192,3 +192,26 @@ def test_reset_slot_zeroes_one_slot_of_every_layer(slot):
     assert torch.equal(conv, want_c) and torch.equal(rec, want_r)
     with pytest.raises(IndexError):
         C.reset_slot(conv, rec, 5)
+
+
+@pytest.mark.parametrize("form", ["layers apart", "slots apart", "rows of 8 bytes", "odd start", "no layers", "fewer conv slots"])
+def test_reset_slot_of_states_that_the_kernel_does_not_take(form):
+    from b200serve.ops import cuda_ops as C
+
+    conv, rec = torch.randn(6, 5, 264, 3, device="cuda").bfloat16(), torch.randn(6, 5, 2, 32, 32, device="cuda")
+    if form == "layers apart":
+        conv, rec = conv[::2], rec[::2]
+    elif form == "slots apart":
+        conv, rec = conv[:, 1:4], rec[:, 1:4]
+    elif form == "rows of 8 bytes":
+        conv = torch.randn(6, 5, 4, 1, device="cuda").bfloat16()
+    elif form == "odd start":
+        rec = torch.randn(6 * 5 * 2048 + 1, device="cuda")[1:].view(6, 5, 2, 32, 32)
+    elif form == "no layers":
+        conv, rec = conv[:0], rec[:0]
+    else:
+        conv = conv[:, :3].contiguous()
+    want_c, want_r = conv.clone(), rec.clone()
+    want_c[:, 2], want_r[:, 2] = 0.0, 0.0
+    C.reset_slot(conv, rec, 2)
+    assert torch.equal(conv, want_c) and torch.equal(rec, want_r)
