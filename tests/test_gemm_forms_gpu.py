@@ -59,21 +59,23 @@ def test_wide_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, p
     wgu, wd = _bf(E + 1, 2 * I, H, scale=0.05, seed=35), _bf(E + 1, H, I, scale=0.05, seed=36)
     if packed:
         wgu, wd = C.pack_weight(wgu, gate_up=True), C.pack_weight(wd)
-    keep = C.GATHER_MAX_BT, C.WIDE_MIN_ROWS
+    keep = C.GATHER_MAX_BT, C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS
     try:
-        C.WIDE_MIN_ROWS = 1
+        C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS = 1, 1 << 30  # one SM per tile on both sides
         wide = C.moe_block(x, router, wgu, wd, E, k, True)
         C.GATHER_MAX_BT = 64
         narrow = C.moe_block(x, router, wgu, wd, E, k, True)
     finally:
-        C.GATHER_MAX_BT, C.WIDE_MIN_ROWS = keep
+        C.GATHER_MAX_BT, C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS = keep
     C.check_errors(x.device)
     assert torch.equal(wide, narrow)
 
 
-@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (31, 64, 32), (32, 64, 32), (33, 64, 32), (32, 300, 7), (700, 40, 3)])
+@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (31, 64, 32), (32, 64, 32), (33, 64, 32), (32, 300, 7), (700, 40, 3), (465, 40, 10),
+                                   (466, 40, 10), (512, 300, 12)])
 def test_routing_and_plan_of_tied_rows(C, T, E, k):
-    """Quantised logits, so that ties are everywhere; the largest table that stays in shared memory, and one beyond it."""
+    """Quantised logits, so that ties are everywhere; the largest table that stays in shared memory, and one beyond it; as many
+    pairs as the last CTA's threads keep between counting and placing, and more."""
     g = torch.Generator(device="cuda").manual_seed(T + E)
     logits = (torch.randn(T, E + 1, device="cuda", generator=g) * 3).round() / 2
     P, dev = k + 1, "cuda"
@@ -157,6 +159,32 @@ def test_two_sm_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I,
     want = C.moe_block(x, router, wgu, wd, E, k, True)
     monkeypatch.setattr(C, "PAIR_MIN_ROWS", 0)
     monkeypatch.setattr(C, "moe_bt", lambda *a: 64)
+    assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
+    C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(300, 32, 8, 2048, 512), (430, 64, 8, 768, 256), (200, 16, 6, 1024, 384), (206, 16, 8, 512, 256)])
+def test_two_sm_expert_tiles_of_128_rows_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, monkeypatch):
+    """50 to 107 rows per expert: eight stages that are used again, several tiles per pair of SMs, both halves of a tile."""
+    assert C.PAIR_MIN_ROWS * E <= T * k < C.PAIR_256_MIN_ROWS * E
+    x = _bf(T, H + 8, seed=T)[:, :H]
+    router = _bf(E + 1, H, scale=0.3, seed=34)
+    router[3] = -4.0 * x.float().mean(0).bfloat16()  # rarely picked
+    wgu = C.pack_weight(_bf(E + 1, 2 * I, H, scale=0.05, seed=35), gate_up=True)
+    wd = C.pack_weight(_bf(E + 1, H, I, scale=0.05, seed=36))
+    got = C.moe_block(x, router, wgu, wd, E, k, True)
+    monkeypatch.setattr(C, "PAIR_MIN_ROWS", 1 << 30)
+    assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), got)
+    C.check_errors(x.device)
+
+
+def test_plan_of_many_pairs_by_one_cta(C, monkeypatch):
+    """Routing and plan as two launches: a single CTA plans more pairs than its threads keep."""
+    T, E, k, H, I = 700, 16, 8, 256, 128
+    x, router = _bf(T, H, seed=T), _bf(E + 1, H, scale=0.3, seed=34)
+    wgu, wd = _bf(E + 1, 2 * I, H, scale=0.05, seed=35), _bf(E + 1, H, I, scale=0.05, seed=36)
+    want = C.moe_block(x, router, wgu, wd, E, k, True)
+    monkeypatch.setattr(C, "ROUTE_PLAN_SPLIT", True)
     assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), want)
     C.check_errors(x.device)
 
