@@ -76,3 +76,19 @@ def test_emulated_kernels_have_no_data_race_and_a_missing_barrier_would_show(tmp
         assert b.returncode == 0, b.stderr[-3000:]
         run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=600)
         assert run.returncode == 0 and run.stdout.startswith("OK") and "ThreadSanitizer" not in run.stderr, run.stderr[-3000:]
+
+
+@pytest.mark.parametrize("tsan", [False, True])
+def test_expert_plan_of_more_pairs_and_wider_tiles_on_the_host(tmp_path, tsan):
+    """More pairs than a CTA's threads keep, eight rows per CTA, tiles of 256 rows; plain and under ThreadSanitizer."""
+    src, exe = ROOT / "tests/emu/plan_sizes_emu.cpp", tmp_path / "plan_sizes_emu"
+    if tsan:
+        if _tsan_build(ROOT / "tests/emu/race_control.cpp", tmp_path / "race_control").returncode:
+            pytest.skip("this toolchain has no ThreadSanitizer")
+        build = _tsan_build(src, exe, ("-DB200_EMU",))
+    else:
+        build = subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-DB200_EMU", "-I", str(ROOT / "tests/emu"), "-x", "c++",
+                                str(src), "-o", str(exe)], capture_output=True, text=True, timeout=300)
+    assert build.returncode == 0, build.stderr[-3000:]
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=600)
+    assert run.returncode == 0 and run.stdout.startswith("OK") and "ThreadSanitizer" not in run.stderr, run.stdout + run.stderr[-3000:]

@@ -59,23 +59,21 @@ def test_wide_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, p
     wgu, wd = _bf(E + 1, 2 * I, H, scale=0.05, seed=35), _bf(E + 1, H, I, scale=0.05, seed=36)
     if packed:
         wgu, wd = C.pack_weight(wgu, gate_up=True), C.pack_weight(wd)
-    keep = C.GATHER_MAX_BT, C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS
+    keep = C.GATHER_MAX_BT, C.WIDE_MIN_ROWS
     try:
-        C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS = 1, 1 << 30  # one SM per tile on both sides
+        C.WIDE_MIN_ROWS = 1
         wide = C.moe_block(x, router, wgu, wd, E, k, True)
         C.GATHER_MAX_BT = 64
         narrow = C.moe_block(x, router, wgu, wd, E, k, True)
     finally:
-        C.GATHER_MAX_BT, C.WIDE_MIN_ROWS, C.PAIR_MIN_ROWS = keep
+        C.GATHER_MAX_BT, C.WIDE_MIN_ROWS = keep
     C.check_errors(x.device)
     assert torch.equal(wide, narrow)
 
 
-@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (31, 64, 32), (32, 64, 32), (33, 64, 32), (32, 300, 7), (700, 40, 3), (465, 40, 10),
-                                   (466, 40, 10), (512, 300, 12)])
+@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (31, 64, 32), (32, 64, 32), (33, 64, 32), (32, 300, 7), (700, 40, 3)])
 def test_routing_and_plan_of_tied_rows(C, T, E, k):
-    """Quantised logits, so that ties are everywhere; the largest table that stays in shared memory, and one beyond it; as many
-    pairs as the last CTA's threads keep between counting and placing, and more."""
+    """Quantised logits, so that ties are everywhere; the largest table that stays in shared memory, and one beyond it."""
     g = torch.Generator(device="cuda").manual_seed(T + E)
     logits = (torch.randn(T, E + 1, device="cuda", generator=g) * 3).round() / 2
     P, dev = k + 1, "cuda"
@@ -176,6 +174,19 @@ def test_two_sm_expert_tiles_of_128_rows_give_the_bits_of_the_64_row_tiles(C, T,
     monkeypatch.setattr(C, "PAIR_MIN_ROWS", 1 << 30)
     assert torch.equal(C.moe_block(x, router, wgu, wd, E, k, True), got)
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(600, 16, 4, 256, 128), (1100, 32, 8, 2048, 512)])
+def test_wide_expert_tiles_of_packed_weights_on_one_sm(C, T, E, k, H, I, monkeypatch):
+    """128-row tiles of one SM against its 64-row tiles, at sizes that otherwise take two SMs per tile."""
+    monkeypatch.setattr(C, "PAIR_MIN_ROWS", 1 << 30)
+    test_wide_expert_tiles_give_the_bits_of_the_64_row_tiles(C, T, E, k, H, I, True)
+
+
+@pytest.mark.parametrize("T,E,k", [(465, 40, 10), (466, 40, 10), (512, 300, 12)])
+def test_routing_and_plan_of_more_pairs_than_threads_keep(C, T, E, k):
+    """As many pairs as the last CTA's threads keep between counting and placing, and more."""
+    test_routing_and_plan_of_tied_rows(C, T, E, k)
 
 
 def test_plan_of_many_pairs_by_one_cta(C, monkeypatch):
