@@ -919,6 +919,10 @@ static DenseForm dense_form(int T, int N, int K, bool packed) {
     if (by4 && tiles(64, 16) <= lim) return {16, 64, 4};
     if (by4 && tiles(64, 32) <= lim) return {32, 64, 4};
     if (by4 && tiles(64, 64) <= lim) return {64, 64, 4};
+    // an odd number of 128-element k-steps, us, 128-row tiles -> these: 257 x 1920 7.5 -> 6.3, 512 x 4224 at 48 rows 13.9 -> 11.1, 2048
+    // x 1152 at 48 5.8 -> 4.9, at 100, as 32 x 64, 6.1 -> 5.8 (x 896 5.1 -> 5.2, x 384 3.6 -> 4.1)
+    if (by2 && tiles(64, 16) <= lim) return {16, 64, 2};
+    if (by2 && K >= 16 * BK && tiles(64, 32) <= lim) return {32, 64, 2};
     return {16, BM, 1};
   }
   if (T > 256) {
@@ -1056,6 +1060,7 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
 static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
                                int max_tiles, int bt, cudaStream_t st) {
   const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
+  if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
   const int rt = bt == 16 && 4 * tiles <= sm_count() ? 32 : 64, kps = rt == 32 ? 4 : 2;
   if (p.K % (kps * BK) || p.N % BM) return 1;
   CUtensorMap tw, tx;

@@ -281,3 +281,15 @@ def test_grouped_launches_refuse_token_tiles_that_no_kernel_has(C):
     torch.cuda.synchronize()
     assert (out == 7.0).all()
     C.check_errors(x.device)
+
+
+@pytest.mark.parametrize("N,K", [(257, 384), (1024, 1152), (2048, 1152), (2048, 896), (4096, 1408)])
+def test_thin_forms_of_an_odd_number_of_stages(C, N, K):
+    """K a multiple of 128 but not of 256: two k-blocks per stage."""
+    w = _bf(N, K, scale=0.05, seed=1)
+    packed = C.pack_weight(w.clone())
+    for T in (16, 17, 48, 64, 100, 129, 200, 256):
+        x = _bf(T, K + 64, seed=T)[:, 32:32 + K]
+        for dt in (None, torch.float32):
+            assert torch.equal(C.linear(x, packed, out_dtype=dt)[:, :N], C.linear(x, w, out_dtype=dt, bt=16)), (T, dt)
+    C.check_errors(w.device)
