@@ -1056,12 +1056,13 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
 // pairs 14.7 -> 9.2, 5 rows 40.5 -> 34.8, 13: 75.3 -> 71.7, 40: 140 -> 132, 128: 176.6 -> 170.2, 256: 179.5 -> 179; 32-row
 // token tiles, 700 rows: 183 -> 180, 1024: 209 -> 191. (Tiles of 32 and 32 for all: 13 rows 73.7, 128: 175; 64-row token tiles
 // are as good with 128 rows: 1300 rows 186 and 190.) The down projection has 16 weight tiles per expert and CTAs enough at
-// one row. Returns 1 when the plain form is to run.
+// one row. Two k-blocks per stage where K has no multiple of four (block of 1 row, 33 experts of 256 x 1152: 128-row tiles 27.5 us,
+// these 21 to 22). Returns 1 when the plain form is to run.
 static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
                                int max_tiles, int bt, cudaStream_t st) {
   const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
   if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
-  const int rt = bt == 16 && 4 * tiles <= sm_count() ? 32 : 64, kps = rt == 32 ? 4 : 2;
+  const int rt = bt == 16 && 4 * tiles <= sm_count() ? 32 : 64, kps = rt == 32 && p.K % (4 * BK) == 0 ? 4 : 2;
   if (p.K % (kps * BK) || p.N % BM) return 1;
   CUtensorMap tw, tx;
   const uint64_t nk = p.K / BK;
@@ -1076,7 +1077,8 @@ static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E
   // with row indices the producer never reads through this map, but it has to be a valid one
   if (make_map_kblocks(&tx, X, gather_rows ? bt : p.T, static_cast<uint64_t>(gather_rows ? ldx : p.K) * 2, nk, BK * 2, bt, kps)) return -1;
   if (bt == 32) return launch<32, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
-  if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 4>(tw, tx, p, max_tiles, st);
+  if (rt == 32 && kps == 4) return launch<16, EPI_SILU_MUL, true, 32, 4>(tw, tx, p, max_tiles, st);
+  if (rt == 32) return launch<16, EPI_SILU_MUL, true, 32, 2>(tw, tx, p, max_tiles, st);
   return launch<16, EPI_SILU_MUL, true, 64, 2>(tw, tx, p, max_tiles, st);
 }
 

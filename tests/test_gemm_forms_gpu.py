@@ -293,3 +293,10 @@ def test_thin_forms_of_an_odd_number_of_stages(C, N, K):
         for dt in (None, torch.float32):
             assert torch.equal(C.linear(x, packed, out_dtype=dt)[:, :N], C.linear(x, w, out_dtype=dt, bt=16)), (T, dt)
     C.check_errors(w.device)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("inter,H", [(256, 1152), (128, 384), (128, 128)])
+def test_expert_block_of_a_few_rows_and_an_odd_number_of_stages(C, T, inter, H):
+    """Tiles of 32 gate and 32 up rows with two k-blocks per stage."""
+    test_expert_block_of_a_few_rows_with_packed_weights(C, T, inter, H)
