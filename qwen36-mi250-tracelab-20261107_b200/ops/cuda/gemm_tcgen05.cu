@@ -979,6 +979,19 @@ static int pair_rows(int T, int N) {
   return best;
 }
 
+// Whether up to 128 rows have too few k-blocks for two SMs per tile: nothing but the launch's ends is left then, and one SM per tile
+// ends sooner where the pairs are mostly busy. Up to nine k-blocks where the rows are cut into several tiles (bf16, x 384, 512, us,
+// pair -> one SM: 9216 at 48 rows 5.3 -> 4.4, 6.1 -> 5.1, at 100 5.7 -> 5.0, 6.5 -> 5.8; at 640 6.5 -> 6.1, at 768 6.9 -> 6.6), up to
+// six where they are one tile (16384 x 256 at 48 rows 4.9 -> 3.9, x 384 5.8 -> 5.1; 12352 x 384 5.0 -> 4.7, x 512 5.6 -> 5.8). fp32
+// rows, whose stores one SM has twice as many of, up to 48 rows (9216 x 384 at 48 rows 5.4 -> 4.8, at 100 5.9 -> 6.0). While the
+// tiles leave half of the pairs idle, or a fifth from 65 rows on, two SMs are the better form (4104 x 384 at 48 rows 3.8 and 4.1, 5120
+// x 384 at 128 rows 4.7 and 5.2).
+static bool pair_too_short(int T, int N, int K, int epi) {
+  const int bt = pair_rows(T, N), cut = (T + bt - 1) / bt;
+  if ((N + 2 * BM - 1) / (2 * BM) * cut <= (T <= 64 ? sm_count() / 4 : sm_count() * 2 / 5)) return false;
+  return cut > 1 ? T <= (epi == EPI_BF16 ? 128 : 48) && K <= 9 * BK : T <= (epi == EPI_BF16 ? 64 : 48) && K <= 6 * BK;
+}
+
 // Whether a dense launch is better off with two SMs per tile, us, best other form -> pair, weights not in L2 (about 10 us of
 // each is the measurement's own):
 //   rows    129           256           257           512           1024          2048          8192
@@ -993,7 +1006,8 @@ static int pair_rows(int T, int N) {
 // picks of 160 rows 192 -> 172 us, of 256 226 -> 206; logits of 160 rows 221 -> 199, of 256 275 -> 240. fp32 rows of fewer
 // weight tiles than SMs are better off from 17 on, x 2048: 16384 at 48 rows 16.1 -> 14.5, at 128 16.3 -> 15.4; 18944 at 17 rows
 // 16.9 -> 15.4, at 64 18.7 -> 16.3 (31104 at 64 rows 24.6 -> 24.9; 62080 at 17 41.7 -> 45.0).
-static bool pair_pays(int T, int N, int epi) {
+static bool pair_pays(int T, int N, int K, int epi) {
+  if (T <= 128 && pair_too_short(T, N, K, epi)) return false;
   if (epi == EPI_ARGMAX || epi == EPI_F32)
     return N > 32 * BM && (T > 128 || (epi == EPI_F32 && T > 16 && N <= BM * sm_count()));
   return N >= 2 * BM && (T > 256 || (T > 16 && N > 32 * BM));
@@ -1109,7 +1123,7 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
   GemmParams p{N, K, T, ldo, out, nullptr, nullptr, up_offset, part_max, part_idx, err, nullptr, CommCtx{}, 0, nullptr, nullptr, splits, nullptr, {}};
   const bool pair_ok = splits == 1 && pair_takes(p, epi, false);
   if (bt == PAIR_FORM && !pair_ok) return -7;
-  if (bt == PAIR_FORM || (bt <= 0 && pair_ok && pair_pays(T, N, epi))) {
+  if (bt == PAIR_FORM || (bt <= 0 && pair_ok && pair_pays(T, N, K, epi))) {
     switch (epi) {
       case EPI_BF16: return launch_pair_dense<EPI_BF16>(X, W, p, ldx, ldw, packed, st);
       case EPI_F32: return launch_pair_dense<EPI_F32>(X, W, p, ldx, ldw, packed, st);

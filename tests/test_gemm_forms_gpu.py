@@ -300,3 +300,17 @@ def test_thin_forms_of_an_odd_number_of_stages(C, N, K):
 def test_expert_block_of_a_few_rows_and_an_odd_number_of_stages(C, T, inter, H):
     """Tiles of 32 gate and 32 up rows with two k-blocks per stage."""
     test_expert_block_of_a_few_rows_with_packed_weights(C, T, inter, H)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("N", [4352, 9216, 16384])
+def test_many_outputs_of_a_few_k_blocks(C, N, packed):
+    """Either side of the number of k-blocks from which two SMs share a tile."""
+    for K in (64, 320, 384, 448, 576, 640):
+        w = _bf(N, K, scale=0.05, seed=1)
+        weights = C.pack_weight(w.clone()) if packed else w
+        for T in (17, 32, 33, 48, 49, 64, 65, 128, 129):
+            x = _bf(T, K, seed=T)
+            for dt in (None, torch.float32):
+                assert torch.equal(C.linear(x, weights, out_dtype=dt), C.linear(x, w, out_dtype=dt, bt=16)), (K, T, dt)
+    C.check_errors(w.device)
