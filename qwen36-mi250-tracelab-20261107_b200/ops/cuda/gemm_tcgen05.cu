@@ -1060,6 +1060,7 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
   if (f.bt == 16 && f.rt == 64 && f.kps == 4) return launch<16, EPI, false, 64, 4>(tw, tx, p, gy, st);
   if (f.bt == 16 && f.rt == 64 && f.kps == 2) return launch<16, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 32 && f.rt == 64 && f.kps == 4) return launch<32, EPI, false, 64, 4>(tw, tx, p, gy, st);
+  if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
   if (f.bt == 64 && f.rt == 64 && f.kps == 4) return launch<64, EPI, false, 64, 4>(tw, tx, p, gy, st);
   return -5;
 }
@@ -1075,7 +1076,6 @@ static int launch_thin_dense(const DenseForm& f, const void* X, const void* W, G
 static int launch_thin_grouped(const void* X, const void* W, GemmParams p, int E, const int* gather_rows, int ldx,
                                int max_tiles, int bt, cudaStream_t st) {
   const long long tiles = static_cast<long long>((p.N + BM - 1) / BM) * p.T;  // p.T: pairs
-  if (f.bt == 32 && f.rt == 64 && f.kps == 2) return launch<32, EPI, false, 64, 2>(tw, tx, p, gy, st);
   const int rt = bt == 16 && 4 * tiles <= sm_count() ? 32 : 64, kps = rt == 32 && p.K % (4 * BK) == 0 ? 4 : 2;
   if (p.K % (kps * BK) || p.N % BM) return 1;
   CUtensorMap tw, tx;
