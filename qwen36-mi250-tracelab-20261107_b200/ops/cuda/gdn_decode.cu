@@ -28,9 +28,10 @@ namespace b200 {
 // that wrote `mixed` and none of them: it released this kernel behind its own wait, so whatever came before it is complete
 // (a fill, a copy, a slot reset, a ring commit or a prefill right in front would still be writing). 72 registers hold the
 // 2048 CTAs of 128 sequences of 8192 channels in one wave. In a step, us, in order -> AHEAD: one sequence 3.4 -> 1.8, 128:
-// 10.4 -> 6.5, 256: 13.8 -> 12.0.
+// 10.4 -> 6.5, 256: 13.8 -> 12.0. The form in order keeps the registers it asks for: alone, conv and step of 13 sequences of two rows
+// took 28.4 us at 72 registers and take 27.4, of 40 sequences 32.9 and 32.1, of 128 96.3 and 96.9.
 template <int KW, bool AHEAD = false>
-__global__ void __launch_bounds__(64, 14)
+__global__ void __launch_bounds__(64, AHEAD ? 14 : 1)
 gdn_conv_step_kernel(const bf16* mixed, int ld, const int* slots, bf16* conv_state, const bf16* conv_w, bf16* out,
                      bf16* ring_conv, int C, int G) {
   // a thread owns 8 consecutive channels: 16-byte loads of the inputs, 48 / 64 contiguous bytes of state / weights
