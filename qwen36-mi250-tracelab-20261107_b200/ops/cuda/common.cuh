@@ -175,7 +175,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
   }
 }
 
-// ------------------------------------------------------------------ TMA (no multicast anywhere)
+// ------------------------------------------------------------------ TMA (loads without multicast)
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }

@@ -13,7 +13,8 @@
 // owner, warps 2..5 = epilogue (one TMEM lane quarter each); the 128-row gate/up tiles have a seventh warp that
 // fetches half of the rows by index. Operand tiles are 64 bf16 wide
 // (128 bytes, TMA 128B swizzle), STAGES deep, guarded by full/empty mbarriers; tcgen05.commit
-// releases a stage when the MMAs that read it have finished. No cluster multicast is used.
+// releases a stage when the MMAs that read it have finished. No load uses cluster multicast; the commits of the two-SM form
+// (gemm_pair.cuh) arrive at both of its CTAs that way.
 //
 // Variants (template): plain store (bf16 or fp32), SiLU(gate)*up over two accumulators,
 // per-tile argmax partials for the LM head, and a grouped mode where a device-side tile table
@@ -1141,7 +1142,7 @@ extern "C" int b200_gemm_dense(const void* X, const void* W, void* out, int T, i
   if (epi == EPI_SILU_MUL && bt > 128) bt = 128;
   CUtensorMap tw, tx;
   if (weight_map(&tw, W, 0, N, w_rows, K, ldw, epi == EPI_SILU_MUL, packed, &p)) return -1;
-  // LM head of 160 rows x 248320 x 2048: 198 -> 177 us (shared memory bounds it at 256 columns)
+  // a single token tile takes no more columns than there are rows (LM head of 160 rows in this form 198 -> 177 us)
   const int gy = (T + bt - 1) / bt;
   if (gy == 1) p.x_rows = (T + 15) / 16 * 16;
   if (make_map(&tx, X, K, T, 0, ldx, 0, gy == 1 ? p.x_rows : bt)) return -1;
